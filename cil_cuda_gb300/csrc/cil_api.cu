@@ -38,6 +38,7 @@ struct HostColony {
   int cap = 0;
   bool uploaded = false;
   double sigma_max = 0.0;
+  int n_seen = 0;  // cells at the upload or the last cil_step's status read
   // oracle-mode mirror
   int n = 0;
   std::vector<int> t0, tsw;
@@ -47,7 +48,7 @@ struct HostColony {
 }  // namespace
 
 struct GraphSlot {
-  int key;                 // cur | meta << 1 | pu << 2 at the first step, | two steps << 3, | last << 4
+  int key;                 // cur | meta << 1 | pu << 2 at the first step, | two steps << 3, | last << 4, lane bits << 5
   uint64_t gen;
   cudaGraphExec_t exec;
   int64_t launches;        // kernels in the graph
@@ -90,6 +91,8 @@ struct cil_handle {
   float4 *d_pk[2] = {nullptr, nullptr};  // mixed: packed elements (coordinates + diameter)
   int *d_sbin[2] = {nullptr, nullptr};
   int2 *d_cyc[2] = {nullptr, nullptr};
+  float4 *d_rec = nullptr;  // FP64 form: FP32 absolute coordinates and diameter per slot
+  int lane_bits = 0;        // FP64 form: log2 of the lanes per element of the force pass
   double *d_sigma_c = nullptr;  // canonical diameters [2 * CC]
   bool need_exact = true;       // next rebuild takes the FP64 reference path
   int pu = 1;                   // which d_pk holds the current packed elements
@@ -178,7 +181,7 @@ cil_status fail(cil_handle *h, cil_status s, const std::string &m) {
 
 void free_all(cil_handle *h) {
   void *ptrs[] = {h->d_col, h->d_cnt, h->d_x[0], h->d_x[1], h->d_sig[0], h->d_sig[1], h->d_eid[0],
-                  h->d_eid[1], h->d_pk[0], h->d_pk[1], h->d_sbin[0], h->d_sbin[1],
+                  h->d_eid[1], h->d_rec, h->d_pk[0], h->d_pk[1], h->d_sbin[0], h->d_sbin[1],
                   h->d_cyc[0], h->d_cyc[1], h->d_sigma_c, h->d_state[0], h->d_state[1], h->d_nbr,
                   h->d_ncnt, h->d_fresh, h->d_spart, h->d_lflat, h->d_lwarp, h->d_oflat, h->d_lstart, h->d_uref, h->d_facc, h->d_ftouch, h->d_skin, h->d_sched, h->d_mlp, h->d_fhead, h->d_fnext, h->d_ts, h->d_anyreb, h->d_vel, h->d_vel2, h->d_frc, h->d_key, h->d_perm,
                   h->d_bcount, h->d_range, h->d_scan_sum, h->d_scan_off, h->d_scan_col,
@@ -332,6 +335,7 @@ RebuildArgs rebuild_args(cil_handle *h) {
   a.sig_out = h->d_sig[1 - h->meta];
   a.eid_out = h->d_eid[1 - h->meta];
   a.pk_out = mixed ? h->d_pk[1 - h->pu] : nullptr;
+  a.rec_out = h->d_rec;
   a.pk_in = mixed ? h->d_pk[h->pu] : nullptr;
   a.skin = nullptr;  // a permuting rebuild re-sorts every colony
   a.permute = 1;
@@ -421,6 +425,7 @@ ForceArgs force_args(cil_handle *h, int noise_mode, int integrate, double *vel, 
   a.x_out = h->d_x[1 - h->cur];
   a.sig = h->d_sig[h->meta];
   a.eid = h->d_eid[h->meta];
+  a.rec = h->d_rec;
   a.pk = h->d_pk[h->pu];
   a.pk_next = h->d_pk[1 - h->pu];
   a.dueq = h->d_dueq;
@@ -769,8 +774,22 @@ cudaEvent_t pool_event(cil_handle *h, size_t i) {
   return h->evpool[i];
 }
 
+// Lanes per element of the FP64 force pass: as many as keep the walk and the pair evaluation of a
+// small colony spread over every SM, up to 8, while the elements give fewer than two warps per
+// scheduler (nsm x 4 x 2 x 32 lanes). From the cells the host knows of (uploaded, or counted by the
+// last cil_step); the forces do not depend on it. Step of the growth colony with 1, 2, 4, 8 lanes:
+// 500 cells 48, 46, 44, 42 us; 4864 cells 61, 56, 57, 61 us; 19456 cells 72, 73, 87, 107 us.
+void set_lane_bits(cil_handle *h) {
+  long long elems = 0;
+  for (int c = 0; c < h->B; ++c) elems += 2ll * h->hc[c].n_seen;
+  int b = 0;
+  while (b < 3 && elems * (2ll << b) <= 2ll * h->nsm * 4 * 32) ++b;
+  h->lane_bits = b;
+}
+
 // Error bits of the colonies' counters as a status (and the handle's message).
 cil_status counter_status(cil_handle *h, const ColonyCounters *k) {
+  for (int c = 0; c < h->B; ++c) h->hc[c].n_seen = k[c].ncell;
   for (int c = 0; c < h->B; ++c) {
     if (k[c].err & kErrNan) return fail(h, CIL_ERR_NAN, "non-finite force in colony " + std::to_string(c));
     if (k[c].err & kErrBox) return fail(h, CIL_ERR_OUT_OF_BOX, "element left the box in colony " + std::to_string(c));
@@ -935,7 +954,7 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
     ForceArgs fa = force_args(h, noise ? (oracle ? 2 : 1) : 0, 1, last ? h->d_vel : nullptr, nullptr);
     fa.heun = heun;
     fa.vel_prev = vel_prev;
-    launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, kTile, h->stream);
+    launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, h->stiles, h->lane_bits, h->stream);
     h->launches += 1;
     h->cur = 1 - h->cur;
     if (h->cfg.precision == CIL_PREC_MIXED) h->pu = 1 - h->pu;
@@ -1011,7 +1030,8 @@ void restore_host_state(cil_handle *h, const HostStepState &s) {
 // caller then replays the graph). On a capture failure the host state is put back, graphs are
 // switched off for the handle and null is returned.
 cudaGraphExec_t steady_graph(cil_handle *h, int nsteps, bool last, int64_t *launches_per_graph) {
-  const int key = h->cur | (h->meta << 1) | (h->pu << 2) | ((nsteps == 2 ? 1 : 0) << 3) | ((last ? 1 : 0) << 4);
+  const int key = h->cur | (h->meta << 1) | (h->pu << 2) | ((nsteps == 2 ? 1 : 0) << 3) | ((last ? 1 : 0) << 4) |
+                  (h->lane_bits << 5);
   for (auto &gs : h->graphs)
     if (gs.key == key && gs.gen == h->graph_gen) {
       HostStepState s = host_state(h);
@@ -1319,6 +1339,7 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
     h->d_cyc[b] = dalloc<int2>(SS);
     if (mixed) h->d_pk[b] = dalloc<float4>(SS);
   }
+  if (!mixed) h->d_rec = dalloc<float4>(SS);
   h->d_sigma_c = dalloc<double>(2 * static_cast<size_t>(h->CC));
   h->d_ts = dalloc<int>(1);
   h->skin_mode = cfg->skin > 0.0;
@@ -1381,7 +1402,7 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
             h->d_slot_of && h->d_t0 && h->d_tsw && h->d_cst && h->d_smflag && h->d_tiles_used && h->d_tiles_live && h->d_tiles_cell &&
             h->d_tiles_pairs &&
             h->d_tile_count && h->d_tile_off && h->d_upchk && h->d_evdone && h->d_dead && h->d_divq && h->d_ts &&
-            (mixed ? (h->d_pk[0] && h->d_pk[1]) : (h->d_sig[0] && h->d_sig[1])) &&
+            (mixed ? (h->d_pk[0] && h->d_pk[1]) : (h->d_sig[0] && h->d_sig[1] && h->d_rec)) &&
             skin_ok;
   if (ok && cfg->rng_mode == CIL_RNG_DSFMT) {
     const size_t nn = 2 * static_cast<size_t>(h->CC) * D + 2 * static_cast<size_t>(h->CC);  // passive, active
@@ -1499,7 +1520,7 @@ cil_status cil_upload(cil_handle *h, int32_t colony, const cil_colony_view *v) {
   std::memcpy(&smax, chk + 2, sizeof smax);
   hc.uploaded = true;
   hc.sigma_max = smax;
-  hc.n = n;
+  hc.n = hc.n_seen = n;
   if (h->cfg.rng_mode == CIL_RNG_DSFMT) {  // the oracle mode's host mirror of the cycles
     hc.t0.assign(v->t0, v->t0 + n);
     hc.tsw.assign(v->tswitch, v->tswitch + n);
@@ -1535,6 +1556,7 @@ cil_status cil_step(cil_handle *h, int32_t nsteps, int64_t *ts_out) {
   if (nsteps < 0) return fail(h, CIL_ERR_CONFIG, "cil_step: negative step count");
   cil_status st = ensure_ready(h);
   if (st != CIL_OK) return st;
+  set_lane_bits(h);
   h->t_rebuild = h->t_force = h->t_events = 0.0;
   h->launches = 0;
   h->graph_steps = 0;
@@ -1632,7 +1654,8 @@ cil_status cil_forces(cil_handle *h, int32_t colony, double *frc) {
   st = do_rebuild(h, true, true);
   if (st != CIL_OK) return st;
   ForceArgs fa = force_args(h, noise ? (oracle ? 2 : 1) : 0, 0, nullptr, h->d_frc);
-  launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, kTile, h->stream);
+  set_lane_bits(h);
+  launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, h->stiles, h->lane_bits, h->stream);
   std::vector<ColonyCounters> k;
   st = check_counters(h, &k);
   if (st != CIL_OK && st != CIL_ERR_NAN) return st;

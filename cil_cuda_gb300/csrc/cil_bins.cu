@@ -294,6 +294,12 @@ __global__ void __launch_bounds__(kTile) k_gather(RebuildArgs a) {
       a.cyc_out[dst] = make_int2(a.t0c[g], a.tswc[g]);
       const double sg = a.sigma_c[e];
       if (a.sig_out) a.sig_out[dst] = sg;
+      if (a.rec_out) {
+        float4 q = make_float4(0.0f, 0.0f, 0.0f, static_cast<float>(sg));
+#pragma unroll
+        for (int d = 0; d < D; ++d) pk_set(q, d, static_cast<float>(x[d]));
+        a.rec_out[dst] = q;
+      }
       if (a.pk_out) {
         int b[D];
         bin_decode<D>(C, nb, b);

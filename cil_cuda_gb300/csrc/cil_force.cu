@@ -1,4 +1,4 @@
-// Fused force + integrate kernels: one thread per binned element.
+// Fused force + integrate kernels over the binned elements.
 //
 // Per element, in the reference's accumulation order (calculForcesPressure,
 // CIL.cu:999-1007):
@@ -23,27 +23,6 @@ namespace cil {
 namespace {
 
 template <int D>
-__device__ __forceinline__ bool neighbor_bin(const ColonyConst &C, const int *bi, const int *o,
-                                             int *nb, double *shift) {
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    int v = bi[d] + o[d];
-    shift[d] = 0.0;
-    if (v < 0) {
-      if (!C.periodic[d]) return false;
-      v += C.ns[d];
-      shift[d] = -C.box[d];
-    } else if (v >= C.ns[d]) {
-      if (!C.periodic[d]) return false;
-      v -= C.ns[d];
-      shift[d] = C.box[d];
-    }
-    nb[d] = v;
-  }
-  return true;
-}
-
-template <int D>
 __device__ __forceinline__ bool neighbor_bin_i(const ColonyConst &C, const int *bi, const int *o, int *nb) {
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -60,38 +39,128 @@ __device__ __forceinline__ bool neighbor_bin_i(const ColonyConst &C, const int *
   return true;
 }
 
+// nint(v / L) (Utils.hpp:173-175) without a division when |v| < L / 4, where v / L lies in
+// (-0.25, 0.25) whatever its rounding: a minimum image leaves v as it is then.
+__device__ __forceinline__ double min_image(double v, double L) {
+  if (fabs(v) < 0.25 * L) return v;
+  return v - static_cast<double>(nint(v / L)) * L;
+}
+
+// fmod(t + L, L) as wrap_like_fmod gives it, its comparisons on the bit patterns (doubles that
+// are not negative order like them), so that the FP64 pipe runs the two additions only.
+__device__ __forceinline__ double wrap_bits(double t, double L) {
+  const double t2 = __dadd_rn(t, L);
+  const long long b = __double_as_longlong(t2), l = __double_as_longlong(L);
+  if (b < 0 || b >= l + 0x0010000000000000ll) return wrap_like_fmod(t, L);  // below 0, at or past 2 L, NaN
+  return b >= l ? t2 - L : t2;
+}
+
+// The law of pair_force with its square root and divisions formed from one reciprocal square
+// root (as pair_f0_fast does in FP32), each within a few units of the last place: GB300's FP64
+// pipe runs 2 lanes a clock per SM, so the law's cost is its count of FP64 instructions.
+//   soft core: q = 1 / (r rc) gives r / rc = r2 q and 1 / r = rc q
+//   Hertz:     y = 1 / r gives r = r2 y, corrected by one Newton residual because sigma_ij - r
+//              cancels; delta^1.5 = delta (delta / sqrt(delta))
+// The other laws, and separations whose square is out of that form's range, take pair_force.
+template <int LAW>
+__device__ __forceinline__ bool pair_force_rsqrt(double r2, double si, double sj, double eps, double rcs, double &f0,
+                                                 double em, double xi, int shifted) {
+  if (LAW == CIL_FORCE_SOFTCORE || LAW == CIL_FORCE_HERTZ) {
+    const double sij = 0.5 * (si + sj);
+    const double rc = rcs * sij;
+    const double rc2 = rc * rc;
+    const int hi = __double2hiint(r2);  // r2 >= 0: the high word orders it to one part in 2^20
+    if (hi < 0x10000000 || hi >= 0x6fffffff || __double2hiint(rc2) < 0x10000000 || __double2hiint(rc2) >= 0x6fffffff)
+      return pair_force<LAW, double>(r2, si, sj, eps, rcs, f0, em, xi, shifted);
+    if (__double_as_longlong(r2) >= __double_as_longlong(rc2)) return false;
+    if (LAW == CIL_FORCE_SOFTCORE) {
+      const double q = rsqrt(r2 * rc2);
+      const double w = 1.0 - r2 * q;
+      f0 = -eps * w * w * (rc * q);
+    } else {
+      const double y = rsqrt(r2);
+      double r = r2 * y;
+      r = __fma_rn(__fma_rn(-r, r, r2), 0.5 * y, r);
+      const double delta = sij - r;
+      const double sq = __double2hiint(delta) >= 0x10000000 ? delta * rsqrt(delta) : sqrt(delta);
+      f0 = -eps * delta * sq * y;
+    }
+    return true;
+  }
+  return pair_force<LAW, double>(r2, si, sj, eps, rcs, f0, em, xi, shifted);
+}
+
+// isfinite by the exponent bits (no FP64 comparison)
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+
+// The FP64 force pass: 2^lane_bits lanes per binned element, blocks of kF64Block threads.
+//
+// What bounds it is the FP64 pipe (2 lanes a clock per SM, 1/64 of FP32), so FP64 runs only for
+// the pairs inside the cutoff and with full warps:
+//   walk    the candidates of the 3^d neighbour bins in rows along the last axis (consecutive bins
+//           hold consecutive slots), tested in FP32 on absolute FP32 coordinates (ForceArgs::rec)
+//           against a cutoff widened by their rounding; the lanes of an element take consecutive
+//           candidates and a ballot keeps the survivors in walk order in shared memory, whatever
+//           the number of lanes, so that an element's sum never depends on it;
+//   pairs   the warp's survivors as one flattened range, a pair per lane (exact FP64 test and law),
+//           results in shared memory;
+//   sums    the element's first lane adds its pairs in walk order, then integrates.
+// Lanes per element: see set_lane_bits (cil_api.cu). When every candidate's separation was formed
+// in FP64 and each lane evaluated its own pairs, a pass took 879 us for 0.5M elements of the 2D
+// growth colony, 376 us for 0.12M of the 3D channel and 42 us for 8192 WCA elements; now 181, 104
+// and 19 us, with the FP64 pipe 70 % active in the first.
+constexpr int kF64Block = 128;
+constexpr int kF64Near = 512;  // survivors held per warp (16 per element at one lane each)
+constexpr int kF64Seg = 256;   // pairs evaluated before their sums are taken
+template <int D>
+struct F64Warp {
+  double res[kF64Seg * D];
+  double x[32 * D];
+  double sig[32];
+  int tt[kF64Near];
+  unsigned char code[kF64Near];
+  unsigned char own[kF64Near];
+};
+
 template <int D, int LAW>
-__global__ void __launch_bounds__(kTile) k_force_fp64(ForceArgs a_) {
+__global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane_bits) {
+  extern __shared__ __align__(16) unsigned char s_f64[];
   ForceArgs a = a_;
   a.ts = *a_.ts_dev;
-  const int total = a.tiles_live[a.B];
-  for (int t = blockIdx.x; t < total; t += gridDim.x) {
-    const int c = colony_of_tile(a.tiles_live, a.B, t);
-    const ColonyConst &C = a.col[c];
-    const int s = C.slot_base + (t - a.tiles_live[c]) * kTile + threadIdx.x;
-    const int nlive = a.cnt[c].nlive;
-    if (s >= C.slot_base + nlive) continue;
-
-    const size_t SS = a.SS;
-    const int e = a.eid[s];
-    if (e < 0) continue;
-    const int g = e >> 1, j = e & 1;
-    double xi[D];
+  const int per_tile = 2 << lane_bits;  // blocks per tile of kTile elements (kTile = 2 kF64Block)
+  const int t = blockIdx.x / per_tile;
+  if (t >= a.tiles_live[a.B]) return;  // uniform per block
+  F64Warp<D> &W = reinterpret_cast<F64Warp<D> *>(s_f64)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31, L = 1 << lane_bits;
+  const int sub = lane & (L - 1), el = lane >> lane_bits;  // lane of the element, element of the warp
+  const int c = colony_of_tile(a.tiles_live, a.B, t);
+  const ColonyConst &C = a.col[c];
+  const int s = C.slot_base + (t - a.tiles_live[c]) * kTile +
+                (((blockIdx.x - t * per_tile) * kF64Block + static_cast<int>(threadIdx.x)) >> lane_bits);
+  const int nlive = a.cnt[c].nlive;
+  const size_t SS = a.SS;
+  const int e = s < C.slot_base + nlive ? a.eid[s] : -1;
+  const bool live = e >= 0;
+  const int g = e >> 1, j = e & 1;
+  double xi[D], F[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) xi[d] = a.x_in[d * SS + s];
-    const double si = a.sig[s];
+  for (int d = 0; d < D; ++d) {
+    xi[d] = live ? a.x_in[d * SS + s] : 0.0;
+    F[d] = 0.0;
+  }
+  const double si = live ? a.sig[s] : 1.0;
+  const int ps = live ? a.slot_of[e ^ 1] : -1;
 
-    double F[D];
+  if (live && sub == 0) {
     // ---- intra-cell: linear spring to the partner + motility along back->front
     {
-      const int ps = a.slot_of[e ^ 1];
       double rij[D];
       double r2 = 0.0;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
         const double xp = a.x_in[d * SS + ps];
         double v = (j == 0) ? xp - xi[d] : xi[d] - xp;  // r1 - r0
-        if (C.periodic[d]) v -= static_cast<double>(nint(v / C.box[d])) * C.box[d];
+        if (C.periodic[d]) v = min_image(v, C.box[d]);
         rij[d] = v;
         r2 += v * v;
       }
@@ -122,7 +191,9 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(ForceArgs a_) {
                           : C.motility[1] * nd + spring * rij[d] * 2.0 + rnd[d] * rij[d];
         }
       } else {
-        const double r = sqrt(r2);
+        const double ir = rsqrt(r2);
+        double r = r2 * ir;
+        r = __fma_rn(__fma_rn(-r, r, r2), 0.5 * ir, r);
         double rest = C.rest0;
         if (C.divide) {
           const int2 cy = a.cyc[s];
@@ -132,11 +203,9 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(ForceArgs a_) {
           rest = C.rest0 + (C.rest1 - C.rest0) * frac;
         }
         const double sp = C.kappa * (r - rest);
+        const double coef = ((j == 0) ? sp - C.motility[0] : C.motility[1] - sp) * ir;
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const double nd = rij[d] / r;
-          F[d] = (j == 0) ? sp * nd - C.motility[0] * nd : -sp * nd + C.motility[1] * nd;
-        }
+        for (int d = 0; d < D; ++d) F[d] = coef * rij[d];
       }
     }
     // ---- walls
@@ -162,10 +231,12 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(ForceArgs a_) {
 #pragma unroll
       for (int d = 0; d < D; ++d) F[d] += C.zeta[j] * (C.noise_amp * static_cast<double>(n[d]));
     }
+  }
 
-    // ---- pair forces
-    const double eps = C.epsilon, rcs = C.rcut_scale;
-    if (C.single_bin) {
+  // ---- pair forces
+  const double eps = C.epsilon, rcs = C.rcut_scale;
+  if (C.single_bin) {
+    if (live && sub == 0) {
       // one bin: all elements, minimum image as BoundingBox::distance (Utils.hpp:536-544)
       for (int tt = C.slot_base; tt < C.slot_base + nlive; ++tt) {
         const int ej = a.eid[tt];
@@ -175,111 +246,206 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(ForceArgs a_) {
 #pragma unroll
         for (int d = 0; d < D; ++d) {
           double v = a.x_in[d * SS + tt] - xi[d];
-          if (C.periodic[d]) v -= static_cast<double>(nint(v / C.box[d])) * C.box[d];
+          if (C.periodic[d]) v = min_image(v, C.box[d]);
           dx[d] = v;
           r2 += v * v;
         }
         double f0;
-        if (pair_force<LAW, double>(r2, si, a.sig[tt], eps, rcs, f0, C.well_eps, C.well_sigma, C.force_shifted)) {
+        if (pair_force_rsqrt<LAW>(r2, si, a.sig[tt], eps, rcs, f0, C.well_eps, C.well_sigma, C.force_shifted)) {
 #pragma unroll
           for (int d = 0; d < D; ++d) F[d] += f0 * dx[d];
         }
       }
-    } else {
-      int bi[D];
-      bin_decode<D>(C, a.sbin[s], bi);
-      // the partners inside the cutoff, in walk order with their neighbour bin: their pair
-      // forces are evaluated kNear at a time after the walk, so the warp runs the FP64 law with
-      // its lanes converged instead of once per candidate (the sums keep the walk order)
-      const float sif = static_cast<float>(si), rcsf = static_cast<float>(rcs);
-      const float xif = static_cast<float>(C.well_sigma);
-      constexpr int kNear = 16;
-      int near_t[kNear];
-      unsigned char near_o[kNear];
-      int nnear = 0;
-      auto pairs = [&]() {
-        for (int k = 0; k < nnear; ++k) {
-          const int tt = near_t[k], code = near_o[k];
-          const int oo[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
-          int nb[D];
-          double shift[D];
-          neighbor_bin<D>(C, bi, oo, nb, shift);
-          double dx[D];
-          double r2 = 0.0;
+    }
+  } else {  // uniform per block
+    if (sub == 0) {
 #pragma unroll
-          for (int d = 0; d < D; ++d) {
-            dx[d] = (__ldg(a.x_in + d * SS + tt) + shift[d]) - xi[d];
-            r2 += dx[d] * dx[d];
-          }
-          double f0;
-          if (pair_force<LAW, double>(r2, si, __ldg(a.sig + tt), eps, rcs, f0, C.well_eps, C.well_sigma,
-                                      C.force_shifted)) {
+      for (int d = 0; d < D; ++d) W.x[el * D + d] = xi[d];
+      W.sig[el] = si;
+    }
+    const int cap = kF64Near >> (5 - lane_bits);  // survivors held per element
+    const int nb0 = el * cap;
+    const unsigned gmask = (L == 32 ? 0xffffffffu : (1u << L) - 1u) << (lane & ~(L - 1));
+    const unsigned below = gmask & ((1u << lane) - 1u);
+    int cnt = 0;  // the element's survivors so far (the same in all its lanes)
+    // the survivors' pairs, the whole warp: flattened, a pair per lane, then the elements' sums
+    auto flush = [&]() {
+      int inc = sub == 0 ? cnt : 0;
 #pragma unroll
-            for (int d = 0; d < D; ++d) F[d] += f0 * dx[d];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, inc, 31);
+      const int end = __shfl_sync(0xffffffffu, inc, lane & ~(L - 1));
+      const int off = end - cnt;
+      for (int k = sub; k < cnt; k += L) W.own[off + k] = static_cast<unsigned char>(el);
+      __syncwarp();
+      for (int S = 0; S < total; S += kF64Seg) {
+        const int E = min(total, S + kF64Seg);
+        for (int f0i = S; f0i < E; f0i += 32) {  // uniform
+          const int f = f0i + lane;
+          const int o = f < E ? W.own[f] : 0;
+          const int offo = __shfl_sync(0xffffffffu, off, o << lane_bits);
+          if (f < E) {
+            const int at = o * cap + (f - offo);
+            const int tt = W.tt[at], code = W.code[at];
+            double dx[D];
+            double r2 = 0.0;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              double xj = __ldg(a.x_in + d * SS + tt);
+              const int k = (code >> (2 * d)) & 3;  // the neighbour's image: 1 below, 2 above
+              if (k) xj = __dadd_rn(xj, k == 1 ? -C.box[d] : C.box[d]);
+              dx[d] = xj - W.x[o * D + d];
+              r2 += dx[d] * dx[d];
+            }
+            double f0 = 0.0;
+            if (!pair_force_rsqrt<LAW>(r2, W.sig[o], __ldg(a.sig + tt), eps, rcs, f0, C.well_eps, C.well_sigma,
+                                       C.force_shifted))
+              f0 = 0.0;
+#pragma unroll
+            for (int d = 0; d < D; ++d) W.res[(f - S) * D + d] = f0 * dx[d];
           }
         }
-        nnear = 0;
-      };
-      int o[3] = {-1, -1, -1};
-      for (o[0] = -1; o[0] <= 1; ++o[0])
-        for (o[1] = -1; o[1] <= 1; ++o[1])
-          for (o[2] = (D == 3 ? -1 : 0); o[2] <= (D == 3 ? 1 : 0); ++o[2]) {
-            int nb[D];
-            double shift[D];
-            if (!neighbor_bin<D>(C, bi, o, nb, shift)) continue;
-            const int2 r = a.range[C.bin_base + bin_id<D>(C, nb)];
-            const unsigned char code = static_cast<unsigned char>((o[0] + 1) + 3 * (o[1] + 1) + 9 * (o[2] + 1));
-            for (int tt = r.x; tt < r.y; ++tt) {
-              const int ej = __ldg(a.eid + tt);
-              if (ej < 0 || (ej >> 1) == g) continue;
-              // a conservative FP32 range test on the FP64 separation (pair_force repeats the
-              // exact test): one FP64 subtraction per axis per candidate, the rest in FP32
-              float r2f = 0.0f;
+        __syncwarp();
+        if (sub == 0) {
+          for (int f = max(off, S); f < min(end, E); ++f)
 #pragma unroll
-              for (int d = 0; d < D; ++d) {
-                const float dx = static_cast<float>((__ldg(a.x_in + d * SS + tt) + shift[d]) - xi[d]);
-                r2f += dx * dx;
-              }
-              if (!pair_maybe_in_range<LAW>(r2f, sif, static_cast<float>(__ldg(a.sig + tt)), rcsf, xif)) continue;
-              near_t[nnear] = tt;
-              near_o[nnear] = code;
-              if (++nnear == kNear) pairs();
+            for (int d = 0; d < D; ++d) F[d] += W.res[(f - S) * D + d];
+        }
+        __syncwarp();
+      }
+      cnt = 0;
+    };
+    int bi[D];
+    bin_decode<D>(C, live ? a.sbin[s] : 0, bi);
+    const float4 me = live ? a.rec[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // FP32 rounds both coordinates, an image's shift and two sums, each by 2^-24 of a value within
+    // max(box, |coordinate|) or so: 2^-21 of their sum bounds a separation's error along an axis
+    float margin[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) margin[d] = 4.76837158e-07f * (static_cast<float>(C.box[d]) + fabsf(pk_c(me, d)));
+    const float rcsf = C.rcs_f, xif = C.well_sigma_f;
+    // the rows of bins (all axes but the last), and per row up to three pieces of the last axis:
+    // one when its three bins are consecutive, each bin of its own at the ends of the axis
+    constexpr int NROW = D == 2 ? 3 : 9;
+    const int last = bi[D - 1], nl = C.ns[D - 1];
+    const bool inner = last > 0 && last < nl - 1;
+    for (int row = 0; row < NROW; ++row) {
+      const int oo[3] = {(D == 2 ? row : row / 3) - 1, (D == 2 ? 0 : row % 3) - 1, 0};
+      int code0 = 0, rowbin = 0;
+      bool ok = live;
+      float sh[D];
+#pragma unroll
+      for (int d = 0; d < D - 1; ++d) {
+        int v = bi[d] + oo[d];
+        sh[d] = 0.0f;
+        if (v < 0) {
+          ok = ok && C.periodic[d];
+          v += C.ns[d];
+          code0 |= 1 << (2 * d);
+          sh[d] = -static_cast<float>(C.box[d]);
+        } else if (v >= C.ns[d]) {
+          ok = ok && C.periodic[d];
+          v -= C.ns[d];
+          code0 |= 2 << (2 * d);
+          sh[d] = static_cast<float>(C.box[d]);
+        }
+        rowbin = rowbin * C.ns[d] + v;
+      }
+      const int2 *rng = a.range + C.bin_base + rowbin * nl;
+      for (int piece = 0; piece < 3; ++piece) {
+        int st = 0, en = 0, code = code0;
+        sh[D - 1] = 0.0f;
+        if (ok) {
+          if (inner) {
+            if (piece == 0) {
+              st = rng[last - 1].x;
+              en = rng[last + 1].y;
+            }
+          } else {
+            int v = last + piece - 1;
+            bool in = true;
+            if (v < 0) {
+              in = C.periodic[D - 1];
+              v += nl;
+              code |= 1 << (2 * (D - 1));
+              sh[D - 1] = -static_cast<float>(C.box[D - 1]);
+            } else if (v >= nl) {
+              in = C.periodic[D - 1];
+              v -= nl;
+              code |= 2 << (2 * (D - 1));
+              sh[D - 1] = static_cast<float>(C.box[D - 1]);
+            }
+            if (in) {
+              st = rng[v].x;
+              en = rng[v].y;
             }
           }
-      pairs();
+        }
+        for (int tt0 = st; __any_sync(0xffffffffu, tt0 < en); tt0 += L) {
+          const int tt = tt0 + sub;
+          bool near = false;
+          if (tt < en && tt != s && tt != ps) {
+            const float4 p = __ldg(a.rec + tt);
+            float r2f = 0.0f;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              const float dx = fmaxf(fabsf((pk_c(p, d) + sh[d]) - pk_c(me, d)) - margin[d], 0.0f);
+              r2f += dx * dx;
+            }
+            near = pair_maybe_reaches<LAW>(r2f, me.w, p.w, rcsf, xif);
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, near);
+          if (near) {
+            const int at = nb0 + cnt + __popc(m & below);
+            W.tt[at] = tt;
+            W.code[at] = static_cast<unsigned char>(code);
+          }
+          cnt += __popc(m & gmask);
+          if (__any_sync(0xffffffffu, cnt + L > cap)) {
+            __syncwarp();
+            flush();
+          }
+        }
+      }
     }
+    __syncwarp();
+    flush();
+  }
+  if (!live || sub != 0) return;
 
-    // ---- checks, integration, outputs
-    bool finite = true;
+  // ---- checks, integration, outputs
+  bool finite = true;
 #pragma unroll
-    for (int d = 0; d < D; ++d) finite = finite && isfinite(F[d]);
-    if (!finite) atomicOr(&a.cnt[c].err, kErrNan);
-    if (a.frc) {
+  for (int d = 0; d < D; ++d) finite = finite && finite_bits(F[d]);
+  if (!finite) atomicOr(&a.cnt[c].err, kErrNan);
+  if (a.frc) {
 #pragma unroll
-      for (int d = 0; d < D; ++d) a.frc[d * SS + s] = F[d];
+    for (int d = 0; d < D; ++d) a.frc[d * SS + s] = F[d];
+  }
+  if (a.integrate) {
+    const double temp = a.heun ? 0.5 * C.temp[j] : C.temp[j];  // (dt/2) / zeta is exact
+    bool inside = true;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const double tnew = __dadd_rn(xi[d], __dmul_rn(temp, F[d]));
+      double xn;
+      if (C.periodic[d]) {
+        xn = wrap_bits(tnew, C.box[d]);
+      } else {
+        xn = tnew;
+        inside = inside && (xn >= 0.0 && xn < C.box[d]);
+      }
+      a.x_out[d * SS + s] = xn;
     }
-    if (a.integrate) {
-      const double temp = a.heun ? 0.5 * C.temp[j] : C.temp[j];  // (dt/2) / zeta is exact
-      bool inside = true;
+    if (!inside) atomicOr(&a.cnt[c].err, kErrBox);
+    if (a.vel) {
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        const double tnew = __dadd_rn(xi[d], __dmul_rn(temp, F[d]));
-        double xn;
-        if (C.periodic[d]) {
-          xn = wrap_like_fmod(tnew, C.box[d]);
-        } else {
-          xn = tnew;
-          inside = inside && (xn >= 0.0 && xn < C.box[d]);
-        }
-        a.x_out[d * SS + s] = xn;
-      }
-      if (!inside) atomicOr(&a.cnt[c].err, kErrBox);
-      if (a.vel) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const double v = F[d] * C.mu_eff[j];
-          a.vel[d * SS + s] = a.heun == 2 ? 0.5 * ((a.vel_prev ? a.vel_prev : a.vel)[d * SS + s] + v) : v;
-        }
+        const double v = F[d] * C.mu_eff[j];
+        a.vel[d * SS + s] = a.heun == 2 ? 0.5 * ((a.vel_prev ? a.vel_prev : a.vel)[d * SS + s] + v) : v;
       }
     }
   }
@@ -1230,9 +1396,15 @@ constexpr size_t mixed_smem_bytes() {
 }
 
 template <int D, int LAW>
-void launch_dl(const ForceArgs &a, int prec, int grid, cudaStream_t s) {
+void launch_dl(const ForceArgs &a, int prec, int grid, int tiles, int lane_bits, cudaStream_t s) {
   if (prec == CIL_PREC_FP64) {
-    k_force_fp64<D, LAW><<<grid, kTile, 0, s>>>(a);
+    constexpr int bytes = kF64Block / 32 * static_cast<int>(sizeof(F64Warp<D>));
+    static bool attr_set = false;  // per instantiation; the attribute is per function
+    if (!attr_set) {
+      cudaFuncSetAttribute(k_force_fp64<D, LAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      attr_set = true;
+    }
+    k_force_fp64<D, LAW><<<tiles * (2 << lane_bits), kF64Block, bytes, s>>>(a, lane_bits);
   } else {
     constexpr size_t bytes = mixed_smem_bytes<D>();
     static bool attr_set = false;  // per instantiation; the attribute is per function
@@ -1246,19 +1418,19 @@ void launch_dl(const ForceArgs &a, int prec, int grid, cudaStream_t s) {
 }
 
 template <int D>
-void launch_d(const ForceArgs &a, int law, int prec, int grid, cudaStream_t s) {
+void launch_d(const ForceArgs &a, int law, int prec, int grid, int tiles, int lane_bits, cudaStream_t s) {
   switch (law) {
     case CIL_FORCE_LJ_WCA:
-      launch_dl<D, CIL_FORCE_LJ_WCA>(a, prec, grid, s);
+      launch_dl<D, CIL_FORCE_LJ_WCA>(a, prec, grid, tiles, lane_bits, s);
       break;
     case CIL_FORCE_SOFTCORE:
-      launch_dl<D, CIL_FORCE_SOFTCORE>(a, prec, grid, s);
+      launch_dl<D, CIL_FORCE_SOFTCORE>(a, prec, grid, tiles, lane_bits, s);
       break;
     case CIL_FORCE_SC:
-      launch_dl<D, CIL_FORCE_SC>(a, prec, grid, s);
+      launch_dl<D, CIL_FORCE_SC>(a, prec, grid, tiles, lane_bits, s);
       break;
     default:
-      launch_dl<D, CIL_FORCE_HERTZ>(a, prec, grid, s);
+      launch_dl<D, CIL_FORCE_HERTZ>(a, prec, grid, tiles, lane_bits, s);
       break;
   }
 }
@@ -1272,12 +1444,12 @@ void launch_force_list_3d(const ForceArgs &a, int law, int grid, int variant, in
   launch_list_d<3>(a, law, grid, variant, block, s);
 }
 
-void launch_force_3d(const ForceArgs &a, int law, int prec, int grid, cudaStream_t s) {
-  launch_d<3>(a, law, prec, grid, s);
+void launch_force_3d(const ForceArgs &a, int law, int prec, int grid, int tiles, int lane_bits, cudaStream_t s) {
+  launch_d<3>(a, law, prec, grid, tiles, lane_bits, s);
 }
 #else
 void launch_force_list_3d(const ForceArgs &a, int law, int grid, int variant, int block, cudaStream_t s);
-void launch_force_3d(const ForceArgs &a, int law, int prec, int grid, cudaStream_t s);
+void launch_force_3d(const ForceArgs &a, int law, int prec, int grid, int tiles, int lane_bits, cudaStream_t s);
 
 void launch_force_list(const ForceArgs &a, int dim, int law, int grid, int variant, int block, cudaStream_t s) {
   if (dim == 2)
@@ -1286,12 +1458,12 @@ void launch_force_list(const ForceArgs &a, int dim, int law, int grid, int varia
     launch_force_list_3d(a, law, grid, variant, block, s);
 }
 
-void launch_force(const ForceArgs &a, int dim, int law, int prec, int grid, int block, cudaStream_t s) {
-  (void)block;
+void launch_force(const ForceArgs &a, int dim, int law, int prec, int grid, int tiles, int lane_bits,
+                  cudaStream_t s) {
   if (dim == 2)
-    launch_d<2>(a, law, prec, grid, s);
+    launch_d<2>(a, law, prec, grid, tiles, lane_bits, s);
   else
-    launch_force_3d(a, law, prec, grid, s);
+    launch_force_3d(a, law, prec, grid, tiles, lane_bits, s);
 }
 #endif
 

@@ -532,27 +532,14 @@ __device__ __forceinline__ bool pair_force(R r2, R si, R sj, R eps, R rcs, R &f0
   }
 }
 
-// The range test of pair_force alone (the same expressions, so the same answer).
-template <int LAW, typename R>
-__device__ __forceinline__ bool pair_in_range(R r2, R si, R sj, R rcs, R xi) {
-  const R sij = R(0.5) * (si + sj);
-  if (LAW == CIL_FORCE_SC)
-    return r2 > rcs * rcs * ((sij - xi) * (sij - xi)) && r2 <= rcs * rcs * ((sij + xi) * (sij + xi));
-  if (LAW == CIL_FORCE_LJ_WCA) return r2 <= (sij * sij) * (rcs * rcs);
-  const R rc = rcs * sij;
-  return r2 < rc * rc && r2 > R(0);
-}
-
-// A superset of pair_in_range in FP32, for a squared separation r2f within a relative 1e-6 of
-// the FP64 one: the bounds are widened by 1e-5, so every pair that pair_force accepts passes.
+// Whether a pair whose separation is at least sqrt(r2f) may be inside pair_force's cutoff: the
+// bound is widened by 1e-5 for the FP32 rounding of the diameters and of the test itself, so every
+// pair that pair_force accepts passes (the soft-core well's lower bound is left to pair_force).
 template <int LAW>
-__device__ __forceinline__ bool pair_maybe_in_range(float r2f, float si, float sj, float rcs, float xi) {
+__device__ __forceinline__ bool pair_maybe_reaches(float r2f, float si, float sj, float rcs, float xi) {
   const float sij = 0.5f * (si + sj);
-  constexpr float up = 1.00001f, dn = 0.99999f;
-  if (LAW == CIL_FORCE_SC)
-    return r2f >= dn * (rcs * rcs * ((sij - xi) * (sij - xi))) && r2f <= up * (rcs * rcs * ((sij + xi) * (sij + xi)));
-  const float rc = rcs * sij;
-  return r2f <= up * (rc * rc);
+  const float rc = LAW == CIL_FORCE_SC ? rcs * (sij + xi) : rcs * sij;
+  return r2f <= 1.00001f * (rc * rc);
 }
 
 // FP32 pair force, branch-free: the law is evaluated for every candidate and masked
@@ -629,6 +616,7 @@ struct RebuildArgs {
   double *sig_out;
   int *eid_out;
   float4 *pk_out;          // mixed: packed elements of the new order, may be null
+  float4 *rec_out;         // FP64 form: FP32 absolute coordinates and diameter, new order; else null
   const float4 *pk_in;     // mixed: packed elements after the last update (relative to sbin_in)
   const int *sbin_in;      // home bin (colony-local id) of each slot
   int *sbin_out;
@@ -666,6 +654,7 @@ struct ForceArgs {
   double *x_out;           // integrated positions (same slots)
   const double *sig;       // FP64 form
   const int *eid;
+  const float4 *rec;       // FP64 form: FP32 absolute coordinates and diameter of every slot
   const float4 *pk;        // mixed: packed elements of this step
   float4 *pk_next;         // mixed: packed elements after the update (same slots)
   const int *sbin;         // home bin of each slot
@@ -857,7 +846,8 @@ void launch_rebuild(const RebuildArgs &a, int grid_slots, cudaStream_t s);
 // elements in the slot pair slot_base + 2 rank, + 1; tombstones dropped); a.tiles_cell must be
 // current; leaves bcount at zero and nslot = 2 ncell
 void launch_cell_resort(const RebuildArgs &a, int grid_cells, cudaStream_t s);
-void launch_force(const ForceArgs &a, int dim, int law, int prec, int grid, int block,
+// tiles: tiles of kTile slots over the capacity; lane_bits: log2 of the lanes per element (FP64 form)
+void launch_force(const ForceArgs &a, int dim, int law, int prec, int grid, int tiles, int lane_bits,
                   cudaStream_t s);
 // skin mode: the cell kernel (one thread per slot pair); block = cells per block (128, 256, 512);
 // a.tiles must be the pair tiles of that block size
