@@ -1509,7 +1509,8 @@ cil_status cil_upload(cil_handle *h, int32_t colony, const cil_colony_view *v) {
   CUDA_TRY(h, cudaMemcpyAsync(st_tsw, v->tswitch, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaMemsetAsync(h->d_upchk, 0, 4 * sizeof(int), h->stream));
   launch_upload(h->d_col, colony, n, D, h->SS, h->d_stage, h->d_x[h->cur], h->d_sigma_c, h->d_t0, h->d_tsw,
-                h->d_vel, h->d_eid[h->meta], h->d_slot_of, h->d_cnt, h->d_upchk, h->stream);
+                h->d_vel, h->d_eid[h->meta], h->d_slot_of, h->d_cnt, h->d_upchk, h->skin_mode ? h->d_sched : nullptr,
+                h->skin_mode ? h->d_spart : nullptr, h->stream);
   CUDA_TRY(h, cudaGetLastError());
   int chk[4] = {0, 0, 0, 0};
   CUDA_TRY(h, cudaMemcpyAsync(chk, h->d_upchk, sizeof chk, cudaMemcpyDeviceToHost, h->stream));
@@ -1545,8 +1546,6 @@ cil_status cil_upload(cil_handle *h, int32_t colony, const cil_colony_view *v) {
   h->obs_ready[colony] = 0;
   h->geometry_ready = false;
   h->need_exact = true;
-  // the scheduler's statistics restart with the new state
-  if (h->skin_mode) CUDA_TRY(h, cudaMemsetAsync(h->d_sched + colony, 0, sizeof(SchedState), h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return CIL_OK;
 }

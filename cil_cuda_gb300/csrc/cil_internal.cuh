@@ -877,7 +877,7 @@ void launch_sm_ops(const EventArgs &a, int colony, int nops, const int *ops, con
                    cudaStream_t s);
 void launch_upload(const ColonyConst *col, int colony, int ncells, int dim, size_t SS, const double *stage,
                    double *x, double *sig_c, int *t0, int *tsw, double *vel, int *eid, int *slot_of,
-                   ColonyCounters *cnt, int *chk, cudaStream_t s);
+                   ColonyCounters *cnt, int *chk, SchedState *sched, StatPart *spart, cudaStream_t s);
 void launch_gather_canonical(int ncells, int dim, size_t SS, int cell_base, const int *slot_of,
                              const double *src, int width, double *dst, cudaStream_t s);
 void launch_observables(const EventArgs &a, int colony, int ncells, int dim, int reset,
