@@ -2,28 +2,26 @@
 //
 // Layout: structure of arrays in index order (cell i at i), FP64. Two complete state sets;
 // a removal (apoptosis, drain) compacts the survivors stably into the other set and the host
-// flips the set index. Positions are double-buffered within a step (the force pass reads one
-// buffer and writes the other).
+// flips the set index. The pair passes read copies in bin order (CyOrdered), so they update the
+// state in place.
 //
 // A step (no host synchronisation; the cell count lives on the device):
-//   bins       k_cy_keys / scan / k_cy_scatter / k_cy_sort: a counting sort of the cells into
+//   bins       k_cy_keys / scan / k_cy_scatter / k_cy_place: a counting sort of the cells into
 //              bins (width set per call from the largest diameter), ascending cell index
-//              inside a bin; the pair search walks +-k bins with k from the colony's largest
-//              diameter of the previous step, so growing cells never outgrow the search; with
-//              FP32 pair arithmetic (precision 1), k_cy_pack writes the FP32 records of the bin
-//              order that the pair loops read instead of the FP64 positions;
-//   forces     k_cy_force: motility along the velocity, passive noise, Hertz contacts with
-//              adhesion and the pressure sum, then the position update with the pressure-
-//              dependent friction, in one thread per cell;
-//   cycle      k_cy_cycle (ODEs, division flag, per-block count) / k_cy_scan_blocks /
-//              k_cy_divide (daughters appended in mother order);
-//   apoptosis  k_cy_apo_mark / scan / k_cy_compact (only with apoptosis on).
-// The DPD integrator: k_dpd_kick_drift (first half kick and the drift), the bins, k_cy_force in
-// its forces-only mode (Fc and the pressure), k_dpd_pair (the pair dissipative and random
-// forces and the second half kick, into the spare velocity buffer), k_dpd_dis (background and
-// pair dissipation at the new velocities), then the same cycle and apoptosis kernels.
-// The file is compiled without FMA contraction, so that the arithmetic is that of the host
-// restatement the tests compare with.
+//              inside a bin, with copies of the positions and diameters in that order; the pair
+//              search walks +-k bins with k from the colony's largest diameter of the previous
+//              step, so growing cells never outgrow the search;
+//   forces     k_cy_force: Hertz contacts with adhesion and the pressure sum, motility along the
+//              velocity, passive noise, the position update with the pressure-dependent friction,
+//              and the cell's cycle (ODEs, division test);
+//   divisions  k_cy_divide (daughters appended in mother order; the step's counts);
+//   apoptosis  k_cy_mark / scan / k_cy_compact (only with apoptosis on).
+// The DPD integrator: k_cy_keys makes the first half kick and the drift, k_cy_force in its
+// forces-only mode gives Fc and the pressure, k_dpd_pair the pair dissipative and random forces and
+// the second half kick (into the spare velocity buffer), k_dpd_dis background and pair dissipation
+// at the new velocities and the cell's cycle; then the same divisions and apoptosis.
+// The file is compiled without FMA contraction: outside the forms of "FP64 arithmetic" below, the
+// arithmetic is that of the host restatement the tests compare with, to a few units of the last place.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,6 +29,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cil_cycle.h"
@@ -75,13 +74,14 @@ struct CyConst {
   double tau_div_mu, tau_div_sigma, tau_mig_mu, tau_mig_sigma;
   double v1, tau_r, tau_v, tau_p;   // tau_* in steps
   double v_s;
+  double growth, inv_vs_tau_v, inv_tau_r, inv_tau_r_neg, inv_p0;  // (v1 - 1) / tau_v, reciprocals
   double p0, beta_vs, rho_ratio, r_maxed_inv, p_shift, p_shift_tau_inv, osm;
   double apop_pressure, apop_duration, apop_rate_step, extr_gamma;
   double apop_steps;  // apop_duration / dt
   double extr_rate;
   // DPD
   int dpd;
-  double kick_div;    // 2 (2 m): updateVel's divisor with the mass argument 2 m
+  double inv_kick_div;  // 1 / (2 (2 m)): updateVel's divisor with the mass argument 2 m
   double sqrt_dt;
   double gamma_d, gamma_b, sigma_r;  // DISDIFCEL, DISBG, sqrt(2 DISDIFCEL kT)
   uint32_t seed_lo, seed_hi;
@@ -96,14 +96,14 @@ struct CySet {
   double *fc, *fd, *fr;  // [D][cap], DPD only (conservative, dissipative, random forces)
 };
 
-// FP32 records of the cells in bin order, for the FP32 pair arithmetic (precision 1): the
-// position relative to the origin of the cell's bin with the diameter, the velocity (DPD), and
-// each cell's place in the bin order. Displacements are then formed in FP32 from bin offsets,
-// with no FP64 operation per candidate.
-struct CyPacked {
-  float4 *pk;  // [q]: x - bin origin per axis (z 0 in 2D), diameter
-  float4 *vk;  // [q]: velocity (DPD)
-  int *qpos;   // [cell]: its place q
+// The cells in bin order, written by k_cy_place for the pair kernels: [q] is the cell at place q.
+struct CyOrdered {
+  double *x;    // [D][cap]
+  double *sig;
+  float4 *rec;  // FP32 position (z 0 in 2D) and diameter, for the range tests
+  float4 *vel;  // FP32 velocity (DPD, precision 1)
+  int *idx;     // the cell's index
+  int *bin;
 };
 
 struct CyCounters {
@@ -112,8 +112,11 @@ struct CyCounters {
   long long ndiv_total;
   long long napo_total;
   unsigned long long sigma_max_bits;  // largest diameter (non-negative doubles order like their bits)
+  unsigned long long sigma_next_bits;  // the same, of the step under way
   int ndiv_step;
   int nrem_step;
+  int ndue;   // cells at phase 1, of the step under way
+  int ndone;  // blocks of k_cy_divide that have finished
 };
 
 constexpr int kErrCapacity = 1;
@@ -163,14 +166,6 @@ __device__ inline double volume_of(double s) { return 4 * kPi * ((s / 2) * (s / 
 __device__ inline double sigma_of_area(double a) { return 2 * sqrt(a / kPi); }
 __device__ inline double sigma_of_volume(double v) { return 2 * cbrt(3 * v / (4 * kPi)); }
 
-__device__ inline double contact_length(double a, double b, double h) {
-  const double ra = a / 2, rb = b / 2;
-  const double q = ra - (2 * rb * h - h * h) / (2 * (ra + rb - h));
-  double t = 2 * sqrt(ra * ra - q * q);
-  const double small_r = (a <= b) ? a : b;
-  return isnan(t) ? small_r : t;
-}
-
 __device__ inline double contact_area(double r, double a, double b) {
   const double ra = a / 2, rb = b / 2;
   const double u = r * r - rb * rb + ra * ra;
@@ -178,9 +173,7 @@ __device__ inline double contact_area(double r, double a, double b) {
   return t > 0 ? kPi * (t * t) : 0.0;
 }
 
-__device__ inline double wrap(double t, double L) {  // fmod(t + L, L)
-  return fmod(t + L, L);
-}
+__device__ inline double wrap(double t, double L) { return cil::wrap_bits(t, L); }  // fmod(t + L, L)
 
 __device__ inline int bin_of(const CyConst &C, const double *xd) {
   int b = 0;
@@ -192,106 +185,7 @@ __device__ inline int bin_of(const CyConst &C, const double *xd) {
   return b;
 }
 
-// The bins around a cell that hold every cell within `radius` of it: k = ceil(radius / bin
-// width) bins on each side, the whole axis (each bin once) when 2k + 1 covers it, clipped at
-// non-periodic walls.
-struct Stencil {
-  int bi[3], lo[3], hi[3];
-};
-
-__device__ inline void stencil_of(const CyConst &C, const double *xi, double radius, Stencil &s) {
-  for (int d = 0; d < 3; ++d) s.bi[d] = s.lo[d] = s.hi[d] = 0;
-  CY_AXES(d, C.D) {
-    int v = static_cast<int>(xi[d] * C.inv_bw[d]);
-    v = v < 0 ? 0 : (v >= C.ns[d] ? C.ns[d] - 1 : v);
-    s.bi[d] = v;
-    const double kk = ceil(radius * C.inv_bw[d]);
-    const int k = (kk >= 0.0 && kk < C.ns[d]) ? static_cast<int>(kk) : C.ns[d];
-    if (2 * k + 1 >= C.ns[d]) {
-      s.lo[d] = -s.bi[d];
-      s.hi[d] = C.ns[d] - 1 - s.bi[d];
-    } else if (C.periodic[d]) {
-      s.lo[d] = -k;
-      s.hi[d] = k;
-    } else {
-      s.lo[d] = s.bi[d] - k < 0 ? -s.bi[d] : -k;
-      s.hi[d] = s.bi[d] + k >= C.ns[d] ? C.ns[d] - 1 - s.bi[d] : k;
-    }
-  }
-}
-
-__device__ inline int stencil_bin(const CyConst &C, const Stencil &s, int o0, int o1, int o2) {
-  const int oo[3] = {o0, o1, o2};
-  int b = 0;
-  CY_AXES(d, C.D) {
-    int v = s.bi[d] + oo[d];
-    if (v < 0) v += C.ns[d];
-    if (v >= C.ns[d]) v -= C.ns[d];
-    b = b * C.ns[d] + v;
-  }
-  return b;
-}
-
-// r_j - r_i at the nearest image (|dd| < L, so Nint(dd / L) is -1, 0 or 1; the two forms differ
-// only at |dd| = L/2, far beyond any contact); returns |r_j - r_i|^2
-__device__ inline double separation(const CyConst &C, const CySet &S, const double *xi, int j, double *rij) {
-  const size_t cap = C.capacity;
-  double r2 = 0.0;
-  CY_AXES(d, C.D) {
-    double dd = S.x[d * cap + j] - xi[d];
-    if (C.periodic[d]) {
-      if (dd > C.half[d])
-        dd -= C.box[d];
-      else if (dd < -C.half[d])
-        dd += C.box[d];
-    }
-    rij[d] = dd;
-    r2 += dd * dd;
-  }
-  return r2;
-}
-
 __device__ inline float f4c(const float4 &v, int d) { return d == 0 ? v.x : (d == 1 ? v.y : v.z); }
-
-// FP32 displacement from the packed record pi to pj, whose bin lies at offset o from pi's, at
-// the nearest image on periodic axes; returns its square length
-__device__ inline float packed_sep(const CyConst &C, const float4 &pi, const float4 &pj, int o0, int o1, int o2,
-                                   float *df) {
-  const int o[3] = {o0, o1, o2};
-  float r2 = 0.0f;
-  CY_AXES(d, C.D) {
-    float v = f4c(pj, d) + static_cast<float>(o[d]) * C.bwf[d] - f4c(pi, d);
-    if (C.periodic[d]) {
-      if (v > C.halff[d])
-        v -= C.boxf[d];
-      else if (v < -C.halff[d])
-        v += C.boxf[d];
-    }
-    df[d] = v;
-    r2 += v * v;
-  }
-  return r2;
-}
-
-// The squared minimum-image separation in FP32 from the FP64 difference, for the walks' range
-// tests: within a relative 1e-6 of separation()'s (a pair near half a box may wrap the other
-// way, and is out of range either way), so bounds widened by 1e-5 let every pair in range pass
-// to the exact FP64 test.
-__device__ inline float separation_f(const CyConst &C, const CySet &S, const double *xi, int j) {
-  const size_t cap = C.capacity;
-  float r2 = 0.0f;
-  CY_AXES(d, C.D) {
-    float v = static_cast<float>(S.x[d * cap + j] - xi[d]);
-    if (C.periodic[d]) {
-      if (v > C.halff[d])
-        v -= C.boxf[d];
-      else if (v < -C.halff[d])
-        v += C.boxf[d];
-    }
-    r2 += v * v;
-  }
-  return r2;
-}
 
 // ---------------------------------------------------------------- block scan
 // Exclusive scan over the block (any multiple of 32 threads up to kTile)
@@ -344,330 +238,609 @@ __global__ void k_cy_chunk_sums(const int *count, int m, int *part) {
   if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-// Exclusive scan of count[0..m) using the scanned chunk sums, into start[0..m] (start[m] =
-// total; the chunks cover index m, count[m] reads as 0)
-__global__ void k_cy_chunk_apply(const int *count, int m, const int *part, int *start) {
+// Exclusive scan of count[0..m) into start[0..m] (start[m] = total; the chunks cover index m,
+// count[m] reads as 0); count is left at zero. part: the chunk sums, scanned when `scanned`, otherwise
+// each block adds those before it itself (a few loads per thread, cheaper than a launch).
+__global__ void k_cy_chunk_apply(int *count, int m, const int *part, int *start, int scanned) {
   const int b0 = blockIdx.x * kScanTile + threadIdx.x * 4;
   int c[4], s = 0;
   for (int q = 0; q < 4; ++q) {
     c[q] = (b0 + q < m) ? count[b0 + q] : 0;
+    if (b0 + q < m) count[b0 + q] = 0;
     s += c[q];
   }
+  int before = 0;
+  if (scanned) {
+    before = part[blockIdx.x];
+  } else {
+    int v = 0;
+    for (int u = threadIdx.x; u < static_cast<int>(blockIdx.x); u += kTile) v += part[u];
+    block_excl_scan(v, &before);
+  }
   int tot;
-  int e = part[blockIdx.x] + block_excl_scan(s, &tot);
+  int e = before + block_excl_scan(s, &tot);
   for (int q = 0; q < 4; ++q) {
     if (b0 + q <= m) start[b0 + q] = e;
     e += c[q];
   }
 }
 
-// ---------------------------------------------------------------- bins
-__global__ void k_cy_clear(int *a, int m) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) a[i] = 0;
+// ---------------------------------------------------------------- FP64 arithmetic
+// GB300's FP64 pipe runs 2 lanes a clock per SM (1/64 of FP32), so the kernels below count FP64
+// instructions: one reciprocal square root per root or quotient, products with constants in place
+// of divisions, comparisons and sign tests on bit patterns.
+
+// 1 / sqrt(a) for normal a > 0: the hardware's approximate reciprocal square root y, then the
+// series 1 / sqrt(1 - e) = 1 + e / 2 + 3 e^2 / 8 + ... with e = 1 - a y^2 (its next term is below
+// 2^-53 for a seed good to 2^-18).
+__device__ inline double rsqrt_pos(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = __fma_rn(-(a * y), y, 1.0);
+  return __fma_rn(__fma_rn(0.375, e, 0.5), y * e, y);
 }
 
-// the bin of every cell, and 1 / (sigma / 2) for the contact pass (the same value it would
-// compute per contact)
-__global__ void k_cy_keys(CyConst C, CySet S, const CyCounters *cnt, int *key, int *count, double *inv_r) {
+// sqrt(a) from y = rsqrt_pos(a): a y and one Newton residual
+__device__ inline double sqrt_from(double a, double y) {
+  const double s = a * y;
+  return __fma_rn(__fma_rn(-s, s, a), 0.5 * y, s);
+}
+
+// 1 / a for normal a: the approximate reciprocal y, then 1 / (1 - e) = 1 + e + e^2 + ... with
+// e = 1 - a y
+__device__ inline double rcp_normal(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = __fma_rn(-a, y, 1.0);
+  return __fma_rn(__fma_rn(e, e, e), y, y);
+}
+
+// positive, and far enough from the ends of the range that the forms above and their products
+// neither overflow nor lose bits (high word: 2^-510 to 2^510)
+__device__ inline bool mid_range(double a) {
+  const int h = __double2hiint(a);
+  return h >= 0x20000000 && h < 0x5fd00000;
+}
+
+__device__ inline bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+
+// ---------------------------------------------------------------- bins
+// A counting sort of the cells into bins: k_cy_keys counts (a cell's arrival rank in its bin comes
+// with the count), the scan gives the bins' starts and leaves the counts at zero for the next call,
+// k_cy_scatter fills the bins in arrival order, k_cy_place gives each cell its place by index in its
+// bin and writes the bin-ordered copies that the pair kernels read.
+
+// DPD's first half kick and drift (updateVelocities then updatePositions, CIL.cu:871-897, 849-866;
+// DPD step, CIL.cu:1055-1056) of the keys' own cells: no pass of its own over the positions.
+__device__ inline double kick(const CyConst &C, double v, double fc, double fd, double fr) {
+  return v + (fc * C.dt + fd * C.dt + fr * C.sqrt_dt) * C.inv_kick_div;  // updateVel (Utils.hpp:568-571)
+}
+
+__global__ void __launch_bounds__(kTile) k_cy_keys(CyConst C, CySet S, const CyCounters *cnt, int *key, int *arrival,
+                                                   int *count, int *dblk, int drift) {
+  if (threadIdx.x == 0) dblk[blockIdx.x] = 0;  // the coming step's divisions per block of cells
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt->n) return;
-  inv_r[i] = 1.0 / (S.sig[i] / 2);
   double xd[3];
-  CY_AXES(d, C.D) xd[d] = S.x[static_cast<size_t>(d) * C.capacity + i];
+  CY_AXES(d, C.D) {
+    const size_t k = static_cast<size_t>(d) * C.capacity + i;
+    xd[d] = S.x[k];
+    if (drift) {
+      const double v = kick(C, S.v[k], S.fc[k], S.fd[k], S.fr[k]);
+      S.v[k] = v;
+      const double t = xd[d] + C.dt * v;
+      xd[d] = C.periodic[d] ? wrap(t, C.box[d]) : t;  // BoundingBox::updatePos
+      S.x[k] = xd[d];
+    }
+  }
   const int b = bin_of(C, xd);
   key[i] = b;
-  atomicAdd(count + b, 1);
+  arrival[i] = atomicAdd(count + b, 1);
 }
 
-__global__ void k_cy_scatter(const CyCounters *cnt, const int *key, const int *start, int *cursor, int *list) {
+__global__ void __launch_bounds__(kTile) k_cy_scatter(const CyCounters *cnt, const int *key, const int *arrival,
+                                                      const int *start, int *tmp) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt->n) return;
-  const int b = key[i];
-  const int pos = start[b] + atomicAdd(cursor + b, 1);
-  list[pos] = i;
+  tmp[start[key[i]] + arrival[i]] = i;
 }
 
-// ascending cell index inside every bin (insertion sort: bins hold a few cells; a bin with
-// more than kBinSortMax cells means overlapping cells and is reported instead of sorted)
-__global__ void k_cy_sort(const int *start, int nbins, int *list, CyCounters *cnt) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbins) return;
-  const int lo = start[b], hi = start[b + 1];
+// The bin order: a cell's place is its bin's start plus the number of smaller indices in the bin
+// (bins hold a few cells; a bin with more than kBinSortMax means overlapping cells and is reported,
+// its cells in arrival order). Written at the place: the index, the bin, the FP64 position and
+// diameter, and the FP32 record (absolute position and diameter) of the range tests.
+__global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounters *cnt, const int *key,
+                                                    const int *arrival, const int *start, const int *tmp,
+                                                    CyOrdered O, int with_vel) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cnt->n) return;
+  const int b = key[i], lo = start[b], hi = start[b + 1];
+  int rank = 0;
   if (hi - lo > kBinSortMax) {
     atomicOr(&cnt->err, kErrCrowded);
-    return;
+    rank = arrival[i];
+  } else {
+    for (int q = lo; q < hi; ++q) rank += tmp[q] < i ? 1 : 0;
   }
-  for (int i = lo + 1; i < hi; ++i) {
-    const int v = list[i];
-    int j = i - 1;
-    while (j >= lo && list[j] > v) {
-      list[j + 1] = list[j];
-      --j;
-    }
-    list[j + 1] = v;
-  }
-}
-
-// The packed records of the bin order (CyPacked); vk only when velocities are wanted
-__global__ void k_cy_pack(CyConst C, CySet S, const CyCounters *cnt, const int *list, CyPacked P, int with_vel) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= cnt->n) return;
-  const int i = list[q];
+  const int q = lo + rank;
   const size_t cap = C.capacity;
-  float rel[3] = {0.0f, 0.0f, 0.0f}, vf[3] = {0.0f, 0.0f, 0.0f};
+  float xf[3] = {0.0f, 0.0f, 0.0f}, vf[3] = {0.0f, 0.0f, 0.0f};
   CY_AXES(d, C.D) {
     const double x = S.x[d * cap + i];
-    int v = static_cast<int>(x * C.inv_bw[d]);
-    v = v < 0 ? 0 : (v >= C.ns[d] ? C.ns[d] - 1 : v);
-    rel[d] = static_cast<float>(x - v * C.bw[d]);
+    O.x[d * cap + q] = x;
+    xf[d] = static_cast<float>(x);
     if (with_vel) vf[d] = static_cast<float>(S.v[d * cap + i]);
   }
-  P.pk[q] = make_float4(rel[0], rel[1], rel[2], static_cast<float>(S.sig[i]));
-  if (with_vel) P.vk[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
-  P.qpos[i] = q;
+  const double sg = S.sig[i];
+  O.sig[q] = sg;
+  O.idx[q] = i;
+  O.bin[q] = b;
+  O.rec[q] = make_float4(xf[0], xf[1], xf[2], static_cast<float>(sg));
+  if (with_vel) O.vel[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
 }
 
-__global__ void k_cy_pack_vel(CyConst C, CySet S, const CyCounters *cnt, const int *list, CyPacked P) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= cnt->n) return;
-  const int i = list[q];
-  const size_t cap = C.capacity;
-  float vf[3] = {0.0f, 0.0f, 0.0f};
-  CY_AXES(d, C.D) vf[d] = static_cast<float>(S.v[d * cap + i]);
-  P.vk[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
+// ---------------------------------------------------------------- the pair walk
+// 2^lane_bits lanes per cell in bin order, no block cooperation. What bounds the pair kernels is the
+// FP64 pipe, so FP64 runs for the pairs in range only, with full warps:
+//   walk    the candidates of the stencil's rows of bins along the last axis (consecutive bins hold
+//           consecutive places), tested in FP32 against a reach widened by the rounding of the
+//           records; a cell's lanes take consecutive candidates and a ballot keeps the survivors in
+//           walk order, so that the sums do not depend on the lane count;
+//   pairs   the warp's survivors as one flattened range, a pair per lane;
+//   sums    a cell's first lane adds its pairs in walk order.
+// One thread per cell with each contact evaluated where it was met took 1079 us for the contacts of
+// 1M cells (2.6 contacts a cell, FP64) and 43 us for 0.15M with FP32 pair terms.
+constexpr int kPairBlock = 128;
+constexpr int kPairNear = 384;  // survivors held per warp (12 per cell at one lane each)
+constexpr int kPairSeg = 128;   // pairs evaluated before their sums are taken
+
+template <int D, int NRES, typename R>
+struct PairWarp {
+  R res[kPairSeg * NRES];
+  double x[32 * D], v[32 * D];
+  double sig[32];
+  int idx[32];
+  int tt[kPairNear];
+  unsigned char own[kPairNear];
+};
+
+// r_j - r_i at the nearest image (|dd| < L, so Nint(dd / L) is -1, 0 or 1; the two forms differ
+// only at |dd| = L/2), the comparison on bit patterns
+__device__ inline double nearest(double dd, double L, double half) {
+  const long long b = __double_as_longlong(dd);
+  if ((b & 0x7fffffffffffffffll) > __double_as_longlong(half)) return b < 0 ? dd + L : dd - L;
+  return dd;
+}
+
+// reach2(me, p): the squared range of a pair in FP32 (an upper bound up to rounding);
+// pair(o, tt, out): the terms of the pair of the warp's cell o and the cell at place tt (in range or
+// not: the exact test is the callee's, which writes zeros out of range); acc: the cell's sums,
+// complete in its first lane. radius: no pair farther apart is in range. Whole warp.
+template <int D, int NRES, typename R, class Reach, class Pair>
+__device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R> &W, const CyOrdered &O,
+                                           const int *start, bool live, int q, int lane_bits, double radius,
+                                           Reach reach2, Pair pair, R *acc) {
+  const int lane = threadIdx.x & 31, L = 1 << lane_bits;
+  const int sub = lane & (L - 1), el = lane >> lane_bits;
+  const unsigned gmask = (L == 32 ? 0xffffffffu : (1u << L) - 1u) << (lane & ~(L - 1));
+  const unsigned below = gmask & ((1u << lane) - 1u);
+  const int cap = kPairNear >> (5 - lane_bits);
+  const int nb0 = el * cap;
+  int cnt = 0;
+  auto flush = [&]() {
+    int inc = sub == 0 ? cnt : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    const int end = __shfl_sync(0xffffffffu, inc, lane & ~(L - 1));
+    const int off = end - cnt;
+    for (int k = sub; k < cnt; k += L) W.own[off + k] = static_cast<unsigned char>(el);
+    __syncwarp();
+    for (int S = 0; S < total; S += kPairSeg) {
+      const int E = min(total, S + kPairSeg);
+      for (int f0 = S; f0 < E; f0 += 32) {  // uniform
+        const int f = f0 + lane;
+        const int o = f < E ? W.own[f] : 0;
+        const int offo = __shfl_sync(0xffffffffu, off, o << lane_bits);
+        if (f < E) pair(o, W.tt[o * cap + (f - offo)], &W.res[(f - S) * NRES]);
+      }
+      __syncwarp();
+      if (sub == 0) {
+        for (int f = max(off, S); f < min(end, E); ++f)
+#pragma unroll
+          for (int k = 0; k < NRES; ++k) acc[k] += W.res[(f - S) * NRES + k];
+      }
+      __syncwarp();
+    }
+    cnt = 0;
+  };
+  // the cell's bin and the bins to search on each side: k = ceil(radius / bin width), the whole axis
+  // (each bin once) when 2k + 1 covers it, clipped at open walls
+  int bi[D], lo[D], hi[D];
+  {
+    int b = live ? O.bin[q] : 0;
+#pragma unroll
+    for (int d = D - 1; d >= 0; --d) {
+      bi[d] = d > 0 ? b % C.ns[d] : b;
+      b /= C.ns[d];
+      const double kk = ceil(radius * C.inv_bw[d]);
+      const int k = (kk >= 0.0 && kk < C.ns[d]) ? static_cast<int>(kk) : C.ns[d];
+      if (2 * k + 1 >= C.ns[d]) {
+        lo[d] = -bi[d];
+        hi[d] = C.ns[d] - 1 - bi[d];
+      } else if (C.periodic[d]) {
+        lo[d] = -k;
+        hi[d] = k;
+      } else {
+        lo[d] = bi[d] - k < 0 ? -bi[d] : -k;
+        hi[d] = bi[d] + k >= C.ns[d] ? C.ns[d] - 1 - bi[d] : k;
+      }
+    }
+  }
+  const float4 me = live ? O.rec[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  // FP32 rounds both positions, the box and the differences, each by 2^-24 of a value within
+  // max(box, |x|) or so: 2^-21 of their sum bounds a separation's error along an axis
+  float margin[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) margin[d] = 4.76837158e-07f * (C.boxf[d] + fabsf(f4c(me, d)));
+  const int nl = C.ns[D - 1];
+  // rows of bins over the other axes; the loop runs to the warp's longest stencil
+  const int n0 = live ? hi[0] - lo[0] + 1 : 0, n1 = D == 3 ? hi[D - 2] - lo[D - 2] + 1 : 1;
+  const int rows = n0 * n1;
+  const int rows_w = __reduce_max_sync(0xffffffffu, rows);
+  for (int row = 0; row < rows_w; ++row) {
+    const bool ok = row < rows;
+    int rb = 0;
+    if (ok) {
+      int v = bi[0] + lo[0] + (D == 3 ? row / n1 : row);
+      if (v < 0) v += C.ns[0];
+      if (v >= C.ns[0]) v -= C.ns[0];
+      rb = v;
+      if (D == 3) {
+        int u = bi[1] + lo[1] + row % n1;
+        if (u < 0) u += C.ns[1];
+        if (u >= C.ns[1]) u -= C.ns[1];
+        rb = rb * C.ns[1] + u;
+      }
+    }
+    // the row's span of the last axis in up to three pieces of consecutive bins: below 0, inside, at
+    // or past the end
+    const int a = bi[D - 1] + lo[D - 1], z = bi[D - 1] + hi[D - 1];
+    const int *rs = start + static_cast<size_t>(rb) * nl;
+    for (int piece = 0; piece < 3; ++piece) {
+      int st = 0, en = 0;
+      if (ok) {
+        if (piece == 0) {
+          if (a < 0) {
+            st = rs[a + nl];
+            en = rs[nl];
+          }
+        } else if (piece == 1) {
+          st = rs[max(a, 0)];
+          en = rs[min(z, nl - 1) + 1];
+        } else if (z >= nl) {
+          st = rs[0];
+          en = rs[z - nl + 1];
+        }
+      }
+      for (int tt0 = st; __any_sync(0xffffffffu, tt0 < en); tt0 += L) {
+        const int tt = tt0 + sub;
+        bool near = false;
+        if (tt < en && tt != q) {
+          const float4 p = __ldg(O.rec + tt);
+          float r2 = 0.0f;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            float dx = fabsf(f4c(p, d) - f4c(me, d));
+            if (C.periodic[d] && dx > C.halff[d]) dx = fabsf(dx - C.boxf[d]);
+            dx = fmaxf(dx - margin[d], 0.0f);
+            r2 += dx * dx;
+          }
+          near = !(r2 > 1.00001f * reach2(me, p));
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, near);
+        if (near) W.tt[nb0 + cnt + __popc(m & below)] = tt;
+        cnt += __popc(m & gmask);
+        if (__any_sync(0xffffffffu, cnt + L > cap)) {
+          __syncwarp();
+          flush();
+        }
+      }
+    }
+  }
+  __syncwarp();
+  flush();
+}
+
+// ---------------------------------------------------------------- the cell cycle of one cell
+// The cycle ODEs at the step's end with pressure p; a cell at phase 1 is counted for k_cy_divide
+// (by its block of kTile cells, so that daughters come in mother order). Returns the bits of the
+// cell's diameter.
+__device__ inline unsigned long long cycle_update(const CyConst &C, const CySet &S, CyCounters *cnt, int *dblk, int i,
+                                                  int ts, double p, double sig) {
+  // cellTPressure (CIL.cu:493-494): every cell is in the dividing state when the species divides
+  S.tp[i] = p < C.apop_pressure ? 0 : S.tp[i] + 1;
+  const double shift = C.p_shift != 0.0 ? C.p_shift * exp(-ts * C.p_shift_tau_inv) : 0.0;
+  double pnd = 0.0;
+  if (shift != 0.0 || __double_as_longlong(p) > 0) {  // fmax(0, p) / p0, the quotient by its residual
+    const double pp = fmax(0., p + shift);
+    pnd = pp * C.inv_p0;
+    pnd = __fma_rn(__fma_rn(-pnd, C.p0, pp), C.inv_p0, pnd);
+  }
+  const double om = S.om[i];
+  double rho = S.rho[i];
+  const double theta = S.theta[i] + om * fmin(C.r_maxed_inv * rho, 1.0);
+  S.theta[i] = theta;
+  const bool d3 = C.D == 3;
+  const double st = S.sigt[i];
+  double vt = d3 ? volume_of(st) : area_of(st);
+  const double vt_prime = (om * kLn2 + C.growth) * rho - (vt - C.v_s) * C.inv_vs_tau_v;
+  vt += vt_prime * vt;
+  double v = vt;  // CYCLE_TAU_P 0 takes the target at once
+  if (C.tau_p != 0) {
+    v = d3 ? volume_of(sig) : area_of(sig);
+    v += -(v - (vt / (1 + C.beta_vs * (C.osm + pnd)))) / C.tau_p;
+  }
+  double sn;
+  if (d3) {
+    S.sigt[i] = sigma_of_volume(vt);
+    sn = sigma_of_volume(v);
+  } else {
+    const double a = vt * (4 / kPi);  // 2 sqrt(vt / pi)
+    const double s = mid_range(a) ? sqrt_from(a, rsqrt_pos(a)) : sigma_of_area(vt);
+    S.sigt[i] = s;
+    sn = C.tau_p == 0 ? s : sigma_of_area(v);
+  }
+  S.sig[i] = sn;
+  const double r_np = (1 - rho - pnd);
+  rho += r_np * (r_np > 0 ? C.inv_tau_r : C.inv_tau_r_neg) * rho;
+  S.rho[i] = rho;
+  if (theta >= 1) {
+    atomicAdd(dblk + i / kTile, 1);
+    atomicAdd(&cnt->ndue, 1);
+  }
+  return static_cast<unsigned long long>(__double_as_longlong(sn));
+}
+
+// the step's largest diameter, one atomic per warp that raises it
+__device__ inline void raise_sigma(CyCounters *cnt, unsigned long long s) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, s, o);
+    s = v > s ? v : s;
+  }
+  if ((threadIdx.x & 31) == 0 && s > *reinterpret_cast<volatile unsigned long long *>(&cnt->sigma_next_bits))
+    atomicMax(&cnt->sigma_next_bits, s);
 }
 
 // ---------------------------------------------------------------- forces + update
-// MIXED: the candidate test and the contact arithmetic in FP32 on the FP64 separation (GB300
-// runs FP64 at a small fraction of its FP32 rate); the forces and the pressure are summed in
-// FP32 over the contacts and added to the FP64 motility and noise; the position update and
-// the cell state stay FP64.
-// mode 0 (Euler): the position update with the pressure-dependent friction follows, into x_out,
-// and the velocity; mode 1 (DPD): the force goes to frc and nothing moves. Draws are keyed by
-// the device step counter + key_off.
-template <bool MIXED>
-// lane_bits: 2^lane_bits threads share a cell (small colonies): lane l takes the l-th of every
-// 2^lane_bits candidates of the flattened bin walk, and the lanes' contact sums are combined by
-// a fixed xor tree (the restatement combines them the same way); lane 0 writes.
-__global__ void __launch_bounds__(kTile) k_cy_force(CyConst C, CySet S, double *x_out, double *frc,
-                                                    CyCounters *cnt, const int *start, const int *list,
-                                                    const int *ts_dev, int mode, int key_off, CyPacked P,
-                                                    int lane_bits, const double *inv_r) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int L = 1 << lane_bits;
-  const int i = t >> lane_bits, lane = t & (L - 1);
-  const int n = cnt->n;
-  if (i >= n) return;  // a cell's lanes leave together (they share a warp)
-  const int ts = *ts_dev + key_off;
-  const size_t cap = C.capacity;
-  const int D = C.D;
-  double xi[3] = {0, 0, 0}, vi[3] = {0, 0, 0}, F[3] = {0, 0, 0};
-  CY_AXES(d, D) {
-    xi[d] = S.x[d * cap + i];
-    vi[d] = S.v[d * cap + i];
-  }
-  const double si = S.sig[i];
-  // ---- motility along the velocity (singleCellForce, MD.cu:600-646)
-  {
-    double v2 = 0.0;
-    CY_AXES(d, D) v2 += vi[d] * vi[d];
-    double vl = sqrt(v2);
-    if (vl == 0.0) {  // a direction at random, length 1e-11 (BIG_TOL_MP)
-      const u32x4 r = draw(C, i, ts, kCyDir, 0);
-      if (D == 2) {
-        const double ang = 6.283185307179586 * u53(r.v[0], r.v[1]);
-        vi[0] = 1e-11 * cos(ang);
-        vi[1] = 1e-11 * sin(ang);
-      } else {
-        const double z = 2.0 * u53(r.v[0], r.v[1]) - 1.0;
-        const double ang = 6.283185307179586 * u53(r.v[2], r.v[3]);
-        const double s = sqrt(1.0 - z * z);
-        vi[0] = 1e-11 * (s * cos(ang));
-        vi[1] = 1e-11 * (s * sin(ang));
-        vi[2] = 1e-11 * z;
-      }
-      v2 = 0.0;
-      CY_AXES(d, D) v2 += vi[d] * vi[d];
-      vl = sqrt(v2);
-    }
-    CY_AXES(d, D) F[d] = C.motility * (vi[d] / vl);
-  }
-  // ---- passive noise (CIL.cu:84-97)
-  if (C.noise_amp > 0.0) {
-    double nz[4];
-    normal2(draw(C, i, ts, kCyNoise, 0), &nz[0], &nz[1]);
-    if (D == 3) normal2(draw(C, i, ts, kCyNoise, 1), &nz[2], &nz[3]);
-    CY_AXES(d, D) F[d] += C.zeta * (C.noise_amp * nz[d]);
-  }
-  // ---- Hertz contacts with adhesion and the pressure (device draft, MD.cu:302-366)
-  double pres = 0.0;
-  double Fc[3] = {0.0, 0.0, 0.0};  // the contacts' share of the force
-  {
-    // bins to search on each side: the largest diameter of the colony over the bin width
-    Stencil st;
-    stencil_of(C, xi, __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)), st);
-    int kflat = 0;  // candidates of the bins walked so far
-    const double c2 = C.hz_c + C.hz_c;
-    const double inv_hz = 1.0 / (0.75 * c2);
-    const double inv_ri = 1.0 / (si / 2);
-    const float sif = static_cast<float>(si), c2f = static_cast<float>(c2), adhf = static_cast<float>(C.adhesion);
-    const float inv_rif = 2.0f / sif;
-    float Ff[3] = {0.0f, 0.0f, 0.0f}, presf = 0.0f;
-    const int qi = MIXED ? P.qpos[i] : 0;
-    const float4 pi4 = MIXED ? P.pk[qi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    // FP64: the candidates that pass the cheap distance test, in walk order (kNear at a time)
-    constexpr int kNear = 16;
-    int near[kNear];
-    int nnear = 0;
-    auto contacts = [&]() {
-      for (int k = 0; k < nnear; ++k) {
-        const int j = near[k];
-        double rij[3] = {0, 0, 0};
-        const double r2 = separation(C, S, xi, j, rij);
-        const double sj = S.sig[j];
-        const double cut = (si + sj) / 2;
-        const double r = sqrt(r2);
-        if (!(r <= cut) || r == 0.0) continue;
-        // the pair's first cell is the one of lower index (the contact length is not
-        // symmetric in the two diameters)
-        const double sa = i < j ? si : sj, sb = i < j ? sj : si;
-        const double h = fmax((si + sj) / 2 - r, 0.0);
-        const double Sr = inv_ri + inv_r[j];
-        // h^1.5 / (0.75 c2 sqrt(S)) as h sqrt(h / S) / (0.75 c2): one square root fewer
-        double fel, f0;
-        if (D == 3) {
-          fel = h * sqrt(h / Sr) * inv_hz;
-          const double A = contact_area(r, sa, sb);
-          const double vol = (A == 0 ? 0 : (4 * kPi * ((sa / 2) * (sa / 2)) / 3));
-          f0 = -fel + C.adhesion * A;
-          if (vol != 0.0) pres -= f0 / vol;
-        } else {
-          const double A = contact_length(sa, sb, h);  // also the contact's volume in 2D
-          if (A != 0.0) {
-            // one reciprocal u = 1 / (S A) gives both h / S = h A u and f0 / A = f0 S u
-            const double u = 1.0 / (Sr * A);
-            fel = h * sqrt(h * (A * u)) * inv_hz;
-            f0 = -fel + C.adhesion * A;
-            pres -= f0 * (Sr * u);
-          } else {
-            fel = h * sqrt(h / Sr) * inv_hz;
-            f0 = -fel;
-          }
-        }
-        CY_AXES(d, D) Fc[d] += f0 * rij[d];
-      }
-      nnear = 0;
-    };
-    for (int o0 = st.lo[0]; o0 <= st.hi[0]; ++o0)
-      for (int o1 = (D > 1 ? st.lo[1] : 0); o1 <= (D > 1 ? st.hi[1] : 0); ++o1)
-        for (int o2 = (D > 2 ? st.lo[2] : 0); o2 <= (D > 2 ? st.hi[2] : 0); ++o2) {
-          const int b = stencil_bin(C, st, o0, o1, o2);
-          const int e0 = start[b], e1 = start[b + 1];
-          const int first = e0 + ((lane - kflat) & (L - 1));
-          kflat += e1 - e0;
-          for (int q = first; q < e1; q += L) {
-            if (MIXED) {
-              if (q == qi) continue;
-              const float4 pj = P.pk[q];
-              float df[3] = {0.0f, 0.0f, 0.0f};
-              const float r2f = packed_sep(C, pi4, pj, o0, o1, o2, df);
-              const float sjf = pj.w;
-              const float cut = 0.5f * (sif + sjf);
-              if (!(r2f <= cut * cut) || r2f == 0.0f) continue;
-              const int j = list[q];
-              const float r = sqrtf(r2f);
-              const float sa = i < j ? sif : sjf, sb = i < j ? sjf : sif;
-              const float h = fmaxf(cut - r, 0.0f);
-              const float fel = (h * sqrtf(h)) / (0.75f * c2f * sqrtf(inv_rif + 2.0f / sjf));
-              float A, vol;
-              if (D == 3) {
-                const float ra = 0.5f * sa, rb = 0.5f * sb;
-                const float u = r2f - rb * rb + ra * ra;
-                const float t = sqrtf(4.0f * r2f * (ra * ra) - u * u) / (2.0f * r);
-                A = t > 0.0f ? static_cast<float>(kPi) * (t * t) : 0.0f;
-                vol = A == 0.0f ? 0.0f : (4.0f * static_cast<float>(kPi) * (ra * ra) / 3.0f);
-              } else {
-                const float ra = 0.5f * sa, rb = 0.5f * sb;
-                const float qq = ra - (2.0f * rb * h - h * h) / (2.0f * (ra + rb - h));
-                const float t = 2.0f * sqrtf(ra * ra - qq * qq);
-                A = isnan(t) ? fminf(sa, sb) : t;
-                vol = A;
-              }
-              const float f0 = -fel + adhf * A;
-              if (vol != 0.0f) presf -= f0 / vol;
-              CY_AXES(d, D) Ff[d] += f0 * df[d];
-              continue;
-            }
-            const int j = list[q];
-            if (j == i) continue;
-            const float cutf = 0.5f * (sif + static_cast<float>(S.sig[j]));
-            if (separation_f(C, S, xi, j) > 1.00001f * (cutf * cutf)) continue;  // out of contact (exact test in contacts())
-            // near candidates are evaluated together after the walk (contacts), so the warp runs
-            // the FP64 contact arithmetic with its lanes converged instead of once per candidate
-            near[nnear++] = j;
-            if (nnear == kNear) contacts();
-          }
-        }
-    if (!MIXED) contacts();
-    if (L > 1) {  // lanes l and l ^ 2^k combine, k from the highest: a fixed tree
-      const unsigned gm = (L == 32 ? 0xffffffffu : ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1)));
-      for (int off = L >> 1; off > 0; off >>= 1) {
-        if (MIXED) {
-          presf += __shfl_xor_sync(gm, presf, off, L);
-          CY_AXES(d, D) Ff[d] += __shfl_xor_sync(gm, Ff[d], off, L);
-        } else {
-          pres += __shfl_xor_sync(gm, pres, off, L);
-          CY_AXES(d, D) Fc[d] += __shfl_xor_sync(gm, Fc[d], off, L);
-        }
-      }
-    }
-    CY_AXES(d, D) F[d] += Fc[d];
-    if (MIXED) {
-      pres += static_cast<double>(presf);
-      CY_AXES(d, D) F[d] += static_cast<double>(Ff[d]);
-    }
-  }
-  if (lane != 0) return;
-  bool finite = true;
-  CY_AXES(d, D) finite = finite && isfinite(F[d]);
-  S.p[i] = pres;
-  if (!finite) atomicOr(&cnt->err, kErrNonFinite);
-  if (mode == 1) {
-    CY_AXES(d, D) frc[d * cap + i] = F[d];
+// The contact of cells a and b (a the lower index) at distance r = 1 / y <= (sa + sb) / 2, the device
+// draft's Hertz law with adhesion and its pressure (MD.cu:302-366): the force along the separation
+// f0 = -fel + adhesion A, fel = h^1.5 / (0.75 c2 sqrt(1/ra + 1/rb)), and f0 / (contact volume).
+// 2D: with h = ra + rb - r the contact length A = 2 sqrt(ra^2 - q^2), q = ra - h (2 rb - h) / (2 r),
+// is 2 sqrt(w (2 ra - w)), w = h (2 rb - h) / (2 r) (no cancellation for small h); the elastic term is
+// h^2 ra rb / (0.75 c2 sqrt(h (ra + rb) ra rb)). Three reciprocal square roots per pair in all.
+__device__ inline void contact(const CyConst &C, double r, double y, double sa, double sb, double inv_hz, double *f0,
+                               double *pr) {
+  const double cut = (sa + sb) / 2;
+  const double h = fmax(cut - r, 0.0);
+  const double ab = 0.25 * (sa * sb);
+  const double g = h * cut * ab;
+  const double fel = mid_range(g) ? h * h * ab * rsqrt_pos(g) * inv_hz
+                                  : h * sqrt(h / (1.0 / (sa / 2) + 1.0 / (sb / 2))) * inv_hz;
+  if (C.D == 3) {
+    const double A = contact_area(r, sa, sb);
+    const double vol = (A == 0 ? 0 : (4 * kPi * ((sa / 2) * (sa / 2)) / 3));
+    *f0 = -fel + C.adhesion * A;
+    *pr = vol != 0.0 ? *f0 / vol : 0.0;
     return;
   }
-  // ---- position update with the pressure-dependent friction (CIL.cu:902-939)
-  const double pnd = pres / C.p0;
-  // pow(x, 0) is 1 for every x
-  const double pw = C.zeta_p_beta == 0.0 ? 1.0 : pow(pnd, C.zeta_p_beta);
-  const double temp = C.dt * 1 / ((C.zeta + C.zeta_p * pw) * area_of(si));
-  CY_AXES(d, D) {
-    const double t = xi[d] + temp * F[d];
-    x_out[d * cap + i] = C.periodic[d] ? wrap(t, C.box[d]) : t;
-    S.v[d * cap + i] = F[d] * (temp / C.dt);
-    if (frc) frc[d * cap + i] = F[d];
+  const double w = h * (sb - h) * (0.5 * y);
+  const double t2 = w * (sa - w);
+  if (mid_range(t2)) {  // A is also the contact's volume in 2D
+    const double z = rsqrt_pos(t2);
+    *f0 = -fel + C.adhesion * (2 * sqrt_from(t2, z));
+    *pr = *f0 * (0.5 * z);
+  } else {
+    const double t = 2 * sqrt(t2);
+    const double A = isnan(t) ? (sa <= sb ? sa : sb) : t;
+    *f0 = -fel + C.adhesion * A;
+    *pr = A != 0.0 ? *f0 / A : 0.0;
   }
+}
+
+// MIXED: the contact arithmetic in FP32 on the FP64 displacement; the forces and the pressure are
+// summed in FP32 over the contacts and added to the FP64 motility and noise; the position update and
+// the cell state stay FP64.
+// mode 0 (Euler): the position update with the pressure-dependent friction follows (in place: the
+// other cells read the bin-ordered copies), then the cell cycle; mode 1: the forces go to frc and
+// nothing moves. Draws are keyed by the device step counter + key_off.
+template <int D, bool MIXED>
+__global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, double *frc, CyCounters *cnt,
+                                                         const int *start, const int *ts_dev, int mode, int key_off,
+                                                         CyOrdered O, int lane_bits, int *dblk) {
+  using R = typename std::conditional<MIXED, float, double>::type;
+  __shared__ PairWarp<D, D + 1, R> s_warp[kPairBlock / 32];
+  PairWarp<D, D + 1, R> &W = s_warp[threadIdx.x >> 5];
+  const int t = blockIdx.x * kPairBlock + threadIdx.x;
+  const int n = cnt->n;
+  const int L = 1 << lane_bits;
+  const int q = t >> lane_bits, lane = threadIdx.x & 31, sub = lane & (L - 1), el = lane >> lane_bits;
+  if ((t & ~31) >> lane_bits >= n) return;  // uniform per warp
+  const bool live = q < n;
+  const size_t cap = C.capacity;
+  const int i = live ? O.idx[q] : 0;
+  double xi[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) xi[d] = live ? O.x[d * cap + q] : 0.0;
+  const double si = live ? O.sig[q] : 1.0;
+  if (sub == 0) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) W.x[el * D + d] = xi[d];
+    W.sig[el] = si;
+    W.idx[el] = i;
+  }
+  __syncwarp();
+  const double c2 = C.hz_c + C.hz_c;
+  const double inv_hz = 1.0 / (0.75 * c2);
+  const float c2f = static_cast<float>(c2), adhf = static_cast<float>(C.adhesion);
+  R acc[D + 1];
+#pragma unroll
+  for (int k = 0; k <= D; ++k) acc[k] = R(0);
+  walk_pairs<D, D + 1, R>(
+      C, W, O, start, live, q, lane_bits, __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)),
+      [](const float4 &a, const float4 &b) {
+        const float cut = 0.5f * (a.w + b.w);
+        return cut * cut;
+      },
+      [&](int o, int tt, R *out) {
+        double rij[D], r2 = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+          if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
+          rij[d] = v;
+          if (!MIXED) r2 = __fma_rn(v, v, r2);
+        }
+        const double so = W.sig[o], sj = __ldg(O.sig + tt);
+        // the pair's first cell is the one of lower index (the contact length is not symmetric in
+        // the two diameters)
+        const bool first = W.idx[o] < __ldg(O.idx + tt);
+#pragma unroll
+        for (int k = 0; k <= D; ++k) out[k] = R(0);
+        if (MIXED) {
+          float df[D], r2f = 0.0f;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            df[d] = static_cast<float>(rij[d]);
+            r2f += df[d] * df[d];
+          }
+          const float sif = static_cast<float>(so), sjf = static_cast<float>(sj);
+          const float cut = 0.5f * (sif + sjf);
+          if (!(r2f <= cut * cut) || r2f == 0.0f) return;
+          const float r = sqrtf(r2f);
+          const float sa = first ? sif : sjf, sb = first ? sjf : sif;
+          const float h = fmaxf(cut - r, 0.0f);
+          const float fel = (h * sqrtf(h)) / (0.75f * c2f * sqrtf(2.0f / sif + 2.0f / sjf));
+          const float ra = 0.5f * sa, rb = 0.5f * sb;
+          float A, vol;
+          if (D == 3) {
+            const float u = r2f - rb * rb + ra * ra;
+            const float t = sqrtf(4.0f * r2f * (ra * ra) - u * u) / (2.0f * r);
+            A = t > 0.0f ? static_cast<float>(kPi) * (t * t) : 0.0f;
+            vol = A == 0.0f ? 0.0f : (4.0f * static_cast<float>(kPi) * (ra * ra) / 3.0f);
+          } else {
+            const float w = h * (sb - h) / (2.0f * r);
+            const float t = 2.0f * sqrtf(w * (sa - w));
+            A = isnan(t) ? fminf(sa, sb) : t;
+            vol = A;
+          }
+          const float f0 = -fel + adhf * A;
+#pragma unroll
+          for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * df[d]);
+          out[D] = static_cast<R>(vol != 0.0f ? -(f0 / vol) : 0.0f);
+        } else {
+          double y, r;
+          if (mid_range(r2)) {
+            y = rsqrt_pos(r2);
+            r = sqrt_from(r2, y);
+          } else {
+            r = sqrt(r2);
+            y = 1.0 / r;
+          }
+          if (!(r <= (so + sj) / 2) || r == 0.0) return;
+          double f0, pr;
+          contact(C, r, y, first ? so : sj, first ? sj : so, inv_hz, &f0, &pr);
+#pragma unroll
+          for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * rij[d]);
+          out[D] = static_cast<R>(-pr);
+        }
+      },
+      acc);
+  unsigned long long sbits = 0ull;
+  if (live && sub == 0) {
+    const int ts = *ts_dev + key_off;
+    double F[D];
+    // ---- motility along the velocity (singleCellForce, MD.cu:600-646)
+    {
+      double vi[D], v2 = 0.0;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        vi[d] = S.v[d * cap + i];
+        v2 += vi[d] * vi[d];
+      }
+      if (mid_range(v2)) {
+        const double m = C.motility * rsqrt_pos(v2);
+#pragma unroll
+        for (int d = 0; d < D; ++d) F[d] = m * vi[d];
+      } else {
+        double vl = sqrt(v2);
+        if (vl == 0.0) {  // a direction at random, length 1e-11 (BIG_TOL_MP)
+          const u32x4 r = draw(C, i, ts, kCyDir, 0);
+          if (D == 2) {
+            const double ang = 6.283185307179586 * u53(r.v[0], r.v[1]);
+            vi[0] = 1e-11 * cos(ang);
+            vi[1] = 1e-11 * sin(ang);
+          } else {
+            const double z = 2.0 * u53(r.v[0], r.v[1]) - 1.0;
+            const double ang = 6.283185307179586 * u53(r.v[2], r.v[3]);
+            const double s = sqrt(1.0 - z * z);
+            vi[0] = 1e-11 * (s * cos(ang));
+            vi[1] = 1e-11 * (s * sin(ang));
+            vi[D - 1] = 1e-11 * z;
+          }
+          v2 = 0.0;
+#pragma unroll
+          for (int d = 0; d < D; ++d) v2 += vi[d] * vi[d];
+          vl = sqrt(v2);
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d) F[d] = C.motility * (vi[d] / vl);
+      }
+    }
+    // ---- passive noise (CIL.cu:84-97)
+    if (C.noise_amp > 0.0) {
+      double nz[4];
+      normal2(draw(C, i, ts, kCyNoise, 0), &nz[0], &nz[1]);
+      if (D == 3) normal2(draw(C, i, ts, kCyNoise, 1), &nz[2], &nz[3]);
+#pragma unroll
+      for (int d = 0; d < D; ++d) F[d] += C.zeta * (C.noise_amp * nz[d]);
+    }
+    bool finite = true;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      F[d] += static_cast<double>(acc[d]);
+      finite = finite && finite_bits(F[d]);
+    }
+    const double pres = static_cast<double>(acc[D]);
+    S.p[i] = pres;
+    if (!finite) atomicOr(&cnt->err, kErrNonFinite);
+    if (mode == 1) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) frc[d * cap + i] = F[d];
+    } else {
+      // ---- position update with the pressure-dependent friction (CIL.cu:902-939)
+      // pow(x, 0) is 1 for every x
+      const double pw = C.zeta_p_beta == 0.0 ? 1.0 : pow(pres / C.p0, C.zeta_p_beta);
+      const double den = (C.zeta + C.zeta_p * pw) * area_of(si);
+      const double mu = mid_range(den) ? rcp_normal(den) : 1.0 / den;
+      const double temp = C.dt * mu;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const double x = xi[d] + temp * F[d];
+        S.x[d * cap + i] = C.periodic[d] ? wrap(x, C.box[d]) : x;
+        S.v[d * cap + i] = F[d] * mu;
+      }
+      if (C.divide) sbits = cycle_update(C, S, cnt, dblk, i, ts + 1, pres, si);
+    }
+  }
+  if (mode == 0 && C.divide) raise_sigma(cnt, sbits);
 }
 
 // ---------------------------------------------------------------- DPD
-__device__ inline double kick(const CyConst &C, double v, double fc, double fd, double fr) {
-  return v + (fc * C.dt + fd * C.dt + fr * C.sqrt_dt) / C.kick_div;  // updateVel (Utils.hpp:568-571)
-}
-
-// updateVelocities then updatePositions (CIL.cu:871-897, 849-866; DPD step, CIL.cu:1055-1056)
-__global__ void __launch_bounds__(kTile) k_dpd_kick_drift(CyConst C, CySet S, const CyCounters *cnt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt->n) return;
-  const size_t cap = C.capacity;
-  CY_AXES(d, C.D) {
-    const size_t k = d * cap + i;
-    const double v = kick(C, S.v[k], S.fc[k], S.fd[k], S.fr[k]);
-    S.v[k] = v;
-    const double x = S.x[k];
-    S.x[k] = C.periodic[d] ? wrap(x + C.dt * v, C.box[d]) : x + v * C.dt;  // BoundingBox::updatePos
-  }
-}
-
 // Two standard normals in FP32 (Box-Muller on 24-bit uniforms) from the four words of one
 // Philox block, the FP32 counterpart of normal2: its uniforms are normal2's rounded to 24 bits
 // (1 - u from the first word, u from the third), so the two agree to FP32 rounding.
@@ -683,234 +856,222 @@ __device__ inline void normal2f(const u32x4 &r, float *n0, float *n1) {
 
 // Pair dissipative and random forces (cellCellDisRanForce, MD.cu:861-905) over the pairs closer
 // than the lower-index cell's diameter; then, with `kick`, the second half kick into v_out.
-// MIXED: the pair terms in FP32 on the FP64 separation and velocity difference, FP32 normals,
-// summed in FP32 per cell; the kick stays FP64.
-template <bool MIXED>
-__global__ void __launch_bounds__(kTile) k_dpd_pair(CyConst C, CySet S, double *v_out, CyCounters *cnt,
-                                                    const int *start, const int *list, const int *ts_dev,
-                                                    int key_off, int kick_on, CyPacked P) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// MIXED: the pair terms in FP32 on the FP64 separation, FP32 velocities and normals, summed in FP32
+// per cell; the kick stays FP64, and the new velocities' records go to vel_out for k_dpd_dis.
+template <int D, bool MIXED>
+__global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, double *v_out, CyCounters *cnt,
+                                                         const int *start, const int *ts_dev, int key_off, int kick_on,
+                                                         CyOrdered O, float4 *vel_out, int lane_bits) {
+  using R = typename std::conditional<MIXED, float, double>::type;
+  __shared__ PairWarp<D, 2 * D, R> s_warp[kPairBlock / 32];
+  PairWarp<D, 2 * D, R> &W = s_warp[threadIdx.x >> 5];
+  const int t = blockIdx.x * kPairBlock + threadIdx.x;
   const int n = cnt->n;
-  if (i >= n) return;
+  const int L = 1 << lane_bits;
+  const int q = t >> lane_bits, lane = threadIdx.x & 31, sub = lane & (L - 1), el = lane >> lane_bits;
+  if ((t & ~31) >> lane_bits >= n) return;  // uniform per warp
+  const bool live = q < n;
   const uint32_t ts = static_cast<uint32_t>(*ts_dev + key_off);
   const size_t cap = C.capacity;
-  const int D = C.D;
-  double xi[3] = {0, 0, 0}, vi[3] = {0, 0, 0}, Fd[3] = {0, 0, 0}, Fr[3] = {0, 0, 0};
-  CY_AXES(d, D) {
-    xi[d] = S.x[d * cap + i];
-    vi[d] = S.v[d * cap + i];
+  const int i = live ? O.idx[q] : 0;
+  double vi[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) vi[d] = live ? S.v[d * cap + i] : 0.0;
+  if (sub == 0) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
+      W.v[el * D + d] = vi[d];
+    }
+    W.sig[el] = live ? O.sig[q] : 1.0;
+    W.idx[el] = i;
   }
-  const double si = S.sig[i];
+  __syncwarp();
   const float gdf = static_cast<float>(C.gamma_d), srf = static_cast<float>(C.sigma_r);
-  float Fdf[3] = {0.0f, 0.0f, 0.0f}, Frf[3] = {0.0f, 0.0f, 0.0f};
-  const int qi = MIXED ? P.qpos[i] : 0;
-  const float4 pi4 = MIXED ? P.pk[qi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const float4 vi4 = MIXED ? P.vk[qi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  // FP64: the candidates in range, in walk order, evaluated kNear at a time after the cheap
-  // distance test, so the warp runs the pair terms (draws, normals, square roots) converged
-  constexpr int kNear = 16;
-  int near[kNear];
-  int nnear = 0;
-  auto pairs = [&]() {
-    for (int k = 0; k < nnear; ++k) {
-      const int j = near[k];
-      double rij[3] = {0, 0, 0};
-      const double r = sqrt(separation(C, S, xi, j, rij));
-      const double rc = i < j ? si : S.sig[j];
-      if (!(r < rc) || r == 0.0) continue;
-      const double ir = 1.0 / r;  // one division for the weight and the unit vector
-      const double w = 1 - r / rc;
-      const uint32_t a = static_cast<uint32_t>(i < j ? i : j), z = static_cast<uint32_t>(i < j ? j : i);
-      double xi_n[4];
-      normal2(philox4x32_10(a, ts, kCyDpd0, z, C.seed_lo, C.seed_hi), &xi_n[0], &xi_n[1]);
-      if (D == 3) normal2(philox4x32_10(a, ts, kCyDpd1, z, C.seed_lo, C.seed_hi), &xi_n[2], &xi_n[3]);
-      const double sw = sqrt(w);
-      CY_AXES(d, D) {
-        const double nd = rij[d] * ir;
-        const double vj = S.v[d * cap + j];
-        Fd[d] -= C.gamma_d * w * ((vi[d] - vj) * nd) * nd;
-        Fr[d] += C.sigma_r * sw * nd * xi_n[d];
-      }
-    }
-    nnear = 0;
-  };
-  Stencil st;
-  stencil_of(C, xi, __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)), st);
-  for (int o0 = st.lo[0]; o0 <= st.hi[0]; ++o0)
-    for (int o1 = (D > 1 ? st.lo[1] : 0); o1 <= (D > 1 ? st.hi[1] : 0); ++o1)
-      for (int o2 = (D > 2 ? st.lo[2] : 0); o2 <= (D > 2 ? st.hi[2] : 0); ++o2) {
-        const int b = stencil_bin(C, st, o0, o1, o2);
-        for (int q = start[b]; q < start[b + 1]; ++q) {
-          const int j = list[q];
-          if (j == i) continue;
-          if (MIXED) {
-            const float4 pj = P.pk[q];
-            float df[3] = {0.0f, 0.0f, 0.0f};
-            const float r2 = packed_sep(C, pi4, pj, o0, o1, o2, df);
-            const float rc = i < j ? pi4.w : pj.w;
-            if (!(r2 < rc * rc) || r2 == 0.0f) continue;
-            const float4 vj4 = P.vk[q];
-            const float rinv = rsqrtf(r2);
-            const float w = 1.0f - r2 * rinv / rc;
-            const uint32_t a = static_cast<uint32_t>(i < j ? i : j), z = static_cast<uint32_t>(i < j ? j : i);
-            float xf[4];
-            normal2f(philox4x32_10(a, ts, kCyDpd0, z, C.seed_lo, C.seed_hi), &xf[0], &xf[1]);
-            if (D == 3) normal2f(philox4x32_10(a, ts, kCyDpd1, z, C.seed_lo, C.seed_hi), &xf[2], &xf[3]);
-            const float sw = sqrtf(w);
-            CY_AXES(d, D) {
-              const float nd = df[d] * rinv;
-              const float dv = f4c(vi4, d) - f4c(vj4, d);
-              Fdf[d] -= gdf * w * (dv * nd) * nd;
-              Frf[d] += srf * sw * nd * xf[d];
-            }
-            continue;
-          }
-          const float rcf = static_cast<float>(i < j ? si : S.sig[j]);
-          if (separation_f(C, S, xi, j) > 1.00001f * (rcf * rcf)) continue;  // out of range (exact test in pairs())
-          near[nnear++] = j;
-          if (nnear == kNear) pairs();
+  R acc[2 * D];
+#pragma unroll
+  for (int k = 0; k < 2 * D; ++k) acc[k] = R(0);
+  walk_pairs<D, 2 * D, R>(
+      C, W, O, start, live, q, lane_bits, __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)),
+      [](const float4 &a, const float4 &b) {
+        const float s = fmaxf(a.w, b.w);
+        return s * s;
+      },
+      [&](int o, int tt, R *out) {
+        double rij[D], r2 = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+          if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
+          rij[d] = v;
+          if (!MIXED) r2 = __fma_rn(v, v, r2);
         }
-      }
-  if (!MIXED) pairs();
-  if (MIXED)
-    CY_AXES(d, D) {
-      Fd[d] = static_cast<double>(Fdf[d]);
-      Fr[d] = static_cast<double>(Frf[d]);
-    }
+        const int io = W.idx[o], j = __ldg(O.idx + tt);
+        const uint32_t a = static_cast<uint32_t>(io < j ? io : j), z = static_cast<uint32_t>(io < j ? j : io);
+#pragma unroll
+        for (int k = 0; k < 2 * D; ++k) out[k] = R(0);
+        if (MIXED) {
+          float df[D], r2f = 0.0f;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            df[d] = static_cast<float>(rij[d]);
+            r2f += df[d] * df[d];
+          }
+          const float rc = io < j ? static_cast<float>(W.sig[o]) : __ldg(O.rec + tt).w;
+          if (!(r2f < rc * rc) || r2f == 0.0f) return;
+          const float4 vj4 = __ldg(O.vel + tt);
+          const float rinv = rsqrtf(r2f);
+          const float w = 1.0f - r2f * rinv / rc;
+          float xf[4];
+          normal2f(philox4x32_10(a, ts, kCyDpd0, z, C.seed_lo, C.seed_hi), &xf[0], &xf[1]);
+          if (D == 3) normal2f(philox4x32_10(a, ts, kCyDpd1, z, C.seed_lo, C.seed_hi), &xf[2], &xf[3]);
+          const float sw = sqrtf(w);
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const float nd = df[d] * rinv;
+            const float dv = static_cast<float>(W.v[o * D + d]) - f4c(vj4, d);
+            out[d] = static_cast<R>(-(gdf * w * (dv * nd) * nd));
+            out[D + d] = static_cast<R>(srf * sw * nd * xf[d]);
+          }
+        } else {
+          const double rc = io < j ? W.sig[o] : __ldg(O.sig + tt);
+          double ir, r;
+          if (mid_range(r2)) {
+            ir = rsqrt_pos(r2);
+            r = sqrt_from(r2, ir);
+          } else {
+            r = sqrt(r2);
+            ir = 1.0 / r;
+          }
+          if (!(r < rc) || r == 0.0) return;
+          const double w = 1 - r / rc;
+          double xn[4];
+          normal2(philox4x32_10(a, ts, kCyDpd0, z, C.seed_lo, C.seed_hi), &xn[0], &xn[1]);
+          if (D == 3) normal2(philox4x32_10(a, ts, kCyDpd1, z, C.seed_lo, C.seed_hi), &xn[2], &xn[3]);
+          const double gw = C.gamma_d * w, sw = C.sigma_r * sqrt(w);
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const double nd = rij[d] * ir;
+            const double vj = __ldg(S.v + d * cap + j);
+            out[d] = static_cast<R>(-(gw * ((W.v[o * D + d] - vj) * nd) * nd));
+            out[D + d] = static_cast<R>(sw * nd * xn[d]);
+          }
+        }
+      },
+      acc);
+  if (!live || sub != 0) return;
   bool finite = true;
-  CY_AXES(d, D) {
+  float vf[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
     const size_t k = d * cap + i;
-    S.fd[k] = Fd[d];
-    S.fr[k] = Fr[d];
+    const double fd = static_cast<double>(acc[d]), fr = static_cast<double>(acc[D + d]);
+    S.fd[k] = fd;
+    S.fr[k] = fr;
     if (kick_on) {
-      const double v = kick(C, vi[d], S.fc[k], Fd[d], Fr[d]);
+      const double v = kick(C, vi[d], S.fc[k], fd, fr);
       v_out[k] = v;
-      finite = finite && isfinite(v);
+      vf[d] = static_cast<float>(v);
+      finite = finite && finite_bits(v);
     }
   }
+  if (MIXED && kick_on) vel_out[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
   if (!finite) atomicOr(&cnt->err, kErrNonFinite);
 }
 
 // Background and pair dissipation at the new velocities (calculDisForces, CIL.cu:294-364:
 // sameCellDisForce zeroes a single-element cell's Fd, cellBackDisForce subtracts gamma_bg v,
-// cellCellDisForce, MD.cu:951-985, with w = 1 - r^2 / sigma_core for r < sigma_core)
-template <bool MIXED>
-__global__ void __launch_bounds__(kTile) k_dpd_dis(CyConst C, CySet S, const CyCounters *cnt, const int *start,
-                                                   const int *list, CyPacked P) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// cellCellDisForce, MD.cu:951-985, with w = 1 - r^2 / sigma_core for r < sigma_core), then the cell
+// cycle.
+template <int D, bool MIXED>
+__global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCounters *cnt, const int *start,
+                                                        const int *ts_dev, CyOrdered O, const float4 *vel,
+                                                        int lane_bits, int *dblk) {
+  using R = typename std::conditional<MIXED, float, double>::type;
+  __shared__ PairWarp<D, D, R> s_warp[kPairBlock / 32];
+  PairWarp<D, D, R> &W = s_warp[threadIdx.x >> 5];
+  const int t = blockIdx.x * kPairBlock + threadIdx.x;
   const int n = cnt->n;
-  if (i >= n) return;
+  const int L = 1 << lane_bits;
+  const int q = t >> lane_bits, lane = threadIdx.x & 31, sub = lane & (L - 1), el = lane >> lane_bits;
+  if ((t & ~31) >> lane_bits >= n) return;  // uniform per warp
+  const bool live = q < n;
   const size_t cap = C.capacity;
-  const int D = C.D;
-  double xi[3] = {0, 0, 0}, vi[3] = {0, 0, 0}, Fd[3] = {0, 0, 0};
-  CY_AXES(d, D) {
-    xi[d] = S.x[d * cap + i];
-    vi[d] = S.v[d * cap + i];
-    Fd[d] = 0;
-    Fd[d] -= C.gamma_b * vi[d];
+  const int i = live ? O.idx[q] : 0;
+  double vi[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) vi[d] = live ? S.v[d * cap + i] : 0.0;
+  if (sub == 0) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
+      W.v[el * D + d] = vi[d];
+    }
   }
+  __syncwarp();
   const double rc = C.sigma_core;
   const float rcf = static_cast<float>(rc), gdf = static_cast<float>(C.gamma_d);
-  float Fdf[3] = {0.0f, 0.0f, 0.0f};
-  const int qi = MIXED ? P.qpos[i] : 0;
-  const float4 pi4 = MIXED ? P.pk[qi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const float4 vi4 = MIXED ? P.vk[qi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const double smax = __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits));
-  // FP64: the candidates in range, in walk order, evaluated kNear at a time after the walk with
-  // the warp's lanes converged (same terms in the same order)
-  constexpr int kNear = 16;
-  int near[kNear];
-  int nnear = 0;
-  auto pairs = [&]() {
-    for (int k = 0; k < nnear; ++k) {
-      const int j = near[k];
-      double rij[3] = {0, 0, 0};
-      const double r = sqrt(separation(C, S, xi, j, rij));
-      if (!(r < rc) || r == 0.0) continue;
-      const double w = 1 - ((r * r) / rc);
-      CY_AXES(d, D) {
-        const double nd = -rij[d] / r;
-        Fd[d] -= C.gamma_d * w * ((vi[d] - S.v[d * cap + j]) * nd) * nd;
-      }
-    }
-    nnear = 0;
-  };
-  Stencil st;
-  stencil_of(C, xi, smax > rc ? smax : rc, st);
-  for (int o0 = st.lo[0]; o0 <= st.hi[0]; ++o0)
-    for (int o1 = (D > 1 ? st.lo[1] : 0); o1 <= (D > 1 ? st.hi[1] : 0); ++o1)
-      for (int o2 = (D > 2 ? st.lo[2] : 0); o2 <= (D > 2 ? st.hi[2] : 0); ++o2) {
-        const int b = stencil_bin(C, st, o0, o1, o2);
-        for (int q = start[b]; q < start[b + 1]; ++q) {
-          if (MIXED) {
-            if (q == qi) continue;
-            const float4 pj = P.pk[q];
-            float df[3] = {0.0f, 0.0f, 0.0f};
-            const float r2 = packed_sep(C, pi4, pj, o0, o1, o2, df);
-            if (!(r2 < rcf * rcf) || r2 == 0.0f) continue;
-            const float4 vj4 = P.vk[q];
-            const float rinv = rsqrtf(r2);
-            const float w = 1.0f - r2 / rcf;
-            CY_AXES(d, D) {
-              const float nd = -df[d] * rinv;
-              const float dv = f4c(vi4, d) - f4c(vj4, d);
-              Fdf[d] -= gdf * w * (dv * nd) * nd;
-            }
-            continue;
-          }
-          const int j = list[q];
-          if (j == i) continue;
-          if (separation_f(C, S, xi, j) > 1.00001f * (rcf * rcf)) continue;  // out of range (exact test in pairs())
-          near[nnear++] = j;
-          if (nnear == kNear) pairs();
+  R acc[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) acc[d] = R(0);
+  walk_pairs<D, D, R>(
+      C, W, O, start, live, q, lane_bits, smax > rc ? smax : rc,
+      [&](const float4 &, const float4 &) { return rcf * rcf; },
+      [&](int o, int tt, R *out) {
+        double rij[D], r2 = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+          if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
+          rij[d] = v;
+          if (!MIXED) r2 = __fma_rn(v, v, r2);
+          out[d] = R(0);
         }
-      }
-  if (!MIXED) pairs();
-  CY_AXES(d, D) S.fd[d * cap + i] = MIXED ? Fd[d] + static_cast<double>(Fdf[d]) : Fd[d];
-}
-
-// ---------------------------------------------------------------- cell cycle and divisions
-__global__ void __launch_bounds__(kTile) k_cy_cycle(CyConst C, CySet S, CyCounters *cnt, const int *ts_dev,
-                                                    int *flag, int *block_count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = cnt->n;
-  const int ts = *ts_dev;
-  int div = 0;
-  if (i < n) {
-    // cellTPressure (CIL.cu:493-494): every cell is in the dividing state when the species divides
-    if (!C.divide || S.p[i] < C.apop_pressure)
-      S.tp[i] = 0;
-    else
-      S.tp[i] += 1;
-    if (C.divide) {
-      const double shift = C.p_shift != 0.0 ? C.p_shift * exp(-ts * C.p_shift_tau_inv) : 0.0;
-      const double pnd = fmax(0., S.p[i] + shift) / C.p0;
-      const double om = S.om[i];
-      double rho = S.rho[i];
-      S.theta[i] += om * fmin(C.r_maxed_inv * rho, 1.0);
-      const bool d3 = C.D == 3;
-      double vt = d3 ? volume_of(S.sigt[i]) : area_of(S.sigt[i]);
-      double v = d3 ? volume_of(S.sig[i]) : area_of(S.sig[i]);
-      const double c0 = om * kLn2 + (C.v1 - 1) / C.tau_v;
-      const double vt_prime = c0 * rho - (((vt - C.v_s) / C.v_s) / C.tau_v);
-      vt += vt_prime * vt;
-      const double v_prime = -(v - (vt / (1 + C.beta_vs * (C.osm + pnd)))) / C.tau_p;
-      v += v_prime;
-      v = C.tau_p == 0 ? vt : v;
-      S.sigt[i] = d3 ? sigma_of_volume(vt) : sigma_of_area(vt);
-      S.sig[i] = d3 ? sigma_of_volume(v) : sigma_of_area(v);
-      const double r_np = (1 - rho - pnd);
-      const double tau_r_pre = r_np > 0 ? 1 : C.rho_ratio;
-      const double r_prime = r_np / (C.tau_r * tau_r_pre);
-      rho += r_prime * rho;
-      S.rho[i] = rho;
-      div = S.theta[i] >= 1 ? 1 : 0;
-    }
-    flag[i] = div;
+        if (MIXED) {
+          float df[D], r2f = 0.0f;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            df[d] = static_cast<float>(rij[d]);
+            r2f += df[d] * df[d];
+          }
+          if (!(r2f < rcf * rcf) || r2f == 0.0f) return;
+          const float4 vj4 = __ldg(vel + tt);
+          const float rinv = rsqrtf(r2f);
+          const float w = 1.0f - r2f / rcf;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const float nd = -df[d] * rinv;
+            const float dv = static_cast<float>(W.v[o * D + d]) - f4c(vj4, d);
+            out[d] = static_cast<R>(-(gdf * w * (dv * nd) * nd));
+          }
+        } else {
+          const int j = __ldg(O.idx + tt);
+          double ir, r;
+          if (mid_range(r2)) {
+            ir = rsqrt_pos(r2);
+            r = sqrt_from(r2, ir);
+          } else {
+            r = sqrt(r2);
+            ir = 1.0 / r;
+          }
+          if (!(r < rc) || r == 0.0) return;
+          const double gw = C.gamma_d * (1 - r2 / rc);
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const double nd = rij[d] * ir;
+            out[d] = static_cast<R>(-(gw * ((W.v[o * D + d] - __ldg(S.v + d * cap + j)) * nd) * nd));
+          }
+        }
+      },
+      acc);
+  unsigned long long sbits = 0ull;
+  if (live && sub == 0) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) S.fd[d * cap + i] = static_cast<double>(acc[d]) - C.gamma_b * vi[d];
+    if (C.divide) sbits = cycle_update(C, S, cnt, dblk, i, *ts_dev + 1, S.p[i], O.sig[q]);
   }
-  int tot;
-  block_excl_scan(div, &tot);
-  if (threadIdx.x == 0) block_count[blockIdx.x] = tot;
+  if (C.divide) raise_sigma(cnt, sbits);
 }
 
 __device__ inline void put_sigma_max(CyCounters *cnt, double s) {
@@ -918,24 +1079,19 @@ __device__ inline void put_sigma_max(CyCounters *cnt, double s) {
 }
 
 // Divisions in mother order: daughter of the k-th dividing cell at n + k (calculDivisionsSingle,
-// CIL.cu:527-600; singleCellDivision, MD.cu:664-718).
-__global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCounters *cnt, const int *ts_dev,
-                                                     const int *flag, const int *block_start, int n_blocks) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = cnt->n;
-  const int ts = *ts_dev;
-  const int f = (i < n) ? flag[i] : 0;
-  int tot;
-  const int rank = block_start[blockIdx.x] + block_excl_scan(f, &tot);
+// CIL.cu:527-600; singleCellDivision, MD.cu:664-718). The blocks take the blocks of kTile cells in
+// turn and pass over those without a dividing cell (dblk). The block that finishes last commits the
+// step: the cell count, the largest diameter and the step counter (every block has read them by then).
+__device__ void divide_block(const CyConst &C, const CySet &S, CyCounters *cnt, int n, int ts, int cb,
+                             const int *dblk) {
+  int before = 0, tot;
+  for (int u = threadIdx.x; u < cb; u += kTile) before += dblk[u];
+  int off;
+  block_excl_scan(before, &off);
+  const int i = cb * kTile + threadIdx.x;
+  const int f = (i < n && S.theta[i] >= 1) ? 1 : 0;
+  const int rank = off + block_excl_scan(f, &tot);
   const size_t cap = C.capacity;
-  {  // the block's largest diameter, one atomic per block
-    __shared__ unsigned long long smax;
-    if (threadIdx.x == 0) smax = 0ull;
-    __syncthreads();
-    if (i < n) atomicMax(&smax, static_cast<unsigned long long>(__double_as_longlong(S.sig[i])));
-    __syncthreads();
-    if (threadIdx.x == 0 && smax) atomicMax(&cnt->sigma_max_bits, smax);
-  }
   if (f) {
     const int inew = n + rank;
     if (inew >= C.capacity) {
@@ -1008,16 +1164,31 @@ __global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCount
   }
 }
 
-__global__ void k_cy_commit_divisions(CyCounters *cnt, const int *block_start, int n_blocks, int capacity) {
-  const int nd = block_start[n_blocks];
-  const int room = capacity - cnt->n;
-  const int add = nd < room ? nd : (room > 0 ? room : 0);
-  cnt->n += add;
-  cnt->ndiv_total += add;
-  cnt->ndiv_step = add;
+__global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCounters *cnt, int *ts_dev,
+                                                     const int *dblk) {
+  const int n = cnt->n, ts = *ts_dev + 1;
+  const int nb = (n + kTile - 1) / kTile;
+  if (cnt->ndue > 0) {
+    for (int cb = blockIdx.x; cb < nb; cb += gridDim.x)
+      if (dblk[cb] > 0) divide_block(C, S, cnt, n, ts, cb, dblk);  // uniform
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&cnt->ndone, 1) == static_cast<int>(gridDim.x) - 1) {
+      const int nd = cnt->ndue, room = C.capacity - n;
+      const int add = nd < room ? nd : (room > 0 ? room : 0);
+      cnt->n = n + add;
+      cnt->ndiv_total += add;
+      cnt->ndiv_step = add;
+      cnt->sigma_max_bits = cnt->sigma_next_bits;
+      cnt->sigma_next_bits = 0ull;
+      cnt->ndue = 0;
+      cnt->ndone = 0;
+      *ts_dev = ts;
+    }
+  }
 }
-
-__global__ void k_cy_reset_smax(CyCounters *cnt) { cnt->sigma_max_bits = 0ull; }
 
 __global__ void k_cy_advance(int *ts) { *ts += 1; }
 
@@ -1158,16 +1329,15 @@ struct cil_cycle {
   cudaStream_t stream = nullptr;
   CySet set[2] = {};
   int cur = 0;
-  double *xs = nullptr;   // position output buffer of the force pass
   double *vs = nullptr;   // velocity output buffer of the DPD pair pass
-  CyPacked P{};           // FP32 records of the bin order (precision 1)
-  double *frc = nullptr;  // last forces (output only)
-  double *inv_r = nullptr;  // 1 / (sigma / 2) per cell, written with the bin keys
+  CyOrdered O{};          // the cells in bin order
+  float4 *vel_next = nullptr;  // the new velocities' records (DPD, precision 1)
+  double *frc = nullptr;  // forces of the last download (output only)
   // captured steps: keyed by the buffer configuration before the step and the bin grid, each
-  // records the configuration after it (a step rotates x / xs, v / vs and the state sets)
+  // records the configuration after it (a step rotates v / vs and the state sets)
   struct Buffers {
     CySet set[2];
-    double *xs, *vs;
+    double *vs;
     int cur;
   };
   struct StepGraph {
@@ -1178,13 +1348,13 @@ struct cil_cycle {
   };
   std::vector<StepGraph> graphs;
   uint64_t grid_gen = 0;
-  int pair_bs = kTile;  // threads per block of the per-cell pair kernels (set per call)
-  int lane_bits = 0;    // log2 of the threads per cell of the contact pass (set per call)
+  int pair_bs = kTile;  // threads per block of the removal kernels (set per call)
+  int lane_bits = 0;    // log2 of the lanes per cell of the pair kernels (set per call)
   CyCounters *cnt = nullptr;
   CyCounters *h_cnt = nullptr;  // pinned
   int *ts_dev = nullptr;
-  int *key = nullptr, *bcount = nullptr, *bstart = nullptr, *cursor = nullptr, *list = nullptr, *part = nullptr;
-  int *flag = nullptr, *blk = nullptr;
+  int *key = nullptr, *arrival = nullptr, *bcount = nullptr, *bstart = nullptr, *tmp = nullptr, *part = nullptr;
+  int *flag = nullptr, *blk = nullptr, *dblk = nullptr;
   int nbins = 0, nparts = 0, nblocks = 0;
   long long nbins_cap = 0;  // bins the arrays hold
   int64_t ts = 0;
@@ -1249,10 +1419,10 @@ int blocks_for(int n) { return n > 0 ? (n + kTile - 1) / kTile : 1; }
 
 constexpr int kNumSMs = 152;  // GB300
 
-// grid of a per-cell pair kernel at h->pair_bs threads per block
+// grid of a removal kernel at h->pair_bs threads per block
 int pair_grid(const cil_cycle *h) { return (h->cap + h->pair_bs - 1) / h->pair_bs; }
 
-// Threads per cell of the contact pass: up to 8, while the colony gives fewer than two warps
+// Lanes per cell of the pair kernels: up to 8, while the colony gives fewer than two warps
 // per scheduler of every SM (152 SMs x 4 x 2 x 32 threads), and while the grid over the
 // capacity stays within 2^24 threads. The restatement uses the same rule.
 int contact_lane_bits(long long ncells, long long capacity) {
@@ -1275,7 +1445,7 @@ void set_bins(cil_cycle *h, double smax, int ncells) {
   CyConst &C = h->C;
   const double w = (smax > h->p.sigma_core ? smax : h->p.sigma_core) * 1.05;
   const int before[3] = {C.ns[0], C.ns[1], C.ns[2]};
-  // blocks of the per-cell pair kernels (FP64-heavy, no block cooperation): small enough that
+  // blocks of the removal kernels (FP64-heavy, no block cooperation): small enough that
   // a small colony still spreads over every SM (two blocks per SM), 32 to kTile threads
   const int bs_before = h->pair_bs, lb_before = h->lane_bits;
   h->lane_bits = contact_lane_bits(ncells, h->cap);
@@ -1310,29 +1480,28 @@ double host_sigma_max(const cil_cycle *h) {
   return s;
 }
 
-// scan of count[0..m) into start[0..m] (start[m] = total)
-void scan_into(cil_cycle *h, const int *count, int m, int *start) {
+// scan of count[0..m) into start[0..m] (start[m] = total), count left at zero. Up to 2048 chunks (2M
+// bins) each block adds the chunk sums before its own; the quadratic cost of that passes a launch's
+// near there.
+void scan_into(cil_cycle *h, int *count, int m, int *start) {
   const int nchunks = m / kScanTile + 1;  // covers index m
+  const int scanned = nchunks > 2048 ? 1 : 0;
   k_cy_chunk_sums<<<nchunks, kTile, 0, h->stream>>>(count, m, h->part);
-  k_cy_scan_small<<<1, kTile, 0, h->stream>>>(h->part, nchunks);
-  k_cy_chunk_apply<<<nchunks, kTile, 0, h->stream>>>(count, m, h->part, start);
-  h->launches += 3;
+  if (scanned) k_cy_scan_small<<<1, kTile, 0, h->stream>>>(h->part, nchunks);
+  k_cy_chunk_apply<<<nchunks, kTile, 0, h->stream>>>(count, m, h->part, start, scanned);
+  h->launches += 2 + scanned;
 }
 
-cil_status bin_cells(cil_cycle *h) {
+// drift: with DPD's first half kick and drift
+cil_status bin_cells(cil_cycle *h, int drift) {
   const CySet &S = h->set[h->cur];
   const int g = blocks_for(h->cap);
-  k_cy_clear<<<256, kTile, 0, h->stream>>>(h->bcount, h->nbins);
-  k_cy_keys<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->key, h->bcount, h->inv_r);
+  k_cy_keys<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->key, h->arrival, h->bcount, h->dblk, drift);
   scan_into(h, h->bcount, h->nbins, h->bstart);
-  k_cy_clear<<<256, kTile, 0, h->stream>>>(h->cursor, h->nbins);
-  k_cy_scatter<<<g, kTile, 0, h->stream>>>(h->cnt, h->key, h->bstart, h->cursor, h->list);
-  k_cy_sort<<<blocks_for(h->nbins), kTile, 0, h->stream>>>(h->bstart, h->nbins, h->list, h->cnt);
-  h->launches += 5;
-  if (h->p.precision == 1) {
-    k_cy_pack<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->list, h->P, h->C.dpd);
-    h->launches += 1;
-  }
+  k_cy_scatter<<<g, kTile, 0, h->stream>>>(h->cnt, h->key, h->arrival, h->bstart, h->tmp);
+  k_cy_place<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->key, h->arrival, h->bstart, h->tmp, h->O,
+                                         h->C.dpd && h->p.precision == 1 ? 1 : 0);
+  h->launches += 3;
   return CIL_OK;
 }
 
@@ -1349,73 +1518,96 @@ cil_status removals(cil_cycle *h, int mode) {
   return CIL_OK;
 }
 
-void launch_force(cil_cycle *h, CySet &S, double *x_out, double *frc, int mode, int key_off) {
-  const int bs = h->pair_bs;
+// blocks of a pair kernel: 2^lane_bits lanes for every cell of the capacity
+int pair_blocks(const cil_cycle *h) {
   const long long threads = static_cast<long long>(h->cap) << h->lane_bits;
-  const int g = static_cast<int>((threads + bs - 1) / bs);
+  return static_cast<int>((threads + kPairBlock - 1) / kPairBlock);
+}
+
+template <int D>
+void launch_force_d(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
+  const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    k_cy_force<true><<<g, bs, 0, h->stream>>>(h->C, S, x_out, frc, h->cnt, h->bstart, h->list, h->ts_dev, mode,
-                                                 key_off, h->P, h->lane_bits, h->inv_r);
+    k_cy_force<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
+                                                         h->O, h->lane_bits, h->dblk);
   else
-    k_cy_force<false><<<g, bs, 0, h->stream>>>(h->C, S, x_out, frc, h->cnt, h->bstart, h->list, h->ts_dev, mode,
-                                                  key_off, h->P, h->lane_bits, h->inv_r);
+    k_cy_force<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
+                                                          h->O, h->lane_bits, h->dblk);
+}
+
+void launch_force(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
+  if (h->C.D == 2)
+    launch_force_d<2>(h, S, frc, mode, key_off);
+  else
+    launch_force_d<3>(h, S, frc, mode, key_off);
   h->launches += 1;
 }
 
-void launch_dpd_pair(cil_cycle *h, CySet &S, int key_off, int kick_on) {
-  const int g = pair_grid(h), bs = h->pair_bs;
+template <int D>
+void launch_dpd_pair_d(cil_cycle *h, CySet &S, int key_off, int kick_on) {
+  const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    k_dpd_pair<true><<<g, bs, 0, h->stream>>>(h->C, S, h->vs, h->cnt, h->bstart, h->list, h->ts_dev, key_off,
-                                                 kick_on, h->P);
+    k_dpd_pair<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off, kick_on,
+                                                         h->O, h->vel_next, h->lane_bits);
   else
-    k_dpd_pair<false><<<g, bs, 0, h->stream>>>(h->C, S, h->vs, h->cnt, h->bstart, h->list, h->ts_dev, key_off,
-                                                  kick_on, h->P);
+    k_dpd_pair<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off,
+                                                          kick_on, h->O, h->vel_next, h->lane_bits);
+}
+
+void launch_dpd_pair(cil_cycle *h, CySet &S, int key_off, int kick_on) {
+  if (h->C.D == 2)
+    launch_dpd_pair_d<2>(h, S, key_off, kick_on);
+  else
+    launch_dpd_pair_d<3>(h, S, key_off, kick_on);
+  h->launches += 1;
+}
+
+template <int D>
+void launch_dpd_dis_d(cil_cycle *h, CySet &S) {
+  const int g = pair_blocks(h);
+  if (h->p.precision == 1)
+    k_dpd_dis<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
+                                                        h->lane_bits, h->dblk);
+  else
+    k_dpd_dis<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
+                                                         h->lane_bits, h->dblk);
+}
+
+void launch_dpd_dis(cil_cycle *h, CySet &S) {
+  if (h->C.D == 2)
+    launch_dpd_dis_d<2>(h, S);
+  else
+    launch_dpd_dis_d<3>(h, S);
+  h->launches += 1;
 }
 
 // Fc, pressure, Fd and Fr at the current positions and velocities (the forces the reference
 // evaluates before its first step, CIL.cu:1096), draws keyed by the current step counter
 void dpd_initial_forces(cil_cycle *h) {
   CySet &S = h->set[h->cur];
-  bin_cells(h);
-  launch_force(h, S, nullptr, S.fc, 1, 0);
+  bin_cells(h, 0);
+  launch_force(h, S, S.fc, 1, 0);
   launch_dpd_pair(h, S, 0, 0);
-  h->launches += 1;
 }
 
 cil_status enqueue_step(cil_cycle *h) {
-  const int g = blocks_for(h->cap);
   CySet &S = h->set[h->cur];
+  bin_cells(h, h->C.dpd);
   if (h->C.dpd) {  // DPD (CIL.cu:1054-1066); this step's draws are keyed by ts + 1
-    k_dpd_kick_drift<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt);
-    bin_cells(h);
-    launch_force(h, S, nullptr, S.fc, 1, 1);
+    launch_force(h, S, S.fc, 1, 1);
     launch_dpd_pair(h, S, 1, 1);
     std::swap(S.v, h->vs);
-    if (h->p.precision == 1) {  // the records take the new velocities
-      k_cy_pack_vel<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->list, h->P);
-      k_dpd_dis<true><<<pair_grid(h), h->pair_bs, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->list, h->P);
-      h->launches += 1;
-    } else {
-      k_dpd_dis<false><<<pair_grid(h), h->pair_bs, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->list, h->P);
-    }
-    h->launches += 3;
+    launch_dpd_dis(h, S);
   } else {
-    bin_cells(h);
-    launch_force(h, S, h->xs, h->frc, 0, 0);
-    std::swap(S.x, h->xs);
+    launch_force(h, S, nullptr, 0, 0);
   }
-  k_cy_advance<<<1, 1, 0, h->stream>>>(h->ts_dev);
   h->ts += 1;
-  h->launches += 1;
-  if (h->C.divide) {
-    const int ge = pair_grid(h), bs = h->pair_bs;  // per-cell event kernels: the pair kernels' blocks
-    k_cy_cycle<<<ge, bs, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev, h->flag, h->blk);
-    k_cy_scan_small<<<1, kTile, 0, h->stream>>>(h->blk, ge);
-    k_cy_reset_smax<<<1, 1, 0, h->stream>>>(h->cnt);
-    k_cy_divide<<<ge, bs, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev, h->flag, h->blk, ge);
-    k_cy_commit_divisions<<<1, 1, 0, h->stream>>>(h->cnt, h->blk, ge, h->cap);
-    h->launches += 5;
+  if (h->C.divide) {  // also moves the step counter
+    k_cy_divide<<<std::min(blocks_for(h->cap), 2 * kNumSMs), kTile, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev, h->dblk);
+  } else {
+    k_cy_advance<<<1, 1, 0, h->stream>>>(h->ts_dev);
   }
+  h->launches += 1;
   if (h->C.apoptosis != CIL_APOP_NONE) removals(h, 1);
   CY_TRY(h, cudaGetLastError());
   return CIL_OK;
@@ -1427,7 +1619,6 @@ cil_cycle::Buffers buffers_of(const cil_cycle *h) {
   cil_cycle::Buffers b{};
   b.set[0] = h->set[0];
   b.set[1] = h->set[1];
-  b.xs = h->xs;
   b.vs = h->vs;
   b.cur = h->cur;
   return b;
@@ -1435,7 +1626,7 @@ cil_cycle::Buffers buffers_of(const cil_cycle *h) {
 
 bool same_buffers(const cil_cycle::Buffers &a, const cil_cycle::Buffers &b) {
   return std::memcmp(&a.set[0], &b.set[0], sizeof(CySet)) == 0 &&
-         std::memcmp(&a.set[1], &b.set[1], sizeof(CySet)) == 0 && a.xs == b.xs && a.vs == b.vs && a.cur == b.cur;
+         std::memcmp(&a.set[1], &b.set[1], sizeof(CySet)) == 0 && a.vs == b.vs && a.cur == b.cur;
 }
 
 // One step through the graph of its buffer configuration: captured from enqueue_step the first
@@ -1447,7 +1638,6 @@ cil_status graph_step(cil_cycle *h) {
       CY_TRY(h, cudaGraphLaunch(g.exec, h->stream));
       h->set[0] = g.after.set[0];
       h->set[1] = g.after.set[1];
-      h->xs = g.after.xs;
       h->vs = g.after.vs;
       h->cur = g.after.cur;
       h->ts += 1;
@@ -1472,7 +1662,6 @@ cil_status graph_step(cil_cycle *h) {
     cudaGetLastError();
     h->set[0] = b.set[0];
     h->set[1] = b.set[1];
-    h->xs = b.xs;
     h->vs = b.vs;
     h->cur = b.cur;
     h->ts = ts0;
@@ -1551,6 +1740,11 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
     C.v_s = p->dim == 3 ? 4 * kPi * (r * r * r) / 3 : kPi * (r * r);  // Sigma2Volume / Sigma2Area
   }
   C.p0 = p->cycle_p0;
+  C.inv_p0 = 1.0 / C.p0;
+  C.growth = (C.v1 - 1) / C.tau_v;
+  C.inv_vs_tau_v = 1.0 / (C.v_s * C.tau_v);
+  C.inv_tau_r = 1.0 / C.tau_r;
+  C.inv_tau_r_neg = 1.0 / (C.tau_r * p->cycle_rho_ratio);
   C.beta_vs = p->cycle_beta_vs;
   C.rho_ratio = p->cycle_rho_ratio;
   C.r_maxed_inv = p->cycle_r_maxed > 0.0 ? 1.0 / p->cycle_r_maxed : 1.0;
@@ -1564,7 +1758,7 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   C.apop_steps = p->apop_duration / p->dt;
   C.extr_rate = p->extr_rate;
   C.dpd = p->integrator == CIL_CYCLE_DPD ? 1 : 0;
-  C.kick_div = 2 * (2 * p->mass);
+  C.inv_kick_div = 1.0 / (2 * (2 * p->mass));
   C.sqrt_dt = std::sqrt(p->dt);
   C.gamma_d = p->dis_diff;
   C.gamma_b = p->dis_bg;
@@ -1600,34 +1794,39 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
     h->vs = h->alloc<double>(D * cap);
     ok = h->vs != nullptr;
   }
-  if (ok && p->precision == 1) {
-    h->P.pk = h->alloc<float4>(cap);
-    h->P.qpos = h->alloc<int>(cap);
-    h->P.vk = C.dpd ? h->alloc<float4>(cap) : nullptr;
-    ok = h->P.pk && h->P.qpos && (!C.dpd || h->P.vk);
+  if (ok && p->precision == 1 && C.dpd) {
+    h->O.vel = h->alloc<float4>(cap);
+    h->vel_next = h->alloc<float4>(cap);
+    ok = h->O.vel && h->vel_next;
   }
   h->nblocks = (capacity + 31) / 32;  // blocks of the per-cell event kernels at their smallest (32 threads)
   h->nparts = (h->nbins_cap + kScanTile - 1) / kScanTile + 1;
   if (ok) {
-    h->xs = h->alloc<double>(D * cap);
     h->frc = h->alloc<double>(D * cap);
-    h->inv_r = h->alloc<double>(cap);
+    h->O.x = h->alloc<double>(D * cap);
+    h->O.sig = h->alloc<double>(cap);
+    h->O.rec = h->alloc<float4>(cap);
+    h->O.idx = h->alloc<int>(cap);
+    h->O.bin = h->alloc<int>(cap);
     h->cnt = h->alloc<CyCounters>(1);
     h->ts_dev = h->alloc<int>(1);
     h->key = h->alloc<int>(cap);
     h->bcount = h->alloc<int>(h->nbins_cap + 1);
     h->bstart = h->alloc<int>(h->nbins_cap + 1);
-    h->cursor = h->alloc<int>(h->nbins_cap + 1);
-    h->list = h->alloc<int>(cap);
+    h->arrival = h->alloc<int>(cap);
+    h->tmp = h->alloc<int>(cap);
+    h->dblk = h->alloc<int>(blocks_for(capacity));
     h->part = h->alloc<int>(h->nparts + 1);
     h->flag = h->alloc<int>(cap);
     h->blk = h->alloc<int>(h->nblocks + 1);
-    ok = h->xs && h->frc && h->inv_r && h->cnt && h->ts_dev && h->key && h->bcount && h->bstart && h->cursor && h->list &&
+    ok = h->frc && h->O.x && h->O.sig && h->O.rec && h->O.idx && h->O.bin && h->cnt && h->ts_dev && h->key &&
+         h->bcount && h->bstart && h->arrival && h->tmp && h->dblk &&
          h->part && h->flag && h->blk &&
          cudaHostAlloc(&h->h_cnt, sizeof(CyCounters), cudaHostAllocDefault) == cudaSuccess;
   }
   if (ok) ok = cudaMemsetAsync(h->cnt, 0, sizeof(CyCounters), h->stream) == cudaSuccess &&
                cudaMemsetAsync(h->ts_dev, 0, sizeof(int), h->stream) == cudaSuccess &&
+               cudaMemsetAsync(h->bcount, 0, sizeof(int) * (h->nbins_cap + 1), h->stream) == cudaSuccess &&
                cudaStreamSynchronize(h->stream) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
@@ -1761,8 +1960,8 @@ cil_status cil_cycle_download(cil_cycle *h, cil_cycle_view *v) {
     // the forces and pressures at the current state, which the reference's Euler step
     // evaluates at its end (CIL.cu:1019) and writes out; the next step's force pass computes
     // the same values again (same positions, velocities and step key)
-    bin_cells(h);
-    launch_force(h, h->set[h->cur], nullptr, h->frc, 1, 0);
+    bin_cells(h, 0);
+    launch_force(h, h->set[h->cur], h->frc, 1, 0);
     h->launches = launches;
     CY_TRY(h, cudaGetLastError());
   }

@@ -46,15 +46,6 @@ __device__ __forceinline__ double min_image(double v, double L) {
   return v - static_cast<double>(nint(v / L)) * L;
 }
 
-// fmod(t + L, L) as wrap_like_fmod gives it, its comparisons on the bit patterns (doubles that
-// are not negative order like them), so that the FP64 pipe runs the two additions only.
-__device__ __forceinline__ double wrap_bits(double t, double L) {
-  const double t2 = __dadd_rn(t, L);
-  const long long b = __double_as_longlong(t2), l = __double_as_longlong(L);
-  if (b < 0 || b >= l + 0x0010000000000000ll) return wrap_like_fmod(t, L);  // below 0, at or past 2 L, NaN
-  return b >= l ? t2 - L : t2;
-}
-
 // The law of pair_force with its square root and divisions formed from one reciprocal square
 // root (as pair_f0_fast does in FP32), each within a few units of the last place: GB300's FP64
 // pipe runs 2 lanes a clock per SM, so the law's cost is its count of FP64 instructions.

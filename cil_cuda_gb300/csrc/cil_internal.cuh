@@ -282,6 +282,15 @@ __device__ __forceinline__ double wrap_like_fmod(double t, double L) {
   return fmod(t2, L);
 }
 
+// fmod(t + L, L) as wrap_like_fmod gives it, its comparisons on the bit patterns (doubles that
+// are not negative order like them), so that the FP64 pipe runs the two additions only.
+__device__ __forceinline__ double wrap_bits(double t, double L) {
+  const double t2 = __dadd_rn(t, L);
+  const long long b = __double_as_longlong(t2), l = __double_as_longlong(L);
+  if (b < 0 || b >= l + 0x0010000000000000ll) return wrap_like_fmod(t, L);  // below 0, at or past 2 L, NaN
+  return b >= l ? t2 - L : t2;
+}
+
 // Colony of a tile: tile_base[c] <= t < tile_base[c+1]
 __device__ __forceinline__ int colony_of_tile(const int *__restrict__ tile_base, int B, int t) {
   int lo = 0, hi = B - 1;
