@@ -61,8 +61,9 @@ struct CyConst {
   double dt;
   int ns[3];
   double bw[3];       // bin width per axis
-  float bwf[3], boxf[3], halff[3];  // FP32 copies for the packed pair arithmetic
+  float boxf[3], halff[3];  // FP32 copies for the range tests
   double half[3];     // box / 2
+  float inv_bwf[3];   // bins per length, rounded up
   double inv_bw[3];
   double sigma_core;
   double hz_c;        // (1 - nu^2) / E
@@ -75,6 +76,8 @@ struct CyConst {
   double v1, tau_r, tau_v, tau_p;   // tau_* in steps
   double v_s;
   double growth, inv_vs_tau_v, inv_tau_r, inv_tau_r_neg, inv_p0;  // (v1 - 1) / tau_v, reciprocals
+  double inv_hz;          // 1 / (0.75 c2), c2 = 2 (1 - nu^2) / E
+  double div_mu2, div_s2; // log-normal parameters of the cycle time
   double p0, beta_vs, rho_ratio, r_maxed_inv, p_shift, p_shift_tau_inv, osm;
   double apop_pressure, apop_duration, apop_rate_step, extr_gamma;
   double apop_steps;  // apop_duration / dt
@@ -99,7 +102,7 @@ struct CySet {
 // The cells in bin order, written by k_cy_place for the pair kernels: [q] is the cell at place q.
 struct CyOrdered {
   double *x;    // [D][cap]
-  double *sig;
+  double *rad;  // radius (sigma / 2, exact)
   float4 *rec;  // FP32 position (z 0 in 2D) and diameter, for the range tests
   float4 *vel;  // FP32 velocity (DPD, precision 1)
   int *idx;     // the cell's index
@@ -123,6 +126,7 @@ constexpr int kErrCapacity = 1;
 constexpr int kErrNonFinite = 2;
 constexpr int kErrOutOfBox = 4;
 constexpr int kErrCrowded = 8;     // a bin holds more than kBinSortMax cells
+constexpr int kDueMax = 1024;      // dividing cells ranked from a queue (more: by a scan of the cells)
 constexpr int kBinSortMax = 256;   // cells a bin may hold (about 1 at the bin width used)
 
 // ---------------------------------------------------------------- draws
@@ -151,13 +155,6 @@ __device__ inline int nint(double a) { return a >= 0.0 ? static_cast<int>(a + 0.
 __device__ inline int span_steps(double x, double dt) {
   const int s = nint(x / dt);
   return s > 1 ? s : 1;
-}
-
-// exp(mu2 + s2 Z), mu2 = log(mu^2 / sqrt(mu^2 + s^2)), s2 = sqrt(log(1 + s^2/mu^2)) (Random.hpp:55-60)
-__device__ inline double lognormal(double mu, double s, double z) {
-  const double mu2 = log((mu * mu) / (sqrt(mu * mu + s * s)));
-  const double s2 = sqrt(log(1 + (s * s) / (mu * mu)));
-  return exp(mu2 + s2 * z);
 }
 
 // ---------------------------------------------------------------- geometry (Utils.hpp:223-256)
@@ -339,43 +336,47 @@ __global__ void __launch_bounds__(kTile) k_cy_keys(CyConst C, CySet S, const CyC
 }
 
 __global__ void __launch_bounds__(kTile) k_cy_scatter(const CyCounters *cnt, const int *key, const int *arrival,
-                                                      const int *start, int *tmp) {
+                                                      const int *start, int2 *tmp) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt->n) return;
-  tmp[start[key[i]] + arrival[i]] = i;
+  const int b = key[i];
+  tmp[start[b] + arrival[i]] = make_int2(i, b);
 }
 
 // The bin order: a cell's place is its bin's start plus the number of smaller indices in the bin
 // (bins hold a few cells; a bin with more than kBinSortMax means overlapping cells and is reported,
 // its cells in arrival order). Written at the place: the index, the bin, the FP64 position and
-// diameter, and the FP32 record (absolute position and diameter) of the range tests.
-__global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounters *cnt, const int *key,
-                                                    const int *arrival, const int *start, const int *tmp,
-                                                    CyOrdered O, int with_vel) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt->n) return;
-  const int b = key[i], lo = start[b], hi = start[b + 1];
-  int rank = 0;
-  if (hi - lo > kBinSortMax) {
-    atomicOr(&cnt->err, kErrCrowded);
-    rank = arrival[i];
-  } else {
-    for (int q = lo; q < hi; ++q) rank += tmp[q] < i ? 1 : 0;
-  }
-  const int q = lo + rank;
+// radius, and the FP32 record (absolute position and diameter) of the range tests. Threads take the
+// cells in arrival order, next to their places: the state is gathered (32 bytes a value where the
+// index order is not the bin order) and the copies are written in full lines (DPD, 0.15M cells: 6.8 us;
+// from the index order, with the copies scattered, 8.2 us).
+__global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounters *cnt, const int *start,
+                                                    const int2 *tmp, CyOrdered O, int with_vel) {
+  const int at = blockIdx.x * blockDim.x + threadIdx.x;
+  if (at >= cnt->n) return;
+  const int2 ib = tmp[at];
+  const int i = ib.x, b = ib.y, lo = start[b], hi = start[b + 1];
   const size_t cap = C.capacity;
-  float xf[3] = {0.0f, 0.0f, 0.0f}, vf[3] = {0.0f, 0.0f, 0.0f};
+  double x[3] = {0.0, 0.0, 0.0};
+  float vf[3] = {0.0f, 0.0f, 0.0f};
   CY_AXES(d, C.D) {
-    const double x = S.x[d * cap + i];
-    O.x[d * cap + q] = x;
-    xf[d] = static_cast<float>(x);
+    x[d] = S.x[d * cap + i];
     if (with_vel) vf[d] = static_cast<float>(S.v[d * cap + i]);
   }
   const double sg = S.sig[i];
-  O.sig[q] = sg;
+  int q = at;
+  if (hi - lo > kBinSortMax) {
+    atomicOr(&cnt->err, kErrCrowded);
+  } else {
+    q = lo;
+    for (int k = lo; k < hi; ++k) q += tmp[k].x < i ? 1 : 0;
+  }
+  CY_AXES(d, C.D) O.x[d * cap + q] = x[d];
+  O.rad[q] = 0.5 * sg;
   O.idx[q] = i;
   O.bin[q] = b;
-  O.rec[q] = make_float4(xf[0], xf[1], xf[2], static_cast<float>(sg));
+  O.rec[q] = make_float4(static_cast<float>(x[0]), static_cast<float>(x[1]), static_cast<float>(x[2]),
+                         static_cast<float>(sg));
   if (with_vel) O.vel[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
 }
 
@@ -388,8 +389,9 @@ __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounte
 //           walk order, so that the sums do not depend on the lane count;
 //   pairs   the warp's survivors as one flattened range, a pair per lane;
 //   sums    a cell's first lane adds its pairs in walk order.
-// One thread per cell with each contact evaluated where it was met took 1079 us for the contacts of
-// 1M cells (2.6 contacts a cell, FP64) and 43 us for 0.15M with FP32 pair terms.
+// The contacts and the cycle of 1M cells (2.6 contacts a cell, FP64) take 498 us, with the FP64 pipe 80 %
+// busy (253 FP64 instructions per cell); one thread per cell with each contact evaluated where it was
+// met took 1079 us, and the cycle's own pass 258 us.
 constexpr int kPairBlock = 128;
 constexpr int kPairNear = 384;  // survivors held per warp (12 per cell at one lane each)
 constexpr int kPairSeg = 128;   // pairs evaluated before their sums are taken
@@ -398,7 +400,8 @@ template <int D, int NRES, typename R>
 struct PairWarp {
   R res[kPairSeg * NRES];
   double x[32 * D], v[32 * D];
-  double sig[32];
+  double rad[32];
+  float dia[32];
   int idx[32];
   int tt[kPairNear];
   unsigned char own[kPairNear];
@@ -418,7 +421,7 @@ __device__ inline double nearest(double dd, double L, double half) {
 // complete in its first lane. radius: no pair farther apart is in range. Whole warp.
 template <int D, int NRES, typename R, class Reach, class Pair>
 __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R> &W, const CyOrdered &O,
-                                           const int *start, bool live, int q, int lane_bits, double radius,
+                                           const int *start, bool live, int q, int lane_bits, float radius,
                                            Reach reach2, Pair pair, R *acc) {
   const int lane = threadIdx.x & 31, L = 1 << lane_bits;
   const int sub = lane & (L - 1), el = lane >> lane_bits;
@@ -457,8 +460,8 @@ __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R
     }
     cnt = 0;
   };
-  // the cell's bin and the bins to search on each side: k = ceil(radius / bin width), the whole axis
-  // (each bin once) when 2k + 1 covers it, clipped at open walls
+  // the cell's bin and the bins to search on each side: k = ceil(radius / bin width) (FP32, rounded
+  // up), the whole axis (each bin once) when 2k + 1 covers it, clipped at open walls
   int bi[D], lo[D], hi[D];
   {
     int b = live ? O.bin[q] : 0;
@@ -466,8 +469,8 @@ __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R
     for (int d = D - 1; d >= 0; --d) {
       bi[d] = d > 0 ? b % C.ns[d] : b;
       b /= C.ns[d];
-      const double kk = ceil(radius * C.inv_bw[d]);
-      const int k = (kk >= 0.0 && kk < C.ns[d]) ? static_cast<int>(kk) : C.ns[d];
+      const float kk = ceilf(__fmul_ru(radius, C.inv_bwf[d]));
+      const int k = (kk >= 0.0f && kk < static_cast<float>(C.ns[d])) ? static_cast<int>(kk) : C.ns[d];
       if (2 * k + 1 >= C.ns[d]) {
         lo[d] = -bi[d];
         hi[d] = C.ns[d] - 1 - bi[d];
@@ -555,20 +558,25 @@ __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R
   flush();
 }
 
+// the colony's largest diameter of the last step, rounded up
+__device__ inline float sigma_max_f(const CyCounters *cnt) {
+  return __double2float_ru(__longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)));
+}
+
 // ---------------------------------------------------------------- the cell cycle of one cell
 // The cycle ODEs at the step's end with pressure p; a cell at phase 1 is counted for k_cy_divide
 // (by its block of kTile cells, so that daughters come in mother order). Returns the bits of the
 // cell's diameter.
-__device__ inline unsigned long long cycle_update(const CyConst &C, const CySet &S, CyCounters *cnt, int *dblk, int i,
-                                                  int ts, double p, double sig) {
+__device__ inline unsigned long long cycle_update(const CyConst &C, const CySet &S, CyCounters *cnt, int *dblk,
+                                                  int *dueq, int i, int ts, double p, double rad) {
   // cellTPressure (CIL.cu:493-494): every cell is in the dividing state when the species divides
   S.tp[i] = p < C.apop_pressure ? 0 : S.tp[i] + 1;
-  const double shift = C.p_shift != 0.0 ? C.p_shift * exp(-ts * C.p_shift_tau_inv) : 0.0;
+  double pp = p;
+  if (C.p_shift != 0.0) pp += C.p_shift * exp(-ts * C.p_shift_tau_inv);
   double pnd = 0.0;
-  if (shift != 0.0 || __double_as_longlong(p) > 0) {  // fmax(0, p) / p0, the quotient by its residual
-    const double pp = fmax(0., p + shift);
+  if (__double_as_longlong(pp) > 0 && !(__double2hiint(pp) > 0x7ff00000)) {  // fmax(0, p) / p0
     pnd = pp * C.inv_p0;
-    pnd = __fma_rn(__fma_rn(-pnd, C.p0, pp), C.inv_p0, pnd);
+    if (finite_bits(pnd)) pnd = __fma_rn(__fma_rn(-pnd, C.p0, pp), C.inv_p0, pnd);
   }
   const double om = S.om[i];
   double rho = S.rho[i];
@@ -576,12 +584,12 @@ __device__ inline unsigned long long cycle_update(const CyConst &C, const CySet 
   S.theta[i] = theta;
   const bool d3 = C.D == 3;
   const double st = S.sigt[i];
-  double vt = d3 ? volume_of(st) : area_of(st);
-  const double vt_prime = (om * kLn2 + C.growth) * rho - (vt - C.v_s) * C.inv_vs_tau_v;
-  vt += vt_prime * vt;
+  double vt = d3 ? volume_of(st) : (kPi / 4) * (st * st);
+  const double vt_prime = __fma_rn(__fma_rn(om, kLn2, C.growth), rho, -((vt - C.v_s) * C.inv_vs_tau_v));
+  vt = __fma_rn(vt_prime, vt, vt);
   double v = vt;  // CYCLE_TAU_P 0 takes the target at once
   if (C.tau_p != 0) {
-    v = d3 ? volume_of(sig) : area_of(sig);
+    v = d3 ? volume_of(2 * rad) : area_of(2 * rad);
     v += -(v - (vt / (1 + C.beta_vs * (C.osm + pnd)))) / C.tau_p;
   }
   double sn;
@@ -596,11 +604,12 @@ __device__ inline unsigned long long cycle_update(const CyConst &C, const CySet 
   }
   S.sig[i] = sn;
   const double r_np = (1 - rho - pnd);
-  rho += r_np * (r_np > 0 ? C.inv_tau_r : C.inv_tau_r_neg) * rho;
+  rho = __fma_rn(r_np * (__double2hiint(r_np) >= 0 ? C.inv_tau_r : C.inv_tau_r_neg), rho, rho);
   S.rho[i] = rho;
   if (theta >= 1) {
     atomicAdd(dblk + i / kTile, 1);
-    atomicAdd(&cnt->ndue, 1);
+    const int at = atomicAdd(&cnt->ndue, 1);
+    if (at < kDueMax) dueq[at] = i;
   }
   return static_cast<unsigned long long>(__double_as_longlong(sn));
 }
@@ -617,38 +626,36 @@ __device__ inline void raise_sigma(CyCounters *cnt, unsigned long long s) {
 }
 
 // ---------------------------------------------------------------- forces + update
-// The contact of cells a and b (a the lower index) at distance r = 1 / y <= (sa + sb) / 2, the device
-// draft's Hertz law with adhesion and its pressure (MD.cu:302-366): the force along the separation
-// f0 = -fel + adhesion A, fel = h^1.5 / (0.75 c2 sqrt(1/ra + 1/rb)), and f0 / (contact volume).
-// 2D: with h = ra + rb - r the contact length A = 2 sqrt(ra^2 - q^2), q = ra - h (2 rb - h) / (2 r),
-// is 2 sqrt(w (2 ra - w)), w = h (2 rb - h) / (2 r) (no cancellation for small h); the elastic term is
-// h^2 ra rb / (0.75 c2 sqrt(h (ra + rb) ra rb)). Three reciprocal square roots per pair in all.
-__device__ inline void contact(const CyConst &C, double r, double y, double sa, double sb, double inv_hz, double *f0,
-                               double *pr) {
-  const double cut = (sa + sb) / 2;
-  const double h = fmax(cut - r, 0.0);
-  const double ab = 0.25 * (sa * sb);
-  const double g = h * cut * ab;
-  const double fel = mid_range(g) ? h * h * ab * rsqrt_pos(g) * inv_hz
-                                  : h * sqrt(h / (1.0 / (sa / 2) + 1.0 / (sb / 2))) * inv_hz;
-  if (C.D == 3) {
-    const double A = contact_area(r, sa, sb);
-    const double vol = (A == 0 ? 0 : (4 * kPi * ((sa / 2) * (sa / 2)) / 3));
+// The contact of cells a and b (radii, a the lower index) at distance r with overlap h = ra + rb - r
+// and half the reciprocal distance hy = 1 / (2 r), the device draft's Hertz law with adhesion and its pressure
+// (MD.cu:302-366): the force along the separation f0 = -fel + adhesion A, fel = h^1.5 / (0.75 c2
+// sqrt(1/ra + 1/rb)), and 2 f0 / (contact volume). 2D: the contact length A = 2 sqrt(ra^2 - q^2),
+// q = ra - h (2 rb - h) / (2 r), is 2 sqrt(w (2 ra - w)), w = h (2 rb - h) / (2 r) (no cancellation for
+// small h); the elastic term is h^2 ra rb / (0.75 c2 sqrt(h (ra + rb) ra rb)). With the separation's,
+// three reciprocal square roots and about 40 FP64 instructions per pair.
+template <int D>
+__device__ inline void contact(const CyConst &C, double r, double h, double hy, double cut, double ra, double rb,
+                               double *f0, double *pr2) {
+  const double u = h * (ra * rb), g = u * cut;
+  const double fel = mid_range(g) ? u * h * (rsqrt_pos(g) * C.inv_hz) : h * sqrt(h / (1.0 / ra + 1.0 / rb)) * C.inv_hz;
+  if (D == 3) {
+    const double A = contact_area(r, 2 * ra, 2 * rb);
+    const double vol = (A == 0 ? 0 : (4 * kPi * (ra * ra) / 3));
     *f0 = -fel + C.adhesion * A;
-    *pr = vol != 0.0 ? *f0 / vol : 0.0;
+    *pr2 = vol != 0.0 ? 2 * (*f0 / vol) : 0.0;
     return;
   }
-  const double w = h * (sb - h) * (0.5 * y);
-  const double t2 = w * (sa - w);
+  const double w = h * hy * __fma_rn(2.0, rb, -h);
+  const double t2 = w * __fma_rn(2.0, ra, -w);
   if (mid_range(t2)) {  // A is also the contact's volume in 2D
     const double z = rsqrt_pos(t2);
-    *f0 = -fel + C.adhesion * (2 * sqrt_from(t2, z));
-    *pr = *f0 * (0.5 * z);
+    *f0 = __fma_rn(2 * C.adhesion, t2 * z, -fel);
+    *pr2 = *f0 * z;
   } else {
     const double t = 2 * sqrt(t2);
-    const double A = isnan(t) ? (sa <= sb ? sa : sb) : t;
+    const double A = isnan(t) ? 2 * (ra <= rb ? ra : rb) : t;
     *f0 = -fel + C.adhesion * A;
-    *pr = A != 0.0 ? *f0 / A : 0.0;
+    *pr2 = A != 0.0 ? 2 * (*f0 / A) : 0.0;
   }
 }
 
@@ -661,7 +668,7 @@ __device__ inline void contact(const CyConst &C, double r, double y, double sa, 
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, double *frc, CyCounters *cnt,
                                                          const int *start, const int *ts_dev, int mode, int key_off,
-                                                         CyOrdered O, int lane_bits, int *dblk) {
+                                                         CyOrdered O, int lane_bits, int *dblk, int *dueq) {
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, D + 1, R> s_warp[kPairBlock / 32];
   PairWarp<D, D + 1, R> &W = s_warp[threadIdx.x >> 5];
@@ -676,22 +683,21 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
   double xi[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) xi[d] = live ? O.x[d * cap + q] : 0.0;
-  const double si = live ? O.sig[q] : 1.0;
+  const double ri = live ? O.rad[q] : 1.0;
   if (sub == 0) {
 #pragma unroll
     for (int d = 0; d < D; ++d) W.x[el * D + d] = xi[d];
-    W.sig[el] = si;
+    W.rad[el] = ri;
+    W.dia[el] = live ? O.rec[q].w : 1.0f;
     W.idx[el] = i;
   }
   __syncwarp();
-  const double c2 = C.hz_c + C.hz_c;
-  const double inv_hz = 1.0 / (0.75 * c2);
-  const float c2f = static_cast<float>(c2), adhf = static_cast<float>(C.adhesion);
+  const float c2f = static_cast<float>(C.hz_c + C.hz_c), adhf = static_cast<float>(C.adhesion);
   R acc[D + 1];
 #pragma unroll
   for (int k = 0; k <= D; ++k) acc[k] = R(0);
   walk_pairs<D, D + 1, R>(
-      C, W, O, start, live, q, lane_bits, __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)),
+      C, W, O, start, live, q, lane_bits, sigma_max_f(cnt),
       [](const float4 &a, const float4 &b) {
         const float cut = 0.5f * (a.w + b.w);
         return cut * cut;
@@ -703,9 +709,8 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
           double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
           if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
           rij[d] = v;
-          if (!MIXED) r2 = __fma_rn(v, v, r2);
+          if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
         }
-        const double so = W.sig[o], sj = __ldg(O.sig + tt);
         // the pair's first cell is the one of lower index (the contact length is not symmetric in
         // the two diameters)
         const bool first = W.idx[o] < __ldg(O.idx + tt);
@@ -718,7 +723,7 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
             df[d] = static_cast<float>(rij[d]);
             r2f += df[d] * df[d];
           }
-          const float sif = static_cast<float>(so), sjf = static_cast<float>(sj);
+          const float sif = W.dia[o], sjf = __ldg(O.rec + tt).w;
           const float cut = 0.5f * (sif + sjf);
           if (!(r2f <= cut * cut) || r2f == 0.0f) return;
           const float r = sqrtf(r2f);
@@ -741,22 +746,26 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
           const float f0 = -fel + adhf * A;
 #pragma unroll
           for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * df[d]);
-          out[D] = static_cast<R>(vol != 0.0f ? -(f0 / vol) : 0.0f);
+          out[D] = static_cast<R>(vol != 0.0f ? f0 / vol : 0.0f);
         } else {
-          double y, r;
+          const double ro = W.rad[o], rj = __ldg(O.rad + tt);
+          double hy, r;
           if (mid_range(r2)) {
-            y = rsqrt_pos(r2);
+            const double y = rsqrt_pos(r2);
             r = sqrt_from(r2, y);
+            hy = 0.5 * y;
           } else {
             r = sqrt(r2);
-            y = 1.0 / r;
+            hy = 0.5 / r;
           }
-          if (!(r <= (so + sj) / 2) || r == 0.0) return;
-          double f0, pr;
-          contact(C, r, y, first ? so : sj, first ? sj : so, inv_hz, &f0, &pr);
+          const double cut = ro + rj, h = cut - r;
+          // h >= 0 and finite (sign and exponent bits), r not 0
+          if (__double2hiint(h) < 0 || !finite_bits(h) || __double_as_longlong(r) == 0) return;
+          double f0, pr2;
+          contact<D>(C, r, h, hy, cut, first ? ro : rj, first ? rj : ro, &f0, &pr2);
 #pragma unroll
           for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * rij[d]);
-          out[D] = static_cast<R>(-pr);
+          out[D] = static_cast<R>(pr2);
         }
       },
       acc);
@@ -770,7 +779,7 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
 #pragma unroll
       for (int d = 0; d < D; ++d) {
         vi[d] = S.v[d * cap + i];
-        v2 += vi[d] * vi[d];
+        v2 = d == 0 ? vi[d] * vi[d] : __fma_rn(vi[d], vi[d], v2);
       }
       if (mid_range(v2)) {
         const double m = C.motility * rsqrt_pos(v2);
@@ -815,7 +824,7 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
       F[d] += static_cast<double>(acc[d]);
       finite = finite && finite_bits(F[d]);
     }
-    const double pres = static_cast<double>(acc[D]);
+    const double pres = MIXED ? -static_cast<double>(acc[D]) : -0.5 * static_cast<double>(acc[D]);
     S.p[i] = pres;
     if (!finite) atomicOr(&cnt->err, kErrNonFinite);
     if (mode == 1) {
@@ -825,16 +834,16 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
       // ---- position update with the pressure-dependent friction (CIL.cu:902-939)
       // pow(x, 0) is 1 for every x
       const double pw = C.zeta_p_beta == 0.0 ? 1.0 : pow(pres / C.p0, C.zeta_p_beta);
-      const double den = (C.zeta + C.zeta_p * pw) * area_of(si);
+      const double den = (C.zeta + C.zeta_p * pw) * (kPi * (ri * ri));
       const double mu = mid_range(den) ? rcp_normal(den) : 1.0 / den;
       const double temp = C.dt * mu;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        const double x = xi[d] + temp * F[d];
+        const double x = __fma_rn(temp, F[d], xi[d]);
         S.x[d * cap + i] = C.periodic[d] ? wrap(x, C.box[d]) : x;
         S.v[d * cap + i] = F[d] * mu;
       }
-      if (C.divide) sbits = cycle_update(C, S, cnt, dblk, i, ts + 1, pres, si);
+      if (C.divide) sbits = cycle_update(C, S, cnt, dblk, dueq, i, ts + 1, pres, ri);
     }
   }
   if (mode == 0 && C.divide) raise_sigma(cnt, sbits);
@@ -883,7 +892,8 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
       W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
       W.v[el * D + d] = vi[d];
     }
-    W.sig[el] = live ? O.sig[q] : 1.0;
+    W.rad[el] = live ? O.rad[q] : 1.0;
+    W.dia[el] = live ? O.rec[q].w : 1.0f;
     W.idx[el] = i;
   }
   __syncwarp();
@@ -892,7 +902,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
 #pragma unroll
   for (int k = 0; k < 2 * D; ++k) acc[k] = R(0);
   walk_pairs<D, 2 * D, R>(
-      C, W, O, start, live, q, lane_bits, __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits)),
+      C, W, O, start, live, q, lane_bits, sigma_max_f(cnt),
       [](const float4 &a, const float4 &b) {
         const float s = fmaxf(a.w, b.w);
         return s * s;
@@ -904,7 +914,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
           double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
           if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
           rij[d] = v;
-          if (!MIXED) r2 = __fma_rn(v, v, r2);
+          if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
         }
         const int io = W.idx[o], j = __ldg(O.idx + tt);
         const uint32_t a = static_cast<uint32_t>(io < j ? io : j), z = static_cast<uint32_t>(io < j ? j : io);
@@ -917,7 +927,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
             df[d] = static_cast<float>(rij[d]);
             r2f += df[d] * df[d];
           }
-          const float rc = io < j ? static_cast<float>(W.sig[o]) : __ldg(O.rec + tt).w;
+          const float rc = io < j ? W.dia[o] : __ldg(O.rec + tt).w;
           if (!(r2f < rc * rc) || r2f == 0.0f) return;
           const float4 vj4 = __ldg(O.vel + tt);
           const float rinv = rsqrtf(r2f);
@@ -934,7 +944,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
             out[D + d] = static_cast<R>(srf * sw * nd * xf[d]);
           }
         } else {
-          const double rc = io < j ? W.sig[o] : __ldg(O.sig + tt);
+          const double rc = 2 * (io < j ? W.rad[o] : __ldg(O.rad + tt));
           double ir, r;
           if (mid_range(r2)) {
             ir = rsqrt_pos(r2);
@@ -986,7 +996,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCounters *cnt, const int *start,
                                                         const int *ts_dev, CyOrdered O, const float4 *vel,
-                                                        int lane_bits, int *dblk) {
+                                                        int lane_bits, int *dblk, int *dueq) {
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, D, R> s_warp[kPairBlock / 32];
   PairWarp<D, D, R> &W = s_warp[threadIdx.x >> 5];
@@ -1011,12 +1021,11 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
   __syncwarp();
   const double rc = C.sigma_core;
   const float rcf = static_cast<float>(rc), gdf = static_cast<float>(C.gamma_d);
-  const double smax = __longlong_as_double(static_cast<long long>(cnt->sigma_max_bits));
   R acc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) acc[d] = R(0);
   walk_pairs<D, D, R>(
-      C, W, O, start, live, q, lane_bits, smax > rc ? smax : rc,
+      C, W, O, start, live, q, lane_bits, fmaxf(sigma_max_f(cnt), __double2float_ru(rc)),
       [&](const float4 &, const float4 &) { return rcf * rcf; },
       [&](int o, int tt, R *out) {
         double rij[D], r2 = 0.0;
@@ -1025,7 +1034,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
           double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
           if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
           rij[d] = v;
-          if (!MIXED) r2 = __fma_rn(v, v, r2);
+          if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
           out[d] = R(0);
         }
         if (MIXED) {
@@ -1069,7 +1078,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
   if (live && sub == 0) {
 #pragma unroll
     for (int d = 0; d < D; ++d) S.fd[d * cap + i] = static_cast<double>(acc[d]) - C.gamma_b * vi[d];
-    if (C.divide) sbits = cycle_update(C, S, cnt, dblk, i, *ts_dev + 1, S.p[i], O.sig[q]);
+    if (C.divide) sbits = cycle_update(C, S, cnt, dblk, dueq, i, *ts_dev + 1, S.p[i], O.rad[q]);
   }
   if (C.divide) raise_sigma(cnt, sbits);
 }
@@ -1079,98 +1088,111 @@ __device__ inline void put_sigma_max(CyCounters *cnt, double s) {
 }
 
 // Divisions in mother order: daughter of the k-th dividing cell at n + k (calculDivisionsSingle,
-// CIL.cu:527-600; singleCellDivision, MD.cu:664-718). The blocks take the blocks of kTile cells in
-// turn and pass over those without a dividing cell (dblk). The block that finishes last commits the
+// CIL.cu:527-600; singleCellDivision, MD.cu:664-718). Up to kDueMax dividing cells are ranked among
+// themselves from their queue; more, by a scan over the cells. The block that finishes last commits the
 // step: the cell count, the largest diameter and the step counter (every block has read them by then).
-__device__ void divide_block(const CyConst &C, const CySet &S, CyCounters *cnt, int n, int ts, int cb,
-                             const int *dblk) {
-  int before = 0, tot;
-  for (int u = threadIdx.x; u < cb; u += kTile) before += dblk[u];
-  int off;
-  block_excl_scan(before, &off);
-  const int i = cb * kTile + threadIdx.x;
-  const int f = (i < n && S.theta[i] >= 1) ? 1 : 0;
-  const int rank = off + block_excl_scan(f, &tot);
+__device__ void divide_one(const CyConst &C, const CySet &S, CyCounters *cnt, int ts, int i, int inew) {
   const size_t cap = C.capacity;
-  if (f) {
-    const int inew = n + rank;
-    if (inew >= C.capacity) {
-      atomicOr(&cnt->err, kErrCapacity);
-    } else {
-      const int D = C.D;
-      const double lmom = S.sig[i];
-      double ldau, newsig;
-      double dr[3] = {0, 0, 0};
-      const u32x4 r0 = draw(C, i, ts, kCyDiv, 0);
-      if (D == 2) {
-        ldau = lmom / sqrt(2.0);
-        newsig = ldau;
-        const double rr = (lmom - ldau) / 2;
-        const double alpha = u53(r0.v[0], r0.v[1]) * 6.283185307179586;
-        dr[0] = rr * sin(alpha);
-        dr[1] = rr * cos(alpha);
-      } else {
-        const double rmom = lmom / 2;
-        const double vmom = 4 * kPi * rmom * rmom * rmom / 3;
-        const double a = 9 * lmom / 4;
-        const double b = -(3 * (lmom * lmom) / 2);
-        const double c = lmom * lmom * lmom / 4 - 3 * vmom / (kPi);
-        ldau = (-b + sqrt(b * b - 4 * a * c)) / (2 * a);
-        newsig = ldau;
-        const double rr = (lmom - ldau) / 2;
-        const double alpha = u53(r0.v[0], r0.v[1]) * 6.283185307179586;
-        const double beta = u53(r0.v[2], r0.v[3]) * 6.283185307179586;
-        dr[0] = rr * sin(alpha) * cos(beta);
-        dr[1] = rr * sin(alpha) * sin(beta);
-        dr[2] = rr * cos(alpha);
-      }
-      CY_AXES(d, D) {
-        const double m = S.x[d * cap + i];
-        double xd = m + dr[d], xm = m + (-dr[d]);
-        if (C.periodic[d]) {
-          xd = wrap(xd, C.box[d]);
-          xm = wrap(xm, C.box[d]);
-        }
-        S.x[d * cap + inew] = xd;
-        S.x[d * cap + i] = xm;
-        S.v[d * cap + inew] = 0.0;
-        S.v[d * cap + i] = 0.0;
-        if (S.fc) {  // resetFrc (CIL.cu:597-598)
-          S.fc[d * cap + inew] = S.fd[d * cap + inew] = S.fr[d * cap + inew] = 0.0;
-          S.fc[d * cap + i] = S.fd[d * cap + i] = S.fr[d * cap + i] = 0.0;
-        }
-      }
-      // cycle times: migration spans (daughter, then mother), log-normal cycle speeds (mother,
-      // then daughter), as the reference draws them
-      double z0, z1, z2, z3;
-      normal2(draw(C, i, ts, kCyDiv, 1), &z0, &z1);
-      normal2(draw(C, i, ts, kCyDiv, 2), &z2, &z3);
-      S.tsw[inew] = ts + span_steps(C.tau_mig_mu + C.tau_mig_sigma * z0, C.dt);
-      S.tsw[i] = ts + span_steps(C.tau_mig_mu + C.tau_mig_sigma * z1, C.dt);
-      S.om[i] = 1.0 / span_steps(lognormal(C.tau_div_mu, C.tau_div_sigma, z2), C.dt);
-      S.om[inew] = 1.0 / span_steps(lognormal(C.tau_div_mu, C.tau_div_sigma, z3), C.dt);
-      S.sig[inew] = newsig;
-      S.sig[i] = newsig;
-      S.sigt[inew] = newsig;
-      S.sigt[i] = newsig;
-      S.t0[inew] = ts;
-      S.t0[i] = ts;
-      S.theta[i] = 0;
-      S.theta[inew] = 0;
-      S.p[inew] = S.p[i];
-      S.rho[inew] = S.rho[i];
-      S.tp[inew] = -1;  // an unused slot of the reference's arrays (Colony.cpp:253)
+  if (inew >= C.capacity) {
+    atomicOr(&cnt->err, kErrCapacity);
+    return;
+  }
+  const int D = C.D;
+  const double lmom = S.sig[i];
+  double ldau, newsig;
+  double dr[3] = {0, 0, 0};
+  const u32x4 r0 = draw(C, i, ts, kCyDiv, 0);
+  if (D == 2) {
+    ldau = lmom / sqrt(2.0);
+    newsig = ldau;
+    const double rr = (lmom - ldau) / 2;
+    const double alpha = u53(r0.v[0], r0.v[1]) * 6.283185307179586;
+    dr[0] = rr * sin(alpha);
+    dr[1] = rr * cos(alpha);
+  } else {
+    const double rmom = lmom / 2;
+    const double vmom = 4 * kPi * rmom * rmom * rmom / 3;
+    const double a = 9 * lmom / 4;
+    const double b = -(3 * (lmom * lmom) / 2);
+    const double c = lmom * lmom * lmom / 4 - 3 * vmom / (kPi);
+    ldau = (-b + sqrt(b * b - 4 * a * c)) / (2 * a);
+    newsig = ldau;
+    const double rr = (lmom - ldau) / 2;
+    const double alpha = u53(r0.v[0], r0.v[1]) * 6.283185307179586;
+    const double beta = u53(r0.v[2], r0.v[3]) * 6.283185307179586;
+    dr[0] = rr * sin(alpha) * cos(beta);
+    dr[1] = rr * sin(alpha) * sin(beta);
+    dr[2] = rr * cos(alpha);
+  }
+  CY_AXES(d, D) {
+    const double m = S.x[d * cap + i];
+    double xd = m + dr[d], xm = m + (-dr[d]);
+    if (C.periodic[d]) {
+      xd = wrap(xd, C.box[d]);
+      xm = wrap(xm, C.box[d]);
+    }
+    S.x[d * cap + inew] = xd;
+    S.x[d * cap + i] = xm;
+    S.v[d * cap + inew] = 0.0;
+    S.v[d * cap + i] = 0.0;
+    if (S.fc) {  // resetFrc (CIL.cu:597-598)
+      S.fc[d * cap + inew] = S.fd[d * cap + inew] = S.fr[d * cap + inew] = 0.0;
+      S.fc[d * cap + i] = S.fd[d * cap + i] = S.fr[d * cap + i] = 0.0;
     }
   }
+  // cycle times: migration spans (daughter, then mother), log-normal cycle speeds (mother,
+  // then daughter), as the reference draws them
+  double z0, z1, z2, z3;
+  normal2(draw(C, i, ts, kCyDiv, 1), &z0, &z1);
+  normal2(draw(C, i, ts, kCyDiv, 2), &z2, &z3);
+  S.tsw[inew] = ts + span_steps(C.tau_mig_mu + C.tau_mig_sigma * z0, C.dt);
+  S.tsw[i] = ts + span_steps(C.tau_mig_mu + C.tau_mig_sigma * z1, C.dt);
+  S.om[i] = 1.0 / span_steps(exp(C.div_mu2 + C.div_s2 * z2), C.dt);
+  S.om[inew] = 1.0 / span_steps(exp(C.div_mu2 + C.div_s2 * z3), C.dt);
+  S.sig[inew] = newsig;
+  S.sig[i] = newsig;
+  S.sigt[inew] = newsig;
+  S.sigt[i] = newsig;
+  S.t0[inew] = ts;
+  S.t0[i] = ts;
+  S.theta[i] = 0;
+  S.theta[inew] = 0;
+  S.p[inew] = S.p[i];
+  S.rho[inew] = S.rho[i];
+  S.tp[inew] = -1;  // an unused slot of the reference's arrays (Colony.cpp:253)
 }
 
 __global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCounters *cnt, int *ts_dev,
-                                                     const int *dblk) {
-  const int n = cnt->n, ts = *ts_dev + 1;
-  const int nb = (n + kTile - 1) / kTile;
-  if (cnt->ndue > 0) {
-    for (int cb = blockIdx.x; cb < nb; cb += gridDim.x)
-      if (dblk[cb] > 0) divide_block(C, S, cnt, n, ts, cb, dblk);  // uniform
+                                                     const int *dblk, const int *dueq) {
+  __shared__ int s_due[kDueMax];
+  const int n = cnt->n, ts = *ts_dev + 1, nd = cnt->ndue;
+  if (nd <= kDueMax) {
+    // the queue's cells (in no particular order): each one's rank is the number of smaller indices
+    const int r = blockIdx.x * kTile + threadIdx.x;
+    if (blockIdx.x * kTile < nd) {  // uniform
+      for (int k = threadIdx.x; k < nd; k += kTile) s_due[k] = dueq[k];
+      __syncthreads();
+      if (r < nd) {
+        const int i = s_due[r];
+        int rank = 0;
+        for (int k = 0; k < nd; ++k) rank += s_due[k] < i ? 1 : 0;
+        divide_one(C, S, cnt, ts, i, n + rank);
+      }
+    }
+  } else {
+    // the blocks of kTile cells in turn, those without a dividing cell passed over
+    const int nb = (n + kTile - 1) / kTile;
+    for (int cb = blockIdx.x; cb < nb; cb += gridDim.x) {
+      if (dblk[cb] == 0) continue;  // uniform
+      int before = 0, off, tot;
+      for (int u = threadIdx.x; u < cb; u += kTile) before += dblk[u];
+      block_excl_scan(before, &tot);
+      off = tot;
+      const int i = cb * kTile + threadIdx.x;
+      const int f = (i < n && S.theta[i] >= 1) ? 1 : 0;
+      const int rank = off + block_excl_scan(f, &tot);
+      if (f) divide_one(C, S, cnt, ts, i, n + rank);
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1353,8 +1375,9 @@ struct cil_cycle {
   CyCounters *cnt = nullptr;
   CyCounters *h_cnt = nullptr;  // pinned
   int *ts_dev = nullptr;
-  int *key = nullptr, *arrival = nullptr, *bcount = nullptr, *bstart = nullptr, *tmp = nullptr, *part = nullptr;
-  int *flag = nullptr, *blk = nullptr, *dblk = nullptr;
+  int *key = nullptr, *arrival = nullptr, *bcount = nullptr, *bstart = nullptr, *part = nullptr;
+  int2 *tmp = nullptr;
+  int *flag = nullptr, *blk = nullptr, *dblk = nullptr, *dueq = nullptr;
   int nbins = 0, nparts = 0, nblocks = 0;
   long long nbins_cap = 0;  // bins the arrays hold
   int64_t ts = 0;
@@ -1467,7 +1490,7 @@ void set_bins(cil_cycle *h, double smax, int ncells) {
       C.bw[d] = 1.0;
       C.inv_bw[d] = 1.0;
     }
-    C.bwf[d] = static_cast<float>(C.bw[d]);
+    C.inv_bwf[d] = std::nextafter(static_cast<float>(C.inv_bw[d]), INFINITY);
     h->nbins *= C.ns[d];
   }
   if (C.ns[0] != before[0] || C.ns[1] != before[1] || C.ns[2] != before[2]) h->grid_gen += 1;
@@ -1499,7 +1522,7 @@ cil_status bin_cells(cil_cycle *h, int drift) {
   k_cy_keys<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->key, h->arrival, h->bcount, h->dblk, drift);
   scan_into(h, h->bcount, h->nbins, h->bstart);
   k_cy_scatter<<<g, kTile, 0, h->stream>>>(h->cnt, h->key, h->arrival, h->bstart, h->tmp);
-  k_cy_place<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->key, h->arrival, h->bstart, h->tmp, h->O,
+  k_cy_place<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->tmp, h->O,
                                          h->C.dpd && h->p.precision == 1 ? 1 : 0);
   h->launches += 3;
   return CIL_OK;
@@ -1529,10 +1552,10 @@ void launch_force_d(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) 
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
     k_cy_force<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
-                                                         h->O, h->lane_bits, h->dblk);
+                                                         h->O, h->lane_bits, h->dblk, h->dueq);
   else
     k_cy_force<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
-                                                          h->O, h->lane_bits, h->dblk);
+                                                          h->O, h->lane_bits, h->dblk, h->dueq);
 }
 
 void launch_force(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
@@ -1567,10 +1590,10 @@ void launch_dpd_dis_d(cil_cycle *h, CySet &S) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
     k_dpd_dis<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
-                                                        h->lane_bits, h->dblk);
+                                                        h->lane_bits, h->dblk, h->dueq);
   else
     k_dpd_dis<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
-                                                         h->lane_bits, h->dblk);
+                                                         h->lane_bits, h->dblk, h->dueq);
 }
 
 void launch_dpd_dis(cil_cycle *h, CySet &S) {
@@ -1603,7 +1626,8 @@ cil_status enqueue_step(cil_cycle *h) {
   }
   h->ts += 1;
   if (h->C.divide) {  // also moves the step counter
-    k_cy_divide<<<std::min(blocks_for(h->cap), 2 * kNumSMs), kTile, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev, h->dblk);
+    k_cy_divide<<<std::min(blocks_for(h->cap), 2 * kNumSMs), kTile, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev,
+                                                                                      h->dblk, h->dueq);
   } else {
     k_cy_advance<<<1, 1, 0, h->stream>>>(h->ts_dev);
   }
@@ -1730,6 +1754,14 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   C.tau_div_sigma = p->tau_div_sigma;
   C.tau_mig_mu = p->tau_mig_mu;
   C.tau_mig_sigma = p->tau_mig_sigma;
+  // the cycle time's log-normal exp(mu2 + s2 Z), mu2 = log(mu^2 / sqrt(mu^2 + s^2)),
+  // s2 = sqrt(log(1 + s^2 / mu^2)) (Random.hpp:55-60)
+  if (p->tau_div_mu != 0.0) {
+    const double mu = p->tau_div_mu, sd = p->tau_div_sigma;
+    C.div_mu2 = std::log((mu * mu) / std::sqrt(mu * mu + sd * sd));
+    C.div_s2 = std::sqrt(std::log(1 + (sd * sd) / (mu * mu)));
+  }
+  C.inv_hz = 1.0 / (0.75 * (C.hz_c + C.hz_c));
   // cycle times in steps (Input.cpp:176-178, CIL.cuh:225-233)
   C.v1 = p->v1;
   C.tau_r = p->cycle_tau_r * p->tau_div_mu / p->dt;
@@ -1804,7 +1836,7 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   if (ok) {
     h->frc = h->alloc<double>(D * cap);
     h->O.x = h->alloc<double>(D * cap);
-    h->O.sig = h->alloc<double>(cap);
+    h->O.rad = h->alloc<double>(cap);
     h->O.rec = h->alloc<float4>(cap);
     h->O.idx = h->alloc<int>(cap);
     h->O.bin = h->alloc<int>(cap);
@@ -1814,13 +1846,14 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
     h->bcount = h->alloc<int>(h->nbins_cap + 1);
     h->bstart = h->alloc<int>(h->nbins_cap + 1);
     h->arrival = h->alloc<int>(cap);
-    h->tmp = h->alloc<int>(cap);
+    h->tmp = h->alloc<int2>(cap);
+    h->dueq = h->alloc<int>(kDueMax);
     h->dblk = h->alloc<int>(blocks_for(capacity));
     h->part = h->alloc<int>(h->nparts + 1);
     h->flag = h->alloc<int>(cap);
     h->blk = h->alloc<int>(h->nblocks + 1);
-    ok = h->frc && h->O.x && h->O.sig && h->O.rec && h->O.idx && h->O.bin && h->cnt && h->ts_dev && h->key &&
-         h->bcount && h->bstart && h->arrival && h->tmp && h->dblk &&
+    ok = h->frc && h->O.x && h->O.rad && h->O.rec && h->O.idx && h->O.bin && h->cnt && h->ts_dev && h->key &&
+         h->bcount && h->bstart && h->arrival && h->tmp && h->dblk && h->dueq &&
          h->part && h->flag && h->blk &&
          cudaHostAlloc(&h->h_cnt, sizeof(CyCounters), cudaHostAllocDefault) == cudaSuccess;
   }
