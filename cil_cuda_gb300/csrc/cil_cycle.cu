@@ -84,8 +84,7 @@ struct CyConst {
   double extr_rate;
   // DPD
   int dpd;
-  double inv_kick_div;  // 1 / (2 (2 m)): updateVel's divisor with the mass argument 2 m
-  double sqrt_dt;
+  double kick_f, kick_r;  // dt and sqrt(dt) over 2 (2 m), updateVel's divisor with the mass argument 2 m
   double gamma_d, gamma_b, sigma_r;  // DISDIFCEL, DISBG, sqrt(2 DISDIFCEL kT)
   uint32_t seed_lo, seed_hi;
   int capacity;
@@ -115,7 +114,7 @@ struct CyCounters {
   long long ndiv_total;
   long long napo_total;
   unsigned long long sigma_max_bits;  // largest diameter (non-negative doubles order like their bits)
-  unsigned long long sigma_next_bits;  // the same, of the step under way
+  unsigned long long sigma_next_bits;  // the same, of the step under way (k_cy_divide)
   int ndiv_step;
   int nrem_step;
   int ndue;   // cells at phase 1, of the step under way
@@ -310,7 +309,8 @@ __device__ inline bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff
 // DPD's first half kick and drift (updateVelocities then updatePositions, CIL.cu:871-897, 849-866;
 // DPD step, CIL.cu:1055-1056) of the keys' own cells: no pass of its own over the positions.
 __device__ inline double kick(const CyConst &C, double v, double fc, double fd, double fr) {
-  return v + (fc * C.dt + fd * C.dt + fr * C.sqrt_dt) * C.inv_kick_div;  // updateVel (Utils.hpp:568-571)
+  // updateVel (Utils.hpp:568-571): v + (fc dt + fd dt + fr sqrt(dt)) / (2 (2 m))
+  return __fma_rn(fr, C.kick_r, __fma_rn(fc + fd, C.kick_f, v));
 }
 
 __global__ void __launch_bounds__(kTile) k_cy_keys(CyConst C, CySet S, const CyCounters *cnt, int *key, int *arrival,
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kTile) k_cy_keys(CyConst C, CySet S, const CyC
     if (drift) {
       const double v = kick(C, S.v[k], S.fc[k], S.fd[k], S.fr[k]);
       S.v[k] = v;
-      const double t = xd[d] + C.dt * v;
+      const double t = __fma_rn(C.dt, v, xd[d]);
       xd[d] = C.periodic[d] ? wrap(t, C.box[d]) : t;  // BoundingBox::updatePos
       S.x[k] = xd[d];
     }
@@ -395,11 +395,13 @@ __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounte
 constexpr int kPairBlock = 128;
 constexpr int kPairNear = 384;  // survivors held per warp (12 per cell at one lane each)
 constexpr int kPairSeg = 128;   // pairs evaluated before their sums are taken
+constexpr int kPairAhead = 4;   // candidates a lane has in flight (one lane per cell)
 
 template <int D, int NRES, typename R>
 struct PairWarp {
   R res[kPairSeg * NRES];
-  double x[32 * D], v[32 * D];
+  double x[32 * D];
+  R v[32 * D];  // velocities (DPD)
   double rad[32];
   float dia[32];
   int idx[32];
@@ -489,70 +491,92 @@ __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R
   float margin[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) margin[d] = 4.76837158e-07f * (C.boxf[d] + fabsf(f4c(me, d)));
-  const int nl = C.ns[D - 1];
+  const int nl = C.ns[D - 1], ahead = lane_bits == 0 ? kPairAhead : 1;
   // rows of bins over the other axes; the loop runs to the warp's longest stencil
   const int n0 = live ? hi[0] - lo[0] + 1 : 0, n1 = D == 3 ? hi[D - 2] - lo[D - 2] + 1 : 1;
   const int rows = n0 * n1;
   const int rows_w = __reduce_max_sync(0xffffffffu, rows);
-  for (int row = 0; row < rows_w; ++row) {
-    const bool ok = row < rows;
-    int rb = 0;
-    if (ok) {
-      int v = bi[0] + lo[0] + (D == 3 ? row / n1 : row);
-      if (v < 0) v += C.ns[0];
-      if (v >= C.ns[0]) v -= C.ns[0];
-      rb = v;
-      if (D == 3) {
-        int u = bi[1] + lo[1] + row % n1;
-        if (u < 0) u += C.ns[1];
-        if (u >= C.ns[1]) u -= C.ns[1];
-        rb = rb * C.ns[1] + u;
-      }
+  // a row's span [a, z] of the last axis is up to three pieces of consecutive bins: inside, below 0 and
+  // at or past the end; the piece inside is loaded a row ahead
+  const int a = bi[D - 1] + lo[D - 1], z = bi[D - 1] + hi[D - 1];
+  const int a1 = max(a, 0), z1 = min(z, nl - 1) + 1;
+  const bool wraps = __any_sync(0xffffffffu, live && (a < 0 || z >= nl));
+  auto row_start = [&](int row) {
+    int v = bi[0] + lo[0] + (D == 3 ? row / n1 : row);
+    if (v < 0) v += C.ns[0];
+    if (v >= C.ns[0]) v -= C.ns[0];
+    if (D == 3) {
+      int u = bi[1] + lo[1] + row % n1;
+      if (u < 0) u += C.ns[1];
+      if (u >= C.ns[1]) u -= C.ns[1];
+      v = v * C.ns[1] + u;
     }
-    // the row's span of the last axis in up to three pieces of consecutive bins: below 0, inside, at
-    // or past the end
-    const int a = bi[D - 1] + lo[D - 1], z = bi[D - 1] + hi[D - 1];
-    const int *rs = start + static_cast<size_t>(rb) * nl;
-    for (int piece = 0; piece < 3; ++piece) {
-      int st = 0, en = 0;
-      if (ok) {
-        if (piece == 0) {
-          if (a < 0) {
-            st = rs[a + nl];
-            en = rs[nl];
-          }
-        } else if (piece == 1) {
-          st = rs[max(a, 0)];
-          en = rs[min(z, nl - 1) + 1];
-        } else if (z >= nl) {
+    return start + static_cast<size_t>(v) * nl;
+  };
+  const int *rs = start;
+  int st = 0, en = 0;
+  if (rows > 0) {
+    rs = row_start(0);
+    st = rs[a1];
+    en = rs[z1];
+  }
+  for (int row = 0; row < rows_w; ++row) {
+    const int *rs_next = start;
+    int st_next = 0, en_next = 0;
+    if (row + 1 < rows) {
+      rs_next = row_start(row + 1);
+      st_next = rs_next[a1];
+      en_next = rs_next[z1];
+    }
+    for (int piece = 0; piece < (wraps ? 3 : 1); ++piece) {
+      if (piece == 1) {
+        st = en = 0;
+        if (row < rows && a < 0) {
+          st = rs[a + nl];
+          en = rs[nl];
+        }
+      } else if (piece == 2) {
+        st = en = 0;
+        if (row < rows && z >= nl) {
           st = rs[0];
           en = rs[z - nl + 1];
         }
       }
-      for (int tt0 = st; __any_sync(0xffffffffu, tt0 < en); tt0 += L) {
-        const int tt = tt0 + sub;
-        bool near = false;
-        if (tt < en && tt != q) {
-          const float4 p = __ldg(O.rec + tt);
+      // candidates in flight: kPairAhead of a lane alone with its cell, or one each of several lanes
+      for (int tt0 = st; __any_sync(0xffffffffu, tt0 < en); tt0 += ahead * L) {
+        float4 p[kPairAhead];
+        bool there[kPairAhead];
+#pragma unroll
+        for (int u = 0; u < kPairAhead; ++u) {
+          const int tt = tt0 + u * L + sub;
+          there[u] = u < ahead && tt < en && tt != q;
+          p[u] = there[u] ? __ldg(O.rec + tt) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < kPairAhead; ++u) {
+          if (u >= ahead) break;
           float r2 = 0.0f;
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            float dx = fabsf(f4c(p, d) - f4c(me, d));
+            float dx = fabsf(f4c(p[u], d) - f4c(me, d));
             if (C.periodic[d] && dx > C.halff[d]) dx = fabsf(dx - C.boxf[d]);
             dx = fmaxf(dx - margin[d], 0.0f);
             r2 += dx * dx;
           }
-          near = !(r2 > 1.00001f * reach2(me, p));
+          const bool near = there[u] && !(r2 > 1.00001f * reach2(me, p[u]));
+          const unsigned m = __ballot_sync(0xffffffffu, near);
+          if (near) W.tt[nb0 + cnt + __popc(m & below)] = tt0 + u * L + sub;
+          cnt += __popc(m & gmask);
         }
-        const unsigned m = __ballot_sync(0xffffffffu, near);
-        if (near) W.tt[nb0 + cnt + __popc(m & below)] = tt;
-        cnt += __popc(m & gmask);
-        if (__any_sync(0xffffffffu, cnt + L > cap)) {
+        if (__any_sync(0xffffffffu, cnt + ahead * L > cap)) {
           __syncwarp();
           flush();
         }
       }
     }
+    rs = rs_next;
+    st = st_next;
+    en = en_next;
   }
   __syncwarp();
   flush();
@@ -569,8 +593,12 @@ __device__ inline float sigma_max_f(const CyCounters *cnt) {
 // cell's diameter.
 __device__ inline unsigned long long cycle_update(const CyConst &C, const CySet &S, CyCounters *cnt, int *dblk,
                                                   int *dueq, int i, int ts, double p, double rad) {
+  // every load before the first store, which the compiler could not move them across
+  const int tp = S.tp[i];
+  const double om = S.om[i], st = S.sigt[i], theta0 = S.theta[i];
+  double rho = S.rho[i];
   // cellTPressure (CIL.cu:493-494): every cell is in the dividing state when the species divides
-  S.tp[i] = p < C.apop_pressure ? 0 : S.tp[i] + 1;
+  S.tp[i] = p < C.apop_pressure ? 0 : tp + 1;
   double pp = p;
   if (C.p_shift != 0.0) pp += C.p_shift * exp(-ts * C.p_shift_tau_inv);
   double pnd = 0.0;
@@ -578,12 +606,9 @@ __device__ inline unsigned long long cycle_update(const CyConst &C, const CySet 
     pnd = pp * C.inv_p0;
     if (finite_bits(pnd)) pnd = __fma_rn(__fma_rn(-pnd, C.p0, pp), C.inv_p0, pnd);
   }
-  const double om = S.om[i];
-  double rho = S.rho[i];
-  const double theta = S.theta[i] + om * fmin(C.r_maxed_inv * rho, 1.0);
+  const double theta = theta0 + om * fmin(C.r_maxed_inv * rho, 1.0);
   S.theta[i] = theta;
   const bool d3 = C.D == 3;
-  const double st = S.sigt[i];
   double vt = d3 ? volume_of(st) : (kPi / 4) * (st * st);
   const double vt_prime = __fma_rn(__fma_rn(om, kLn2, C.growth), rho, -((vt - C.v_s) * C.inv_vs_tau_v));
   vt = __fma_rn(vt_prime, vt, vt);
@@ -614,15 +639,15 @@ __device__ inline unsigned long long cycle_update(const CyConst &C, const CySet 
   return static_cast<unsigned long long>(__double_as_longlong(sn));
 }
 
-// the step's largest diameter, one atomic per warp that raises it
-__device__ inline void raise_sigma(CyCounters *cnt, unsigned long long s) {
+// the largest diameter of the warp's cells, for k_cy_divide (all the warps of a colony that fits the
+// chip at once would meet at one address)
+__device__ inline void warp_sigma(unsigned long long *part, unsigned long long s) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long v = __shfl_xor_sync(0xffffffffu, s, o);
     s = v > s ? v : s;
   }
-  if ((threadIdx.x & 31) == 0 && s > *reinterpret_cast<volatile unsigned long long *>(&cnt->sigma_next_bits))
-    atomicMax(&cnt->sigma_next_bits, s);
+  if ((threadIdx.x & 31) == 0) part[(blockIdx.x * kPairBlock + threadIdx.x) >> 5] = s;
 }
 
 // ---------------------------------------------------------------- forces + update
@@ -668,7 +693,8 @@ __device__ inline void contact(const CyConst &C, double r, double h, double hy, 
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, double *frc, CyCounters *cnt,
                                                          const int *start, const int *ts_dev, int mode, int key_off,
-                                                         CyOrdered O, int lane_bits, int *dblk, int *dueq) {
+                                                         CyOrdered O, int lane_bits, int *dblk, int *dueq,
+                                                         unsigned long long *sig_part) {
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, D + 1, R> s_warp[kPairBlock / 32];
   PairWarp<D, D + 1, R> &W = s_warp[threadIdx.x >> 5];
@@ -846,7 +872,7 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
       if (C.divide) sbits = cycle_update(C, S, cnt, dblk, dueq, i, ts + 1, pres, ri);
     }
   }
-  if (mode == 0 && C.divide) raise_sigma(cnt, sbits);
+  if (mode == 0 && C.divide) warp_sigma(sig_part, sbits);
 }
 
 // ---------------------------------------------------------------- DPD
@@ -890,7 +916,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
-      W.v[el * D + d] = vi[d];
+      W.v[el * D + d] = static_cast<R>(vi[d]);
     }
     W.rad[el] = live ? O.rad[q] : 1.0;
     W.dia[el] = live ? O.rec[q].w : 1.0f;
@@ -996,7 +1022,8 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCounters *cnt, const int *start,
                                                         const int *ts_dev, CyOrdered O, const float4 *vel,
-                                                        int lane_bits, int *dblk, int *dueq) {
+                                                        int lane_bits, int *dblk, int *dueq,
+                                                         unsigned long long *sig_part) {
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, D, R> s_warp[kPairBlock / 32];
   PairWarp<D, D, R> &W = s_warp[threadIdx.x >> 5];
@@ -1015,7 +1042,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
-      W.v[el * D + d] = vi[d];
+      W.v[el * D + d] = static_cast<R>(vi[d]);
     }
   }
   __syncwarp();
@@ -1080,7 +1107,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
     for (int d = 0; d < D; ++d) S.fd[d * cap + i] = static_cast<double>(acc[d]) - C.gamma_b * vi[d];
     if (C.divide) sbits = cycle_update(C, S, cnt, dblk, dueq, i, *ts_dev + 1, S.p[i], O.rad[q]);
   }
-  if (C.divide) raise_sigma(cnt, sbits);
+  if (C.divide) warp_sigma(sig_part, sbits);
 }
 
 __device__ inline void put_sigma_max(CyCounters *cnt, double s) {
@@ -1091,14 +1118,15 @@ __device__ inline void put_sigma_max(CyCounters *cnt, double s) {
 // CIL.cu:527-600; singleCellDivision, MD.cu:664-718). Up to kDueMax dividing cells are ranked among
 // themselves from their queue; more, by a scan over the cells. The block that finishes last commits the
 // step: the cell count, the largest diameter and the step counter (every block has read them by then).
-__device__ void divide_one(const CyConst &C, const CySet &S, CyCounters *cnt, int ts, int i, int inew) {
+// The division of cell i into i and inew: divide_places (positions, velocities, forces, diameters) and
+// divide_times (cycles), which touch different arrays, so that two warps run their chains at once. The
+// loads come before the stores, which the compiler could not move them across.
+__device__ void divide_places(const CyConst &C, const CySet &S, int ts, int i, int inew) {
   const size_t cap = C.capacity;
-  if (inew >= C.capacity) {
-    atomicOr(&cnt->err, kErrCapacity);
-    return;
-  }
   const int D = C.D;
   const double lmom = S.sig[i];
+  double x[3] = {0, 0, 0};
+  CY_AXES(d, D) x[d] = S.x[d * cap + i];
   double ldau, newsig;
   double dr[3] = {0, 0, 0};
   const u32x4 r0 = draw(C, i, ts, kCyDiv, 0);
@@ -1125,7 +1153,7 @@ __device__ void divide_one(const CyConst &C, const CySet &S, CyCounters *cnt, in
     dr[2] = rr * cos(alpha);
   }
   CY_AXES(d, D) {
-    const double m = S.x[d * cap + i];
+    const double m = x[d];
     double xd = m + dr[d], xm = m + (-dr[d]);
     if (C.periodic[d]) {
       xd = wrap(xd, C.box[d]);
@@ -1140,43 +1168,63 @@ __device__ void divide_one(const CyConst &C, const CySet &S, CyCounters *cnt, in
       S.fc[d * cap + i] = S.fd[d * cap + i] = S.fr[d * cap + i] = 0.0;
     }
   }
+  S.sig[inew] = newsig;
+  S.sig[i] = newsig;
+  S.sigt[inew] = newsig;
+  S.sigt[i] = newsig;
+}
+
+__device__ void divide_times(const CyConst &C, const CySet &S, int ts, int i, int inew) {
   // cycle times: migration spans (daughter, then mother), log-normal cycle speeds (mother,
-  // then daughter), as the reference draws them
-  double z0, z1, z2, z3;
-  normal2(draw(C, i, ts, kCyDiv, 1), &z0, &z1);
+  // then daughter), as the reference draws them (a span without spread needs no draw)
+  const double p = S.p[i], rho = S.rho[i];
+  double z0 = 0.0, z1 = 0.0, z2, z3;
+  if (C.tau_mig_sigma != 0.0) normal2(draw(C, i, ts, kCyDiv, 1), &z0, &z1);
   normal2(draw(C, i, ts, kCyDiv, 2), &z2, &z3);
   S.tsw[inew] = ts + span_steps(C.tau_mig_mu + C.tau_mig_sigma * z0, C.dt);
   S.tsw[i] = ts + span_steps(C.tau_mig_mu + C.tau_mig_sigma * z1, C.dt);
   S.om[i] = 1.0 / span_steps(exp(C.div_mu2 + C.div_s2 * z2), C.dt);
   S.om[inew] = 1.0 / span_steps(exp(C.div_mu2 + C.div_s2 * z3), C.dt);
-  S.sig[inew] = newsig;
-  S.sig[i] = newsig;
-  S.sigt[inew] = newsig;
-  S.sigt[i] = newsig;
   S.t0[inew] = ts;
   S.t0[i] = ts;
   S.theta[i] = 0;
   S.theta[inew] = 0;
-  S.p[inew] = S.p[i];
-  S.rho[inew] = S.rho[i];
+  S.p[inew] = p;
+  S.rho[inew] = rho;
   S.tp[inew] = -1;  // an unused slot of the reference's arrays (Colony.cpp:253)
 }
 
 __global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCounters *cnt, int *ts_dev,
-                                                     const int *dblk, const int *dueq) {
+                                                     const int *dblk, const int *dueq,
+                                                     const unsigned long long *sig_part, int lane_bits) {
   __shared__ int s_due[kDueMax];
+  __shared__ unsigned long long s_sig;
   const int n = cnt->n, ts = *ts_dev + 1, nd = cnt->ndue;
+  if (threadIdx.x == 0) s_sig = 0ull;
+  __syncthreads();
+  {  // the step's largest diameter (before the divisions halve the dividing cells)
+    const int nw = static_cast<int>(((static_cast<long long>(n) << lane_bits) + 31) >> 5);
+    unsigned long long m = 0ull;
+    for (int k = blockIdx.x * kTile + threadIdx.x; k < nw; k += gridDim.x * kTile) m = sig_part[k] > m ? sig_part[k] : m;
+    if (m) atomicMax(&s_sig, m);
+  }
   if (nd <= kDueMax) {
-    // the queue's cells (in no particular order): each one's rank is the number of smaller indices
-    const int r = blockIdx.x * kTile + threadIdx.x;
-    if (blockIdx.x * kTile < nd) {  // uniform
+    // the queue's cells (in no particular order): each one's rank is the number of smaller indices;
+    // the block's first half takes the places, the second the times
+    constexpr int kHalf = kTile / 2;
+    if (blockIdx.x * kHalf < nd) {  // uniform
       for (int k = threadIdx.x; k < nd; k += kTile) s_due[k] = dueq[k];
       __syncthreads();
-      if (r < nd) {
+      for (int r = blockIdx.x * kHalf + threadIdx.x % kHalf; r < nd; r += gridDim.x * kHalf) {
         const int i = s_due[r];
         int rank = 0;
         for (int k = 0; k < nd; ++k) rank += s_due[k] < i ? 1 : 0;
-        divide_one(C, S, cnt, ts, i, n + rank);
+        if (n + rank >= C.capacity)
+          atomicOr(&cnt->err, kErrCapacity);
+        else if (threadIdx.x < kHalf)
+          divide_places(C, S, ts, i, n + rank);
+        else
+          divide_times(C, S, ts, i, n + rank);
       }
     }
   } else {
@@ -1191,11 +1239,17 @@ __global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCount
       const int i = cb * kTile + threadIdx.x;
       const int f = (i < n && S.theta[i] >= 1) ? 1 : 0;
       const int rank = off + block_excl_scan(f, &tot);
-      if (f) divide_one(C, S, cnt, ts, i, n + rank);
+      if (f && n + rank >= C.capacity) {
+        atomicOr(&cnt->err, kErrCapacity);
+      } else if (f) {
+        divide_places(C, S, ts, i, n + rank);
+        divide_times(C, S, ts, i, n + rank);
+      }
     }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    if (s_sig) atomicMax(&cnt->sigma_next_bits, s_sig);
     __threadfence();
     if (atomicAdd(&cnt->ndone, 1) == static_cast<int>(gridDim.x) - 1) {
       const int nd = cnt->ndue, room = C.capacity - n;
@@ -1203,8 +1257,7 @@ __global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCount
       cnt->n = n + add;
       cnt->ndiv_total += add;
       cnt->ndiv_step = add;
-      cnt->sigma_max_bits = cnt->sigma_next_bits;
-      cnt->sigma_next_bits = 0ull;
+      cnt->sigma_max_bits = atomicExch(&cnt->sigma_next_bits, 0ull);
       cnt->ndue = 0;
       cnt->ndone = 0;
       *ts_dev = ts;
@@ -1378,6 +1431,7 @@ struct cil_cycle {
   int *key = nullptr, *arrival = nullptr, *bcount = nullptr, *bstart = nullptr, *part = nullptr;
   int2 *tmp = nullptr;
   int *flag = nullptr, *blk = nullptr, *dblk = nullptr, *dueq = nullptr;
+  unsigned long long *sig_part = nullptr;  // the step's largest diameter per warp of the pair kernel
   int nbins = 0, nparts = 0, nblocks = 0;
   long long nbins_cap = 0;  // bins the arrays hold
   int64_t ts = 0;
@@ -1552,10 +1606,10 @@ void launch_force_d(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) 
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
     k_cy_force<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
-                                                         h->O, h->lane_bits, h->dblk, h->dueq);
+                                                         h->O, h->lane_bits, h->dblk, h->dueq, h->sig_part);
   else
     k_cy_force<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
-                                                          h->O, h->lane_bits, h->dblk, h->dueq);
+                                                          h->O, h->lane_bits, h->dblk, h->dueq, h->sig_part);
 }
 
 void launch_force(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
@@ -1590,10 +1644,10 @@ void launch_dpd_dis_d(cil_cycle *h, CySet &S) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
     k_dpd_dis<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
-                                                        h->lane_bits, h->dblk, h->dueq);
+                                                        h->lane_bits, h->dblk, h->dueq, h->sig_part);
   else
     k_dpd_dis<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
-                                                         h->lane_bits, h->dblk, h->dueq);
+                                                         h->lane_bits, h->dblk, h->dueq, h->sig_part);
 }
 
 void launch_dpd_dis(cil_cycle *h, CySet &S) {
@@ -1627,7 +1681,8 @@ cil_status enqueue_step(cil_cycle *h) {
   h->ts += 1;
   if (h->C.divide) {  // also moves the step counter
     k_cy_divide<<<std::min(blocks_for(h->cap), 2 * kNumSMs), kTile, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev,
-                                                                                      h->dblk, h->dueq);
+                                                                                      h->dblk, h->dueq, h->sig_part,
+                                                                                      h->lane_bits);
   } else {
     k_cy_advance<<<1, 1, 0, h->stream>>>(h->ts_dev);
   }
@@ -1790,8 +1845,8 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   C.apop_steps = p->apop_duration / p->dt;
   C.extr_rate = p->extr_rate;
   C.dpd = p->integrator == CIL_CYCLE_DPD ? 1 : 0;
-  C.inv_kick_div = 1.0 / (2 * (2 * p->mass));
-  C.sqrt_dt = std::sqrt(p->dt);
+  C.kick_f = p->dt / (2 * (2 * p->mass));
+  C.kick_r = std::sqrt(p->dt) / (2 * (2 * p->mass));
   C.gamma_d = p->dis_diff;
   C.gamma_b = p->dis_bg;
   C.sigma_r = std::sqrt(2 * p->dis_diff * p->kbt);  // Sigma (MD.cu:872)
@@ -1848,12 +1903,13 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
     h->arrival = h->alloc<int>(cap);
     h->tmp = h->alloc<int2>(cap);
     h->dueq = h->alloc<int>(kDueMax);
+    h->sig_part = h->alloc<unsigned long long>(cap / 4 + kPairBlock / 32);  // up to 8 lanes per cell
     h->dblk = h->alloc<int>(blocks_for(capacity));
     h->part = h->alloc<int>(h->nparts + 1);
     h->flag = h->alloc<int>(cap);
     h->blk = h->alloc<int>(h->nblocks + 1);
     ok = h->frc && h->O.x && h->O.rad && h->O.rec && h->O.idx && h->O.bin && h->cnt && h->ts_dev && h->key &&
-         h->bcount && h->bstart && h->arrival && h->tmp && h->dblk && h->dueq &&
+         h->bcount && h->bstart && h->arrival && h->tmp && h->dblk && h->dueq && h->sig_part &&
          h->part && h->flag && h->blk &&
          cudaHostAlloc(&h->h_cnt, sizeof(CyCounters), cudaHostAllocDefault) == cudaSuccess;
   }

@@ -91,3 +91,33 @@ def test_cells_that_outgrow_their_bins_within_a_call(gpu_lib, oracle_lib, growth
     st["theta"][:] = 0.0
     st["angvel"][:] = 1e-6
     _check(prm, st, n, steps=30)
+
+
+@pytest.mark.parametrize("integrator", [0, G.CYCLE_DPD])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [1, 33, 600, 1023, 1024, 1025, 3000])
+def test_many_cells_divide_at_once(gpu_lib, oracle_lib, n, dim, integrator):
+    # every cell reaches phase 1 in the same step (queue and scan of k_cy_divide, daughters in mother
+    # order), then half of the colony's capacity is used
+    from oracle import oracle as O
+    L = max(6.0, (3.0 * n) ** (1.0 / dim))
+    box = [L, L, L]
+    prm = _params(dim, box, integrator)
+    st = _state(n, box, dim, seed=n)
+    st["theta"] = np.full(n, 0.999)
+    st["rho"] = np.ones(n)
+    eng = G.CycleEngine(prm, 2 * n, seed=7)
+    eng.upload(**st)
+    eng.step(1)
+    g = eng.download()
+    eng.close()
+    o = O.CycleOracle(prm, 2 * n, 7)
+    o.set_state(**st)
+    assert o.step(1) == 0
+    s = o.state()
+    assert g["ncells"] == s["ncells"] == 2 * n
+    for k in ("pos", "sigma", "sigma_t", "theta", "rho", "angvel", "vel"):
+        d = np.asarray(g[k]) - np.asarray(s[k])
+        if k == "pos":
+            d -= np.round(d / L) * L
+        assert np.abs(d).max() <= TOL * max(1.0, np.abs(s[k]).max()), k
