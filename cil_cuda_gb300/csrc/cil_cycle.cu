@@ -1393,6 +1393,32 @@ __global__ void k_cy_sigma_max(CyConst C, CySet S, CyCounters *cnt) {
   if (threadIdx.x == 0 && smax) put_sigma_max(cnt, __longlong_as_double(static_cast<long long>(smax)));
 }
 
+// ---------------------------------------------------------------- host copies
+// The host's vectors are [cell][axis], the device's [axis][cap]: staged as the host has them and
+// rearranged here, so that a copy from or into pinned memory runs at the link's rate (a host loop and
+// pageable copies took 5.8 of the 13.1 ms of a 1M-cell leg of 10 steps).
+__global__ void __launch_bounds__(kTile) k_cy_from_host(const double *staged, int n, int D, size_t cap, double *dst) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  CY_AXES(d, D) dst[d * cap + i] = staged[static_cast<size_t>(i) * D + d];
+}
+
+__global__ void __launch_bounds__(kTile) k_cy_to_host(const double *src, int n, int D, size_t cap, double *staged) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  CY_AXES(d, D) staged[static_cast<size_t>(i) * D + d] = src[d * cap + i];
+}
+
+// a staged position outside [0, box) sets *bad
+__global__ void __launch_bounds__(kTile) k_cy_check_staged(CyConst C, const double *staged, int n, int *bad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  CY_AXES(d, C.D) {
+    const double x = staged[static_cast<size_t>(i) * C.D + d];
+    if (!(x >= 0.0 && x < C.box[d])) *bad = 1;
+  }
+}
+
 }  // namespace
 
 // ================================================================ host side
@@ -1723,6 +1749,16 @@ cil_status graph_step(cil_cycle *h) {
       h->launches += g.nodes;
       return CIL_OK;
     }
+  // graphs of earlier grids serve no more (a grid's number never comes back), and none of them is in
+  // flight: a grid changes between calls, which end with the stream idle
+  for (size_t k = 0; k < h->graphs.size();) {
+    if (h->graphs[k].grid != h->grid_gen) {
+      cudaGraphExecDestroy(h->graphs[k].exec);
+      h->graphs.erase(h->graphs.begin() + static_cast<std::ptrdiff_t>(k));
+    } else {
+      ++k;
+    }
+  }
   if (h->graphs.size() >= kMaxStepGraphs) return enqueue_step(h);
   const int64_t l0 = h->launches, ts0 = h->ts;
   if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -1943,46 +1979,49 @@ cil_status cil_cycle_upload(cil_cycle *h, const cil_cycle_view *v) {
   if (!h || !v || !v->pos) return CIL_ERR_CONFIG;
   if (v->ncells < 0 || v->ncells > h->cap) return h->fail(CIL_ERR_CAPACITY, "cil_cycle_upload: more cells than the capacity");
   CY_TRY(h, cudaSetDevice(h->device));
-  const int n = v->ncells, D = h->C.D;
-  const size_t cap = h->cap;
+  const int n = v->ncells, D = h->C.D, g = blocks_for(n);
+  const size_t cap = h->cap, vec = sizeof(double) * static_cast<size_t>(n) * D;
+  // staged and checked before any of the state is written (O.x and the outputs of the last download
+  // are free between calls)
+  double *st_pos = h->O.x, *st_vel = h->frc;
+  int bad = 0, *d_bad = h->dueq;
+  if (n > 0) {
+    CY_TRY(h, cudaMemcpyAsync(st_pos, v->pos, vec, cudaMemcpyHostToDevice, h->stream));
+    CY_TRY(h, cudaMemsetAsync(d_bad, 0, sizeof(int), h->stream));
+    k_cy_check_staged<<<g, kTile, 0, h->stream>>>(h->C, st_pos, n, d_bad);
+    CY_TRY(h, cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    if (v->vel) CY_TRY(h, cudaMemcpyAsync(st_vel, v->vel, vec, cudaMemcpyHostToDevice, h->stream));
+    CY_TRY(h, cudaStreamSynchronize(h->stream));
+  }
+  if (bad) return h->fail(CIL_ERR_OUT_OF_BOX, "Input Positions Out of Bounds!");
   h->cur = 0;
   CySet &S = h->set[0];
-  std::vector<double> t(static_cast<size_t>(n));
-  for (int d = 0; d < D; ++d) {
-    for (int i = 0; i < n; ++i) {
-      const double x = v->pos[static_cast<size_t>(i) * D + d];
-      if (!(x >= 0.0 && x < h->C.box[d])) return h->fail(CIL_ERR_OUT_OF_BOX, "Input Positions Out of Bounds!");
-      t[i] = x;
-    }
-    CY_TRY(h, cudaMemcpy(S.x + d * cap, t.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-    CY_TRY(h, cudaMemset(S.v + d * cap, 0, sizeof(double) * cap));
-    if (v->vel) {
-      for (int i = 0; i < n; ++i) t[i] = v->vel[static_cast<size_t>(i) * D + d];
-      CY_TRY(h, cudaMemcpy(S.v + d * cap, t.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-    }
+  CY_TRY(h, cudaMemsetAsync(S.v, 0, sizeof(double) * D * cap, h->stream));
+  if (n > 0) {
+    k_cy_from_host<<<g, kTile, 0, h->stream>>>(st_pos, n, D, cap, S.x);
+    if (v->vel) k_cy_from_host<<<g, kTile, 0, h->stream>>>(st_vel, n, D, cap, S.v);
   }
   auto up = [&](double *dst, const double *src) -> cudaError_t {
-    return src ? cudaMemcpy(dst, src, sizeof(double) * n, cudaMemcpyHostToDevice) : cudaSuccess;
+    return src ? cudaMemcpyAsync(dst, src, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream) : cudaSuccess;
   };
   CY_TRY(h, up(S.sig, v->sigma));
   CY_TRY(h, up(S.sigt, v->sigma_t ? v->sigma_t : v->sigma));
   CY_TRY(h, up(S.theta, v->theta));
   CY_TRY(h, up(S.rho, v->rho));
   CY_TRY(h, up(S.om, v->angvel));
-  CY_TRY(h, cudaMemset(S.p, 0, sizeof(double) * cap));
+  CY_TRY(h, cudaMemsetAsync(S.p, 0, sizeof(double) * cap, h->stream));
   if (v->pressure) CY_TRY(h, up(S.p, v->pressure));
   CyCounters c{};
   c.n = n;
-  CY_TRY(h, cudaMemcpy(h->cnt, &c, sizeof(c), cudaMemcpyHostToDevice));
+  CY_TRY(h, cudaMemcpyAsync(h->cnt, &c, sizeof(c), cudaMemcpyHostToDevice, h->stream));
   const int ts = v->ts;
-  CY_TRY(h, cudaMemcpy(h->ts_dev, &ts, sizeof(int), cudaMemcpyHostToDevice));
+  CY_TRY(h, cudaMemcpyAsync(h->ts_dev, &ts, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   h->ts = ts;
   const int fill_sigma = v->sigma ? 0 : 1;
   const int fill_cycle = (v->theta && v->rho && v->angvel) ? 0 : 1;
   k_cy_init_status<<<blocks_for(h->cap), kTile, 0, h->stream>>>(h->C, S, h->cnt, ts, fill_sigma, fill_cycle);
   if (v->tpressure) {
-    CY_TRY(h, cudaStreamSynchronize(h->stream));
-    CY_TRY(h, cudaMemcpy(S.tp, v->tpressure, sizeof(int) * n, cudaMemcpyHostToDevice));
+    CY_TRY(h, cudaMemcpyAsync(S.tp, v->tpressure, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
   }
   k_cy_sigma_max<<<blocks_for(h->cap), kTile, 0, h->stream>>>(h->C, S, h->cnt);
   CY_TRY(h, cudaGetLastError());
@@ -2061,20 +2100,14 @@ cil_status cil_cycle_download(cil_cycle *h, cil_cycle_view *v) {
   if (n > v->capacity) return h->fail(CIL_ERR_CAPACITY, "cil_cycle_download: host arrays too small");
   const CySet &S = h->set[h->cur];
   const size_t cap = h->cap;
-  std::vector<double> t(static_cast<size_t>(n) * D);
+  // rearranged in O.x (free between steps), one vector after the other on the stream
   auto vec = [&](double *dst, const double *src) -> cudaError_t {
-    if (!dst) return cudaSuccess;
-    for (int d = 0; d < D; ++d) {
-      const cudaError_t e = cudaMemcpy(t.data() + static_cast<size_t>(d) * n, src + d * cap, sizeof(double) * n,
-                                       cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) return e;
-    }
-    for (int i = 0; i < n; ++i)
-      for (int d = 0; d < D; ++d) dst[static_cast<size_t>(i) * D + d] = t[static_cast<size_t>(d) * n + i];
-    return cudaSuccess;
+    if (!dst || n == 0) return cudaSuccess;
+    k_cy_to_host<<<blocks_for(n), kTile, 0, h->stream>>>(src, n, D, cap, h->O.x);
+    return cudaMemcpyAsync(dst, h->O.x, sizeof(double) * static_cast<size_t>(n) * D, cudaMemcpyDeviceToHost, h->stream);
   };
   auto sca = [&](void *dst, const void *src, size_t es) -> cudaError_t {
-    return dst ? cudaMemcpy(dst, src, es * n, cudaMemcpyDeviceToHost) : cudaSuccess;
+    return dst ? cudaMemcpyAsync(dst, src, es * n, cudaMemcpyDeviceToHost, h->stream) : cudaSuccess;
   };
   CY_TRY(h, vec(v->pos, S.x));
   CY_TRY(h, vec(v->vel, S.v));
@@ -2095,6 +2128,7 @@ cil_status cil_cycle_download(cil_cycle *h, cil_cycle_view *v) {
     for (double *f : {v->force_dis, v->force_ran})
       if (f) std::fill(f, f + static_cast<size_t>(n) * D, 0.0);
   }
+  CY_TRY(h, cudaStreamSynchronize(h->stream));
   return st;
 }
 

@@ -121,3 +121,32 @@ def test_many_cells_divide_at_once(gpu_lib, oracle_lib, n, dim, integrator):
         if k == "pos":
             d -= np.round(d / L) * L
         assert np.abs(d).max() <= TOL * max(1.0, np.abs(s[k]).max()), k
+
+
+@pytest.mark.parametrize("integrator", [0, G.CYCLE_DPD])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 1000])
+def test_state_comes_back_as_uploaded(gpu_lib, n, dim, integrator):
+    L = max(6.0, (3.0 * n) ** (1.0 / dim))
+    box = [L, L + 1.0, L + 2.0]
+    st = _state(n, box, dim, seed=n)
+    eng = G.CycleEngine(_params(dim, box, integrator), n + 5, seed=1)
+    keys = ("pos", "vel", "sigma", "theta", "rho", "angvel")
+    for _ in range(2):
+        eng.upload(**st)
+        g = eng.download()
+        assert g["ncells"] == n
+        for k in keys:
+            np.testing.assert_array_equal(g[k], st[k])
+        st["pos"] = st["pos"][::-1].copy()
+    eng.upload(**st)
+    for d in range(dim):  # refused, and the state stays
+        bad = dict(st, pos=st["pos"].copy(), sigma=2 * st["sigma"])
+        bad["pos"][n // 2, d] = box[d]
+        with pytest.raises(G.CilError) as e:
+            eng.upload(**bad)
+        assert e.value.status == 5
+        g = eng.download()
+        for k in keys:
+            np.testing.assert_array_equal(g[k], st[k])
+    eng.close()
