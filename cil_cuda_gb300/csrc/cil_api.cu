@@ -95,6 +95,9 @@ struct cil_handle {
   int lane_bits = 0;        // FP64 form: log2 of the lanes per element of the force pass
   double *d_sigma_c = nullptr;  // canonical diameters [2 * CC]
   bool need_exact = true;       // next rebuild takes the FP64 reference path
+  bool due_events = false;      // Philox draws, no crawling/dividing cells: events from the due-cell queues
+  bool scanned = false;         // a colony's scan blocks are many: their sums scanned by a launch of its own
+  int *d_scandone = nullptr;
   int pu = 1;                   // which d_pk holds the current packed elements
   // skin mode
   bool skin_mode = false;
@@ -140,9 +143,9 @@ struct cil_handle {
   int *d_tiles_pairs = nullptr;  // skin mode: tiles over slot pairs (the cell-major force kernel)
   int *d_tile_count = nullptr, *d_tile_off = nullptr;
   int *d_upchk = nullptr;     // upload checks: bad-value bits, largest diameter (double bits)
-  int *d_dueq = nullptr;      // skin mode, Philox: cells due to divide, per colony (due_base)
+  int *d_dueq = nullptr;      // Philox: cells due to divide, per colony (due_base)
   size_t due_total = 0;
-  int *d_evdone = nullptr;    // skin mode, Philox: colonies whose events are done this step
+  int *d_evdone = nullptr;    // Philox: colonies whose events are done this step
   int *d_dead = nullptr;
   int *d_divq = nullptr;  // division queue [CC]
   double *d_obs = nullptr;  // com_prev, disp, vref: 3 * D * CC
@@ -186,7 +189,7 @@ void free_all(cil_handle *h) {
                   h->d_ncnt, h->d_fresh, h->d_spart, h->d_lflat, h->d_lwarp, h->d_oflat, h->d_lstart, h->d_uref, h->d_facc, h->d_ftouch, h->d_skin, h->d_sched, h->d_mlp, h->d_fhead, h->d_fnext, h->d_ts, h->d_anyreb, h->d_vel, h->d_vel2, h->d_frc, h->d_key, h->d_perm,
                   h->d_bcount, h->d_range, h->d_scan_sum, h->d_scan_off, h->d_scan_col,
                   h->d_slot_of, h->d_t0, h->d_tsw, h->d_tiles_used, h->d_tiles_live, h->d_tiles_pairs,
-                  h->d_tiles_cell, h->d_tile_count, h->d_tile_off, h->d_upchk, h->d_dueq, h->d_evdone, h->d_dead, h->d_divq, h->d_obs,
+                  h->d_tiles_cell, h->d_tile_count, h->d_tile_off, h->d_upchk, h->d_dueq, h->d_evdone, h->d_scandone, h->d_dead, h->d_divq, h->d_obs,
                   h->d_partials, h->d_stage, h->d_noise, h->d_oracle_i, h->d_oracle_d};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -298,6 +301,10 @@ cil_status setup_geometry(cil_handle *h) {
       CUDA_TRY(h, cudaMemsetAsync(h->d_fhead, 0xff, sizeof(unsigned long long) * h->NBpad, h->stream));
     }
   }
+  // forms that rebuild every step: up to 4096 scan blocks (4M bins) a block of the scan adds the sums
+  // before its own itself: 33 MB read from L2 at most, about a launch's time
+  h->scanned = h->skin_mode;
+  for (int c = 0; c < h->B; ++c) h->scanned = h->scanned || h->cc[c].nbins_pad / kScanItems > 4096;
   std::vector<int> scol(h->nscan);
   for (int c = 0; c < h->B; ++c)
     for (int i = 0; i < h->cc[c].nbins_pad / kScanItems; ++i) scol[h->cc[c].scan_base + i] = c;
@@ -356,6 +363,9 @@ RebuildArgs rebuild_args(cil_handle *h) {
   a.perm = h->d_perm;
   a.scan_sum = h->d_scan_sum;
   a.scan_off = h->d_scan_off;
+  a.scanned = h->scanned ? 1 : 0;
+  a.scan_done = h->d_scandone;
+  a.tiles_live_out = h->d_tiles_live;  // of a permuting rebuild
   a.slot_of = h->d_slot_of;
   a.dim = h->D;
   return a;
@@ -380,8 +390,14 @@ cil_status do_rebuild(cil_handle *h, bool carry_vel = false, bool exact = false,
     a.vel_in = h->d_vel;
     a.vel_out = h->d_vel2;
   }
-  launch_tiles(h->d_col, h->d_cnt, h->B, 0, h->d_tiles_used, h->stream);
+  // the events of the last step left the tile table over the used slots (k_events_due; a re-sort since
+  // then only drops slots, which the keys pass over)
+  if (h->need_exact || !h->due_events) {
+    launch_tiles(h->d_col, h->d_cnt, h->B, 0, h->d_tiles_used, h->stream);
+    h->launches += 1;
+  }
   launch_rebuild(a, h->grid_slots, h->stream);
+  h->launches += h->scanned ? 6 : 5;  // keys, scan (2 or 3), scatter, gather
   h->cur = 1 - h->cur;
   h->meta = 1 - h->meta;
   if (h->cfg.precision == CIL_PREC_MIXED) h->pu = 1 - h->pu;
@@ -403,6 +419,7 @@ cil_status do_cell_resort(cil_handle *h) {
   a.skin = nullptr;
   a.any_rebuild = nullptr;
   a.permute = 0;
+  a.tiles_live_out = nullptr;
   launch_tiles(h->d_col, h->d_cnt, h->B, 2, h->d_tiles_cell, h->stream);
   launch_cell_resort(a, h->grid_cells, h->stream);
   h->cur = 1 - h->cur;
@@ -495,6 +512,7 @@ EventArgs event_args(cil_handle *h) {
   a.dueq = h->d_dueq;
   a.ev_done = h->d_evdone;
   a.any_rebuild = h->d_anyreb;
+  a.tiles_used = h->skin_mode ? nullptr : h->d_tiles_used;
   a.dead = h->d_dead;
   a.divq = h->d_divq;
   if (h->d_obs) {
@@ -823,10 +841,11 @@ cil_status enqueue_step(cil_handle *h, bool last, bool timed, size_t e0) {
     if (st != CIL_OK) return st;
   }
   const bool philox = h->cfg.rng_mode != CIL_RNG_DSFMT;
-  // skin mode, Philox: one event kernel over the force kernel's due-cell queues, which also
-  // moves the step counter; otherwise a step-end launch (the step counter and, in Philox mode,
-  // the cell tile table) and the tile-wise event kernels
-  const bool due_events = philox && h->skin_mode;
+  // Philox: one event kernel over the force kernel's due-cell queues, which also moves the step
+  // counter; otherwise (the reference's draws, or crawling/dividing cells, whose divisions do not
+  // come from a cycle's end) a step-end launch (the step counter and, in Philox mode, the cell tile
+  // table) and the tile-wise event kernels
+  const bool due_events = h->due_events;
   if (!due_events) {
     launch_advance_ts(h->d_ts, h->d_anyreb, h->stream, h->d_cnt, h->B, philox ? h->d_tiles_cell : nullptr);
     h->launches += 1;
@@ -841,8 +860,8 @@ cil_status enqueue_step(cil_handle *h, bool last, bool timed, size_t e0) {
     launch_events_due(event_args(h), h->D, h->stream);
     h->launches += 1;
   } else {
-    launch_events_fast(event_args(h), h->grid_cells, h->D, h->stream, h->any_cell_sm);
-    h->launches += h->any_cell_sm ? 4 : 3;
+    launch_events_fast(event_args(h), h->grid_cells, h->D, h->stream);
+    h->launches += 4;
     if (h->any_swell) {
       launch_sm_swell_all(event_args(h), h->grid_cells, h->stream);
       h->launches += 1;
@@ -925,6 +944,7 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
     ra.any_rebuild = h->d_anyreb;
     ra.ts_dev = h->d_ts;
     ra.state_out = nullptr;
+    ra.tiles_live_out = nullptr;
     launch_rebuild(ra, h->grid_slots, rs);  // slot count unchanged: tile tables stay
     launch_skin_lists(skin_args(h, 0), h->D, h->cfg.force_law, h->grid_slots, rs);
     launch_list_flatten(skin_args(h, 0), h->grid_slots, rs);
@@ -949,11 +969,11 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
     }
     st = do_rebuild(h, false, false, vel_prev);
     if (st != CIL_OK) return st;
-    h->launches += 10;
     if (before_force) CUDA_TRY(h, cudaEventRecord(before_force, h->stream));
     ForceArgs fa = force_args(h, noise ? (oracle ? 2 : 1) : 0, 1, last ? h->d_vel : nullptr, nullptr);
     fa.heun = heun;
     fa.vel_prev = vel_prev;
+    fa.collect_due = (h->due_events && heun != 1) ? 1 : 0;  // the step's events read the due-cell queue
     launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, h->stiles, h->lane_bits, h->stream);
     h->launches += 1;
     h->cur = 1 - h->cur;
@@ -1359,11 +1379,10 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
     h->d_fresh = dalloc<int>(static_cast<size_t>(h->B) * kFreshCap);
     h->d_fnext = dalloc<unsigned long long>(SS);
     h->d_anyreb = dalloc<int>(4);
-    h->d_dueq = dalloc<int>(h->due_total);
     h->d_skin = dalloc<ColonySkin>(h->B);
     h->d_sched = dalloc<SchedState>(h->B);
     skin_ok = h->d_state[0] && h->d_state[1] && h->d_nbr && h->d_ncnt && h->d_uref && h->d_facc && h->d_ftouch &&
-              h->d_dueq && h->d_spart && h->d_lflat && h->d_oflat && h->d_lstart && h->d_lwarp &&
+              h->d_spart && h->d_lflat && h->d_oflat && h->d_lstart && h->d_lwarp &&
               h->d_fresh &&
               h->d_fnext && h->d_anyreb && h->d_skin && h->d_sched;
   }
@@ -1395,13 +1414,16 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
   h->d_tile_off = dalloc<int>(h->ctiles + 1);
   h->d_upchk = dalloc<int>(4);
   h->d_evdone = dalloc<int>(1);
+  h->d_scandone = dalloc<int>(1);
+  h->due_events = cfg->rng_mode != CIL_RNG_DSFMT && (h->skin_mode || !h->any_cell_sm);
+  if (h->due_events || h->skin_mode) h->d_dueq = dalloc<int>(h->due_total);
   h->d_dead = dalloc<int>(static_cast<size_t>(h->B) * kDeadCap);
   h->d_divq = dalloc<int>(static_cast<size_t>(h->CC));
   bool ok = h->d_col && h->d_cnt && h->d_x[0] && h->d_x[1] && h->d_eid[0] && h->d_eid[1] && h->d_sbin[0] &&
             h->d_sbin[1] && h->d_cyc[0] && h->d_cyc[1] && h->d_sigma_c && h->d_vel && h->d_key && h->d_perm &&
             h->d_slot_of && h->d_t0 && h->d_tsw && h->d_cst && h->d_smflag && h->d_tiles_used && h->d_tiles_live && h->d_tiles_cell &&
             h->d_tiles_pairs &&
-            h->d_tile_count && h->d_tile_off && h->d_upchk && h->d_evdone && h->d_dead && h->d_divq && h->d_ts &&
+            h->d_tile_count && h->d_tile_off && h->d_upchk && h->d_evdone && h->d_scandone && (h->d_dueq || !(h->due_events || h->skin_mode)) && h->d_dead && h->d_divq && h->d_ts &&
             (mixed ? (h->d_pk[0] && h->d_pk[1]) : (h->d_sig[0] && h->d_sig[1] && h->d_rec)) &&
             skin_ok;
   if (ok && cfg->rng_mode == CIL_RNG_DSFMT) {
@@ -1417,6 +1439,7 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
     return CIL_ERR_CUDA;
   }
   cudaMemsetAsync(h->d_evdone, 0, sizeof(int), h->stream);
+  cudaMemsetAsync(h->d_scandone, 0, sizeof(int), h->stream);
   // static parts of the colony table (bases, capacities, physics); the bin geometry is
   // filled in once every colony has been uploaded
   cudaMemcpyAsync(h->d_col, h->cc.data(), sizeof(ColonyConst) * h->B, cudaMemcpyHostToDevice, h->stream);

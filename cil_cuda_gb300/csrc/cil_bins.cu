@@ -6,10 +6,9 @@
 //   scan     per colony exclusive scan of the histogram -> range[b] = (first, end) slot
 //   scatter  one thread per element: claim a slot inside its bin (atomic countdown, which
 //            also returns the histogram to zero for the next rebuild)
-//   sort     one thread per bin: order the bin's entries by element id (deterministic
-//            result independent of the atomic order)
-//   gather   one thread per destination slot: copy position, diameter, id; update slot_of;
-//            write FP32 bin-local coordinates for the mixed-precision pair kernel
+//   gather   one thread per binned element: its rank by element id inside its bin (deterministic
+//            result independent of the atomic order) gives its slot; copy position, diameter, id;
+//            update slot_of; write FP32 bin-local coordinates for the mixed-precision pair kernel
 #include "cil_internal.cuh"
 
 namespace cil {
@@ -108,9 +107,9 @@ __global__ void __launch_bounds__(kTile) k_bin_keys(RebuildArgs a) {
     const int c = colony_of_tile(a.tiles_used, a.B, t);
     const ColonyConst &C = a.col[c];
     const int s = C.slot_base + (t - a.tiles_used[c]) * kTile + threadIdx.x;
-    if (s >= C.slot_base + a.cnt[c].nslot) continue;
-    int k = -1;
-    if (a.eid_in[s] >= 0) {
+    if (s >= C.slot_base + C.slot_cap) continue;
+    int k = -1;  // also for the rest of the last tile: the scatter takes whole tiles
+    if (s < C.slot_base + a.cnt[c].nslot && a.eid_in[s] >= 0) {
       int b[D];
       if (a.exact) {
         double x[D];
@@ -158,7 +157,7 @@ __global__ void __launch_bounds__(kTile) k_scan_partial(RebuildArgs a) {
   }
 }
 
-// one block per colony: exclusive scan of its scan-block sums; nlive = nslot = total
+// one block per colony with many scan blocks: exclusive scan of its scan-block sums
 __global__ void __launch_bounds__(kTile) k_scan_colony(RebuildArgs a) {
   if (no_rebuild(a)) return;
   const int c = blockIdx.x;
@@ -174,24 +173,32 @@ __global__ void __launch_bounds__(kTile) k_scan_colony(RebuildArgs a) {
     if (i < nsb) a.scan_off[C.scan_base + i] = carry + ex;
     carry += total;
   }
-  if (threadIdx.x == 0) {
-    a.cnt[c].nlive = carry;
-    if (a.permute) a.cnt[c].nslot = carry;
-  }
 }
 
-// per scan block: bin ranges
+// Per scan block: bin ranges. Without a.scanned the block adds the sums of its colony's scan blocks
+// before its own itself (a few loads per thread) instead of taking them from k_scan_colony: a launch
+// less (1.6-2 us of a step) against 4 bytes times half the square of the colony's scan blocks read
+// from L2. The last scan block of a colony has its total: nlive (and, re-sorting, nslot); the last
+// colony to have its total writes the tile table over the live slots (a.tiles_live_out).
 __global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
   if (no_rebuild(a)) return;
-  const int sb = blockIdx.x;
-  if (skip_colony(a, a.scan_col[sb])) return;
-  const ColonyConst &C = a.col[a.scan_col[sb]];
+  const int sb = blockIdx.x, c = a.scan_col[sb];
+  if (skip_colony(a, c)) return;
+  const ColonyConst &C = a.col[c];
   const int b0 = C.bin_base + (sb - C.scan_base) * kScanItems + threadIdx.x * 4;
   const int4 v = *reinterpret_cast<const int4 *>(a.bcount + b0);
   const int sum = v.x + v.y + v.z + v.w;
+  int before = 0;
+  if (a.scanned) {
+    before = a.scan_off[sb];
+  } else {
+    int part = 0;
+    for (int i = C.scan_base + static_cast<int>(threadIdx.x); i < sb; i += kTile) part += a.scan_sum[i];
+    block_excl_scan(part, &before);
+  }
   int total;
   const int ex = block_excl_scan(sum, &total);
-  int start = C.slot_base + a.scan_off[sb] + ex;
+  int start = C.slot_base + before + ex;
   int2 *r = a.range + b0;
   r[0] = make_int2(start, start + v.x);
   start += v.x;
@@ -200,6 +207,33 @@ __global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
   r[2] = make_int2(start, start + v.z);
   start += v.z;
   r[3] = make_int2(start, start + v.w);
+  if (sb != C.scan_base + C.nbins_pad / kScanItems - 1) return;  // uniform
+  __shared__ int s_last;
+  if (threadIdx.x == 0) {
+    a.cnt[c].nlive = before + total;
+    if (a.permute) a.cnt[c].nslot = before + total;
+    s_last = 0;
+    if (a.tiles_live_out) {
+      __threadfence();
+      s_last = atomicAdd(a.scan_done, 1) == a.B - 1 ? 1 : 0;
+    }
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  int carry = 0;
+  for (int base = 0; base < a.B; base += kTile) {
+    const int k = base + static_cast<int>(threadIdx.x);
+    const int nt = k < a.B ? (__ldcg(&a.cnt[k].nlive) + kTile - 1) / kTile : 0;
+    int tot;
+    const int e = block_excl_scan(nt, &tot);
+    if (k < a.B) a.tiles_live_out[k] = carry + e;
+    carry += tot;
+  }
+  if (threadIdx.x == 0) {
+    a.tiles_live_out[a.B] = carry;
+    *a.scan_done = 0;
+  }
 }
 
 __global__ void __launch_bounds__(kTile) k_scatter(RebuildArgs a) {
@@ -221,56 +255,24 @@ __global__ void __launch_bounds__(kTile) k_scatter(RebuildArgs a) {
   }
 }
 
-// Orders each bin's entries by element id. Bins hold a few elements: up to 8 are sorted in
-// registers (insertion into a register array, then one coalesced write-back); larger bins
-// fall back to an in-place insertion sort.
-__global__ void __launch_bounds__(kTile) k_sort_bins(RebuildArgs a, int nbins_total) {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nbins_total; b += gridDim.x * blockDim.x) {
-    const int2 r = a.range[b];
-    const int n = r.y - r.x;
-    if (n < 2) continue;
-    if (n <= 8) {
-      unsigned long long v[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = i < n ? a.perm[r.x + i] : ~0ull;
-#pragma unroll
-      for (int i = 1; i < 8; ++i)
-#pragma unroll
-        for (int k = i; k > 0; --k) {
-          const unsigned long long lo = v[k - 1] < v[k] ? v[k - 1] : v[k];
-          const unsigned long long hi = v[k - 1] < v[k] ? v[k] : v[k - 1];
-          v[k - 1] = lo;
-          v[k] = hi;
-        }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (i < n) a.perm[r.x + i] = v[i];
-    } else {
-      for (int i = r.x + 1; i < r.y; ++i) {
-        const unsigned long long v = a.perm[i];
-        int j = i - 1;
-        while (j >= r.x && a.perm[j] > v) {
-          a.perm[j + 1] = a.perm[j];
-          --j;
-        }
-        a.perm[j + 1] = v;
-      }
-    }
-  }
-}
-
+// The bins hold a few elements: each one's rank among the ids of its bin is a few loads next to its own
+// (a pass that sorted every bin first took 10 us of a step with 0.4M elements).
 template <int D>
 __global__ void __launch_bounds__(kTile) k_gather(RebuildArgs a) {
   const int total = a.tiles_live[a.B];
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int c = colony_of_tile(a.tiles_live, a.B, t);
     const ColonyConst &C = a.col[c];
-    const int dst = C.slot_base + (t - a.tiles_live[c]) * kTile + threadIdx.x;
-    if (dst >= C.slot_base + a.cnt[c].nlive) continue;
-    const unsigned long long v = a.perm[dst];
+    const int at = C.slot_base + (t - a.tiles_live[c]) * kTile + threadIdx.x;
+    if (at >= C.slot_base + a.cnt[c].nlive) continue;
+    const unsigned long long v = a.perm[at];
     const int src = static_cast<int>(v & 0xffffffffu);
     const int e = static_cast<int>(v >> 32);
     const int g = e >> 1;
+    const int bin = a.key[src];
+    const int2 r = a.range[bin];
+    int dst = r.x;
+    for (int k = r.x; k < r.y; ++k) dst += a.perm[k] < v ? 1 : 0;
     double x[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -284,11 +286,9 @@ __global__ void __launch_bounds__(kTile) k_gather(RebuildArgs a) {
     a.eid_out[dst] = e;
     a.slot_of[e] = dst;
     if (a.state_out) {
-      // skin mode: the new order is the bin order, so a bin's members are its own slots
       a.state_out[dst] = kSlotNormal;
-      a.perm[dst] = (static_cast<unsigned long long>(static_cast<uint32_t>(e)) << 32) | static_cast<uint32_t>(dst);
     }
-    const int nb = a.key[src] - C.bin_base;  // colony-local bin of the element
+    const int nb = bin - C.bin_base;  // colony-local bin of the element
     a.sbin_out[dst] = nb;
     if (a.exact) {
       a.cyc_out[dst] = make_int2(a.t0c[g], a.tswc[g]);
@@ -324,14 +324,15 @@ __global__ void __launch_bounds__(kTile) k_gather(RebuildArgs a) {
   }
 }
 
-// marks the slots past the used range as empty so that the scatter pass sees key -1
-__global__ void __launch_bounds__(kTile) k_clear_tail_keys(RebuildArgs a) {
-  const int c = blockIdx.y;
-  const ColonyConst &C = a.col[c];
-  const int used = a.cnt[c].nslot;
-  for (int i = used + blockIdx.x * blockDim.x + threadIdx.x; i < ((used + kTile - 1) / kTile) * kTile;
-       i += gridDim.x * blockDim.x)
-    if (i < C.slot_cap) a.key[C.slot_base + i] = -1;
+// skin mode, after a re-sort into bin order: a bin's members are its own slots
+__global__ void __launch_bounds__(kTile) k_own_slots(RebuildArgs a) {
+  const int total = a.tiles_live[a.B];
+  for (int t = blockIdx.x; t < total; t += gridDim.x) {
+    const int c = colony_of_tile(a.tiles_live, a.B, t);
+    const int s = a.col[c].slot_base + (t - a.tiles_live[c]) * kTile + threadIdx.x;
+    if (s < a.col[c].slot_base + a.cnt[c].nlive)
+      a.perm[s] = (static_cast<unsigned long long>(static_cast<uint32_t>(a.eid_out[s])) << 32) | static_cast<uint32_t>(s);
+  }
 }
 
 // ---------------------------------------------------------------- cell-major slot re-sort
@@ -469,28 +470,30 @@ void launch_tiles(const ColonyConst *, ColonyCounters *cnt, int B, int which, in
   k_tiles<<<1, kTile, 0, s>>>(cnt, B, which, tiles, which2, tiles2, per2);
 }
 
+static void launch_scan(const RebuildArgs &a, cudaStream_t s) {
+  k_scan_partial<<<a.nscan, kTile, 0, s>>>(a);
+  if (a.scanned) k_scan_colony<<<a.B, kTile, 0, s>>>(a);
+  k_scan_final<<<a.nscan, kTile, 0, s>>>(a);
+}
+
 void launch_rebuild(const RebuildArgs &a, int grid_slots, cudaStream_t s) {
   // keys + histogram over the used slots (tiles_used must be current); a non-permuting
   // rebuild (skin mode) gets its keys from the in-place rebin kernel instead
   if (a.permute) {
-    k_clear_tail_keys<<<dim3(1, a.B), kTile, 0, s>>>(a);
     if (a.dim == 2)
       k_bin_keys<2><<<grid_slots, kTile, 0, s>>>(a);
     else
       k_bin_keys<3><<<grid_slots, kTile, 0, s>>>(a);
   }
-  k_scan_partial<<<a.nscan, kTile, 0, s>>>(a);
-  k_scan_colony<<<a.B, kTile, 0, s>>>(a);
-  k_scan_final<<<a.nscan, kTile, 0, s>>>(a);
+  launch_scan(a, s);
   k_scatter<<<grid_slots, kTile, 0, s>>>(a);
   if (!a.permute) return;  // the bin index (range + perm) is all a list rebuild needs
-  if (a.skin == nullptr)   // bin order by element id: deterministic sums (FP64 / plain forms)
-    k_sort_bins<<<(a.nscan * kScanItems + kTile - 1) / kTile, kTile, 0, s>>>(a, a.nscan * kScanItems);
-  k_tiles<<<1, kTile, 0, s>>>(a.cnt, a.B, 1, const_cast<int *>(a.tiles_live), 0, nullptr, 2 * kTile);
+  // bin order by element id: deterministic sums (FP64 / plain forms)
   if (a.dim == 2)
     k_gather<2><<<grid_slots, kTile, 0, s>>>(a);
   else
     k_gather<3><<<grid_slots, kTile, 0, s>>>(a);
+  if (a.state_out) k_own_slots<<<grid_slots, kTile, 0, s>>>(a);
 }
 
 void launch_cell_resort(const RebuildArgs &a, int grid_cells, cudaStream_t s) {
@@ -498,9 +501,7 @@ void launch_cell_resort(const RebuildArgs &a, int grid_cells, cudaStream_t s) {
     k_cell_keys<2><<<grid_cells, kTile, 0, s>>>(a);
   else
     k_cell_keys<3><<<grid_cells, kTile, 0, s>>>(a);
-  k_scan_partial<<<a.nscan, kTile, 0, s>>>(a);
-  k_scan_colony<<<a.B, kTile, 0, s>>>(a);
-  k_scan_final<<<a.nscan, kTile, 0, s>>>(a);
+  launch_scan(a, s);
   k_cell_scatter<<<grid_cells, kTile, 0, s>>>(a);
   if (a.dim == 2)
     k_cell_gather<2><<<grid_cells, kTile, 0, s>>>(a);

@@ -365,17 +365,22 @@ __global__ void __launch_bounds__(kTile) k_div_rank(EventArgs a_) {
   }
 }
 
+// Cell src becomes cell dst. Every load before the first store: the compiler cannot move a load across a
+// store that may alias it, and each such pair would wait for memory in turn.
 __device__ void move_cell(const EventArgs &a, const ColonyConst &C, int dst, int src, int D) {
   const int gd = C.cell_base + dst, gs = C.cell_base + src;
-  a.t0[gd] = a.t0[gs];
-  a.tsw[gd] = a.tsw[gs];
-  a.cst[gd] = a.cst[gs];
-  a.sigma_c[2 * gd] = a.sigma_c[2 * gs];
-  a.sigma_c[2 * gd + 1] = a.sigma_c[2 * gs + 1];
+  const int t0 = a.t0[gs], tsw = a.tsw[gs], cst = a.cst[gs];
+  const double s0 = a.sigma_c[2 * gs], s1 = a.sigma_c[2 * gs + 1];
+  const int sl[2] = {a.slot_of[2 * gs], a.slot_of[2 * gs + 1]};
+  a.t0[gd] = t0;
+  a.tsw[gd] = tsw;
+  a.cst[gd] = cst;
+  a.sigma_c[2 * gd] = s0;
+  a.sigma_c[2 * gd + 1] = s1;
+#pragma unroll
   for (int j = 0; j < 2; ++j) {
-    const int sl = a.slot_of[2 * gs + j];
-    a.eid[sl] = 2 * gd + j;
-    a.slot_of[2 * gd + j] = sl;
+    a.eid[sl[j]] = 2 * gd + j;
+    a.slot_of[2 * gd + j] = sl[j];
   }
   if (a.obs_disp) {
     for (int d = 0; d < D; ++d) {
@@ -705,14 +710,16 @@ __device__ void block_bitonic_sort(int *v, int P) {
 constexpr int kDueSort = 2048;  // due cells sorted in shared memory (more: in the queue itself)
 constexpr int kDueRank = 512;   // up to this many: sorted by ranks instead of a sorting network
 
-// Skin mode, Philox: the step's events from the due-cell queues, one block per colony. The
-// force pass appended the cells whose cycle ends at this step (in no particular order); the
-// block sorts them by cell index, so the first ndiv_allowed in cell order divide (within the
-// colony's cell and slot room; the ranking of the tile-wise kernels), places the divisions
-// (one thread each: draws, FP64 placement of the four elements, new cycles; daughters take
-// cells n + rank and slots nslot + 2 rank), then the colony's apoptoses (apo_colony). The
-// kernel reads the step as *ts_dev + 1; the block that finishes last writes it back and
-// clears the next step's any-rebuild flag (in place of a step-counter launch).
+// Philox mode: the step's events from the due-cell queues, one block per colony. The force pass
+// appended the cells whose cycle ends at this step (in no particular order); the block sorts them by
+// cell index, so the first ndiv_allowed in cell order divide (within the colony's cell and slot room;
+// the ranking of the tile-wise kernels), places the divisions (one thread each: draws, FP64 placement
+// of the four elements, new cycles; daughters take cells n + rank and slots nslot + 2 rank), then the
+// colony's apoptoses (apo_colony). The kernel reads the step as *ts_dev + 1; the block that finishes
+// last writes it back (in place of a step-counter launch) and, in skin mode, clears the next step's
+// any-rebuild flag, otherwise writes the tile table over the used slots for the next step's keys.
+// In the forms without lists this replaced a step-counter, a counting, a ranking and a placing launch
+// (growth, 0.2M cells: 15.7 us a step and four gaps).
 template <int D>
 __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
   EventArgs a = a_;
@@ -798,16 +805,36 @@ __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
   }
   __syncthreads();
   apo_colony(a, c, D, true, s_k, s_vic[threadIdx.x & 31], s_kk);
+  __shared__ int s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
     // the last colony's block moves the step counter (every block has read it by then)
-    __threadfence();
-    if (atomicAdd(a.ev_done, 1) == a.B - 1) {
-      a.any_rebuild[a.ts & 1] = 0;
+    int last = 1;
+    if (a.B > 1) {
+      __threadfence();
+      last = atomicAdd(a.ev_done, 1) == a.B - 1 ? 1 : 0;
+      if (last) __threadfence();
+    }
+    if (last) {
+      if (a.any_rebuild) a.any_rebuild[a.ts & 1] = 0;
       *a.ts_dev = a.ts;
       *a.ev_done = 0;
     }
+    s_last = last;
   }
+  if (!a.tiles_used) return;  // uniform
+  __syncthreads();
+  if (!s_last) return;
+  int carry = 0;
+  for (int base = 0; base < a.B; base += kTile) {
+    const int k = base + static_cast<int>(threadIdx.x);
+    const int v = k < a.B ? (__ldcg(&a.cnt[k].nslot) + kTile - 1) / kTile : 0;
+    int total;
+    const int ex = block_excl_scan_ev(v, &total);
+    if (k < a.B) a.tiles_used[k] = carry + ex;
+    carry += total;
+  }
+  if (threadIdx.x == 0) a.tiles_used[a.B] = carry;
 }
 
 // oracle mode: divisions in the host's order with host-drawn axes and cycle lengths
@@ -1042,10 +1069,10 @@ void launch_advance_ts(int *ts_dev, int *any_rebuild, cudaStream_t s, const Colo
   k_step_end<<<1, kTile, 0, s>>>(ts_dev, any_rebuild, cnt, B, tiles_cell);
 }
 
-void launch_events_fast(const EventArgs &a, int grid_cells, int dim, cudaStream_t s, bool cell_states) {
+void launch_events_fast(const EventArgs &a, int grid_cells, int dim, cudaStream_t s) {
   k_div_count<<<grid_cells, kTile, 0, s>>>(a);
   k_div_rank<<<grid_cells, kTile, 0, s>>>(a);
-  if (cell_states) launch_sm_philox(a, grid_cells, s);
+  launch_sm_philox(a, grid_cells, s);
   if (dim == 2)
     k_events_exec<2><<<a.B, kTile, 0, s>>>(a);
   else

@@ -84,6 +84,20 @@ __device__ __forceinline__ bool pair_force_rsqrt(double r2, double si, double sj
 // isfinite by the exponent bits (no FP64 comparison)
 __device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
+// Forms without lists: back elements whose cell's cycle ends at the coming events (step ts + 1) put it
+// into the colony's due-cell queue, one atomic per warp. Whole warp.
+__device__ __forceinline__ void collect_due(const ForceArgs &a, const ColonyConst &C, int c, bool back, int s, int e) {
+  if (!a.collect_due || !C.divide) return;  // uniform
+  const bool due = back && a.cyc[s].y == a.ts + 1;
+  const unsigned dm = __ballot_sync(0xffffffffu, due);
+  if (!dm) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(dm) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(&a.cnt[c].ndue, __popc(dm));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (due) a.dueq[C.due_base + base + __popc(dm & ((1u << lane) - 1u))] = (e >> 1) - C.cell_base;
+}
+
 // The FP64 force pass: 2^lane_bits lanes per binned element, blocks of kF64Block threads.
 //
 // What bounds it is the FP64 pipe (2 lanes a clock per SM, 1/64 of FP32), so FP64 runs only for
@@ -141,6 +155,7 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
   }
   const double si = live ? a.sig[s] : 1.0;
   const int ps = live ? a.slot_of[e ^ 1] : -1;
+  collect_due(a, C, c, live && sub == 0 && j == 0, s, e);
 
   if (live && sub == 0) {
     // ---- intra-cell: linear spring to the partner + motility along back->front
@@ -628,6 +643,8 @@ __global__ void __launch_bounds__(kTile) k_force_mixed(ForceArgs a_) {
     const bool live = e >= 0;
     const int g = live ? (e >> 1) : -1;
     const int j = e & 1;
+
+    collect_due(a, C, c, live && j == 0, s, e);
 
     float ui[D], F[D];
     float si = 0.0f, w = 0.0f;

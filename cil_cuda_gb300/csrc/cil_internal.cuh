@@ -259,7 +259,7 @@ struct ColonyCounters {
   int ndiv_step;      // divisions this step
   int ndead;          // apoptoses recorded this step (list length, may exceed kDeadCap)
   int ndiv_allowed;   // divisions that fit the capacity this step
-  int ndue;           // skin mode, Philox: cells due to divide at the coming events (force kernel)
+  int ndue;           // Philox: cells due to divide at the coming events (force kernel)
   long long ndiv_total;
   long long napo_total;
 };
@@ -646,6 +646,9 @@ struct RebuildArgs {
   unsigned long long *perm;
   int *scan_sum;
   int *scan_off;
+  int scanned;             // scan_off comes from k_scan_colony (colonies with many scan blocks)
+  int *scan_done;          // colonies whose total is known, of the scan under way
+  int *tiles_live_out;     // tiles_live, written by the scan; null: not wanted
   int *slot_of;
   const double *vel_in;    // optional: carry velocities through the permutation
   double *vel_out;
@@ -698,7 +701,7 @@ struct ForceArgs {
   int noise_mode;          // 0 none, 1 philox, 2 uploaded
   int integrate;
   int heun;                // 0 Euler step; 1, 2: first, second half step of a Heun step
-  // skin mode, Philox, the step's last force pass: cells due to divide at step ts + 1 are
+  // Philox, the step's last force pass: cells due to divide at step ts + 1 are
   // appended to the colony's due-cell queue (dueq + col[c].due_base, count cnt[c].ndue)
   int collect_due;
   int *dueq;
@@ -738,11 +741,12 @@ struct EventArgs {
   unsigned char *smflag;   // per cell: the division criterion is met (oracle mode, state machine)
   int *tile_count;
   int *tile_off;
-  // skin mode, Philox: the cells due to divide, appended by the force kernel (colony c's at
+  int *tiles_used;         // forms without lists: the next step's tile table over the used slots, or null
+  // Philox: the cells due to divide, appended by the force kernel (colony c's at
   // dueq + col[c].due_base, count cnt[c].ndue), and the event kernel's finished-colony count
   int *dueq;
   int *ev_done;
-  int *any_rebuild;        // the any-rebuild flags (the next step's is cleared)
+  int *any_rebuild;        // skin mode: the any-rebuild flags (the next step's is cleared)
   int *dead;               // [B * kDeadCap]
   int *divq;               // [CC] per colony: the cells dividing this step, in rank order
   double *obs_com_prev;    // [D * CC] or null
@@ -871,7 +875,7 @@ void launch_fresh_pairs(const SkinArgs &a, int dim, int law, cudaStream_t s);
 void launch_advance_ts(int *ts_dev, int *any_rebuild, cudaStream_t s, const ColonyCounters *cnt = nullptr, int B = 0,
                        int *tiles_cell = nullptr);
 int mlp_param_count();
-void launch_events_fast(const EventArgs &a, int grid_cells, int dim, cudaStream_t s, bool cell_states);
+void launch_events_fast(const EventArgs &a, int grid_cells, int dim, cudaStream_t s);
 void launch_events_due(const EventArgs &a, int dim, cudaStream_t s);
 void launch_divisions_list(const EventArgs &a, int colony, int n0, int ndiv, const int *mothers,
                            const double *dirs, const int *spans, int dim, cudaStream_t s);
