@@ -70,7 +70,6 @@ struct cil_handle {
   int ctiles = 0;      // max cell tiles
   int grid_slots = 0;  // persistent grid for slot kernels
   int grid_cells = 0;
-  int grid_force = 0;
   int stiles = 0;      // tiles over the slot capacity
   int ptiles = 0;      // tiles over the slot pairs of the capacity (grid of the list force kernel)
   int cell_block = 256;  // threads (cells) per block of the list force kernel
@@ -974,7 +973,7 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
     fa.heun = heun;
     fa.vel_prev = vel_prev;
     fa.collect_due = (h->due_events && heun != 1) ? 1 : 0;  // the step's events read the due-cell queue
-    launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, h->stiles, h->lane_bits, h->stream);
+    launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->stiles, h->lane_bits, h->stream);
     h->launches += 1;
     h->cur = 1 - h->cur;
     if (h->cfg.precision == CIL_PREC_MIXED) h->pu = 1 - h->pu;
@@ -1474,7 +1473,6 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
   }
   h->grid_slots = std::max(1, std::min(h->nsm * 8, static_cast<int>((SS + kTile - 1) / kTile)));
   h->grid_cells = std::max(1, std::min(h->nsm * 8, h->ctiles));
-  h->grid_force = h->grid_slots;
   {
     // the upload and download staging, sized for the largest colony here rather than at the
     // first upload (an allocation would otherwise sit inside the first cil_upload)
@@ -1677,7 +1675,7 @@ cil_status cil_forces(cil_handle *h, int32_t colony, double *frc) {
   if (st != CIL_OK) return st;
   ForceArgs fa = force_args(h, noise ? (oracle ? 2 : 1) : 0, 0, nullptr, h->d_frc);
   set_lane_bits(h);
-  launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->grid_force, h->stiles, h->lane_bits, h->stream);
+  launch_force(fa, h->D, h->cfg.force_law, h->cfg.precision, h->stiles, h->lane_bits, h->stream);
   std::vector<ColonyCounters> k;
   st = check_counters(h, &k);
   if (st != CIL_OK && st != CIL_ERR_NAN) return st;

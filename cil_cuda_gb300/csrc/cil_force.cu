@@ -22,23 +22,6 @@ namespace cil {
 
 namespace {
 
-template <int D>
-__device__ __forceinline__ bool neighbor_bin_i(const ColonyConst &C, const int *bi, const int *o, int *nb) {
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    int v = bi[d] + o[d];
-    if (v < 0) {
-      if (!C.periodic[d]) return false;
-      v += C.ns[d];
-    } else if (v >= C.ns[d]) {
-      if (!C.periodic[d]) return false;
-      v -= C.ns[d];
-    }
-    nb[d] = v;
-  }
-  return true;
-}
-
 // nint(v / L) (Utils.hpp:173-175) without a division when |v| < L / 4, where v / L lies in
 // (-0.25, 0.25) whatever its rounding: a minimum image leaves v as it is then.
 __device__ __forceinline__ double min_image(double v, double L) {
@@ -610,226 +593,138 @@ __device__ __forceinline__ void mixed_integrate(const ForceArgs &a, const Colony
   }
 }
 
-// Mixed-precision step without lists, one CTA per tile of kTile consecutive binned elements:
-//  1. each thread: its element's intra-cell, wall and noise force (FP32) and the ranges of
-//     its 3^d neighbour bins, staged in shared memory with the candidate count;
-//  2. a block scan turns the counts into one list of (element, candidate) pairs and every
-//     thread evaluates an equal contiguous chunk of it, so lanes stay converged whatever
-//     the bin occupancies; partial sums are added into the element's shared accumulator;
-//  3. each thread adds its element's pair force and integrates.
+// Mixed-precision step without lists, one thread per binned element: its intra-cell, wall and noise
+// force, then the pair forces over the rows of bins around it, summed in slot order, then the update.
+// The three bins of a row along the last axis hold consecutive slots, so a row is one range of records
+// (kMixedAhead in flight) that the warp's elements, neighbours in bin order, share in L1; which of the
+// three bins a candidate is in follows from its slot. The law is branch-free and costs about what the
+// record's load does, so candidates out of range are evaluated and masked, and the cell's own two
+// elements are told by their slots. 0.4M elements of the 2D growth colony: 26 us; staging the bin
+// ranges in shared memory and sharing out a block's candidates evenly (element ids loaded per
+// candidate, partial sums by shared atomics) took 49.6 us.
+constexpr int kMixedAhead = 4;
+
 template <int D, int LAW>
-__global__ void __launch_bounds__(kTile) k_force_mixed(ForceArgs a_) {
+__global__ void __launch_bounds__(kTile, 4) k_force_mixed(ForceArgs a_) {
   ForceArgs a = a_;
   a.ts = *a_.ts_dev;
-  constexpr int NB = (D == 2) ? 9 : 27;
-  extern __shared__ int smem[];
-  int *s_start = smem;                       // [NB][kTile]
-  int *s_cnt = s_start + NB * kTile;         // [NB][kTile]
-  int *s_off = s_cnt + NB * kTile;           // [kTile + 1]
-  int *s_g = s_off + kTile + 1;              // [kTile]
-  float *s_u = reinterpret_cast<float *>(s_g + kTile);  // [D][kTile]
-  float *s_si = s_u + D * kTile;             // [kTile]
-  float *s_F = s_si + kTile;                 // [D][kTile]
-  __shared__ int s_total;
-
-  const int tid = threadIdx.x;
-  const int total = a.tiles_live[a.B];
-  for (int t = blockIdx.x; t < total; t += gridDim.x) {
-    const int c = colony_of_tile(a.tiles_live, a.B, t);
-    const ColonyConst &C = a.col[c];
-    const int s = C.slot_base + (t - a.tiles_live[c]) * kTile + tid;
-    const int nlive = a.cnt[c].nlive;
-    const int e = s < C.slot_base + nlive ? a.eid[s] : -1;
-    const bool live = e >= 0;
-    const int g = live ? (e >> 1) : -1;
-    const int j = e & 1;
-
-    collect_due(a, C, c, live && j == 0, s, e);
-
-    float ui[D], F[D];
-    float si = 0.0f, w = 0.0f;
-    int bi[D];
+  const int t = blockIdx.x;
+  if (t >= a.tiles_live[a.B]) return;  // uniform per block
+  const int c = colony_of_tile(a.tiles_live, a.B, t);
+  const ColonyConst &C = a.col[c];
+  const int s = C.slot_base + (t - a.tiles_live[c]) * kTile + static_cast<int>(threadIdx.x);
+  const int nlive = a.cnt[c].nlive;
+  const int e = s < C.slot_base + nlive ? a.eid[s] : -1;
+  const bool live = e >= 0;
+  const int j = e & 1;
+  collect_due(a, C, c, live && j == 0, s, e);
+  if (!live) return;
+  const float4 pi = a.pk[s];
+  float ui[D], F[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      ui[d] = 0.0f;
-      F[d] = 0.0f;
-      bi[d] = 0;
+  for (int d = 0; d < D; ++d) ui[d] = pk_c(pi, d);
+  const float si = fabsf(pi.w);
+  int bi[D];
+  bin_decode<D>(C, a.sbin[s], bi);
+  mixed_own_forces<D>(a, C, s, e, ui, bi, si, F);
+  const float eps = C.eps_f, rcs = C.rcs_f;
+  if (C.single_bin) {
+    // one bin only (tiny boxes): every element, FP32 minimum image
+    const int g = e >> 1;
+    for (int tt = C.slot_base; tt < C.slot_base + nlive; ++tt) {
+      const int ej = a.eid[tt];
+      const float4 pj = a.pk[tt];
+      float dx[D];
+      float r2 = 0.0f;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        float v = pk_c(pj, d) - ui[d];
+        if (C.periodic[d]) v -= rintf(v * C.inv_bwf[d]) * C.bwf[d];
+        dx[d] = v;
+        r2 += v * v;
+      }
+      const float f0 = pair_f0_fast<LAW>(r2, si, pj.w, eps, rcs, ej >= 0 && (ej >> 1) != g, C.well_eps_f, C.well_sigma_f, C.force_shifted);
+#pragma unroll
+      for (int d = 0; d < D; ++d) F[d] += f0 * dx[d];
     }
-    int ncand = 0;
-    if (live) {
-      const float4 pi = a.pk[s];
+  } else {
+    const int ps = a.slot_of[e ^ 1];
+    float acc[D];
 #pragma unroll
-      for (int d = 0; d < D; ++d) ui[d] = pk_c(pi, d);
-      w = pi.w;
-      si = fabsf(w);
-      bin_decode<D>(C, a.sbin[s], bi);
-      mixed_own_forces<D>(a, C, s, e, ui, bi, si, F);
-      // ---- neighbour bin ranges
-      if (!C.single_bin) {
+    for (int d = 0; d < D; ++d) acc[d] = 0.0f;
+    constexpr int NROW = D == 2 ? 3 : 9;
+    const int last = bi[D - 1], nl = C.ns[D - 1];
+    const bool inner = last > 0 && last < nl - 1;
+    const float bwl = C.bwf[D - 1];
+    for (int row = 0; row < NROW; ++row) {
+      const int oo[3] = {(D == 2 ? row : row / 3) - 1, (D == 2 ? 0 : row % 3) - 1, 0};
+      int rowbin = 0;
+      bool ok = true;
+      float ofs[D];  // the row's bin origins relative to the element
 #pragma unroll
-        for (int o = 0; o < NB; ++o) {
-          int off[3] = {o / (D == 2 ? 3 : 9) - 1, (D == 2 ? o % 3 : (o / 3) % 3) - 1, (D == 2 ? 0 : o % 3 - 1)};
-          int nb[D];
-          int st = 0, n = 0;
-          if (neighbor_bin_i<D>(C, bi, off, nb)) {
-            const int2 r = a.range[C.bin_base + bin_id<D>(C, nb)];
-            st = r.x;
-            n = r.y - r.x;
+      for (int d = 0; d < D - 1; ++d) {
+        int v = bi[d] + oo[d];
+        if (v < 0) {
+          ok = ok && C.periodic[d];
+          v += C.ns[d];
+        } else if (v >= C.ns[d]) {
+          ok = ok && C.periodic[d];
+          v -= C.ns[d];
+        }
+        rowbin = rowbin * C.ns[d] + v;
+        ofs[d] = static_cast<float>(oo[d]) * C.bwf[d] - ui[d];
+      }
+      ofs[D - 1] = -ui[D - 1];
+      if (!ok) continue;
+      const int2 *rng = a.range + C.bin_base + rowbin * nl;
+      for (int piece = 0; piece < (inner ? 1 : 3); ++piece) {
+        // [st, en) with the bins' bounds: below m0 the bin before the element's, from m1 on the one after
+        int st, en, m0, m1;
+        if (inner) {
+          const int2 r0 = rng[last - 1], r1 = rng[last + 1];
+          st = r0.x;
+          m0 = r0.y;
+          m1 = r1.x;
+          en = r1.y;
+        } else {
+          int v = last + piece - 1;
+          if (v < 0 || v >= nl) {
+            if (!C.periodic[D - 1]) continue;
+            v += v < 0 ? nl : -nl;
           }
-          s_start[o * kTile + tid] = st;
-          s_cnt[o * kTile + tid] = n;
-          ncand += n;
+          const int2 r = rng[v];
+          st = r.x;
+          en = r.y;
+          m0 = piece == 0 ? en : st;
+          m1 = piece == 2 ? st : en;
         }
-      }
-    }
-    if (!live || C.single_bin) {
+        for (int t0 = st; t0 < en; t0 += kMixedAhead) {
+          float4 pj[kMixedAhead];
 #pragma unroll
-      for (int o = 0; o < NB; ++o) s_cnt[o * kTile + tid] = 0;
-    }
+          for (int u = 0; u < kMixedAhead; ++u) pj[u] = __ldg(a.pk + min(t0 + u, en - 1));
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      s_u[d * kTile + tid] = ui[d];
-      s_F[d * kTile + tid] = 0.0f;
-    }
-    s_si[tid] = si;
-    s_g[tid] = g;
-    // ---- pair list offsets
-    {
-      const int lane = tid & 31, wid = tid >> 5;
-      int inc = ncand;
+          for (int u = 0; u < kMixedAhead; ++u) {
+            const int tt = t0 + u;
+            const float ol = ofs[D - 1] + (tt < m0 ? -bwl : (tt >= m1 ? bwl : 0.0f));
+            float dx[D];
+            float r2 = 0.0f;
 #pragma unroll
-      for (int q = 1; q < 32; q <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, inc, q);
-        if (lane >= q) inc += v;
-      }
-      __shared__ int ws[kTile / 32];
-      if (lane == 31) ws[wid] = inc;
-      __syncthreads();
-      if (wid == 0) {
-        int wv = lane < kTile / 32 ? ws[lane] : 0;
-#pragma unroll
-        for (int q = 1; q < 32; q <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, wv, q);
-          if (lane >= q) wv += v;
-        }
-        if (lane < kTile / 32) ws[lane] = wv;
-        if (lane == kTile / 32 - 1) s_total = wv;
-      }
-      __syncthreads();
-      s_off[tid] = (wid > 0 ? ws[wid - 1] : 0) + inc - ncand;
-      __syncthreads();
-    }
-    // ---- pair chunk of this thread
-    const int npairs = s_total;
-    const float eps = C.eps_f, rcs = C.rcs_f;
-    if (npairs > 0) {
-      const int q = (npairs + kTile - 1) / kTile;
-      int p = tid * q;
-      const int p1 = min(p + q, npairs);
-      if (p < p1) {
-        // home element: largest i with s_off[i] <= p
-        int lo = 0, hi = kTile - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (s_off[mid] <= p)
-            lo = mid;
-          else
-            hi = mid - 1;
-        }
-        int i = lo;
-        int k = p - s_off[i];
-        int o = 0;
-        while (k >= s_cnt[o * kTile + i]) {
-          k -= s_cnt[o * kTile + i];
-          ++o;
-        }
-        int tt = s_start[o * kTile + i] + k;
-        int rem = s_cnt[o * kTile + i] - k;
-        float uh[D], offv[D], acc[D];
-        float sh = s_si[i];
-        int gh = s_g[i];
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          uh[d] = s_u[d * kTile + i];
-          acc[d] = 0.0f;
-        }
-        auto set_off = [&](int oo) {
-          const int o0 = oo / (D == 2 ? 3 : 9) - 1;
-          const int o1 = (D == 2 ? oo % 3 : (oo / 3) % 3) - 1;
-          offv[0] = static_cast<float>(o0) * C.bwf[0] - uh[0];
-          offv[1] = static_cast<float>(o1) * C.bwf[1] - uh[1];
-          if (D == 3) offv[D - 1] = static_cast<float>(oo % 3 - 1) * C.bwf[D - 1] - uh[D - 1];
-        };
-        set_off(o);
-        for (;;) {
-          const int ej = __ldg(a.eid + tt);
-          const float4 pj = __ldg(a.pk + tt);
-          float dx[D];
-          float r2 = 0.0f;
-#pragma unroll
-          for (int d = 0; d < D; ++d) {
-            dx[d] = pk_c(pj, d) + offv[d];
-            r2 += dx[d] * dx[d];
-          }
-          const float f0 = pair_f0_fast<LAW>(r2, sh, pj.w, eps, rcs, ej >= 0 && (ej >> 1) != gh, C.well_eps_f, C.well_sigma_f, C.force_shifted);
-#pragma unroll
-          for (int d = 0; d < D; ++d) acc[d] += f0 * dx[d];
-          if (++p >= p1) break;
-          ++tt;
-          --rem;
-          while (rem == 0) {
-            if (++o == NB) {
-#pragma unroll
-              for (int d = 0; d < D; ++d) {
-                atomicAdd(&s_F[d * kTile + i], acc[d]);
-                acc[d] = 0.0f;
-              }
-              ++i;
-              o = 0;
-              sh = s_si[i];
-              gh = s_g[i];
-#pragma unroll
-              for (int d = 0; d < D; ++d) uh[d] = s_u[d * kTile + i];
+            for (int d = 0; d < D; ++d) {
+              dx[d] = pk_c(pj[u], d) + (d == D - 1 ? ol : ofs[d]);
+              r2 += dx[d] * dx[d];
             }
-            rem = s_cnt[o * kTile + i];
-            tt = s_start[o * kTile + i];
-            if (rem) set_off(o);
+            const float f0 = pair_f0_fast<LAW>(r2, si, pj[u].w, eps, rcs, tt < en && tt != s && tt != ps, C.well_eps_f, C.well_sigma_f, C.force_shifted);
+#pragma unroll
+            for (int d = 0; d < D; ++d) acc[d] += f0 * dx[d];
           }
         }
-#pragma unroll
-        for (int d = 0; d < D; ++d) atomicAdd(&s_F[d * kTile + i], acc[d]);
       }
     }
-    __syncthreads();
-
-    if (live) {
-      if (C.single_bin) {
-        // one bin only (tiny boxes): every element, FP32 minimum image
-        for (int tt = C.slot_base; tt < C.slot_base + nlive; ++tt) {
-          const int ej = a.eid[tt];
-          const float4 pj = a.pk[tt];
-          float dx[D];
-          float r2 = 0.0f;
 #pragma unroll
-          for (int d = 0; d < D; ++d) {
-            float v = pk_c(pj, d) - ui[d];
-            if (C.periodic[d]) v -= rintf(v * C.inv_bwf[d]) * C.bwf[d];
-            dx[d] = v;
-            r2 += v * v;
-          }
-          const float f0 = pair_f0_fast<LAW>(r2, si, pj.w, eps, rcs, ej >= 0 && (ej >> 1) != g, C.well_eps_f, C.well_sigma_f, C.force_shifted);
-#pragma unroll
-          for (int d = 0; d < D; ++d) F[d] += f0 * dx[d];
-        }
-      } else {
-#pragma unroll
-        for (int d = 0; d < D; ++d) F[d] += s_F[d * kTile + tid];
-      }
-      float dstep[D];
-      mixed_integrate<D>(a, C, c, s, j, ui, w, F, dstep);
-    }
-    __syncthreads();
+    for (int d = 0; d < D; ++d) F[d] += acc[d];
   }
+  float dstep[D];
+  mixed_integrate<D>(a, C, c, s, j, ui, pi.w, F, dstep);
 }
 
 // Asynchronous global -> shared copies (cp.async, sm_80 and later): issued early, waited for
@@ -1398,13 +1293,8 @@ void launch_list_d(const ForceArgs &a, int law, int grid, int variant, int block
   }
 }
 
-template <int D>
-constexpr size_t mixed_smem_bytes() {
-  return sizeof(int) * ((D == 2 ? 9 : 27) * kTile * 2 + kTile + 1 + kTile) + sizeof(float) * (2 * D * kTile + kTile);
-}
-
 template <int D, int LAW>
-void launch_dl(const ForceArgs &a, int prec, int grid, int tiles, int lane_bits, cudaStream_t s) {
+void launch_dl(const ForceArgs &a, int prec, int tiles, int lane_bits, cudaStream_t s) {
   if (prec == CIL_PREC_FP64) {
     constexpr int bytes = kF64Block / 32 * static_cast<int>(sizeof(F64Warp<D>));
     static bool attr_set = false;  // per instantiation; the attribute is per function
@@ -1414,31 +1304,24 @@ void launch_dl(const ForceArgs &a, int prec, int grid, int tiles, int lane_bits,
     }
     k_force_fp64<D, LAW><<<tiles * (2 << lane_bits), kF64Block, bytes, s>>>(a, lane_bits);
   } else {
-    constexpr size_t bytes = mixed_smem_bytes<D>();
-    static bool attr_set = false;  // per instantiation; the attribute is per function
-    if (!attr_set) {
-      cudaFuncSetAttribute(k_force_mixed<D, LAW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(bytes));
-      attr_set = true;
-    }
-    k_force_mixed<D, LAW><<<grid, kTile, bytes, s>>>(a);
+    k_force_mixed<D, LAW><<<tiles, kTile, 0, s>>>(a);
   }
 }
 
 template <int D>
-void launch_d(const ForceArgs &a, int law, int prec, int grid, int tiles, int lane_bits, cudaStream_t s) {
+void launch_d(const ForceArgs &a, int law, int prec, int tiles, int lane_bits, cudaStream_t s) {
   switch (law) {
     case CIL_FORCE_LJ_WCA:
-      launch_dl<D, CIL_FORCE_LJ_WCA>(a, prec, grid, tiles, lane_bits, s);
+      launch_dl<D, CIL_FORCE_LJ_WCA>(a, prec, tiles, lane_bits, s);
       break;
     case CIL_FORCE_SOFTCORE:
-      launch_dl<D, CIL_FORCE_SOFTCORE>(a, prec, grid, tiles, lane_bits, s);
+      launch_dl<D, CIL_FORCE_SOFTCORE>(a, prec, tiles, lane_bits, s);
       break;
     case CIL_FORCE_SC:
-      launch_dl<D, CIL_FORCE_SC>(a, prec, grid, tiles, lane_bits, s);
+      launch_dl<D, CIL_FORCE_SC>(a, prec, tiles, lane_bits, s);
       break;
     default:
-      launch_dl<D, CIL_FORCE_HERTZ>(a, prec, grid, tiles, lane_bits, s);
+      launch_dl<D, CIL_FORCE_HERTZ>(a, prec, tiles, lane_bits, s);
       break;
   }
 }
@@ -1452,12 +1335,12 @@ void launch_force_list_3d(const ForceArgs &a, int law, int grid, int variant, in
   launch_list_d<3>(a, law, grid, variant, block, s);
 }
 
-void launch_force_3d(const ForceArgs &a, int law, int prec, int grid, int tiles, int lane_bits, cudaStream_t s) {
-  launch_d<3>(a, law, prec, grid, tiles, lane_bits, s);
+void launch_force_3d(const ForceArgs &a, int law, int prec, int tiles, int lane_bits, cudaStream_t s) {
+  launch_d<3>(a, law, prec, tiles, lane_bits, s);
 }
 #else
 void launch_force_list_3d(const ForceArgs &a, int law, int grid, int variant, int block, cudaStream_t s);
-void launch_force_3d(const ForceArgs &a, int law, int prec, int grid, int tiles, int lane_bits, cudaStream_t s);
+void launch_force_3d(const ForceArgs &a, int law, int prec, int tiles, int lane_bits, cudaStream_t s);
 
 void launch_force_list(const ForceArgs &a, int dim, int law, int grid, int variant, int block, cudaStream_t s) {
   if (dim == 2)
@@ -1466,12 +1349,12 @@ void launch_force_list(const ForceArgs &a, int dim, int law, int grid, int varia
     launch_force_list_3d(a, law, grid, variant, block, s);
 }
 
-void launch_force(const ForceArgs &a, int dim, int law, int prec, int grid, int tiles, int lane_bits,
+void launch_force(const ForceArgs &a, int dim, int law, int prec, int tiles, int lane_bits,
                   cudaStream_t s) {
   if (dim == 2)
-    launch_d<2>(a, law, prec, grid, tiles, lane_bits, s);
+    launch_d<2>(a, law, prec, tiles, lane_bits, s);
   else
-    launch_force_3d(a, law, prec, grid, tiles, lane_bits, s);
+    launch_force_3d(a, law, prec, tiles, lane_bits, s);
 }
 #endif
 

@@ -860,7 +860,7 @@ void launch_rebuild(const RebuildArgs &a, int grid_slots, cudaStream_t s);
 // current; leaves bcount at zero and nslot = 2 ncell
 void launch_cell_resort(const RebuildArgs &a, int grid_cells, cudaStream_t s);
 // tiles: tiles of kTile slots over the capacity; lane_bits: log2 of the lanes per element (FP64 form)
-void launch_force(const ForceArgs &a, int dim, int law, int prec, int grid, int tiles, int lane_bits,
+void launch_force(const ForceArgs &a, int dim, int law, int prec, int tiles, int lane_bits,
                   cudaStream_t s);
 // skin mode: the cell kernel (one thread per slot pair); block = cells per block (128, 256, 512);
 // a.tiles must be the pair tiles of that block size
