@@ -344,6 +344,7 @@ RebuildArgs rebuild_args(cil_handle *h) {
   a.rec_out = h->d_rec;
   a.pk_in = mixed ? h->d_pk[h->pu] : nullptr;
   a.skin = nullptr;  // a permuting rebuild re-sorts every colony
+  a.dep = (h->cfg.flags & CIL_FLAG_REBUILD_NODE) == 0;
   a.permute = 1;
   a.state_out = h->skin_mode ? h->d_state[1 - h->meta] : nullptr;
   a.sbin_in = h->d_sbin[h->meta];
@@ -564,6 +565,7 @@ SkinArgs skin_args(cil_handle *h, int force_rebuild) {
   a.skin_min = h->sched_skin_min;
   a.skin_max = static_cast<float>(h->cfg.skin);
   a.interval_scale = h->sched_interval_scale;
+  a.dep = (h->cfg.flags & CIL_FLAG_REBUILD_NODE) == 0;
   a.grid = h->nsm * 16;  // fresh-pair kernel: 64 warps per SM over all colonies' fresh elements
   return a;
 }

@@ -102,6 +102,7 @@ __device__ __forceinline__ void fast_bin(const ColonyConst &C, int home, const f
 
 template <int D>
 __global__ void __launch_bounds__(kTile) k_bin_keys(RebuildArgs a) {
+  enter_step_kernel();
   const int total = a.tiles_used[a.B];
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int c = colony_of_tile(a.tiles_used, a.B, t);
@@ -138,6 +139,7 @@ __device__ __forceinline__ bool no_rebuild(const RebuildArgs &a) {
 }
 
 __global__ void __launch_bounds__(kTile) k_scan_partial(RebuildArgs a) {
+  enter_step_kernel();
   if (no_rebuild(a)) return;
   const int sb = blockIdx.x;
   if (skip_colony(a, a.scan_col[sb])) return;
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(kTile) k_scan_partial(RebuildArgs a) {
 
 // one block per colony with many scan blocks: exclusive scan of its scan-block sums
 __global__ void __launch_bounds__(kTile) k_scan_colony(RebuildArgs a) {
+  enter_step_kernel();
   if (no_rebuild(a)) return;
   const int c = blockIdx.x;
   if (skip_colony(a, c)) return;
@@ -181,6 +184,7 @@ __global__ void __launch_bounds__(kTile) k_scan_colony(RebuildArgs a) {
 // from L2. The last scan block of a colony has its total: nlive (and, re-sorting, nslot); the last
 // colony to have its total writes the tile table over the live slots (a.tiles_live_out).
 __global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
+  enter_step_kernel();
   if (no_rebuild(a)) return;
   const int sb = blockIdx.x, c = a.scan_col[sb];
   if (skip_colony(a, c)) return;
@@ -237,6 +241,7 @@ __global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
 }
 
 __global__ void __launch_bounds__(kTile) k_scatter(RebuildArgs a) {
+  enter_step_kernel();
   if (no_rebuild(a)) return;
   const int total = a.tiles_used[a.B];
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
@@ -259,6 +264,7 @@ __global__ void __launch_bounds__(kTile) k_scatter(RebuildArgs a) {
 // (a pass that sorted every bin first took 10 us of a step with 0.4M elements).
 template <int D>
 __global__ void __launch_bounds__(kTile) k_gather(RebuildArgs a) {
+  enter_step_kernel();
   const int total = a.tiles_live[a.B];
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int c = colony_of_tile(a.tiles_live, a.B, t);
@@ -326,6 +332,7 @@ __global__ void __launch_bounds__(kTile) k_gather(RebuildArgs a) {
 
 // skin mode, after a re-sort into bin order: a bin's members are its own slots
 __global__ void __launch_bounds__(kTile) k_own_slots(RebuildArgs a) {
+  enter_step_kernel();
   const int total = a.tiles_live[a.B];
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int c = colony_of_tile(a.tiles_live, a.B, t);
@@ -471,9 +478,9 @@ void launch_tiles(const ColonyConst *, ColonyCounters *cnt, int B, int which, in
 }
 
 static void launch_scan(const RebuildArgs &a, cudaStream_t s) {
-  k_scan_partial<<<a.nscan, kTile, 0, s>>>(a);
-  if (a.scanned) k_scan_colony<<<a.B, kTile, 0, s>>>(a);
-  k_scan_final<<<a.nscan, kTile, 0, s>>>(a);
+  launch_step(a.dep, a.nscan, kTile, 0, s, k_scan_partial, a);
+  if (a.scanned) launch_step(a.dep, a.B, kTile, 0, s, k_scan_colony, a);
+  launch_step(a.dep, a.nscan, kTile, 0, s, k_scan_final, a);
 }
 
 void launch_rebuild(const RebuildArgs &a, int grid_slots, cudaStream_t s) {
@@ -481,19 +488,19 @@ void launch_rebuild(const RebuildArgs &a, int grid_slots, cudaStream_t s) {
   // rebuild (skin mode) gets its keys from the in-place rebin kernel instead
   if (a.permute) {
     if (a.dim == 2)
-      k_bin_keys<2><<<grid_slots, kTile, 0, s>>>(a);
+      launch_step(a.dep, grid_slots, kTile, 0, s, k_bin_keys<2>, a);
     else
-      k_bin_keys<3><<<grid_slots, kTile, 0, s>>>(a);
+      launch_step(a.dep, grid_slots, kTile, 0, s, k_bin_keys<3>, a);
   }
   launch_scan(a, s);
-  k_scatter<<<grid_slots, kTile, 0, s>>>(a);
+  launch_step(a.dep, grid_slots, kTile, 0, s, k_scatter, a);
   if (!a.permute) return;  // the bin index (range + perm) is all a list rebuild needs
   // bin order by element id: deterministic sums (FP64 / plain forms)
   if (a.dim == 2)
-    k_gather<2><<<grid_slots, kTile, 0, s>>>(a);
+    launch_step(a.dep, grid_slots, kTile, 0, s, k_gather<2>, a);
   else
-    k_gather<3><<<grid_slots, kTile, 0, s>>>(a);
-  if (a.state_out) k_own_slots<<<grid_slots, kTile, 0, s>>>(a);
+    launch_step(a.dep, grid_slots, kTile, 0, s, k_gather<3>, a);
+  if (a.state_out) launch_step(a.dep, grid_slots, kTile, 0, s, k_own_slots, a);
 }
 
 void launch_cell_resort(const RebuildArgs &a, int grid_cells, cudaStream_t s) {

@@ -226,6 +226,7 @@ __global__ void k_cy_scan_small(int *count, int m) {
 
 // Block sums of kScanTile-sized chunks (4 per thread)
 __global__ void k_cy_chunk_sums(const int *count, int m, int *part) {
+  cil::enter_step_kernel();
   const int b0 = blockIdx.x * kScanTile + threadIdx.x * 4;
   int s = 0;
   for (int q = 0; q < 4; ++q) s += (b0 + q < m) ? count[b0 + q] : 0;
@@ -238,6 +239,7 @@ __global__ void k_cy_chunk_sums(const int *count, int m, int *part) {
 // count[m] reads as 0); count is left at zero. part: the chunk sums, scanned when `scanned`, otherwise
 // each block adds those before it itself (a few loads per thread, cheaper than a launch).
 __global__ void k_cy_chunk_apply(int *count, int m, const int *part, int *start, int scanned) {
+  cil::enter_step_kernel();
   const int b0 = blockIdx.x * kScanTile + threadIdx.x * 4;
   int c[4], s = 0;
   for (int q = 0; q < 4; ++q) {
@@ -315,6 +317,7 @@ __device__ inline double kick(const CyConst &C, double v, double fc, double fd, 
 
 __global__ void __launch_bounds__(kTile) k_cy_keys(CyConst C, CySet S, const CyCounters *cnt, int *key, int *arrival,
                                                    int *count, int *dblk, int drift) {
+  cil::enter_step_kernel();
   if (threadIdx.x == 0) dblk[blockIdx.x] = 0;  // the coming step's divisions per block of cells
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt->n) return;
@@ -337,6 +340,7 @@ __global__ void __launch_bounds__(kTile) k_cy_keys(CyConst C, CySet S, const CyC
 
 __global__ void __launch_bounds__(kTile) k_cy_scatter(const CyCounters *cnt, const int *key, const int *arrival,
                                                       const int *start, int2 *tmp) {
+  cil::enter_step_kernel();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt->n) return;
   const int b = key[i];
@@ -352,6 +356,7 @@ __global__ void __launch_bounds__(kTile) k_cy_scatter(const CyCounters *cnt, con
 // from the index order, with the copies scattered, 8.2 us).
 __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounters *cnt, const int *start,
                                                     const int2 *tmp, CyOrdered O, int with_vel) {
+  cil::enter_step_kernel();
   const int at = blockIdx.x * blockDim.x + threadIdx.x;
   if (at >= cnt->n) return;
   const int2 ib = tmp[at];
@@ -695,6 +700,7 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
                                                          const int *start, const int *ts_dev, int mode, int key_off,
                                                          CyOrdered O, int lane_bits, int *dblk, int *dueq,
                                                          unsigned long long *sig_part) {
+  cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, D + 1, R> s_warp[kPairBlock / 32];
   PairWarp<D, D + 1, R> &W = s_warp[threadIdx.x >> 5];
@@ -897,6 +903,7 @@ template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, double *v_out, CyCounters *cnt,
                                                          const int *start, const int *ts_dev, int key_off, int kick_on,
                                                          CyOrdered O, float4 *vel_out, int lane_bits) {
+  cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, 2 * D, R> s_warp[kPairBlock / 32];
   PairWarp<D, 2 * D, R> &W = s_warp[threadIdx.x >> 5];
@@ -1024,6 +1031,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
                                                         const int *ts_dev, CyOrdered O, const float4 *vel,
                                                         int lane_bits, int *dblk, int *dueq,
                                                          unsigned long long *sig_part) {
+  cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
   __shared__ PairWarp<D, D, R> s_warp[kPairBlock / 32];
   PairWarp<D, D, R> &W = s_warp[threadIdx.x >> 5];
@@ -1197,6 +1205,7 @@ __device__ void divide_times(const CyConst &C, const CySet &S, int ts, int i, in
 __global__ void __launch_bounds__(kTile) k_cy_divide(CyConst C, CySet S, CyCounters *cnt, int *ts_dev,
                                                      const int *dblk, const int *dueq,
                                                      const unsigned long long *sig_part, int lane_bits) {
+  cil::enter_step_kernel();
   __shared__ int s_due[kDueMax];
   __shared__ unsigned long long s_sig;
   const int n = cnt->n, ts = *ts_dev + 1, nd = cnt->ndue;
@@ -1589,9 +1598,9 @@ double host_sigma_max(const cil_cycle *h) {
 void scan_into(cil_cycle *h, int *count, int m, int *start) {
   const int nchunks = m / kScanTile + 1;  // covers index m
   const int scanned = nchunks > 2048 ? 1 : 0;
-  k_cy_chunk_sums<<<nchunks, kTile, 0, h->stream>>>(count, m, h->part);
+  cil::launch_step(true, nchunks, kTile, 0, h->stream, k_cy_chunk_sums, count, m, h->part);
   if (scanned) k_cy_scan_small<<<1, kTile, 0, h->stream>>>(h->part, nchunks);
-  k_cy_chunk_apply<<<nchunks, kTile, 0, h->stream>>>(count, m, h->part, start, scanned);
+  cil::launch_step(true, nchunks, kTile, 0, h->stream, k_cy_chunk_apply, count, m, h->part, start, scanned);
   h->launches += 2 + scanned;
 }
 
@@ -1599,10 +1608,10 @@ void scan_into(cil_cycle *h, int *count, int m, int *start) {
 cil_status bin_cells(cil_cycle *h, int drift) {
   const CySet &S = h->set[h->cur];
   const int g = blocks_for(h->cap);
-  k_cy_keys<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->key, h->arrival, h->bcount, h->dblk, drift);
+  cil::launch_step(true, g, kTile, 0, h->stream, k_cy_keys, h->C, S, h->cnt, h->key, h->arrival, h->bcount, h->dblk, drift);
   scan_into(h, h->bcount, h->nbins, h->bstart);
-  k_cy_scatter<<<g, kTile, 0, h->stream>>>(h->cnt, h->key, h->arrival, h->bstart, h->tmp);
-  k_cy_place<<<g, kTile, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->tmp, h->O,
+  cil::launch_step(true, g, kTile, 0, h->stream, k_cy_scatter, h->cnt, h->key, h->arrival, h->bstart, h->tmp);
+  cil::launch_step(true, g, kTile, 0, h->stream, k_cy_place, h->C, S, h->cnt, h->bstart, h->tmp, h->O,
                                          h->C.dpd && h->p.precision == 1 ? 1 : 0);
   h->launches += 3;
   return CIL_OK;
@@ -1631,10 +1640,10 @@ template <int D>
 void launch_force_d(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    k_cy_force<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_cy_force<D, true>, h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
                                                          h->O, h->lane_bits, h->dblk, h->dueq, h->sig_part);
   else
-    k_cy_force<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_cy_force<D, false>, h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
                                                           h->O, h->lane_bits, h->dblk, h->dueq, h->sig_part);
 }
 
@@ -1650,10 +1659,10 @@ template <int D>
 void launch_dpd_pair_d(cil_cycle *h, CySet &S, int key_off, int kick_on) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    k_dpd_pair<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off, kick_on,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_pair<D, true>, h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off, kick_on,
                                                          h->O, h->vel_next, h->lane_bits);
   else
-    k_dpd_pair<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_pair<D, false>, h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off,
                                                           kick_on, h->O, h->vel_next, h->lane_bits);
 }
 
@@ -1669,10 +1678,10 @@ template <int D>
 void launch_dpd_dis_d(cil_cycle *h, CySet &S) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    k_dpd_dis<D, true><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_dis<D, true>, h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
                                                         h->lane_bits, h->dblk, h->dueq, h->sig_part);
   else
-    k_dpd_dis<D, false><<<g, kPairBlock, 0, h->stream>>>(h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_dis<D, false>, h->C, S, h->cnt, h->bstart, h->ts_dev, h->O, h->vel_next,
                                                          h->lane_bits, h->dblk, h->dueq, h->sig_part);
 }
 
@@ -1706,7 +1715,7 @@ cil_status enqueue_step(cil_cycle *h) {
   }
   h->ts += 1;
   if (h->C.divide) {  // also moves the step counter
-    k_cy_divide<<<std::min(blocks_for(h->cap), 2 * kNumSMs), kTile, 0, h->stream>>>(h->C, S, h->cnt, h->ts_dev,
+    cil::launch_step(true, std::min(blocks_for(h->cap), 2 * kNumSMs), kTile, 0, h->stream, k_cy_divide, h->C, S, h->cnt, h->ts_dev,
                                                                                       h->dblk, h->dueq, h->sig_part,
                                                                                       h->lane_bits);
   } else {

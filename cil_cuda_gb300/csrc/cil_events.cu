@@ -722,6 +722,7 @@ constexpr int kDueRank = 512;   // up to this many: sorted by ranks instead of a
 // (growth, 0.2M cells: 15.7 us a step and four gaps).
 template <int D>
 __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
+  enter_step_kernel();
   EventArgs a = a_;
   a.ts = *a_.ts_dev + 1;
   const int c = blockIdx.x;
@@ -1081,9 +1082,9 @@ void launch_events_fast(const EventArgs &a, int grid_cells, int dim, cudaStream_
 
 void launch_events_due(const EventArgs &a, int dim, cudaStream_t s) {
   if (dim == 2)
-    k_events_due<2><<<a.B, kTile, 0, s>>>(a);
+    launch_step(true, a.B, kTile, 0, s, k_events_due<2>, a);
   else
-    k_events_due<3><<<a.B, kTile, 0, s>>>(a);
+    launch_step(true, a.B, kTile, 0, s, k_events_due<3>, a);
 }
 
 // The crawling/dividing cells, oracle mode: per cell of the colony, whether a dividing cell's

@@ -112,6 +112,7 @@ struct F64Warp {
 
 template <int D, int LAW>
 __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane_bits) {
+  enter_step_kernel();
   extern __shared__ __align__(16) unsigned char s_f64[];
   ForceArgs a = a_;
   a.ts = *a_.ts_dev;
@@ -606,6 +607,7 @@ constexpr int kMixedAhead = 4;
 
 template <int D, int LAW>
 __global__ void __launch_bounds__(kTile, 4) k_force_mixed(ForceArgs a_) {
+  enter_step_kernel();
   ForceArgs a = a_;
   a.ts = *a_.ts_dev;
   const int t = blockIdx.x;
@@ -899,6 +901,7 @@ __device__ __forceinline__ void pairs_finish(const ForceArgs &a, const ColonyCon
 // list build, in no list) arrive through facc from k_fresh_pairs.
 template <int D, int LAW, int UNROLL, int MINB, int TILE>
 __global__ void __launch_bounds__(TILE, MINB) k_force_cells(const ForceArgs a) {
+  enter_step_kernel();
   constexpr int SEG = pair_seg<D, MINB, TILE>();
   extern __shared__ __align__(16) unsigned char s_pairs[];
   __shared__ ColonyConst sC;
@@ -1241,7 +1244,7 @@ void launch_cells_t(const ForceArgs &a, int grid, cudaStream_t s) {
                          bytes);
     attr_set = true;
   }
-  k_force_cells<D, LAW, UNROLL, MINB, TILE><<<grid, TILE, bytes, s>>>(a);
+  launch_step(true, grid, TILE, bytes, s, k_force_cells<D, LAW, UNROLL, MINB, TILE>, a);
 }
 
 // MINB is the CTAs per SM at 256 threads; 128-thread blocks keep its threads per SM (hence the
@@ -1302,9 +1305,9 @@ void launch_dl(const ForceArgs &a, int prec, int tiles, int lane_bits, cudaStrea
       cudaFuncSetAttribute(k_force_fp64<D, LAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
       attr_set = true;
     }
-    k_force_fp64<D, LAW><<<tiles * (2 << lane_bits), kF64Block, bytes, s>>>(a, lane_bits);
+    launch_step(true, tiles * (2 << lane_bits), kF64Block, bytes, s, k_force_fp64<D, LAW>, a, lane_bits);
   } else {
-    k_force_mixed<D, LAW><<<tiles, kTile, 0, s>>>(a);
+    launch_step(true, tiles, kTile, 0, s, k_force_mixed<D, LAW>, a);
   }
 }
 

@@ -264,6 +264,35 @@ struct ColonyCounters {
   long long napo_total;
 };
 
+// ---------------------------------------------------------------- launches of a step
+// The kernels of a step are launched with programmatic stream serialisation: a kernel's blocks are
+// brought onto the SMs while the one before it drains, and wait there (enter_step_kernel, the first
+// statement of every such kernel) until it has completed and its writes are visible. They release the
+// next kernel only then, so at most two kernels of a step are resident and a kernel's completion
+// implies that of all before it. A leg of 100 steps takes 3.00 ms instead of 3.39 for 300 cells in lists (11
+// launches a step) and 15.25 instead of 15.67 for 1M; 50 steps of 1024 cell-cycle cells 1.53 instead of
+// 1.64. `dep` false (kernels in and after a conditional graph node): an ordinary launch, in which the two
+// instructions do nothing.
+__device__ __forceinline__ void enter_step_kernel() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+template <class... P, class... A>
+void launch_step(bool dep, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void (*kernel)(P...), A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = dep ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------- small device helpers
 
 // Utils.hpp:173-175
@@ -638,6 +667,7 @@ struct RebuildArgs {
   const ColonySkin *skin;  // skin mode: colonies without rebuild_now are skipped; else null
   const int *any_rebuild;  // skin mode: [2] per step parity, 0 = no colony rebuilds (kernels return); else null
   const int *ts_dev;
+  bool dep;                // launch_step's
   int permute;             // 1: slots are re-sorted (data moves); 0: only the bin index is rebuilt
   unsigned char *state_out;// skin mode, permuting: slot states of the new order
   int *key;
@@ -805,6 +835,7 @@ struct SkinArgs {
   const float *mlp;
   int use_interval;
   float skin_min, skin_max, interval_scale;
+  bool dep;                // launch_step's
 };
 
 // ---------------------------------------------------------------- scheduler network

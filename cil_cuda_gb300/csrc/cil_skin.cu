@@ -121,6 +121,7 @@ __device__ __forceinline__ int skin_begin_colony(const SkinArgs &a, int c) {
 // one warp per colony: the decision, then (rebuilding colony, scheduler installed) the
 // network on the colony's features sets the skin of the new lists and the cadence
 __global__ void k_skin_begin(SkinArgs a) {
+  enter_step_kernel();
   if (blockIdx.x == 0 && a.tiles_used_out) {
     // the step's tile tables (slots: kTile per tile; slot pairs: pair_tile slots per tile),
     // block 0, before any thread returns
@@ -225,6 +226,7 @@ __global__ void k_skin_begin(SkinArgs a) {
 
 template <int D>
 __global__ void __launch_bounds__(kTile) k_skin_rebin(SkinArgs a) {
+  enter_step_kernel();
   if (a.any_rebuild && a.any_rebuild[*a.ts_dev & 1] == 0) return;  // uniform
   const int total = a.tiles[a.B];
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
@@ -277,6 +279,7 @@ constexpr int kListMinBlocks = D == 2 ? 8 : 3;
 
 template <int D, int LAW>
 __global__ void __launch_bounds__(kTile, kListMinBlocks<D>) k_skin_lists(SkinArgs a) {
+  enter_step_kernel();
   constexpr int NB = (D == 2) ? 9 : 27;
   if (a.any_rebuild && a.any_rebuild[*a.ts_dev & 1] == 0) return;  // uniform, before any barrier
   __shared__ unsigned s_occ_sum, s_occ_max, s_cnt;
@@ -425,6 +428,7 @@ __global__ void __launch_bounds__(kTile, kListMinBlocks<D>) k_skin_lists(SkinArg
 constexpr int kFlatSeg = 1024;
 
 __global__ void __launch_bounds__(128) k_list_flatten(SkinArgs a) {
+  enter_step_kernel();
   __shared__ __align__(16) int s_ent[4][kFlatSeg];
   __shared__ __align__(16) unsigned char s_own[4][kFlatSeg];
   const int total = a.tiles[a.B];
@@ -497,6 +501,7 @@ constexpr int kFreshBlock = 128, kFreshWarps = kFreshBlock / 32;
 
 template <int D, int LAW>
 __global__ void __launch_bounds__(kFreshBlock) k_fresh_pairs(SkinArgs a) {
+  enter_step_kernel();
   constexpr int NB = (D == 2) ? 9 : 27;
   // the fresh sets of all colonies as one flattened range (inclusive prefix of their sizes)
   extern __shared__ int s_pref[];  // [B], sized at launch (all blocks resident in one wave)
@@ -651,16 +656,16 @@ template <int D>
 void lists_d(const SkinArgs &a, int law, int grid, cudaStream_t s) {
   switch (law) {
     case CIL_FORCE_LJ_WCA:
-      k_skin_lists<D, CIL_FORCE_LJ_WCA><<<grid, kTile, 0, s>>>(a);
+      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_LJ_WCA>, a);
       break;
     case CIL_FORCE_SOFTCORE:
-      k_skin_lists<D, CIL_FORCE_SOFTCORE><<<grid, kTile, 0, s>>>(a);
+      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_SOFTCORE>, a);
       break;
     case CIL_FORCE_SC:
-      k_skin_lists<D, CIL_FORCE_SC><<<grid, kTile, 0, s>>>(a);
+      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_SC>, a);
       break;
     default:
-      k_skin_lists<D, CIL_FORCE_HERTZ><<<grid, kTile, 0, s>>>(a);
+      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_HERTZ>, a);
       break;
   }
 }
@@ -670,16 +675,16 @@ void fresh_d(const SkinArgs &a, int law, cudaStream_t s) {
   const int grid = a.grid;
   switch (law) {
     case CIL_FORCE_LJ_WCA:
-      k_fresh_pairs<D, CIL_FORCE_LJ_WCA><<<grid, kFreshBlock, sizeof(int) * a.B, s>>>(a);
+      launch_step(a.dep, grid, kFreshBlock, sizeof(int) * a.B, s, k_fresh_pairs<D, CIL_FORCE_LJ_WCA>, a);
       break;
     case CIL_FORCE_SOFTCORE:
-      k_fresh_pairs<D, CIL_FORCE_SOFTCORE><<<grid, kFreshBlock, sizeof(int) * a.B, s>>>(a);
+      launch_step(a.dep, grid, kFreshBlock, sizeof(int) * a.B, s, k_fresh_pairs<D, CIL_FORCE_SOFTCORE>, a);
       break;
     case CIL_FORCE_SC:
-      k_fresh_pairs<D, CIL_FORCE_SC><<<grid, kFreshBlock, sizeof(int) * a.B, s>>>(a);
+      launch_step(a.dep, grid, kFreshBlock, sizeof(int) * a.B, s, k_fresh_pairs<D, CIL_FORCE_SC>, a);
       break;
     default:
-      k_fresh_pairs<D, CIL_FORCE_HERTZ><<<grid, kFreshBlock, sizeof(int) * a.B, s>>>(a);
+      launch_step(a.dep, grid, kFreshBlock, sizeof(int) * a.B, s, k_fresh_pairs<D, CIL_FORCE_HERTZ>, a);
       break;
   }
 }
@@ -687,17 +692,17 @@ void fresh_d(const SkinArgs &a, int law, cudaStream_t s) {
 }  // namespace
 
 void launch_skin_begin(const SkinArgs &a, cudaStream_t s) {
-  k_skin_begin<<<(32 * a.B + 127) / 128, 128, 0, s>>>(a);
+  launch_step(a.dep, (32 * a.B + 127) / 128, 128, 0, s, k_skin_begin, a);
 }
 
 void launch_skin_rebin(const SkinArgs &a, int dim, int grid, cudaStream_t s) {
   if (dim == 2)
-    k_skin_rebin<2><<<grid, kTile, 0, s>>>(a);
+    launch_step(a.dep, grid, kTile, 0, s, k_skin_rebin<2>, a);
   else
-    k_skin_rebin<3><<<grid, kTile, 0, s>>>(a);
+    launch_step(a.dep, grid, kTile, 0, s, k_skin_rebin<3>, a);
 }
 
-void launch_list_flatten(const SkinArgs &a, int grid, cudaStream_t s) { k_list_flatten<<<grid, 128, 0, s>>>(a); }
+void launch_list_flatten(const SkinArgs &a, int grid, cudaStream_t s) { launch_step(a.dep, grid, 128, 0, s, k_list_flatten, a); }
 
 void launch_skin_lists(const SkinArgs &a, int dim, int law, int grid, cudaStream_t s) {
   if (dim == 2)
