@@ -101,7 +101,9 @@ struct cil_handle {
   // skin mode
   bool skin_mode = false;
   unsigned char *d_state[2] = {nullptr, nullptr};
-  int *d_nbr = nullptr, *d_ncnt = nullptr, *d_fresh = nullptr;
+  unsigned long long *d_nmask = nullptr;  // list candidates per slot (k_skin_lists)
+  float4 *d_brec = nullptr;               // the records in bin order
+  int *d_ncnt = nullptr, *d_fresh = nullptr;
   int *d_lflat = nullptr, *d_lwarp = nullptr;  // the lists flattened per warp of 32 cells
   StatPart *d_spart = nullptr;                 // displacement statistics slots [B][kStatSlots]
   unsigned char *d_oflat = nullptr;
@@ -184,7 +186,7 @@ cil_status fail(cil_handle *h, cil_status s, const std::string &m) {
 void free_all(cil_handle *h) {
   void *ptrs[] = {h->d_col, h->d_cnt, h->d_x[0], h->d_x[1], h->d_sig[0], h->d_sig[1], h->d_eid[0],
                   h->d_eid[1], h->d_rec, h->d_pk[0], h->d_pk[1], h->d_sbin[0], h->d_sbin[1],
-                  h->d_cyc[0], h->d_cyc[1], h->d_sigma_c, h->d_state[0], h->d_state[1], h->d_nbr,
+                  h->d_cyc[0], h->d_cyc[1], h->d_sigma_c, h->d_state[0], h->d_state[1], h->d_nmask, h->d_brec,
                   h->d_ncnt, h->d_fresh, h->d_spart, h->d_lflat, h->d_lwarp, h->d_oflat, h->d_lstart, h->d_uref, h->d_facc, h->d_ftouch, h->d_skin, h->d_sched, h->d_mlp, h->d_fhead, h->d_fnext, h->d_ts, h->d_anyreb, h->d_vel, h->d_vel2, h->d_frc, h->d_key, h->d_perm,
                   h->d_bcount, h->d_range, h->d_scan_sum, h->d_scan_off, h->d_scan_col,
                   h->d_slot_of, h->d_t0, h->d_tsw, h->d_tiles_used, h->d_tiles_live, h->d_tiles_pairs,
@@ -449,7 +451,6 @@ ForceArgs force_args(cil_handle *h, int noise_mode, int integrate, double *vel, 
   if (h->skin_mode) {
     a.tiles = h->d_tiles_pairs;
     a.skin = h->d_skin;
-    a.nbr = h->d_nbr;
     a.ncnt = h->d_ncnt;
     a.lflat = h->d_lflat;
     a.oflat = h->d_oflat;
@@ -543,7 +544,8 @@ SkinArgs skin_args(cil_handle *h, int force_rebuild) {
   a.sbin = h->d_sbin[h->meta];
   a.range = h->d_range;
   a.perm = h->d_perm;
-  a.nbr = h->d_nbr;
+  a.nmask = h->d_nmask;
+  a.brec = h->d_brec;
   a.ncnt = h->d_ncnt;
   a.lflat = h->d_lflat;
   a.oflat = h->d_oflat;
@@ -946,9 +948,9 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
     ra.ts_dev = h->d_ts;
     ra.state_out = nullptr;
     ra.tiles_live_out = nullptr;
+    ra.brec = h->d_brec;
     launch_rebuild(ra, h->grid_slots, rs);  // slot count unchanged: tile tables stay
     launch_skin_lists(skin_args(h, 0), h->D, h->cfg.force_law, h->grid_slots, rs);
-    launch_list_flatten(skin_args(h, 0), h->grid_slots, rs);
     if (use_cond) {
       cudaGraph_t body = nullptr;
       CUDA_TRY(h, cudaStreamEndCapture(h->side, &body));
@@ -1367,7 +1369,8 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
   bool skin_ok = true;
   if (h->skin_mode) {
     for (int b = 0; b < 2; ++b) h->d_state[b] = dalloc<unsigned char>(SS);
-    h->d_nbr = dalloc<int>(static_cast<size_t>(kListCap) * SS);
+    h->d_nmask = dalloc<unsigned long long>(SS);
+    h->d_brec = dalloc<float4>(SS);
     h->d_ncnt = dalloc<int>(SS);
     h->d_lflat = dalloc<int>(static_cast<size_t>(kListCap) * SS);
     h->d_oflat = dalloc<unsigned char>(static_cast<size_t>(kListCap) * SS);
@@ -1382,7 +1385,7 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
     h->d_anyreb = dalloc<int>(4);
     h->d_skin = dalloc<ColonySkin>(h->B);
     h->d_sched = dalloc<SchedState>(h->B);
-    skin_ok = h->d_state[0] && h->d_state[1] && h->d_nbr && h->d_ncnt && h->d_uref && h->d_facc && h->d_ftouch &&
+    skin_ok = h->d_state[0] && h->d_state[1] && h->d_nmask && h->d_brec && h->d_ncnt && h->d_uref && h->d_facc && h->d_ftouch &&
               h->d_spart && h->d_lflat && h->d_oflat && h->d_lstart && h->d_lwarp &&
               h->d_fresh &&
               h->d_fnext && h->d_anyreb && h->d_skin && h->d_sched;

@@ -257,6 +257,11 @@ __global__ void __launch_bounds__(kTile) k_scatter(RebuildArgs a) {
     const int pos = a.range[k].x + atomicSub(a.bcount + k, 1) - 1;
     a.perm[pos] = (static_cast<unsigned long long>(static_cast<uint32_t>(a.eid_in[s])) << 32) |
                   static_cast<uint32_t>(s);
+    if (a.brec) {
+      float4 p = a.pk_in[s];
+      if (a.dim == 2) p.z = __int_as_float(s);  // the record's unused word
+      a.brec[pos] = p;
+    }
   }
 }
 

@@ -654,6 +654,7 @@ struct RebuildArgs {
   double *sig_out;
   int *eid_out;
   float4 *pk_out;          // mixed: packed elements of the new order, may be null
+  float4 *brec;            // skin mode, bin index of a list build: the records in bin order; else null
   float4 *rec_out;         // FP64 form: FP32 absolute coordinates and diameter, new order; else null
   const float4 *pk_in;     // mixed: packed elements after the last update (relative to sbin_in)
   const int *sbin_in;      // home bin (colony-local id) of each slot
@@ -706,7 +707,6 @@ struct ForceArgs {
   // skin mode (null otherwise)
   const int *tiles;        // skin mode: tiles over slot pairs (k_force_cells)
   ColonySkin *skin;
-  const int *nbr;          // Verlet lists [kListCap][SS]
   const int *ncnt;
   // the lists per warp of 32 cells (64 slots from w0), flattened: entries and their owners
   // (element of the warp) at w0 * kListCap, element starts per slot, entries per warp
@@ -804,7 +804,8 @@ struct SkinArgs {
   int *sbin;
   const int2 *range;
   const unsigned long long *perm;
-  int *nbr;
+  unsigned long long *nmask;  // per slot: which of its first 64 candidates are in its list
+  const float4 *brec;         // the records in bin order (at the places of perm; 2D: z holds the slot)
   int *ncnt;
   int *lflat;              // flattened lists per warp of 32 cells (see ForceArgs)
   unsigned char *oflat;
@@ -899,7 +900,6 @@ void launch_force_list(const ForceArgs &a, int dim, int law, int grid, int varia
 void launch_skin_begin(const SkinArgs &a, cudaStream_t s);
 void launch_skin_rebin(const SkinArgs &a, int dim, int grid, cudaStream_t s);
 void launch_skin_lists(const SkinArgs &a, int dim, int law, int grid, cudaStream_t s);
-void launch_list_flatten(const SkinArgs &a, int grid, cudaStream_t s);
 void launch_fresh_pairs(const SkinArgs &a, int dim, int law, cudaStream_t s);
 // the device step counter advance; with tiles_cell also the tile table over the cells of the
 // step's events

@@ -9,9 +9,11 @@
 //   k_skin_rebin   rebuilding colonies: new home bin of every slot from its FP32 local
 //                  coordinate (in place, no data movement) and the bin histogram
 //   (scan + scatter of cil_bins.cu give range[] and perm[] for the rebuilding colonies)
-//   k_skin_lists   rebuilding colonies: Verlet list of every live slot from the 3^d bins;
-//                  entries are slot | (neighbour-bin index << 27); same-cell elements are
-//                  excluded; uref = u; every slot becomes "normal"
+//   k_skin_lists   rebuilding colonies: which of the 3^d bins' elements are in the Verlet list of every
+//                  live slot (a bit per candidate), same-cell elements excluded; uref = u; every slot
+//                  becomes "normal"
+//   k_list_flatten the lists' entries, slot | (neighbour-bin offset code << 26), per warp of the force
+//                  kernel
 //   k_fresh_pairs  elements created or moved by a division since the last build ("fresh")
 //                  are in no list: each searches the bins of the last build for normal
 //                  partners (Newton's third law onto them through facc) and the per-bin
@@ -266,21 +268,91 @@ __global__ void __launch_bounds__(kTile) k_skin_rebin(SkinArgs a) {
   }
 }
 
-// Latency-bound (two dependent loads per batch of candidates): many resident warps with short
-// batches beat few warps with long ones. One list build (with the rebin and scan launches) of
-// the 2M-particle 2D colony took 0.603 ms with batches of 8 at 2 CTAs per SM (108 registers),
-// 0.440 ms with 4 at 4 CTAs and 0.420 ms with 2 at 8 CTAs (32 registers); of the 4M-particle
-// 3D channel, 2.64 ms with 8 at 1 CTA, 1.55 ms with 2 at 2 CTAs and 1.43 ms with 2 at 3 CTAs
-// (3D keeps the 27 bin ranges in registers, so it runs fewer CTAs per SM).
+// The candidates of a list build: the rows of bins around an element's bin, as ranges of the bin order
+// (SkinArgs::brec and perm, written by k_scatter), in the order of the 3^d offsets. A row's three bins
+// along the last axis hold consecutive places; at the ends of the axis they are three ranges.
+// f(range start, end, m0, m1, row): places below m0 are in the bin before the element's on the last
+// axis, those from m1 on in the one after.
+template <int D, class F>
+__device__ __forceinline__ void candidate_rows(const ColonyConst &C, const int2 *range, const int *bi, F f) {
+  constexpr int NROW = D == 2 ? 3 : 9;
+  const int last = bi[D - 1], nl = C.ns[D - 1];
+  const bool inner = last > 0 && last < nl - 1;
+  for (int row = 0; row < NROW; ++row) {
+    const int oo[2] = {(D == 2 ? row : row / 3) - 1, row % 3 - 1};
+    int rowbin = 0;
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < D - 1; ++d) {
+      int v = bi[d] + oo[d];
+      if (v < 0) {
+        ok = ok && C.periodic[d];
+        v += C.ns[d];
+      } else if (v >= C.ns[d]) {
+        ok = ok && C.periodic[d];
+        v -= C.ns[d];
+      }
+      rowbin = rowbin * C.ns[d] + v;
+    }
+    if (!ok) continue;
+    const int2 *rng = range + C.bin_base + rowbin * nl;
+    for (int piece = 0; piece < (inner ? 1 : 3); ++piece) {
+      int st, en, m0, m1;
+      if (inner) {
+        const int2 r0 = rng[last - 1], r1 = rng[last + 1];
+        st = r0.x;
+        m0 = r0.y;
+        m1 = r1.x;
+        en = r1.y;
+      } else {
+        int v = last + piece - 1;
+        if (v < 0 || v >= nl) {
+          if (!C.periodic[D - 1]) continue;
+          v += v < 0 ? nl : -nl;
+        }
+        const int2 r = rng[v];
+        st = r.x;
+        en = r.y;
+        m0 = piece == 0 ? en : st;
+        m1 = piece == 2 ? st : en;
+      }
+      f(st, en, m0, m1, row);
+    }
+  }
+}
+
+// The slot of the candidate at a place of the bin order: in 2D its record's unused z word, else perm's
 template <int D>
-constexpr int kListBatch = 2;
-template <int D>
-constexpr int kListMinBlocks = D == 2 ? 8 : 3;
+__device__ __forceinline__ int candidate_slot(const SkinArgs &a, int at, float z) {
+  return D == 2 ? __float_as_int(z) : static_cast<int>(a.perm[at] & 0xffffffffu);
+}
+
+// whether the candidate with record p, l bins away along the last axis (-1, 0, 1), is within reach
+template <int D, int LAW>
+__device__ __forceinline__ bool list_reaches(const ColonyConst &C, const float *ui, float si, float skin,
+                                             const float4 &p, int row, int l) {
+  const int oo[3] = {(D == 2 ? row : row / 3) - 1, D == 2 ? l : row % 3 - 1, l};
+  float r2 = 0.0f;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float dx = pk_c(p, d) + (static_cast<float>(oo[d]) * C.bwf[d] - ui[d]);
+    r2 += dx * dx;
+  }
+  const float cut = law_cutoff_f<LAW>(C, si, fabsf(p.w)) + skin;
+  return r2 < cut * cut;
+}
+
+// Bound by its round trips to L2, so the candidates' records are read as ranges, in the bin order's own
+// copy, with kListAhead in flight: one round trip per batch. Through the bin order's slots (slot, then
+// element id and record, two in flight) a build of the 2M-element 2D colony took 400 us and its
+// flattening 119, of the 0.8M-element 3D channel 650 and 101 us, and of the few colonies of a sweep that
+// rebuild in a step 19.2 and 5.7 us; now 250 and 184, 327 and 245, 10.2 and 7.1 us (the flattening finds
+// the entries from a mask of candidates instead of reading them from 256 bytes a slot).
+constexpr int kListAhead = 4;
 
 template <int D, int LAW>
-__global__ void __launch_bounds__(kTile, kListMinBlocks<D>) k_skin_lists(SkinArgs a) {
+__global__ void __launch_bounds__(kTile, 4) k_skin_lists(SkinArgs a) {
   enter_step_kernel();
-  constexpr int NB = (D == 2) ? 9 : 27;
   if (a.any_rebuild && a.any_rebuild[*a.ts_dev & 1] == 0) return;  // uniform, before any barrier
   __shared__ unsigned s_occ_sum, s_occ_max, s_cnt;
   __shared__ unsigned long long s_pairs;
@@ -308,8 +380,7 @@ __global__ void __launch_bounds__(kTile, kListMinBlocks<D>) k_skin_lists(SkinArg
       if (e < 0 || a.state[s] == kSlotDead) {
         a.ncnt[s] = 0;
       } else {
-        const int g = e >> 1;
-        float4 pi = a.pk[s];
+        const float4 pi = a.pk[s];
         float ui[D];
 #pragma unroll
         for (int d = 0; d < D; ++d) ui[d] = pk_c(pi, d);
@@ -317,66 +388,33 @@ __global__ void __launch_bounds__(kTile, kListMinBlocks<D>) k_skin_lists(SkinArg
         const float skin = S.skin;
         int bi[D];
         bin_decode<D>(C, a.sbin[s], bi);
-        // the 3^d bin ranges, loaded together; candidates are then taken as one flattened
-        // range in batches of kLB, so each batch costs two round trips (slots, then records)
-        constexpr int kLB = kListBatch<D>;
-        int start[NB], pre[NB + 1];
-        pre[0] = 0;
+        constexpr int kMid = D == 2 ? 1 : 4;  // the element's own row
+        unsigned long long mask = 0ull;       // the first 64 candidates (k_list_flatten tests the others again)
+        int k = 0;
+        candidate_rows<D>(C, a.range, bi, [&](int st, int en, int m0, int m1, int row) {
+          if (row == kMid) occ += static_cast<unsigned>(m1 - m0);  // the home bin (0 in the other pieces)
+          for (int t0 = st; t0 < en; t0 += kListAhead) {
+            float4 pj[kListAhead];
+            int tj[kListAhead];
 #pragma unroll
-        for (int o = 0; o < NB; ++o) {
-          int off[3];
-          nb_offsets<D>(o, off);
-          int nb[D];
-          int2 r = make_int2(0, 0);
-          if (nb_bin<D>(C, bi, off, nb)) r = a.range[C.bin_base + bin_id<D>(C, nb)];
-          start[o] = r.x;
-          pre[o + 1] = pre[o] + (r.y - r.x);
-          if (o == NB / 2) occ = static_cast<unsigned>(r.y - r.x);  // the home bin
-        }
-        const int ncand = pre[NB];
-        for (int k0 = 0; k0 < ncand; k0 += kLB) {
-          int tt[kLB], oo[kLB];
-#pragma unroll
-          for (int q = 0; q < kLB; ++q) {
-            const int kq = k0 + q;
-            int o = 0, base = start[0];  // select chain: constant indices keep the arrays in registers
-#pragma unroll
-            for (int b = 1; b < NB; ++b) {
-              if (kq >= pre[b]) {
-                o = b;
-                base = start[b] - pre[b];
-              }
+            for (int u = 0; u < kListAhead; ++u) {
+              const int at = min(t0 + u, en - 1);
+              pj[u] = __ldg(a.brec + at);
+              tj[u] = candidate_slot<D>(a, at, pj[u].z);
             }
-            oo[q] = o;
-            tt[q] = kq < ncand ? static_cast<int>(a.perm[base + kq] & 0xffffffffu) : -1;
-          }
-          int ej[kLB];
-          float4 pj[kLB];
 #pragma unroll
-          for (int q = 0; q < kLB; ++q) {
-            ej[q] = tt[q] >= 0 ? a.eid[tt[q]] : -2;
-            pj[q] = tt[q] >= 0 ? a.pk[tt[q]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          }
-#pragma unroll
-          for (int q = 0; q < kLB; ++q) {
-            if (tt[q] < 0 || tt[q] == s || (ej[q] >> 1) == g) continue;
-            int off[3];
-            nb_offsets<D>(oo[q], off);
-            float r2 = 0.0f;
-#pragma unroll
-            for (int d = 0; d < D; ++d) {
-              const float dx = pk_c(pj[q], d) + (static_cast<float>(off[d]) * C.bwf[d] - ui[d]);
-              r2 += dx * dx;
+            for (int u = 0; u < kListAhead; ++u) {
+              const int at = t0 + u;
+              const int l = at < m0 ? -1 : (at >= m1 ? 1 : 0);
+              // a cell's two elements sit in one slot pair
+              const bool in = at < en && (tj[u] >> 1) != (s >> 1) && list_reaches<D, LAW>(C, ui, si, skin, pj[u], row, l);
+              if (in && k + u < 64) mask |= 1ull << (k + u);
+              n += in ? 1 : 0;
             }
-            const float cut = law_cutoff_f<LAW>(C, si, fabsf(pj[q].w)) + skin;
-            if (r2 < cut * cut) {
-              if (n < kListCap)
-                a.nbr[static_cast<size_t>(n) * SS + s] =
-                    tt[q] | static_cast<int>(list_offset_code(oo[q], D) << kListSlotBits);
-              ++n;
-            }
+            k += min(kListAhead, en - t0);
           }
-        }
+        });
+        a.nmask[s] = mask;
         a.ncnt[s] = n < kListCap ? n : kListCap;
         if (D == 2) {
           a.pk[s].z = uref_pack2(C.uq_scale, ui[0], ui[1]);  // list reference in the record
@@ -418,77 +456,117 @@ __global__ void __launch_bounds__(kTile, kListMinBlocks<D>) k_skin_lists(SkinArg
   }
 }
 
-// After a list build, the lists of each warp of the force kernel (32 cells = 64 slots from a
+// After k_skin_lists, the lists of each warp of the force kernel (32 cells = 64 slots from a
 // 64-aligned first slot w0) as one contiguous range in the warp's flattened order (element by
 // element, each list in order) at w0 * kListCap, with the owner (element of the warp) of every
 // entry, each element's start in the range (lstart) and the warp's entry count (lwarp): the force
-// kernel then copies a warp's entries and owners with a few 16-byte copies per lane. One block of
-// 128 threads per tile of kTile slots (4 warps of 64 slots), rebuilding colonies only; each warp
-// assembles segments of kFlatSeg entries in shared memory and stores them with 16-byte stores.
+// kernel then copies a warp's entries and owners with a few 16-byte copies per lane. A thread per slot
+// of a tile, rebuilding colonies only; the two warps of 64 slots assemble segments of kFlatSeg entries
+// in shared memory and store them with 16-byte stores.
 constexpr int kFlatSeg = 1024;
+constexpr int kFlatAhead = 4;  // entries whose slots a thread has in flight
 
-__global__ void __launch_bounds__(128) k_list_flatten(SkinArgs a) {
+template <int D, int LAW>
+__global__ void __launch_bounds__(kTile) k_list_flatten(SkinArgs a) {
   enter_step_kernel();
-  __shared__ __align__(16) int s_ent[4][kFlatSeg];
-  __shared__ __align__(16) unsigned char s_own[4][kFlatSeg];
+  if (a.any_rebuild && a.any_rebuild[*a.ts_dev & 1] == 0) return;  // uniform
+  constexpr int NU = kTile / 64;
+  __shared__ __align__(16) int s_ent[NU][kFlatSeg];
+  __shared__ __align__(16) unsigned char s_own[NU][kFlatSeg];
+  __shared__ int s_tot[kTile / 32];
   const int total = a.tiles[a.B];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, unit = threadIdx.x >> 6, el = threadIdx.x & 63;
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int c = colony_of_tile(a.tiles, a.B, t);
     if (!a.skin[c].rebuild_now) continue;  // uniform per block
     const ColonyConst &C = a.col[c];
-    const int s0 = C.slot_base + (t - a.tiles[c]) * kTile + 2 * threadIdx.x;
+    const int s = C.slot_base + (t - a.tiles[c]) * kTile + static_cast<int>(threadIdx.x);
     const int nslot = a.cnt[c].nslot;
-    const int2 n = s0 < C.slot_base + nslot ? *reinterpret_cast<const int2 *>(a.ncnt + s0) : make_int2(0, 0);
-    const int cnt = n.x + n.y;
-    int inc = cnt;
+    const bool used = s < C.slot_base + nslot;
+    const int n = used ? a.ncnt[s] : 0;
+    const unsigned long long mask = used ? a.nmask[s] : 0ull;
+    const int home = used ? a.sbin[s] : 0;
+    int inc = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += v;
     }
-    const int T = __shfl_sync(0xffffffffu, inc, 31);
-    const int st0 = inc - cnt, st1 = st0 + n.x;
-    const int w0 = s0 - 2 * lane;
-    if (s0 < C.slot_base + C.slot_cap)
-      *reinterpret_cast<ushort2 *>(a.lstart + s0) =
-          make_ushort2(static_cast<unsigned short>(st0), static_cast<unsigned short>(st1));
-    if (lane == 31) a.lwarp[w0 >> 6] = inc;
+    if (lane == 31) s_tot[wid] = inc;
+    __syncthreads();
+    const int T = s_tot[2 * unit] + s_tot[2 * unit + 1];
+    const int st = (wid & 1 ? s_tot[wid - 1] : 0) + inc - n;
+    const int w0 = s - el;
+    if (s < C.slot_base + C.slot_cap) a.lstart[s] = static_cast<unsigned short>(st);
+    if (el == 0) a.lwarp[w0 >> 6] = T;
     if (t == a.tiles[c] && threadIdx.x == 0) a.skin[c].nslot_built = nslot;
     int *dst = a.lflat + static_cast<size_t>(w0) * kListCap;
     unsigned char *dso = a.oflat + static_cast<size_t>(w0) * kListCap;
-    int *se = s_ent[wid];
-    unsigned char *so = s_own[wid];
-    for (int S = 0; S < T; S += kFlatSeg) {  // uniform per warp
+    int *se = s_ent[unit];
+    unsigned char *so = s_own[unit];
+    int most = 0;
+#pragma unroll
+    for (int u = 0; u < NU; ++u) most = max(most, s_tot[2 * u] + s_tot[2 * u + 1]);
+    for (int S = 0; S < most; S += kFlatSeg) {  // uniform per block
       const int E = min(T, S + kFlatSeg);
-      // this lane's entries of the segment, read row by row (the list rows are SS apart)
+      if (n > 0 && st < E && st + n > S) {
+        // the element's entries of the segment, from its candidate mask
+        int bi[D];
+        bin_decode<D>(C, home, bi);
+        int k = 0, m = 0;  // candidate, entry
+        auto put = [&](int at, int slot, int m0, int m1, int row) {
+          if (m < n && st + m >= S && st + m < E) {
+            const int l = at < m0 ? 0 : (at >= m1 ? 2 : 1);
+            se[st + m - S] = slot | static_cast<int>(list_offset_code(row * 3 + l, D) << kListSlotBits);
+            so[st + m - S] = static_cast<unsigned char>(el);
+          }
+          ++m;
+        };
+        candidate_rows<D>(C, a.range, bi, [&](int rs, int re, int m0, int m1, int row) {
+          const int len = re - rs;
+          if (k < 64) {
+            unsigned long long bits = mask >> k;
+            if (len < 64) bits &= (1ull << len) - 1ull;
+            while (bits) {
+              int at[kFlatAhead], slot[kFlatAhead];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int st = j ? st1 : st0, nj = j ? n.y : n.x;
-        const int k0 = max(S - st, 0), k1 = min(E - st, nj);
-        for (int k = k0; k < k1; k += 4) {
-          int v[4];
+              for (int u = 0; u < kFlatAhead; ++u) {
+                at[u] = bits ? rs + __ffsll(static_cast<long long>(bits)) - 1 : -1;
+                bits &= bits - 1ull;
+                slot[u] = at[u] >= 0 ? candidate_slot<D>(a, at[u], D == 2 ? __ldg(&a.brec[at[u]].z) : 0.0f) : 0;
+              }
 #pragma unroll
-          for (int q = 0; q < 4; ++q) v[q] = k + q < k1 ? __ldg(a.nbr + static_cast<size_t>(k + q) * a.SS + s0 + j) : 0;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (k + q < k1) {
-              se[st + k + q - S] = v[q];
-              so[st + k + q - S] = static_cast<unsigned char>(2 * lane + j);
+              for (int u = 0; u < kFlatAhead; ++u)
+                if (at[u] >= 0) put(at[u], slot[u], m0, m1, row);
             }
           }
-        }
+          if (k + len > 64) {  // candidates past the mask, tested again
+            const float4 pi = a.pk[s];
+            float ui[D];
+#pragma unroll
+            for (int d = 0; d < D; ++d) ui[d] = pk_c(pi, d);
+            for (int at = rs + max(64 - k, 0); at < re; ++at) {
+              const int l = at < m0 ? -1 : (at >= m1 ? 1 : 0);
+              const int slot = candidate_slot<D>(a, at, a.brec[at].z);
+              if ((slot >> 1) != (s >> 1) &&
+                  list_reaches<D, LAW>(C, ui, fabsf(pi.w), a.skin[c].skin, a.brec[at], row, l))
+                put(at, slot, m0, m1, row);
+            }
+          }
+          k += len;
+        });
       }
-      __syncwarp();
+      __syncthreads();
       // 16-byte stores of the segment (rounded up to 4 entries / 16 owners: within the warp's
       // 64 kListCap entries and within the shared segment)
       const int ne = (E - S + 3) >> 2, no = (E - S + 15) >> 4;
-      for (int i = lane; i < ne; i += 32)
+      for (int i = el; i < ne; i += 64)
         *reinterpret_cast<int4 *>(dst + S + 4 * i) = *reinterpret_cast<const int4 *>(se + 4 * i);
-      for (int i = lane; i < no; i += 32)
+      for (int i = el; i < no; i += 64)
         *reinterpret_cast<int4 *>(dso + S + 16 * i) = *reinterpret_cast<const int4 *>(so + 16 * i);
-      __syncwarp();
+      __syncthreads();
     }
+    __syncthreads();  // s_tot is free for the next tile
   }
 }
 
@@ -652,20 +730,26 @@ __global__ void __launch_bounds__(kFreshBlock) k_fresh_pairs(SkinArgs a) {
   }
 }
 
+template <int D, int LAW>
+void lists_dl(const SkinArgs &a, int grid, cudaStream_t s) {
+  launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, LAW>, a);
+  launch_step(a.dep, grid, kTile, 0, s, k_list_flatten<D, LAW>, a);
+}
+
 template <int D>
 void lists_d(const SkinArgs &a, int law, int grid, cudaStream_t s) {
   switch (law) {
     case CIL_FORCE_LJ_WCA:
-      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_LJ_WCA>, a);
+      lists_dl<D, CIL_FORCE_LJ_WCA>(a, grid, s);
       break;
     case CIL_FORCE_SOFTCORE:
-      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_SOFTCORE>, a);
+      lists_dl<D, CIL_FORCE_SOFTCORE>(a, grid, s);
       break;
     case CIL_FORCE_SC:
-      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_SC>, a);
+      lists_dl<D, CIL_FORCE_SC>(a, grid, s);
       break;
     default:
-      launch_step(a.dep, grid, kTile, 0, s, k_skin_lists<D, CIL_FORCE_HERTZ>, a);
+      lists_dl<D, CIL_FORCE_HERTZ>(a, grid, s);
       break;
   }
 }
@@ -701,8 +785,6 @@ void launch_skin_rebin(const SkinArgs &a, int dim, int grid, cudaStream_t s) {
   else
     launch_step(a.dep, grid, kTile, 0, s, k_skin_rebin<3>, a);
 }
-
-void launch_list_flatten(const SkinArgs &a, int grid, cudaStream_t s) { launch_step(a.dep, grid, 128, 0, s, k_list_flatten, a); }
 
 void launch_skin_lists(const SkinArgs &a, int dim, int law, int grid, cudaStream_t s) {
   if (dim == 2)
