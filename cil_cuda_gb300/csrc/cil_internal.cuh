@@ -59,7 +59,6 @@ struct ColonySkin {
   int nfresh;          // entries in the fresh list
   int nrebuild;        // list rebuilds so far
   int ntrip;           // rebuilds requested by the guard
-  unsigned maxdisp2;   // largest |u - uref|^2 of the last step (float bits)
   int list_overflow;   // elements whose list was truncated at the last build
   int last_interval;   // steps between the last two rebuilds
   long long npairs;    // list entries at the last build
@@ -86,8 +85,6 @@ struct SchedState {
   float occ_sum;          // sum over elements of their home-bin occupancy at the last list build
   int occ_count;          // elements counted into occ_sum
   float occ_max;          // largest bin occupancy at the last list build (float bits, atomicMax)
-  float step_sum;         // sum over elements of |displacement| in the last step
-  float step_max;         // largest |displacement| in the last step (float bits, atomicMax)
   float div_rate;         // divisions per cell per step, moving average over ~100 steps
   float apo_rate;         // apoptoses per cell per step, moving average over ~100 steps
   float trip_share;       // share of guard-triggered rebuilds, moving average over ~10 rebuilds

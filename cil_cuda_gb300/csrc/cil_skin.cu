@@ -55,27 +55,36 @@ __device__ __forceinline__ bool nb_bin(const ColonyConst &C, const int *bi, cons
 
 __device__ __forceinline__ float log_disp(float d) { return 0.25f * log10f(fmaxf(d, 1e-8f)) + 1.0f; }
 
+// What the decision of a colony reads, loaded before the first store of the kernel (the compiler
+// cannot move a load across a store that may alias it, and each would wait for memory in turn).
+struct BeginState {
+  ColonySkin S;
+  SchedState Q;
+  int ncell;
+  long long ndiv, napo;
+};
+
 // per colony (lane 0 of the colony's warp): the rebuild decision and, at a rebuild, the
-// scheduler's features; returns whether the colony rebuilds this step
-__device__ __forceinline__ int skin_begin_colony(const SkinArgs &a, int c) {
+// scheduler's features (into x); returns whether the colony rebuilds this step. dmax, smax, ssum: the
+// last force pass's displacement statistics.
+__device__ __forceinline__ int skin_begin_colony(const SkinArgs &a, int c, const BeginState &B, float dmax, float smax,
+                                                 float ssum) {
   ColonySkin &S = a.skin[c];
-  int need = S.need;
+  int need = B.S.need;
   if (a.force_rebuild) need |= 8;
-  if (S.interval > 0 && S.steps_since >= S.interval) need |= 4;
+  if (B.S.interval > 0 && B.S.steps_since >= B.S.interval) need |= 4;
   const int now = need != 0 ? 1 : 0;
   S.rebuild_now = now;
   SchedState &Q = a.sched[c];
-  const ColonyCounters &K = a.cnt[c];
-  const float n = fmaxf(static_cast<float>(K.ncell), 1.0f);
-  {
-    // event rates per cell per step, moving averages over ~100 steps
-    const float dr = static_cast<float>(K.ndiv_total - Q.ndiv_prev) / n;
-    const float ar = static_cast<float>(K.napo_total - Q.napo_prev) / n;
-    Q.ndiv_prev = K.ndiv_total;
-    Q.napo_prev = K.napo_total;
-    Q.div_rate = 0.99f * Q.div_rate + 0.01f * dr;
-    Q.apo_rate = 0.99f * Q.apo_rate + 0.01f * ar;
-  }
+  const float n = fmaxf(static_cast<float>(B.ncell), 1.0f);
+  // event rates per cell per step, moving averages over ~100 steps
+  const float dr = static_cast<float>(B.ndiv - B.Q.ndiv_prev) / n;
+  const float ar = static_cast<float>(B.napo - B.Q.napo_prev) / n;
+  const float div_rate = 0.99f * B.Q.div_rate + 0.01f * dr, apo_rate = 0.99f * B.Q.apo_rate + 0.01f * ar;
+  Q.ndiv_prev = B.ndiv;
+  Q.napo_prev = B.napo;
+  Q.div_rate = div_rate;
+  Q.apo_rate = apo_rate;
   if (now) {
     // features of the decision taken at this rebuild:
     //   0 log(cells)/14              1 mean home-bin occupancy/10   2 max bin occupancy/20
@@ -85,38 +94,35 @@ __device__ __forceinline__ int skin_begin_colony(const SkinArgs &a, int c) {
     //   9 largest displacement from the list reference / (skin/2)
     //   10 share of guard-triggered rebuilds   11 fresh elements / elements x10
     const float ne = 2.0f * n;
-    const float disp = sqrtf(__uint_as_float(S.maxdisp2));
-    const float occn = fmaxf(static_cast<float>(Q.occ_count), 1.0f);
+    const float disp = sqrtf(dmax);
+    const float occn = fmaxf(static_cast<float>(B.Q.occ_count), 1.0f);
+    const float trip = 0.9f * B.Q.trip_share + ((need & 1) ? 0.1f : 0.0f);
     float *x = Q.features;
     x[0] = logf(n) / 14.0f;
-    x[1] = Q.occ_sum / occn / 10.0f;
-    x[2] = Q.occ_max / 20.0f;
-    x[3] = log_disp(Q.step_sum / ne);
-    x[4] = log_disp(Q.step_max);
-    x[5] = Q.div_rate * 1e4f;
-    x[6] = Q.apo_rate * 1e4f;
-    x[7] = S.skin;
-    x[8] = log1pf(static_cast<float>(S.steps_since)) / 5.0f;
-    x[9] = S.skin > 0.0f ? disp / (0.5f * S.skin) : 0.0f;
-    Q.trip_share = 0.9f * Q.trip_share + ((need & 1) ? 0.1f : 0.0f);
-    x[10] = Q.trip_share;
-    x[11] = 10.0f * static_cast<float>(S.nfresh) / ne;
+    x[1] = B.Q.occ_sum / occn / 10.0f;
+    x[2] = B.Q.occ_max / 20.0f;
+    x[3] = log_disp(ssum / ne);
+    x[4] = log_disp(smax);
+    x[5] = div_rate * 1e4f;
+    x[6] = apo_rate * 1e4f;
+    x[7] = B.S.skin;
+    x[8] = log1pf(static_cast<float>(B.S.steps_since)) / 5.0f;
+    x[9] = B.S.skin > 0.0f ? disp / (0.5f * B.S.skin) : 0.0f;
+    x[10] = trip;
+    x[11] = 10.0f * static_cast<float>(B.S.nfresh) / ne;
+    Q.trip_share = trip;
     Q.occ_sum = 0.0f;
     Q.occ_max = 0.0f;
     Q.occ_count = 0;
-    if (need & 1) S.ntrip += 1;
-    S.last_interval = S.steps_since;
-    S.steps_since = 0;
-    S.nrebuild += 1;
+    if (need & 1) S.ntrip = B.S.ntrip + 1;
+    S.last_interval = B.S.steps_since;
+    S.nrebuild = B.S.nrebuild + 1;
     S.nfresh = 0;
     S.npairs = 0;
     S.list_overflow = 0;
     S.need = 0;
   }
-  Q.step_sum = 0.0f;
-  Q.step_max = 0.0f;
-  S.steps_since += 1;
-  S.maxdisp2 = 0u;
+  S.steps_since = (now ? 0 : B.S.steps_since) + 1;
   return now;
 }
 
@@ -124,6 +130,19 @@ __device__ __forceinline__ int skin_begin_colony(const SkinArgs &a, int c) {
 // network on the colony's features sets the skin of the new lists and the cadence
 __global__ void k_skin_begin(SkinArgs a) {
   enter_step_kernel();
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const bool have = c < a.B;  // uniform per warp
+  BeginState bs;
+  StatPart part{};
+  if (have) {
+    part = a.spart[c * kStatSlots + (threadIdx.x & 31)];
+    bs.S = a.skin[c];
+    bs.Q = a.sched[c];
+    bs.ncell = a.cnt[c].ncell;
+    bs.ndiv = a.cnt[c].ndiv_total;
+    bs.napo = a.cnt[c].napo_total;
+  }
+  const int parity = *a.ts_dev & 1;
   if (blockIdx.x == 0 && a.tiles_used_out) {
     // the step's tile tables (slots: kTile per tile; slot pairs: pair_tile slots per tile),
     // block 0, before any thread returns
@@ -167,36 +186,25 @@ __global__ void k_skin_begin(SkinArgs a) {
       a.tiles_pairs_out[a.B] = carry1;
     }
   }
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (c >= a.B) return;  // uniform per warp
+  if (!have) return;
   const int lane = threadIdx.x & 31;
   int now = 0;
-  {
-    // the last force pass's displacement statistics, folded from the colony's slots
-    StatPart &P = a.spart[c * kStatSlots + lane];
-    const unsigned dmax = __reduce_max_sync(0xffffffffu, P.dmax);
-    const unsigned smax = __reduce_max_sync(0xffffffffu, P.smax);
-    float ssum = P.ssum;
+  // the last force pass's displacement statistics, folded from the colony's slots
+  const unsigned dmax = __reduce_max_sync(0xffffffffu, part.dmax);
+  const unsigned smax = __reduce_max_sync(0xffffffffu, part.smax);
+  float ssum = part.ssum;
 #pragma unroll
-    for (int q = 16; q > 0; q >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, q);
-    P.dmax = 0u;
-    P.smax = 0u;
-    P.ssum = 0.0f;
-    if (lane == 0) {
-      a.skin[c].maxdisp2 = dmax;
-      a.sched[c].step_max = __uint_as_float(smax);
-      a.sched[c].step_sum = ssum;
-    }
-  }
+  for (int q = 16; q > 0; q >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, q);
+  a.spart[c * kStatSlots + lane] = StatPart{};
   if (lane == 0) {
-    now = skin_begin_colony(a, c);
-    if (now && a.any_rebuild) atomicOr(&a.any_rebuild[*a.ts_dev & 1], 1);
+    now = skin_begin_colony(a, c, bs, __uint_as_float(dmax), __uint_as_float(smax), ssum);
+    if (now && a.any_rebuild) atomicOr(&a.any_rebuild[parity], 1);
     if (a.use_cond) {
       // the last colony to decide sets the step's rebuild node (one caller: no racing sets)
       __threadfence();
       if (atomicAdd(&a.any_rebuild[2], 1) == a.B - 1) {
         __threadfence();
-        const int any = atomicOr(&a.any_rebuild[*a.ts_dev & 1], 0);
+        const int any = atomicOr(&a.any_rebuild[parity], 0);
         cudaGraphSetConditional(a.cond, any != 0 ? 1u : 0u);
         if (any) atomicAdd(&a.any_rebuild[3], 1);
         atomicExch(&a.any_rebuild[2], 0);
