@@ -11,9 +11,12 @@
 // Order inside a bin: ascending element id, as cil_bins reports it. It comes out of a stable
 // LSD radix sort of the bin keys (keys are produced in element order): one pass of 10-bit
 // digits when the grid has at most 1024 bins, two passes otherwise. Each pass is a per-tile
-// digit histogram, one exclusive scan over (digit, tile), and a scatter in which each tile
-// ranks its elements stably with warp matches. The work is linear in the element count
-// whatever the bin occupancy; a grid collapsed to one bin costs the same as any other.
+// digit histogram (the first with the keys), one exclusive scan over (digit, tile), and a scatter in
+// which each tile ranks its elements stably with warp matches. The work is linear in the element count
+// whatever the bin occupancy; a grid collapsed to one bin costs the same as any other. Bound by
+// latency (20 MB move for 1M elements): a tile is shared by eight warps, each ranking its part against
+// its own counters, and the launches overlap (launch_step). 1M elements in 0.46M bins: NA1 us a call;
+// with one warp per tile and 14 launches 145 us.
 //
 // Limits: at most kMaxElems elements and kMaxBins bins per call (about 14.7 MB of scratch,
 // held by every GPU that loads the library until the process exits).
@@ -39,7 +42,9 @@ constexpr int kNaTile = 256;
 constexpr int kNaScan = 1024;        // entries per scan block
 constexpr int kDigitBits = 10;       // radix digit: 1024 buckets
 constexpr int kDigits = 1 << kDigitBits;
-constexpr int kRadixTile = 2048;     // elements per radix tile (one warp, 64 chunks of 32)
+constexpr int kRadixTile = 2048;     // elements per radix tile (8 warps, 8 chunks of 32 each)
+constexpr int kRadixWarps = kNaTile / 32;
+constexpr int kRadixChunks = kRadixTile / kNaTile;
 constexpr int kMaxTiles = kMaxElems / kRadixTile;
 constexpr int kIdBits = 20;          // element id field of a packed pass-0 entry (kMaxElems = 2^20)
 constexpr int kMaxDevices = 64;
@@ -50,7 +55,8 @@ static __device__ __align__(256) int g_na_key[kMaxElems];                 // bin
 static __device__ __align__(256) int g_na_alt[kMaxElems];                 // pass 0 out: id | high digit << 20
 static __device__ __align__(256) int g_na_count[kMaxBins + kNaScan];      // bin counts (+ end sentinel room)
 static __device__ __align__(256) int g_na_hist[kDigits * kMaxTiles];      // [digit][tile] counts -> offsets
-static __device__ __align__(256) int g_na_part[kMaxBins / kNaScan + 1];   // scan partials
+static __device__ __align__(256) int g_na_part[kMaxBins / kNaScan + 1];   // scan partials (bin counts)
+static __device__ __align__(256) int g_na_part_hist[kMaxTiles];           // scan partials (first histogram)
 
 struct Scratch {
   int *key;
@@ -58,6 +64,7 @@ struct Scratch {
   int *count;
   int *hist;
   int *part;
+  int *part_hist;
 };
 
 struct NaGeom {
@@ -67,22 +74,40 @@ struct NaGeom {
 };
 
 __global__ void k_na_clear(int *count, int nbins_pad) {
+  enter_step_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nbins_pad; i += gridDim.x * blockDim.x) count[i] = 0;
 }
 
-__global__ void k_na_keys(const double *__restrict__ pos, int n, NaGeom g, int *key, int *count) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  int ls[3] = {0, 0, 0};
-  for (int d = 0; d < g.dim; ++d) {
-    const double x = pos[static_cast<size_t>(e) * g.dim + d];
-    int v = static_cast<int>(__dmul_rn(__dmul_rn(x, g.ih[d]), static_cast<double>(g.ns[d])));
-    v = v < g.ns[d] - 1 ? v : g.ns[d] - 1;
-    ls[d] = v > 0 ? v : 0;
+// per radix tile: the elements' bins, the bin counts, and the histogram of the first pass's digits,
+// written digit-major (hist[digit * ntiles + tile]) so that one exclusive scan gives every (digit, tile)
+// its first output position
+__global__ void __launch_bounds__(kNaTile) k_na_keys(const double *__restrict__ pos, int n, NaGeom g, int ntiles, int *key,
+                                                     int *count, int *hist) {
+  enter_step_kernel();
+  __shared__ int h[kDigits];
+  for (int d = threadIdx.x; d < kDigits; d += kNaTile) h[d] = 0;
+  __syncthreads();
+  const int e0 = blockIdx.x * kRadixTile + threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < kRadixChunks; ++q) {
+    const int e = e0 + q * kNaTile;
+    if (e >= n) continue;
+    int ls[3] = {0, 0, 0};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      if (d >= g.dim) continue;
+      const double x = pos[static_cast<size_t>(e) * g.dim + d];
+      int v = static_cast<int>(__dmul_rn(__dmul_rn(x, g.ih[d]), static_cast<double>(g.ns[d])));
+      v = v < g.ns[d] - 1 ? v : g.ns[d] - 1;
+      ls[d] = v > 0 ? v : 0;
+    }
+    const int b = g.dim == 2 ? ls[0] * g.ns[1] + ls[1] : (ls[0] * g.ns[1] + ls[1]) * g.ns[2] + ls[2];
+    key[e] = b;
+    atomicAdd(count + b, 1);
+    atomicAdd(h + (b & (kDigits - 1)), 1);
   }
-  const int b = g.dim == 2 ? ls[0] * g.ns[1] + ls[1] : (ls[0] * g.ns[1] + ls[1]) * g.ns[2] + ls[2];
-  key[e] = b;
-  atomicAdd(count + b, 1);
+  __syncthreads();
+  for (int d = threadIdx.x; d < kDigits; d += kNaTile) hist[d * ntiles + blockIdx.x] = h[d];
 }
 
 __device__ __forceinline__ int na_block_scan(int v, int *total) {
@@ -110,34 +135,44 @@ __device__ __forceinline__ int na_block_scan(int v, int *total) {
   return base + inc - v;
 }
 
-// per scan block: the sum of its kNaScan counts
-__global__ void k_na_partial(const int *count, int *part) {
-  const int4 v = reinterpret_cast<const int4 *>(count + blockIdx.x * kNaScan)[threadIdx.x];
+// sums of the scan blocks (kNaScan entries) of a (na blocks, sums to pa) and of b (the other blocks, to pb)
+__global__ void __launch_bounds__(kNaTile) k_na_partial(const int *a, int na, int *pa, const int *b, int *pb) {
+  enter_step_kernel();
+  const bool first = static_cast<int>(blockIdx.x) < na;
+  const int blk = first ? blockIdx.x : blockIdx.x - na;
+  const int4 v = reinterpret_cast<const int4 *>((first ? a : b) + blk * kNaScan)[threadIdx.x];
   int tot;
   na_block_scan(v.x + v.y + v.z + v.w, &tot);
-  if (threadIdx.x == 0) part[blockIdx.x] = tot;
+  if (threadIdx.x == 0) (first ? pa : pb)[blk] = tot;
 }
 
-// one block: exclusive scan of the partials
-__global__ void k_na_scan_parts(int *part, int nparts) {
-  int carry = 0;
-  for (int base = 0; base < nparts; base += kNaTile) {
-    const int i = base + threadIdx.x;
-    const int v = i < nparts ? part[i] : 0;
-    int tot;
-    const int ex = na_block_scan(v, &tot);
-    if (i < nparts) part[i] = carry + ex;
-    carry += tot;
-  }
+// the sum of the scan blocks before blk (at most about 1000: a few loads per thread)
+__device__ __forceinline__ int na_before(const int *part, int blk) {
+  int v = 0, tot;
+  for (int i = threadIdx.x; i < blk; i += kNaTile) v += part[i];
+  na_block_scan(v, &tot);
+  return tot;
 }
 
-// bin starts from the bin counts and their scanned scan-block sums
-__global__ void k_na_starts(const int *count, const int *part, int nbins, int *bin_start) {
-  const int b0 = blockIdx.x * kNaScan + threadIdx.x * 4;
-  const int4 v = *reinterpret_cast<const int4 *>(count + b0);
+// blocks below na: bin starts from the bin counts; the others: in-place exclusive scan of the (digit,
+// tile) counts
+__global__ void __launch_bounds__(kNaTile) k_na_offsets(const int *count, int na, const int *pa, int nbins, int *bin_start,
+                                                        int *hist, const int *ph) {
+  enter_step_kernel();
+  const bool bins = static_cast<int>(blockIdx.x) < na;
+  const int blk = bins ? blockIdx.x : blockIdx.x - na;
+  const int before = na_before(bins ? pa : ph, blk);
+  int4 *p = reinterpret_cast<int4 *>(const_cast<int *>(bins ? count : hist) + blk * kNaScan) + threadIdx.x;
+  const int4 v = *p;
   int tot;
-  int s = part[blockIdx.x] + na_block_scan(v.x + v.y + v.z + v.w, &tot);
+  int s = before + na_block_scan(v.x + v.y + v.z + v.w, &tot);
+  if (!bins) {
+    *p = make_int4(s, s + v.x, s + v.x + v.y, s + v.x + v.y + v.z);
+    return;
+  }
+  const int b0 = blk * kNaScan + threadIdx.x * 4;
   const int c[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int b = b0 + q;
     if (b <= nbins) bin_start[b] = s;  // bins past nbins are empty: bin_start[nbins] = n
@@ -145,67 +180,74 @@ __global__ void k_na_starts(const int *count, const int *part, int nbins, int *b
   }
 }
 
-// in-place exclusive scan of a count array whose scan-block sums are already scanned in part[]
-__global__ void k_na_offsets(int *v, const int *part) {
-  int4 *p = reinterpret_cast<int4 *>(v + blockIdx.x * kNaScan) + threadIdx.x;
-  const int4 c = *p;
-  int tot;
-  const int s = part[blockIdx.x] + na_block_scan(c.x + c.y + c.z + c.w, &tot);
-  *p = make_int4(s, s + c.x, s + c.x + c.y, s + c.x + c.y + c.z);
-}
+// radix digit of a word in pass `pass` (0: low 10 bits of the key, 1: high 10 bits, read from the
+// packed pass-0 output)
+__device__ __forceinline__ int na_digit(int pass, int v) { return pass == 0 ? (v & (kDigits - 1)) : (v >> kIdBits); }
 
-// radix digit of element i in pass `pass` (0: low 10 bits of the key, 1: high 10 bits, read
-// from the packed pass-0 output)
-__device__ __forceinline__ int na_digit(int pass, const int *src, int i) {
-  const int v = src[i];
-  return pass == 0 ? (v & (kDigits - 1)) : (v >> kIdBits);
-}
-
-// per radix tile: digit histogram, written digit-major (hist[digit * ntiles + tile]) so that
-// one exclusive scan gives every (digit, tile) its first output position
-__global__ void __launch_bounds__(32) k_na_hist(int pass, const int *src, int n, int ntiles, int *hist) {
+// per radix tile: the second pass's digit histogram
+__global__ void __launch_bounds__(kNaTile) k_na_hist(const int *src, int n, int ntiles, int *hist) {
+  enter_step_kernel();
   __shared__ int h[kDigits];
-  const int lane = threadIdx.x;
-  for (int d = lane; d < kDigits; d += 32) h[d] = 0;
-  __syncwarp();
-  const int i0 = blockIdx.x * kRadixTile;
-  const int i1 = min(n, i0 + kRadixTile);
-  for (int i = i0 + lane; i < i1; i += 32) atomicAdd(h + na_digit(pass, src, i), 1);
-  __syncwarp();
-  for (int d = lane; d < kDigits; d += 32) hist[d * ntiles + blockIdx.x] = h[d];
+  for (int d = threadIdx.x; d < kDigits; d += kNaTile) h[d] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kRadixChunks; ++q) {
+    const int i = blockIdx.x * kRadixTile + q * kNaTile + threadIdx.x;
+    if (i < n) atomicAdd(h + na_digit(1, src[i]), 1);
+  }
+  __syncthreads();
+  for (int d = threadIdx.x; d < kDigits; d += kNaTile) hist[d * ntiles + blockIdx.x] = h[d];
 }
 
-// per radix tile, in element order 32 at a time: each element's place is its (digit, tile)
-// offset plus the elements of the same digit before it in the tile (warp match + popcount),
-// so the scatter is stable. Pass 0 of two writes id | high digit << 20 into alt; the last pass
-// writes element ids into the caller's array.
-__global__ void __launch_bounds__(32) k_na_rank_scatter(int pass, int last, const int *src, int n, int ntiles,
-                                                        const int *hist, int *alt, int *elems) {
-  __shared__ int cur[kDigits];
-  const int lane = threadIdx.x;
-  for (int d = lane; d < kDigits; d += 32) cur[d] = hist[d * ntiles + blockIdx.x];
+// Per radix tile, each warp takes kRadixChunks x 32 consecutive elements: an element's rank among
+// those of its digit in the warp's part (warp match + popcount over the warp's own counters, in element
+// order), then the warps' counters become their first places (the (digit, tile) offset plus the earlier
+// warps' counts), so the scatter is stable. Pass 0 of two writes id | high digit << 20 into alt; the
+// last pass writes element ids into the caller's array.
+__global__ void __launch_bounds__(kNaTile) k_na_rank_scatter(int pass, int last, const int *src, int n, int ntiles,
+                                                             const int *hist, int *alt, int *elems) {
+  enter_step_kernel();
+  __shared__ int cur[kRadixWarps][kDigits];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * kRadixTile + w * (kRadixChunks * 32) + lane;
+  int v[kRadixChunks], rank[kRadixChunks];
+#pragma unroll
+  for (int q = 0; q < kRadixChunks; ++q) v[q] = i0 + q * 32 < n ? src[i0 + q * 32] : -1;
+  for (int d = lane; d < kDigits; d += 32) cur[w][d] = 0;
   __syncwarp();
   const unsigned lt = (1u << lane) - 1u;
-  const int i0 = blockIdx.x * kRadixTile;
-  const int i1 = min(n, i0 + kRadixTile);
-  for (int base = i0; base < i1; base += 32) {
-    const int i = base + lane;
-    const bool valid = i < i1;
-    const int v = valid ? src[i] : 0;
-    const int d = valid ? (pass == 0 ? (v & (kDigits - 1)) : (v >> kIdBits)) : -1;
+#pragma unroll
+  for (int q = 0; q < kRadixChunks; ++q) {
+    const bool valid = i0 + q * 32 < n;
+    const int d = valid ? na_digit(pass, v[q]) : -1;
     const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int at = valid ? cur[d] : 0;  // every lane reads before any leader advances
+    const int at = valid ? cur[w][d] : 0;  // every lane reads before any leader advances
     __syncwarp();
-    if (valid && lane == __ffs(peers) - 1) cur[d] = at + __popc(peers);
+    if (valid && lane == __ffs(peers) - 1) cur[w][d] = at + __popc(peers);
     __syncwarp();
-    if (valid) {
-      const int pos = at + __popc(peers & lt);
-      const int id = pass == 0 ? i : (v & ((1 << kIdBits) - 1));
-      if (last)
-        elems[pos] = id;
-      else
-        alt[pos] = id | ((v >> kDigitBits) << kIdBits);
+    rank[q] = at + __popc(peers & lt);
+  }
+  __syncthreads();
+  for (int d = threadIdx.x; d < kDigits; d += kNaTile) {
+    int off = hist[d * ntiles + blockIdx.x];
+#pragma unroll
+    for (int k = 0; k < kRadixWarps; ++k) {
+      const int c = cur[k][d];
+      cur[k][d] = off;
+      off += c;
     }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kRadixChunks; ++q) {
+    const int i = i0 + q * 32;
+    if (i >= n) continue;
+    const int at = cur[w][na_digit(pass, v[q])] + rank[q];
+    const int id = pass == 0 ? i : (v[q] & ((1 << kIdBits) - 1));
+    if (last)
+      elems[at] = id;
+    else
+      alt[at] = id | ((v[q] >> kDigitBits) << kIdBits);
   }
 }
 
@@ -222,7 +264,8 @@ cil_status na_scratch(int dev, Scratch *out) {
         cudaGetSymbolAddress(reinterpret_cast<void **>(&s.alt), g_na_alt) != cudaSuccess ||
         cudaGetSymbolAddress(reinterpret_cast<void **>(&s.count), g_na_count) != cudaSuccess ||
         cudaGetSymbolAddress(reinterpret_cast<void **>(&s.hist), g_na_hist) != cudaSuccess ||
-        cudaGetSymbolAddress(reinterpret_cast<void **>(&s.part), g_na_part) != cudaSuccess)
+        cudaGetSymbolAddress(reinterpret_cast<void **>(&s.part), g_na_part) != cudaSuccess ||
+        cudaGetSymbolAddress(reinterpret_cast<void **>(&s.part_hist), g_na_part_hist) != cudaSuccess)
       return CIL_ERR_CUDA;
     g_na_scratch[dev] = s;
     g_na_ready[dev] = true;
@@ -278,25 +321,24 @@ extern "C" cil_status cil_bin_elements_noalloc(const double *pos, int32_t n_elem
   cil_status st = na_scratch(dev, &sc);
   if (st != CIL_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  k_na_clear<<<(nbins_pad + kNaTile - 1) / kNaTile, kNaTile, 0, s>>>(sc.count, nbins_pad);
-  if (n_elems > 0) k_na_keys<<<(n_elems + kNaTile - 1) / kNaTile, kNaTile, 0, s>>>(pos, n_elems, g, sc.key, sc.count);
-  k_na_partial<<<nparts, kNaTile, 0, s>>>(sc.count, sc.part);
-  k_na_scan_parts<<<1, kNaTile, 0, s>>>(sc.part, nparts);
-  k_na_starts<<<nparts, kNaTile, 0, s>>>(sc.count, sc.part, nbins, bin_start);
+  const int ntiles = (n_elems + kRadixTile - 1) / kRadixTile;
+  const int hparts = ntiles;  // kDigits * ntiles entries, kNaScan per scan block
+  launch_step(false, (nbins_pad + kNaTile - 1) / kNaTile, kNaTile, 0, s, k_na_clear, sc.count, nbins_pad);  // after the caller's work
+  if (n_elems > 0) launch_step(true, ntiles, kNaTile, 0, s, k_na_keys, pos, n_elems, g, ntiles, sc.key, sc.count, sc.hist);
+  launch_step(true, nparts + hparts, kNaTile, 0, s, k_na_partial, sc.count, nparts, sc.part, sc.hist, sc.part_hist);
+  launch_step(true, nparts + hparts, kNaTile, 0, s, k_na_offsets, sc.count, nparts, sc.part, nbins, bin_start, sc.hist,
+              sc.part_hist);
   if (n_elems > 0) {
     // stable radix sort of the keys by bin: one pass of 10-bit digits for grids of at most
     // 1024 bins, two otherwise (ntiles <= 512, so the histogram scan has <= 512 blocks)
-    const int ntiles = (n_elems + kRadixTile - 1) / kRadixTile;
     const int npass = nbins <= kDigits ? 1 : 2;
-    const int hparts = ntiles;  // kDigits * ntiles entries, kNaScan per scan block
-    for (int pass = 0; pass < npass; ++pass) {
-      const int *src = pass == 0 ? sc.key : sc.alt;
-      k_na_hist<<<ntiles, 32, 0, s>>>(pass, src, n_elems, ntiles, sc.hist);
-      k_na_partial<<<hparts, kNaTile, 0, s>>>(sc.hist, sc.part);
-      k_na_scan_parts<<<1, kNaTile, 0, s>>>(sc.part, hparts);
-      k_na_offsets<<<hparts, kNaTile, 0, s>>>(sc.hist, sc.part);
-      k_na_rank_scatter<<<ntiles, 32, 0, s>>>(pass, pass == npass - 1, src, n_elems, ntiles, sc.hist, sc.alt,
-                                              elems);
+    launch_step(true, ntiles, kNaTile, 0, s, k_na_rank_scatter, 0, npass == 1, sc.key, n_elems, ntiles, sc.hist, sc.alt,
+                elems);
+    if (npass == 2) {
+      launch_step(true, ntiles, kNaTile, 0, s, k_na_hist, sc.alt, n_elems, ntiles, sc.hist);
+      launch_step(true, hparts, kNaTile, 0, s, k_na_partial, sc.hist, hparts, sc.part, sc.hist, sc.part);
+      launch_step(true, hparts, kNaTile, 0, s, k_na_offsets, sc.count, 0, sc.part, nbins, bin_start, sc.hist, sc.part);
+      launch_step(true, ntiles, kNaTile, 0, s, k_na_rank_scatter, 1, 1, sc.alt, n_elems, ntiles, sc.hist, sc.alt, elems);
     }
   }
   if (cudaGetLastError() != cudaSuccess) return CIL_ERR_CUDA;
