@@ -15,7 +15,7 @@
 // which each tile ranks its elements stably with warp matches. The work is linear in the element count
 // whatever the bin occupancy; a grid collapsed to one bin costs the same as any other. Bound by
 // latency (20 MB move for 1M elements): a tile is shared by eight warps, each ranking its part against
-// its own counters, and the launches overlap (launch_step). 1M elements in 0.46M bins: NA1 us a call;
+// its own counters, and the launches overlap (launch_step). 1M elements in 0.46M bins: 91 us a call;
 // with one warp per tile and 14 launches 145 us.
 //
 // Limits: at most kMaxElems elements and kMaxBins bins per call (about 14.7 MB of scratch,
