@@ -64,6 +64,7 @@ struct CyConst {
   float boxf[3], halff[3];  // FP32 copies for the range tests
   double half[3];     // box / 2
   float inv_bwf[3];   // bins per length, rounded up
+  float scalef[3];    // and to the nearest
   double inv_bw[3];
   double sigma_core;
   double hz_c;        // (1 - nu^2) / E
@@ -174,7 +175,7 @@ __device__ inline double wrap(double t, double L) { return cil::wrap_bits(t, L);
 __device__ inline int bin_of(const CyConst &C, const double *xd) {
   int b = 0;
   CY_AXES(d, C.D) {
-    int v = static_cast<int>(xd[d] * C.inv_bw[d]);
+    int v = cil::floor_scaled(xd[d], C.scalef[d], [&] { return xd[d] * C.inv_bw[d]; });
     v = v < 0 ? 0 : (v >= C.ns[d] ? C.ns[d] - 1 : v);
     b = b * C.ns[d] + v;
   }
@@ -1579,6 +1580,7 @@ void set_bins(cil_cycle *h, double smax, int ncells) {
       C.bw[d] = 1.0;
       C.inv_bw[d] = 1.0;
     }
+    C.scalef[d] = static_cast<float>(C.inv_bw[d]);
     C.inv_bwf[d] = std::nextafter(static_cast<float>(C.inv_bw[d]), INFINITY);
     h->nbins *= C.ns[d];
   }

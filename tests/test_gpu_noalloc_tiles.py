@@ -50,6 +50,36 @@ def test_tile_edges(gpu_lib, n, dim, bins):
     np.testing.assert_array_equal(elems.cpu().numpy()[:n], want)
 
 
+@pytest.mark.parametrize("L,width", [(1.0, 0.001), (1254.3, 1.31), (3e-5, 1e-6), (7.7e5, 1.0), (100.0, 1.0)])
+def test_positions_next_to_the_bins_edges(gpu_lib, L, width):
+    # one FP64 step to either side of an edge, and parts of an FP32 step: where the FP32 product cannot
+    # tell the bin
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(8)
+    box = np.array([L, 40.0 * width])
+    n = 20000
+    ns0 = int(L / (width + min(box) * 1e-8))
+    x = rng.integers(0, ns0, n) * (L / ns0)
+    x *= 1.0 + rng.choice([0.0, 1e-16, -1e-16, 3e-16, -3e-16, 1e-12, -1e-12, 1e-8, -1e-8, 1e-7, -1e-7, 1e-6, -1e-6], n)
+    x[:4] = [0.0, 5e-324, 1e-40, np.nextafter(L, 0.0)]
+    pos = np.stack([np.clip(x, 0.0, np.nextafter(L, 0.0)), rng.random(n) * box[1]], axis=1)
+    p = torch.from_numpy(pos).cuda()
+    ns, start, elems = _call(torch, p, box, width, 1 << 20) if ns0 * 39 <= 1 << 20 else (None, None, None)
+    if ns is None:  # too many bins along with the other axis: one wide axis less
+        box = np.array([L, 3.2 * width])
+        pos[:, 1] = rng.random(n) * box[1]
+        p = torch.from_numpy(pos).cuda()
+        if ns0 * 3 > 1 << 20:
+            width *= 4.0
+            box[1] = 3.2 * width
+            pos[:, 1] = rng.random(n) * box[1]
+            p = torch.from_numpy(pos).cuda()
+        ns, start, elems = _call(torch, p, box, width, 1 << 20)
+    want_start, want = _expected(pos, box, ns)
+    np.testing.assert_array_equal(start.cpu().numpy()[:len(want_start)], want_start)
+    np.testing.assert_array_equal(elems.cpu().numpy()[:n], want)
+
+
 def test_captured_on_a_stream_of_the_callers(gpu_lib):
     torch = pytest.importorskip("torch")
     n, box = 5000, np.array([120.0, 120.0])
