@@ -20,7 +20,7 @@
 // forces-only mode gives Fc and the pressure, k_dpd_pair the pair dissipative and random forces and
 // the second half kick (into the spare velocity buffer), k_dpd_dis background and pair dissipation
 // at the new velocities and the cell's cycle; then the same divisions and apoptosis.
-// The file is compiled without FMA contraction: outside the forms of "FP64 arithmetic" below, the
+// The file is compiled without FMA contraction: outside the forms of "FP64 arithmetic" (cil_internal.cuh), the
 // arithmetic is that of the host restatement the tests compare with, to a few units of the last place.
 #include <cuda_runtime.h>
 
@@ -42,7 +42,12 @@
 namespace {
 
 using cil::kTile;
+using cil::finite_bits;
+using cil::mid_range;
 using cil::philox4x32_10;
+using cil::rcp_normal;
+using cil::rsqrt_pos;
+using cil::sqrt_from;
 using cil::u32x4;
 
 constexpr double kPi = 3.14159265358979323846;
@@ -263,45 +268,6 @@ __global__ void k_cy_chunk_apply(int *count, int m, const int *part, int *start,
     e += c[q];
   }
 }
-
-// ---------------------------------------------------------------- FP64 arithmetic
-// GB300's FP64 pipe runs 2 lanes a clock per SM (1/64 of FP32), so the kernels below count FP64
-// instructions: one reciprocal square root per root or quotient, products with constants in place
-// of divisions, comparisons and sign tests on bit patterns.
-
-// 1 / sqrt(a) for normal a > 0: the hardware's approximate reciprocal square root y, then the
-// series 1 / sqrt(1 - e) = 1 + e / 2 + 3 e^2 / 8 + ... with e = 1 - a y^2 (its next term is below
-// 2^-53 for a seed good to 2^-18).
-__device__ inline double rsqrt_pos(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = __fma_rn(-(a * y), y, 1.0);
-  return __fma_rn(__fma_rn(0.375, e, 0.5), y * e, y);
-}
-
-// sqrt(a) from y = rsqrt_pos(a): a y and one Newton residual
-__device__ inline double sqrt_from(double a, double y) {
-  const double s = a * y;
-  return __fma_rn(__fma_rn(-s, s, a), 0.5 * y, s);
-}
-
-// 1 / a for normal a: the approximate reciprocal y, then 1 / (1 - e) = 1 + e + e^2 + ... with
-// e = 1 - a y
-__device__ inline double rcp_normal(double a) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = __fma_rn(-a, y, 1.0);
-  return __fma_rn(__fma_rn(e, e, e), y, y);
-}
-
-// positive, and far enough from the ends of the range that the forms above and their products
-// neither overflow nor lose bits (high word: 2^-510 to 2^510)
-__device__ inline bool mid_range(double a) {
-  const int h = __double2hiint(a);
-  return h >= 0x20000000 && h < 0x5fd00000;
-}
-
-__device__ inline bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
 // ---------------------------------------------------------------- bins
 // A counting sort of the cells into bins: k_cy_keys counts (a cell's arrival rank in its bin comes

@@ -23,49 +23,63 @@ namespace cil {
 namespace {
 
 // nint(v / L) (Utils.hpp:173-175) without a division when |v| < L / 4, where v / L lies in
-// (-0.25, 0.25) whatever its rounding: a minimum image leaves v as it is then.
+// (-0.25, 0.25) whatever its rounding: a minimum image leaves v as it is then. L / 4 by its exponent,
+// the comparison on bit patterns.
 __device__ __forceinline__ double min_image(double v, double L) {
-  if (fabs(v) < 0.25 * L) return v;
+  const long long quarter = __double_as_longlong(L) - 0x0020000000000000ll;
+  if ((__double_as_longlong(v) & 0x7fffffffffffffffll) < quarter) return v;
   return v - static_cast<double>(nint(v / L)) * L;
 }
 
-// The law of pair_force with its square root and divisions formed from one reciprocal square
-// root (as pair_f0_fast does in FP32), each within a few units of the last place: GB300's FP64
-// pipe runs 2 lanes a clock per SM, so the law's cost is its count of FP64 instructions.
+// The law of pair_force without its constant factor (pair_scale), with its roots and quotients formed
+// from one reciprocal or reciprocal square root (as pair_f0_fast does in FP32), each within a few units
+// of the last place; 0 out of range. hi = sigma_i / 2, sj = sigma_j. About 20 FP64 instructions for the
+// soft core with the displacement, where the form with sqrt and divisions took 50 and one with the
+// library's rsqrt 28.
 //   soft core: q = 1 / (r rc) gives r / rc = r2 q and 1 / r = rc q
 //   Hertz:     y = 1 / r gives r = r2 y, corrected by one Newton residual because sigma_ij - r
-//              cancels; delta^1.5 = delta (delta / sqrt(delta))
-// The other laws, and separations whose square is out of that form's range, take pair_force.
+//              cancels; delta^1.5 = delta^2 / sqrt(delta)
+//   LJ:        1 / r2
+// The other laws, and squares out of those forms' range, take pair_force.
 template <int LAW>
-__device__ __forceinline__ bool pair_force_rsqrt(double r2, double si, double sj, double eps, double rcs, double &f0,
-                                                 double em, double xi, int shifted) {
-  if (LAW == CIL_FORCE_SOFTCORE || LAW == CIL_FORCE_HERTZ) {
-    const double sij = 0.5 * (si + sj);
-    const double rc = rcs * sij;
-    const double rc2 = rc * rc;
-    const int hi = __double2hiint(r2);  // r2 >= 0: the high word orders it to one part in 2^20
-    if (hi < 0x10000000 || hi >= 0x6fffffff || __double2hiint(rc2) < 0x10000000 || __double2hiint(rc2) >= 0x6fffffff)
-      return pair_force<LAW, double>(r2, si, sj, eps, rcs, f0, em, xi, shifted);
-    if (__double_as_longlong(r2) >= __double_as_longlong(rc2)) return false;
-    if (LAW == CIL_FORCE_SOFTCORE) {
-      const double q = rsqrt(r2 * rc2);
-      const double w = 1.0 - r2 * q;
-      f0 = -eps * w * w * (rc * q);
-    } else {
-      const double y = rsqrt(r2);
-      double r = r2 * y;
-      r = __fma_rn(__fma_rn(-r, r, r2), 0.5 * y, r);
-      const double delta = sij - r;
-      const double sq = __double2hiint(delta) >= 0x10000000 ? delta * rsqrt(delta) : sqrt(delta);
-      f0 = -eps * delta * sq * y;
-    }
-    return true;
-  }
-  return pair_force<LAW, double>(r2, si, sj, eps, rcs, f0, em, xi, shifted);
+__device__ __forceinline__ double pair_scale(double eps) {
+  return LAW == CIL_FORCE_LJ_WCA ? 24.0 * eps : (LAW == CIL_FORCE_SC ? 1.0 : -eps);
 }
 
-// isfinite by the exponent bits (no FP64 comparison)
-__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+template <int LAW>
+__device__ __forceinline__ double pair_force_lean(double r2, double hi, double sj, double eps, double rcs, double em,
+                                                  double xi, int shifted) {
+  const double sij = __fma_rn(0.5, sj, hi);
+  if (LAW == CIL_FORCE_SOFTCORE || LAW == CIL_FORCE_HERTZ) {
+    const double rc = rcs * sij;
+    const double rc2 = rc * rc;
+    if (mid_range(r2) && mid_range(rc2)) {
+      if (__double_as_longlong(r2) >= __double_as_longlong(rc2)) return 0.0;
+      if (LAW == CIL_FORCE_SOFTCORE) {
+        const double q = rsqrt_pos(r2 * rc2);
+        const double w = __fma_rn(-r2, q, 1.0);
+        return (w * w) * (rc * q);
+      }
+      const double y = rsqrt_pos(r2);
+      const double delta = sij - sqrt_from(r2, y);
+      if (mid_range(delta)) return (delta * delta) * (rsqrt_pos(delta) * y);
+      return delta * sqrt(delta) * y;
+    }
+  } else if (LAW == CIL_FORCE_LJ_WCA) {
+    const double sij2 = sij * sij;
+    const double rc2 = sij2 * (rcs * rcs);
+    if (!shifted && mid_range(r2) && mid_range(rc2)) {
+      if (__double_as_longlong(r2) > __double_as_longlong(rc2)) return 0.0;
+      const double ir2 = rcp_normal(r2);
+      const double s2 = sij2 * ir2;
+      const double s6 = s2 * s2 * s2;
+      return (s6 * ir2) * __fma_rn(-2.0, s6, 1.0);
+    }
+  }
+  double f0 = 0.0;
+  const double unit = LAW == CIL_FORCE_LJ_WCA ? 1.0 / 24.0 : (LAW == CIL_FORCE_SC ? eps : -1.0);
+  return pair_force<LAW, double>(r2, 2.0 * hi, sj, unit, rcs, f0, em, xi, shifted) ? f0 : 0.0;
+}
 
 // Forms without lists: back elements whose cell's cycle ends at the coming events (step ts + 1) put it
 // into the colony's due-cell queue, one atomic per warp. Whole warp.
@@ -99,19 +113,19 @@ __device__ __forceinline__ void collect_due(const ForceArgs &a, const ColonyCons
 // and 19 us, with the FP64 pipe 70 % active in the first.
 constexpr int kF64Block = 128;
 constexpr int kF64Near = 512;  // survivors held per warp (16 per element at one lane each)
-constexpr int kF64Seg = 256;   // pairs evaluated before their sums are taken
+constexpr int kF64Seg = 128;   // pairs evaluated before their sums are taken
 template <int D>
 struct F64Warp {
   double res[kF64Seg * D];
   double x[32 * D];
-  double sig[32];
+  double hs[32];  // half diameters
   int tt[kF64Near];
   unsigned char code[kF64Near];
   unsigned char own[kF64Near];
 };
 
-template <int D, int LAW>
-__global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane_bits) {
+template <int D, int LAW, int AHEAD>
+__global__ void __launch_bounds__(kF64Block, 8) k_force_fp64(ForceArgs a_, int lane_bits) {
   enter_step_kernel();
   extern __shared__ __align__(16) unsigned char s_f64[];
   ForceArgs a = a_;
@@ -181,16 +195,25 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
                           : C.motility[1] * nd + spring * rij[d] * 2.0 + rnd[d] * rij[d];
         }
       } else {
-        const double ir = rsqrt(r2);
-        double r = r2 * ir;
-        r = __fma_rn(__fma_rn(-r, r, r2), 0.5 * ir, r);
+        double ir, r;
+        if (mid_range(r2)) {
+          ir = rsqrt_pos(r2);
+          r = sqrt_from(r2, ir);
+        } else {
+          r = sqrt(r2);
+          ir = 1.0 / r;
+        }
         double rest = C.rest0;
         if (C.divide) {
           const int2 cy = a.cyc[s];
-          const int span = cy.y - cy.x;
-          double frac = span > 0 ? static_cast<double>(a.ts - cy.x) / static_cast<double>(span) : 1.0;
-          frac = fmin(1.0, fmax(0.0, frac));
-          rest = C.rest0 + (C.rest1 - C.rest0) * frac;
+          const int span = cy.y - cy.x, age = a.ts - cy.x;
+          double frac = 1.0;  // age / span within [0, 1], the quotient by its residual
+          if (span > 0 && age < span) {
+            const double m = static_cast<double>(span), p = static_cast<double>(age > 0 ? age : 0), im = rcp_normal(m);
+            frac = p * im;
+            frac = __fma_rn(__fma_rn(-frac, m, p), im, frac);
+          }
+          rest = __fma_rn(C.rest1 - C.rest0, frac, C.rest0);
         }
         const double sp = C.kappa * (r - rest);
         const double coef = ((j == 0) ? sp - C.motility[0] : C.motility[1] - sp) * ir;
@@ -219,12 +242,15 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
       box_muller(w[0], w[1], n[0], n[1]);
       if (D == 3) box_muller(w[2], w[3], n[2], n[3]);
 #pragma unroll
-      for (int d = 0; d < D; ++d) F[d] += C.zeta[j] * (C.noise_amp * static_cast<double>(n[d]));
+      for (int d = 0; d < D; ++d) F[d] = __fma_rn(C.zeta[j] * C.noise_amp, static_cast<double>(n[d]), F[d]);
     }
   }
 
   // ---- pair forces
-  const double eps = C.epsilon, rcs = C.rcut_scale;
+  const double eps = C.epsilon, rcs = C.rcut_scale, hs = 0.5 * si;
+  double P[D];  // the pair forces without the law's factor
+#pragma unroll
+  for (int d = 0; d < D; ++d) P[d] = 0.0;
   if (C.single_bin) {
     if (live && sub == 0) {
       // one bin: all elements, minimum image as BoundingBox::distance (Utils.hpp:536-544)
@@ -240,18 +266,16 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
           dx[d] = v;
           r2 += v * v;
         }
-        double f0;
-        if (pair_force_rsqrt<LAW>(r2, si, a.sig[tt], eps, rcs, f0, C.well_eps, C.well_sigma, C.force_shifted)) {
+        const double f0 = pair_force_lean<LAW>(r2, hs, a.sig[tt], eps, rcs, C.well_eps, C.well_sigma, C.force_shifted);
 #pragma unroll
-          for (int d = 0; d < D; ++d) F[d] += f0 * dx[d];
-        }
+        for (int d = 0; d < D; ++d) P[d] = __fma_rn(f0, dx[d], P[d]);
       }
     }
   } else {  // uniform per block
     if (sub == 0) {
 #pragma unroll
       for (int d = 0; d < D; ++d) W.x[el * D + d] = xi[d];
-      W.sig[el] = si;
+      W.hs[el] = hs;
     }
     const int cap = kF64Near >> (5 - lane_bits);  // survivors held per element
     const int nb0 = el * cap;
@@ -290,10 +314,8 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
               dx[d] = xj - W.x[o * D + d];
               r2 += dx[d] * dx[d];
             }
-            double f0 = 0.0;
-            if (!pair_force_rsqrt<LAW>(r2, W.sig[o], __ldg(a.sig + tt), eps, rcs, f0, C.well_eps, C.well_sigma,
-                                       C.force_shifted))
-              f0 = 0.0;
+            const double f0 = pair_force_lean<LAW>(r2, W.hs[o], __ldg(a.sig + tt), eps, rcs, C.well_eps, C.well_sigma,
+                                                   C.force_shifted);
 #pragma unroll
             for (int d = 0; d < D; ++d) W.res[(f - S) * D + d] = f0 * dx[d];
           }
@@ -302,7 +324,7 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
         if (sub == 0) {
           for (int f = max(off, S); f < min(end, E); ++f)
 #pragma unroll
-            for (int d = 0; d < D; ++d) F[d] += W.res[(f - S) * D + d];
+            for (int d = 0; d < D; ++d) P[d] += W.res[(f - S) * D + d];
         }
         __syncwarp();
       }
@@ -317,84 +339,95 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
 #pragma unroll
     for (int d = 0; d < D; ++d) margin[d] = 4.76837158e-07f * (static_cast<float>(C.box[d]) + fabsf(pk_c(me, d)));
     const float rcsf = C.rcs_f, xif = C.well_sigma_f;
-    // the rows of bins (all axes but the last), and per row up to three pieces of the last axis:
-    // one when its three bins are consecutive, each bin of its own at the ends of the axis
+    // the rows of bins (all axes but the last), and per row one range of the last axis where its three
+    // bins are consecutive, each bin of its own at the ends of the axis. A row's range is loaded a row
+    // ahead (of the piece inside, at the ends: the element's own bin and its neighbours inside).
     constexpr int NROW = D == 2 ? 3 : 9;
     const int last = bi[D - 1], nl = C.ns[D - 1];
-    const bool inner = last > 0 && last < nl - 1;
-    for (int row = 0; row < NROW; ++row) {
-      const int oo[3] = {(D == 2 ? row : row / 3) - 1, (D == 2 ? 0 : row % 3) - 1, 0};
-      int code0 = 0, rowbin = 0;
-      bool ok = live;
-      float sh[D];
+    const bool wraps = __any_sync(0xffffffffu, live && (last == 0 || last == nl - 1));
+    const int lo = max(last - 1, 0), hi = min(last + 1, nl - 1);
+    struct Row {
+      const int2 *rng;
+      int st, en, code;
+      bool ok;
+    };
+    auto load_row = [&](int row) {
+      const int oo[2] = {(D == 2 ? row : row / 3) - 1, row % 3 - 1};
+      Row r;
+      r.ok = live && row < NROW;
+      r.code = 0;
+      int rowbin = 0;
 #pragma unroll
       for (int d = 0; d < D - 1; ++d) {
         int v = bi[d] + oo[d];
-        sh[d] = 0.0f;
         if (v < 0) {
-          ok = ok && C.periodic[d];
+          r.ok = r.ok && C.periodic[d];
           v += C.ns[d];
-          code0 |= 1 << (2 * d);
-          sh[d] = -static_cast<float>(C.box[d]);
+          r.code |= 1 << (2 * d);
         } else if (v >= C.ns[d]) {
-          ok = ok && C.periodic[d];
+          r.ok = r.ok && C.periodic[d];
           v -= C.ns[d];
-          code0 |= 2 << (2 * d);
-          sh[d] = static_cast<float>(C.box[d]);
+          r.code |= 2 << (2 * d);
         }
         rowbin = rowbin * C.ns[d] + v;
       }
-      const int2 *rng = a.range + C.bin_base + rowbin * nl;
-      for (int piece = 0; piece < 3; ++piece) {
-        int st = 0, en = 0, code = code0;
-        sh[D - 1] = 0.0f;
-        if (ok) {
-          if (inner) {
-            if (piece == 0) {
-              st = rng[last - 1].x;
-              en = rng[last + 1].y;
-            }
-          } else {
-            int v = last + piece - 1;
-            bool in = true;
-            if (v < 0) {
-              in = C.periodic[D - 1];
-              v += nl;
-              code |= 1 << (2 * (D - 1));
-              sh[D - 1] = -static_cast<float>(C.box[D - 1]);
-            } else if (v >= nl) {
-              in = C.periodic[D - 1];
-              v -= nl;
-              code |= 2 << (2 * (D - 1));
-              sh[D - 1] = static_cast<float>(C.box[D - 1]);
-            }
-            if (in) {
-              st = rng[v].x;
-              en = rng[v].y;
-            }
+      r.rng = a.range + C.bin_base + rowbin * nl;
+      r.st = r.en = 0;
+      if (r.ok) {
+        r.st = r.rng[lo].x;
+        r.en = r.rng[hi].y;
+      }
+      return r;
+    };
+    Row next = load_row(0);
+    for (int row = 0; row < NROW; ++row) {
+      const Row r = next;
+      next = load_row(row + 1);
+      for (int piece = 0; piece < (wraps ? 2 : 1); ++piece) {
+        // piece 0: the bins inside the axis; piece 1: the bin past its end, through the boundary
+        int st = r.st, en = r.en, code = r.code;
+        if (piece == 1) {
+          st = en = 0;
+          if (r.ok && C.periodic[D - 1] && (last == 0 || last == nl - 1)) {
+            const int2 q = r.rng[last == 0 ? nl - 1 : 0];
+            st = q.x;
+            en = q.y;
+            code |= (last == 0 ? 1 : 2) << (2 * (D - 1));
           }
         }
-        for (int tt0 = st; __any_sync(0xffffffffu, tt0 < en); tt0 += L) {
-          const int tt = tt0 + sub;
-          bool near = false;
-          if (tt < en && tt != s && tt != ps) {
-            const float4 p = __ldg(a.rec + tt);
+        float sh[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const int k = (code >> (2 * d)) & 3;
+          sh[d] = k == 0 ? 0.0f : (k == 1 ? -static_cast<float>(C.box[d]) : static_cast<float>(C.box[d]));
+        }
+        for (int tt0 = st; __any_sync(0xffffffffu, tt0 < en); tt0 += AHEAD * L) {
+          float4 p[AHEAD];
+          bool there[AHEAD];
+#pragma unroll
+          for (int u = 0; u < AHEAD; ++u) {
+            const int tt = tt0 + u * L + sub;
+            there[u] = tt < en && tt != s && tt != ps;
+            p[u] = there[u] ? __ldg(a.rec + tt) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          }
+#pragma unroll
+          for (int u = 0; u < AHEAD; ++u) {
             float r2f = 0.0f;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-              const float dx = fmaxf(fabsf((pk_c(p, d) + sh[d]) - pk_c(me, d)) - margin[d], 0.0f);
+              const float dx = fmaxf(fabsf((pk_c(p[u], d) + sh[d]) - pk_c(me, d)) - margin[d], 0.0f);
               r2f += dx * dx;
             }
-            near = pair_maybe_reaches<LAW>(r2f, me.w, p.w, rcsf, xif);
+            const bool near = there[u] && pair_maybe_reaches<LAW>(r2f, me.w, p[u].w, rcsf, xif);
+            const unsigned m = __ballot_sync(0xffffffffu, near);
+            if (near) {
+              const int at = nb0 + cnt + __popc(m & below);
+              W.tt[at] = tt0 + u * L + sub;
+              W.code[at] = static_cast<unsigned char>(code);
+            }
+            cnt += __popc(m & gmask);
           }
-          const unsigned m = __ballot_sync(0xffffffffu, near);
-          if (near) {
-            const int at = nb0 + cnt + __popc(m & below);
-            W.tt[at] = tt;
-            W.code[at] = static_cast<unsigned char>(code);
-          }
-          cnt += __popc(m & gmask);
-          if (__any_sync(0xffffffffu, cnt + L > cap)) {
+          if (__any_sync(0xffffffffu, cnt + AHEAD * L > cap)) {
             __syncwarp();
             flush();
           }
@@ -405,6 +438,8 @@ __global__ void __launch_bounds__(kF64Block) k_force_fp64(ForceArgs a_, int lane
     flush();
   }
   if (!live || sub != 0) return;
+#pragma unroll
+  for (int d = 0; d < D; ++d) F[d] = __fma_rn(pair_scale<LAW>(eps), P[d], F[d]);
 
   // ---- checks, integration, outputs
   bool finite = true;
@@ -1300,12 +1335,12 @@ template <int D, int LAW>
 void launch_dl(const ForceArgs &a, int prec, int tiles, int lane_bits, cudaStream_t s) {
   if (prec == CIL_PREC_FP64) {
     constexpr int bytes = kF64Block / 32 * static_cast<int>(sizeof(F64Warp<D>));
-    static bool attr_set = false;  // per instantiation; the attribute is per function
-    if (!attr_set) {
-      cudaFuncSetAttribute(k_force_fp64<D, LAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-      attr_set = true;
-    }
-    launch_step(true, tiles * (2 << lane_bits), kF64Block, bytes, s, k_force_fp64<D, LAW>, a, lane_bits);
+    static_assert(bytes <= 48 * 1024, "within the default shared memory of a block");
+    // a lane alone with its element has 4 candidates in flight; lanes that share one have one each
+    if (lane_bits == 0)
+      launch_step(true, 2 * tiles, kF64Block, bytes, s, k_force_fp64<D, LAW, 4>, a, lane_bits);
+    else
+      launch_step(true, tiles * (2 << lane_bits), kF64Block, bytes, s, k_force_fp64<D, LAW, 1>, a, lane_bits);
   } else {
     launch_step(true, tiles, kTile, 0, s, k_force_mixed<D, LAW>, a);
   }

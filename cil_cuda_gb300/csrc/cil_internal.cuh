@@ -317,6 +317,45 @@ __device__ __forceinline__ double wrap_bits(double t, double L) {
   return b >= l ? t2 - L : t2;
 }
 
+// ---------------------------------------------------------------- FP64 arithmetic
+// GB300's FP64 pipe runs 2 lanes a clock per SM (1/64 of FP32), so the FP64 kernels count FP64
+// instructions: one reciprocal square root per root or quotient, products with constants in place
+// of divisions, comparisons and sign tests on bit patterns.
+
+// 1 / sqrt(a) for normal a > 0: the hardware's approximate reciprocal square root y, then the
+// series 1 / sqrt(1 - e) = 1 + e / 2 + 3 e^2 / 8 + ... with e = 1 - a y^2 (its next term is below
+// 2^-53 for a seed good to 2^-18).
+__device__ __forceinline__ double rsqrt_pos(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = __fma_rn(-(a * y), y, 1.0);
+  return __fma_rn(__fma_rn(0.375, e, 0.5), y * e, y);
+}
+
+// sqrt(a) from y = rsqrt_pos(a): a y and one Newton residual
+__device__ __forceinline__ double sqrt_from(double a, double y) {
+  const double s = a * y;
+  return __fma_rn(__fma_rn(-s, s, a), 0.5 * y, s);
+}
+
+// 1 / a for normal a: the approximate reciprocal y, then 1 / (1 - e) = 1 + e + e^2 + ... with
+// e = 1 - a y
+__device__ __forceinline__ double rcp_normal(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = __fma_rn(-a, y, 1.0);
+  return __fma_rn(__fma_rn(e, e, e), y, y);
+}
+
+// positive, and far enough from the ends of the range that the forms above and their products
+// neither overflow nor lose bits (high word: 2^-510 to 2^510)
+__device__ __forceinline__ bool mid_range(double a) {
+  const int h = __double2hiint(a);
+  return h >= 0x20000000 && h < 0x5fd00000;
+}
+
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+
 // Colony of a tile: tile_base[c] <= t < tile_base[c+1]
 __device__ __forceinline__ int colony_of_tile(const int *__restrict__ tile_base, int B, int t) {
   int lo = 0, hi = B - 1;
