@@ -48,7 +48,7 @@ struct HostColony {
 }  // namespace
 
 struct GraphSlot {
-  int key;                 // cur | meta << 1 | pu << 2 at the first step, | two steps << 3, | last << 4, lane bits << 5
+  int key;                 // cur | meta << 1 | pu << 2 at the first step, | two steps << 3, | last << 4, lane bits << 5, many << 7
   uint64_t gen;
   cudaGraphExec_t exec;
   int64_t launches;        // kernels in the graph
@@ -93,6 +93,7 @@ struct cil_handle {
   int2 *d_cyc[2] = {nullptr, nullptr};
   float4 *d_rec = nullptr;  // FP64 form: FP32 absolute coordinates and diameter per slot
   int lane_bits = 0;        // FP64 form: log2 of the lanes per element of the force pass
+  bool many = false;        // the list force kernel's form for many cells (set_lane_bits)
   double *d_sigma_c = nullptr;  // canonical diameters [2 * CC]
   bool need_exact = true;       // next rebuild takes the FP64 reference path
   bool due_events = false;      // Philox draws, no crawling/dividing cells: events from the due-cell queues
@@ -807,6 +808,12 @@ void set_lane_bits(cil_handle *h) {
   int b = 0;
   while (b < 3 && elems * (2ll << b) <= 2ll * h->nsm * 4 * 32) ++b;
   h->lane_bits = b;
+  // The list force kernel's default form for more cells than one wave of its first form holds (6
+  // blocks of 128 threads an SM): with a third more warps an SM the pass hides more of its loads (legs
+  // of 1M cells 14.89 -> 14.44 ms, of the 0.4M-cell 3D channel 5.20 -> 5.09, of a sweep of 0.29M 33.8 ->
+  // 33.2), but segments shrink from 544 to 352 entries, which a colony that does not fill the chip pays
+  // for (300 cells 2.80 -> 2.90 ms).
+  h->many = elems / 2 > 6ll * 128 * h->nsm;
 }
 
 // Error bits of the colonies' counters as a status (and the handle's message).
@@ -988,7 +995,8 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
   ForceArgs fa = force_args(h, noise ? (oracle ? 2 : 1) : 0, 1, last ? h->d_vel : nullptr, nullptr);
   fa.heun = heun;
   fa.collect_due = (!oracle && heun != 1) ? 1 : 0;  // the step's events read the due-cell queue
-  launch_force_list(fa, h->D, h->cfg.force_law, h->ptiles, h->list_variant, h->cell_block, h->stream);  // skin mode
+  const int variant = h->list_variant == 0 && h->many ? 4 : h->list_variant;
+  launch_force_list(fa, h->D, h->cfg.force_law, h->ptiles, variant, h->cell_block, h->stream);  // skin mode
   h->launches += 1;
   h->cur = 1 - h->cur;
   if (h->cfg.precision == CIL_PREC_MIXED) h->pu = 1 - h->pu;
@@ -1055,7 +1063,7 @@ void restore_host_state(cil_handle *h, const HostStepState &s) {
 // switched off for the handle and null is returned.
 cudaGraphExec_t steady_graph(cil_handle *h, int nsteps, bool last, int64_t *launches_per_graph) {
   const int key = h->cur | (h->meta << 1) | (h->pu << 2) | ((nsteps == 2 ? 1 : 0) << 3) | ((last ? 1 : 0) << 4) |
-                  (h->lane_bits << 5);
+                  (h->lane_bits << 5) | ((h->many ? 1 : 0) << 7);
   for (auto &gs : h->graphs)
     if (gs.key == key && gs.gen == h->graph_gen) {
       HostStepState s = host_state(h);

@@ -1298,12 +1298,15 @@ template <int D, int LAW>
 void launch_list_dl(const ForceArgs &a, int grid, int variant, int block, cudaStream_t s) {
   // cell-major slots, one thread per cell, the warp's list entries flattened; variants
   // (chunks of 32 entries in flight per warp, CTAs per SM at 256 threads): 0 (4, 3), 1 (2, 3),
-  // 2 (1, 3), 3 (1, 4); block: 128, 256 or 512 threads (cells per block). The reference's
-  // soft-core well is compiled in the default variant only.
+  // 2 (1, 3), 3 (1, 4), 4 (4, 4) in 2D and (2, 4) in 3D, which the default takes for many cells
+  // (set_lane_bits in cil_api.cu); block: 128, 256 or 512 threads (cells per block). The reference's
+  // soft-core well is compiled in the first variant only.
   if (LAW == CIL_FORCE_SC || variant == 0) {
     launch_cells<D, LAW, 4, 3>(a, grid, block, s);
   } else if constexpr (LAW != CIL_FORCE_SC) {
-    if (variant == 1) {
+    if (variant == 4) {
+      launch_cells<D, LAW, D == 2 ? 4 : 2, 4>(a, grid, block, s);
+    } else if (variant == 1) {
       launch_cells<D, LAW, 2, 3>(a, grid, block, s);
     } else if (variant == 2) {
       launch_cells<D, LAW, 1, 3>(a, grid, block, s);
