@@ -56,9 +56,14 @@ __device__ __forceinline__ void place(const ColonyConst &C, const double *master
   for (int d = 0; d < D; ++d) {
     const double a = __dadd_rn(master[d], __dmul_rn(radius, dir[d]));
     const double b = __dadd_rn(master[d], __dmul_rn(-radius, dir[d]));
-    m_out[d] = C.periodic[d] ? wrap_like_fmod(a, C.box[d]) : a;
-    s_out[d] = C.periodic[d] ? wrap_like_fmod(b, C.box[d]) : b;
+    m_out[d] = C.periodic[d] ? wrap_bits(a, C.box[d]) : a;
+    s_out[d] = C.periodic[d] ? wrap_bits(b, C.box[d]) : b;
   }
+}
+
+// the slots of cell g's two elements
+__device__ __forceinline__ int2 cell_slots(const EventArgs &a, int g) {
+  return *reinterpret_cast<const int2 *>(a.slot_of + 2 * static_cast<size_t>(g));
 }
 
 // Division of cell i into i (mother, its slots sb, sf) and k (daughter, new slots s0, s0+1):
@@ -73,10 +78,10 @@ __device__ __forceinline__ void place(const ColonyConst &C, const double *master
 template <int D>
 __device__ void divide_cell(const EventArgs &a, const ColonyConst &C, int c, int i, int k,
                             const double *dir_m, const double *dir_d, int tsw_d, int tsw_m,
-                            int nslot0, int rank) {
+                            int nslot0, int rank, int2 own) {
   const size_t SS = a.SS;
   const int g = C.cell_base + i, gk = C.cell_base + k;
-  const int sb = a.slot_of[2 * g], sf = a.slot_of[2 * g + 1];
+  const int sb = own.x, sf = own.y;
   const int s0 = C.slot_base + nslot0 + 2 * rank;
   const int slots[4] = {sb, sf, s0, s0 + 1};
   // ---- loads
@@ -139,9 +144,15 @@ __device__ void divide_cell(const EventArgs &a, const ColonyConst &C, int c, int
   if (skin) {
     ColonySkin &S = a.skin[c];
     const bool push[4] = {!was_fresh_b, !was_fresh_f, true, true};
-    const int npush = 2 + (was_fresh_b ? 0 : 1) + (was_fresh_f ? 0 : 1);
     if (was_fresh_b || was_fresh_f) atomicOr(&S.need, 2);
-    const int idx0 = atomicAdd(&S.nfresh, npush);
+    // one reservation for the lanes of the warp that are here: two entries each (the daughter's), and
+    // the mother's that were not fresh
+    const unsigned here = __activemask(), below = here & ((1u << (threadIdx.x & 31)) - 1u);
+    const unsigned pb = __ballot_sync(here, push[0]), pf = __ballot_sync(here, push[1]);
+    const int first = __ffs(here) - 1;
+    int idx0 = 0;
+    if (below == 0u) idx0 = atomicAdd(&S.nfresh, 2 * __popc(here) + __popc(pb) + __popc(pf));
+    idx0 = __shfl_sync(here, idx0, first) + 2 * __popc(below) + __popc(pb & below) + __popc(pf & below);
     const unsigned epoch = static_cast<unsigned>(S.nrebuild);
     unsigned long long prev[4];
     bool listed[4];
@@ -515,7 +526,7 @@ __device__ int apo_count(const EventArgs &a, const ColonyConst &C, ColonyCounter
 // leaves tombstones and moves tail cells into the holes. With planned (k_events_due), the
 // counts are committed and k (and, for k <= 32, warp 0's victims sdv / kk) were drawn already.
 __device__ void apo_colony(const EventArgs &a, int c, int D, bool planned = false, int k_planned = 0,
-                           int sdv_planned = 0, int kk_planned = 0) {
+                           int sdv_planned = 0, int kk_planned = 0, int n1_planned = 0) {
   __shared__ int sd[kDeadCap];
   __shared__ int s_n1, s_k;
   const ColonyConst &C = a.col[c];
@@ -527,7 +538,7 @@ __device__ void apo_colony(const EventArgs &a, int c, int D, bool planned = fals
       K.nslot += 2 * add;
       K.ndiv_total += add;
     }
-    s_n1 = K.ncell;
+    s_n1 = planned ? n1_planned : K.ncell;
     s_k = planned ? k_planned : apo_count(a, C, K, K.ncell);
   }
   __syncthreads();
@@ -681,7 +692,7 @@ __global__ void __launch_bounds__(kTile) k_events_exec(EventArgs a_) {
     division_draws<D>(a, i, dm, dd, span_d, span_m, C);
     // crawling/dividing cells: migration spans, the mother's added to her own time (CIL.cu:403, 424)
     const int tm = C.cell_sm ? a.tsw[C.cell_base + i] + span_m : a.ts + span_m;
-    divide_cell<D>(a, C, c, i, n + r, dm, dd, a.ts + span_d, tm, nslot, r);
+    divide_cell<D>(a, C, c, i, n + r, dm, dd, a.ts + span_d, tm, nslot, r, cell_slots(a, C.cell_base + i));
   }
   __syncthreads();  // every division is placed, and visible to the whole block
   apo_colony(a, c, D);
@@ -711,13 +722,15 @@ constexpr int kDueSort = 2048;  // due cells sorted in shared memory (more: in t
 constexpr int kDueRank = 512;   // up to this many: sorted by ranks instead of a sorting network
 
 // Philox mode: the step's events from the due-cell queues, one block per colony. The force pass
-// appended the cells whose cycle ends at this step (in no particular order); the block sorts them by
-// cell index, so the first ndiv_allowed in cell order divide (within the colony's cell and slot room;
-// the ranking of the tile-wise kernels), places the divisions (one thread each: draws, FP64 placement
-// of the four elements, new cycles; daughters take cells n + rank and slots nslot + 2 rank), then the
+// appended the cells whose cycle ends at this step (in no particular order); the block ranks them by
+// cell index (up to kDueRank among themselves, more by a sort), so the first ndiv_allowed in cell order
+// divide (within the colony's cell and slot room; the ranking of the tile-wise kernels), places the
+// divisions (one thread each: draws, FP64 placement of the four elements, new cycles; daughters take
+// cells n + rank and slots nslot + 2 rank), then the
 // colony's apoptoses (apo_colony). The kernel reads the step as *ts_dev + 1; the block that finishes
 // last writes it back (in place of a step-counter launch) and, in skin mode, clears the next step's
 // any-rebuild flag, otherwise writes the tile table over the used slots for the next step's keys.
+// A chain of round trips to memory: what a division needs is asked for as soon as its address is known.
 // In the forms without lists this replaced a step-counter, a counting, a ranking and a placing launch
 // (growth, 0.2M cells: 15.7 us a step and four gaps).
 template <int D>
@@ -728,24 +741,23 @@ __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
   const int c = blockIdx.x;
   const ColonyConst &C = a.col[c];
   ColonyCounters &K = a.cnt[c];
-  __shared__ int s_key[kDueSort], s_sorted[kDueRank];
-  __shared__ int s_allowed;
-  const int n = K.ncell;
-  const int nd = min(K.ndue, n);
+  __shared__ __align__(16) int s_key[kDueSort];
+  // the counters and this thread's entry of the queue in one round trip (what lies past the queue's
+  // entries is not used)
+  const int n = K.ncell, nslot = K.nslot, ndue = K.ndue;
   int *q = a.dueq + C.due_base;  // capacity: a power of two >= cell_cap
+  const int own = static_cast<int>(threadIdx.x) < C.cell_cap ? q[threadIdx.x] : 0;
+  const int nd = min(ndue, n);
+  // room for the cells and for their two element slots each (skin mode appends daughters
+  // behind removed elements until the next slot re-sort)
+  const int room = min(C.cell_cap - n, (C.slot_cap - nslot) / 2);
+  const int allowed = max(min(nd, room), 0);
   int *keys = s_key;
-  if (nd <= kDueRank) {
-    // the keys are distinct cell indices: each one's rank is the number of smaller keys, so
-    // one pass over the shared keys (and two barriers) sorts them
-    for (int i = threadIdx.x; i < nd; i += blockDim.x) s_key[i] = q[i];
+  const bool ranked = nd <= kDueRank;
+  if (ranked) {
+    for (int i = threadIdx.x; i < ((nd + 3) & ~3); i += blockDim.x)
+      s_key[i] = i >= nd ? 0x7fffffff : (i == static_cast<int>(threadIdx.x) ? own : q[i]);
     __syncthreads();
-    for (int i = threadIdx.x; i < nd; i += blockDim.x) {
-      const int v = s_key[i];
-      int r = 0;
-      for (int j = 0; j < nd; ++j) r += s_key[j] < v ? 1 : 0;
-      s_sorted[r] = v;
-    }
-    keys = s_sorted;
   } else {
     int P = 1;
     while (P < nd) P <<= 1;
@@ -758,23 +770,13 @@ __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
     __syncthreads();
     block_bitonic_sort(keys, P);
   }
-  if (threadIdx.x == 0) {
-    // room for the cells and for their two element slots each (skin mode appends daughters
-    // behind removed elements until the next slot re-sort)
-    const int room_cells = C.cell_cap - n;
-    const int room_slots = (C.slot_cap - K.nslot) / 2;
-    const int room = room_cells < room_slots ? room_cells : room_slots;
-    int allowed = nd < room ? nd : room;
-    if (allowed < 0) allowed = 0;
+  if (threadIdx.x == 0) {  // every thread has read the counters
     if (allowed < nd) K.err |= kErrCap;
     K.ndiv_step = nd;
     K.ndiv_allowed = allowed;
     K.ndead = 0;
     K.ndue = 0;  // for the next step's force pass
-    s_allowed = allowed;
   }
-  __syncthreads();
-  const int allowed = s_allowed, nslot = K.nslot;
   // the apoptosis draws depend only on the cell count after the divisions: the last warp draws
   // them (and, for k <= 32, picks the victims) while the other warps place the divisions
   __shared__ int s_k, s_kk, s_vic[32];
@@ -791,12 +793,23 @@ __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
       s_kk = kk;
     }
   }
-  for (int r = threadIdx.x; r < allowed; r += blockDim.x) {
+  for (int r = threadIdx.x; r < (ranked ? nd : allowed); r += blockDim.x) {
     const int i = keys[r];
+    const int2 sl = cell_slots(a, C.cell_base + i);  // on its way during the ranking and the draws
+    int rank = r;
+    if (ranked) {  // the keys are distinct cell indices: a key's rank is the number of smaller ones
+      rank = 0;
+      const int4 *k4 = reinterpret_cast<const int4 *>(s_key);
+      for (int j = 0; 4 * j < nd; ++j) {
+        const int4 v = k4[j];
+        rank += (v.x < i ? 1 : 0) + (v.y < i ? 1 : 0) + (v.z < i ? 1 : 0) + (v.w < i ? 1 : 0);
+      }
+      if (rank >= allowed) continue;
+    }
     double dm[D], dd[D];
     int span_d, span_m;
     division_draws<D>(a, i, dm, dd, span_d, span_m, C);
-    divide_cell<D>(a, C, c, i, n + r, dm, dd, a.ts + span_d, a.ts + span_m, nslot, r);
+    divide_cell<D>(a, C, c, i, n + rank, dm, dd, a.ts + span_d, a.ts + span_m, nslot, rank, sl);
   }
   __syncthreads();  // every division is placed, and visible to the whole block
   if (threadIdx.x == 0) {
@@ -804,8 +817,10 @@ __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
     K.nslot = nslot + 2 * allowed;
     K.ndiv_total += allowed;
   }
-  __syncthreads();
-  apo_colony(a, c, D, true, s_k, s_vic[threadIdx.x & 31], s_kk);
+  if (s_k > 0) {  // uniform
+    __syncthreads();
+    apo_colony(a, c, D, true, s_k, s_vic[threadIdx.x & 31], s_kk, n + allowed);
+  }
   __shared__ int s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -852,7 +867,7 @@ __global__ void k_div_list(EventArgs a_, int c, int n0, int ndiv, const int *mot
     return;
   }
   divide_cell<D>(a, C, c, mothers[r], n0 + r, dirs + (2 * r) * D, dirs + (2 * r + 1) * D, tsws[2 * r],
-                 tsws[2 * r + 1], a.cnt[c].nslot, r);
+                 tsws[2 * r + 1], a.cnt[c].nslot, r, cell_slots(a, C.cell_base + mothers[r]));
 }
 
 // oracle mode: commit divisions, then the sequential removals removeCell(i) in order
