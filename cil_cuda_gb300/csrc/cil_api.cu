@@ -280,7 +280,8 @@ cil_status setup_geometry(cil_handle *h) {
       }
     }
   }
-  if (bin_base != h->NBpad) {
+  bool regrid = bin_base != h->NBpad;  // other bin arrays or scan grid: captured steps hold the old ones
+  if (regrid) {
     cudaFree(h->d_bcount);
     cudaFree(h->d_range);
     cudaFree(h->d_scan_sum);
@@ -306,8 +307,10 @@ cil_status setup_geometry(cil_handle *h) {
   }
   // forms that rebuild every step: up to 4096 scan blocks (4M bins) a block of the scan adds the sums
   // before its own itself: 33 MB read from L2 at most, about a launch's time
-  h->scanned = h->skin_mode;
-  for (int c = 0; c < h->B; ++c) h->scanned = h->scanned || h->cc[c].nbins_pad / kScanItems > 4096;
+  bool scanned = h->skin_mode;
+  for (int c = 0; c < h->B; ++c) scanned = scanned || h->cc[c].nbins_pad / kScanItems > 4096;
+  regrid = regrid || scanned != h->scanned;
+  h->scanned = scanned;
   std::vector<int> scol(h->nscan);
   for (int c = 0; c < h->B; ++c)
     for (int i = 0; i < h->cc[c].nbins_pad / kScanItems; ++i) scol[h->cc[c].scan_base + i] = c;
@@ -316,7 +319,15 @@ cil_status setup_geometry(cil_handle *h) {
   CUDA_TRY(h, cudaMemcpyAsync(h->d_scan_col, scol.data(), sizeof(int) * h->nscan, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaMemcpyAsync(h->d_col, h->cc.data(), sizeof(ColonyConst) * h->B, cudaMemcpyHostToDevice, h->stream));
   h->geometry_ready = true;
-  h->graph_gen += 1;  // captured graphs hold the old bin arrays
+  // The geometry is in device memory, so captured steps go on serving a state uploaded into the same bin
+  // arrays (they were captured again for every upload: 40-70 us of a leg). Those of other arrays make
+  // room; none is in flight, since an upload ends with the stream idle.
+  if (regrid) {
+    h->graph_gen += 1;
+    for (auto &gs : h->graphs)
+      if (gs.exec) cudaGraphExecDestroy(gs.exec);
+    h->graphs.clear();
+  }
   return CIL_OK;
 }
 

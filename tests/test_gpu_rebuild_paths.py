@@ -71,3 +71,36 @@ def test_bins_and_forces_of_small_and_huge_grids(gpu_lib, oracle_lib, box):
     ref = ora.compute_forces()
     assert np.abs(eng.forces(0) - ref).max() <= 1e-12 * max(1.0, np.abs(ref).max())
     eng.close()
+
+
+@pytest.mark.parametrize("precision,skin", [(G.PREC_FP64, 0.0), (G.PREC_MIXED, 0.0), (G.PREC_MIXED, 0.3)])
+def test_captured_steps_across_uploads(gpu_lib, precision, skin):
+    # states of other boxes' fill, diameters and sizes into one engine, in turn: same bin arrays (captured
+    # steps go on), more bins or fewer (captured again); each leg as in an engine of its own
+    p = S.growth_params(box=60.0, dt=1e-3, div_tau_mu=0.2, div_tau_sigma=0.02, apop_rate=0.5)
+    states = [S.disk_colony(n, p, seed=n) for n in (300, 500, 120)]
+    states.append(dict(states[0], sigma=states[0]["sigma"] * 0.5))   # twice the bins per axis
+    order = [0, 0, 1, 3, 1, 2, 3, 0]
+
+    def leg(eng, st):
+        eng.upload(0, **st)
+        eng.step(21)
+        eng.step(8)
+        return eng.download(0)
+
+    def engine():
+        return G.Engine([p], [4000], precision=precision, rng=G.RNG_PHILOX, seed=6, skin=skin)
+
+    eng = engine()
+    for k in order:
+        a = leg(eng, states[k])
+        fresh = engine()
+        b = leg(fresh, states[k])
+        fresh.close()
+        assert a["ncells"] == b["ncells"]
+        np.testing.assert_array_equal(a["tswitch"], b["tswitch"])
+        d = a["pos"] - b["pos"]
+        d -= np.round(d / 60.0) * 60.0
+        assert np.abs(d).max() <= (0.0 if precision == G.PREC_FP64 else 1e-5)
+    assert eng.graph_info()["graph_steps"] > 0
+    eng.close()
