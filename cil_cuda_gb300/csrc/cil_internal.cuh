@@ -911,7 +911,9 @@ __device__ __forceinline__ float mlp_silu(float z) { return z / (1.0f + expf(-z)
 
 // The network on one input, evaluated by one whole warp (every lane calls it): lane l owns
 // hidden units l and l + 32; every lane holds x; both outputs are returned to all lanes.
-// Weights are read from global memory (they stay in L2).
+// Weights are read from global memory (they stay in L2), a row of the hidden layer as 16-byte words with
+// 32 inputs' weights in flight, summed in input order; a word at a time left a wait for every few of the
+// 64 inputs (a sweep rebuilds some colony in most steps).
 __device__ __forceinline__ void mlp_forward_warp(const float *__restrict__ w, const float *x, float *y) {
   const int lane = threadIdx.x & 31;
   float h1[2], h2[2];
@@ -924,10 +926,25 @@ __device__ __forceinline__ void mlp_forward_warp(const float *__restrict__ w, co
     h1[q] = mlp_silu(z);
   }
   float z2[2] = {__ldg(w + kMlpB2 + lane), __ldg(w + kMlpB2 + lane + 32)};
-  for (int v = 0; v < kMlpH; ++v) {
-    const float hv = __shfl_sync(0xffffffffu, v < 32 ? h1[0] : h1[1], v & 31);
+  constexpr int kAhead = 8;  // 16-byte words per row in flight
+  static_assert(kMlpW2 % 4 == 0 && kMlpH % (4 * kAhead) == 0, "rows in 16-byte words");
+  for (int v0 = 0; v0 < kMlpH; v0 += 4 * kAhead) {
+    float4 r[2][kAhead];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) z2[q] += __ldg(w + kMlpW2 + (lane + 32 * q) * kMlpH + v) * hv;
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+        r[q][k] = __ldg(reinterpret_cast<const float4 *>(w + kMlpW2 + (lane + 32 * q) * kMlpH + v0) + k);
+#pragma unroll
+    for (int k = 0; k < 4 * kAhead; ++k) {
+      const int v = v0 + k;
+      const float hv = __shfl_sync(0xffffffffu, v < 32 ? h1[0] : h1[1], v & 31);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float4 &f = r[q][k >> 2];
+        z2[q] += ((k & 3) == 0 ? f.x : (k & 3) == 1 ? f.y : (k & 3) == 2 ? f.z : f.w) * hv;
+      }
+    }
   }
 #pragma unroll
   for (int q = 0; q < 2; ++q) h2[q] = mlp_silu(z2[q]);
