@@ -16,9 +16,9 @@
 //              and the cell's cycle (ODEs, division test);
 //   divisions  k_cy_divide (daughters appended in mother order; the step's counts);
 //   apoptosis  k_cy_mark / scan / k_cy_compact (only with apoptosis on).
-// The DPD integrator: k_cy_keys makes the first half kick and the drift, k_cy_force in its
-// forces-only mode gives Fc and the pressure, k_dpd_pair the pair dissipative and random forces and
-// the second half kick (into the spare velocity buffer), k_dpd_dis background and pair dissipation
+// The DPD integrator: k_cy_keys makes the first half kick and the drift, k_dpd_forces the conservative
+// forces and the pressure, the pair dissipative and random forces and the second half kick (into the
+// spare velocity buffer), k_dpd_dis background and pair dissipation
 // at the new velocities and the cell's cycle; then the same divisions and apoptosis.
 // The file is compiled without FMA contraction: outside the forms of "FP64 arithmetic" (cil_internal.cuh), the
 // arithmetic is that of the host restatement the tests compare with, to a few units of the last place.
@@ -73,6 +73,7 @@ struct CyConst {
   double inv_bw[3];
   double sigma_core;
   double hz_c;        // (1 - nu^2) / E
+  float c2f, adhf, gdf, srf;  // FP32: 2 hz_c, adhesion, gamma_d, sigma_r
   double adhesion;
   double motility, zeta, zeta_p, zeta_p_beta;
   double noise_amp;   // sqrt(2 D) / sqrt(dt)
@@ -366,12 +367,12 @@ __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounte
 // met took 1079 us, and the cycle's own pass 258 us.
 constexpr int kPairBlock = 128;
 constexpr int kPairNear = 384;  // survivors held per warp (12 per cell at one lane each)
-constexpr int kPairSeg = 128;   // pairs evaluated before their sums are taken
 constexpr int kPairAhead = 4;   // candidates a lane has in flight (one lane per cell)
 
 template <int D, int NRES, typename R>
 struct PairWarp {
-  R res[kPairSeg * NRES];
+  static constexpr int kSeg = NRES > 6 ? 64 : 128;  // pairs evaluated before their sums are taken
+  R res[kSeg * NRES];
   double x[32 * D];
   R v[32 * D];  // velocities (DPD)
   double rad[32];
@@ -416,8 +417,9 @@ __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R
     const int off = end - cnt;
     for (int k = sub; k < cnt; k += L) W.own[off + k] = static_cast<unsigned char>(el);
     __syncwarp();
-    for (int S = 0; S < total; S += kPairSeg) {
-      const int E = min(total, S + kPairSeg);
+    constexpr int kSeg = PairWarp<D, NRES, R>::kSeg;
+    for (int S = 0; S < total; S += kSeg) {
+      const int E = min(total, S + kSeg);
       for (int f0 = S; f0 < E; f0 += 32) {  // uniform
         const int f = f0 + lane;
         const int o = f < E ? W.own[f] : 0;
@@ -656,16 +658,129 @@ __device__ inline void contact(const CyConst &C, double r, double h, double hy, 
   }
 }
 
+// The terms of the pair at displacement rij (r2 its square, FP64 form): the contact force on the cell,
+// and in out[D] the pressure term, -f0 / volume doubled (FP64) or f0 / volume (MIXED); zeros out of
+// contact. The warp's cell o and the cell at place tt; first: the cell has the lower index.
+template <int D, bool MIXED, int NRES, typename R>
+__device__ __forceinline__ void contact_terms(const CyConst &C, const CyOrdered &O, const PairWarp<D, NRES, R> &W, int o,
+                                              int tt, const double *rij, double r2, bool first, R *out) {
+  // the pair's first cell is the one of lower index (the contact length is not symmetric in
+  // the two diameters)
+#pragma unroll
+  for (int k = 0; k <= D; ++k) out[k] = R(0);
+  if (MIXED) {
+    float df[D], r2f = 0.0f;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      df[d] = static_cast<float>(rij[d]);
+      r2f += df[d] * df[d];
+    }
+    const float sif = W.dia[o], sjf = __ldg(O.rec + tt).w;
+    const float cut = 0.5f * (sif + sjf);
+    if (!(r2f <= cut * cut) || r2f == 0.0f) return;
+    const float r = sqrtf(r2f);
+    const float sa = first ? sif : sjf, sb = first ? sjf : sif;
+    const float h = fmaxf(cut - r, 0.0f);
+    const float fel = (h * sqrtf(h)) / (0.75f * C.c2f * sqrtf(2.0f / sif + 2.0f / sjf));
+    const float ra = 0.5f * sa, rb = 0.5f * sb;
+    float A, vol;
+    if (D == 3) {
+      const float u = r2f - rb * rb + ra * ra;
+      const float t = sqrtf(4.0f * r2f * (ra * ra) - u * u) / (2.0f * r);
+      A = t > 0.0f ? static_cast<float>(kPi) * (t * t) : 0.0f;
+      vol = A == 0.0f ? 0.0f : (4.0f * static_cast<float>(kPi) * (ra * ra) / 3.0f);
+    } else {
+      const float w = h * (sb - h) / (2.0f * r);
+      const float t = 2.0f * sqrtf(w * (sa - w));
+      A = isnan(t) ? fminf(sa, sb) : t;
+      vol = A;
+    }
+    const float f0 = -fel + C.adhf * A;
+#pragma unroll
+    for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * df[d]);
+    out[D] = static_cast<R>(vol != 0.0f ? f0 / vol : 0.0f);
+  } else {
+    const double ro = W.rad[o], rj = __ldg(O.rad + tt);
+    double hy, r;
+    if (mid_range(r2)) {
+      const double y = rsqrt_pos(r2);
+      r = sqrt_from(r2, y);
+      hy = 0.5 * y;
+    } else {
+      r = sqrt(r2);
+      hy = 0.5 / r;
+    }
+    const double cut = ro + rj, h = cut - r;
+    // h >= 0 and finite (sign and exponent bits), r not 0
+    if (__double2hiint(h) < 0 || !finite_bits(h) || __double_as_longlong(r) == 0) return;
+    double f0, pr2;
+    contact<D>(C, r, h, hy, cut, first ? ro : rj, first ? rj : ro, &f0, &pr2);
+#pragma unroll
+    for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * rij[d]);
+    out[D] = static_cast<R>(pr2);
+  }
+}
+
+// Motility along the velocity and passive noise of cell i
+template <int D>
+__device__ __forceinline__ void own_force(const CyConst &C, const CySet &S, int i, int ts, double *F) {
+  const size_t cap = C.capacity;
+  // ---- motility along the velocity (singleCellForce, MD.cu:600-646)
+  {
+    double vi[D], v2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      vi[d] = S.v[d * cap + i];
+      v2 = d == 0 ? vi[d] * vi[d] : __fma_rn(vi[d], vi[d], v2);
+    }
+    if (mid_range(v2)) {
+      const double m = C.motility * rsqrt_pos(v2);
+#pragma unroll
+      for (int d = 0; d < D; ++d) F[d] = m * vi[d];
+    } else {
+      double vl = sqrt(v2);
+      if (vl == 0.0) {  // a direction at random, length 1e-11 (BIG_TOL_MP)
+        const u32x4 r = draw(C, i, ts, kCyDir, 0);
+        if (D == 2) {
+          const double ang = 6.283185307179586 * u53(r.v[0], r.v[1]);
+          vi[0] = 1e-11 * cos(ang);
+          vi[1] = 1e-11 * sin(ang);
+        } else {
+          const double z = 2.0 * u53(r.v[0], r.v[1]) - 1.0;
+          const double ang = 6.283185307179586 * u53(r.v[2], r.v[3]);
+          const double s = sqrt(1.0 - z * z);
+          vi[0] = 1e-11 * (s * cos(ang));
+          vi[1] = 1e-11 * (s * sin(ang));
+          vi[D - 1] = 1e-11 * z;
+        }
+        v2 = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) v2 += vi[d] * vi[d];
+        vl = sqrt(v2);
+      }
+#pragma unroll
+      for (int d = 0; d < D; ++d) F[d] = C.motility * (vi[d] / vl);
+    }
+  }
+  // ---- passive noise (CIL.cu:84-97)
+  if (C.noise_amp > 0.0) {
+    double nz[4];
+    normal2(draw(C, i, ts, kCyNoise, 0), &nz[0], &nz[1]);
+    if (D == 3) normal2(draw(C, i, ts, kCyNoise, 1), &nz[2], &nz[3]);
+#pragma unroll
+    for (int d = 0; d < D; ++d) F[d] += C.zeta * (C.noise_amp * nz[d]);
+  }
+}
+
 // MIXED: the contact arithmetic in FP32 on the FP64 displacement; the forces and the pressure are
 // summed in FP32 over the contacts and added to the FP64 motility and noise; the position update and
 // the cell state stay FP64.
 // mode 0 (Euler): the position update with the pressure-dependent friction follows (in place: the
 // other cells read the bin-ordered copies), then the cell cycle; mode 1: the forces go to frc and
-// nothing moves. Draws are keyed by the device step counter + key_off.
+// nothing moves. Draws are keyed by the device step counter.
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, double *frc, CyCounters *cnt,
-                                                         const int *start, const int *ts_dev, int mode, int key_off,
-                                                         CyOrdered O, int lane_bits, int *dblk, int *dueq,
+                                                         const int *start, const int *ts_dev, int mode, CyOrdered O, int lane_bits, int *dblk, int *dueq,
                                                          unsigned long long *sig_part) {
   cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
@@ -691,7 +806,6 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
     W.idx[el] = i;
   }
   __syncwarp();
-  const float c2f = static_cast<float>(C.hz_c + C.hz_c), adhf = static_cast<float>(C.adhesion);
   R acc[D + 1];
 #pragma unroll
   for (int k = 0; k <= D; ++k) acc[k] = R(0);
@@ -710,113 +824,14 @@ __global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, dou
           rij[d] = v;
           if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
         }
-        // the pair's first cell is the one of lower index (the contact length is not symmetric in
-        // the two diameters)
-        const bool first = W.idx[o] < __ldg(O.idx + tt);
-#pragma unroll
-        for (int k = 0; k <= D; ++k) out[k] = R(0);
-        if (MIXED) {
-          float df[D], r2f = 0.0f;
-#pragma unroll
-          for (int d = 0; d < D; ++d) {
-            df[d] = static_cast<float>(rij[d]);
-            r2f += df[d] * df[d];
-          }
-          const float sif = W.dia[o], sjf = __ldg(O.rec + tt).w;
-          const float cut = 0.5f * (sif + sjf);
-          if (!(r2f <= cut * cut) || r2f == 0.0f) return;
-          const float r = sqrtf(r2f);
-          const float sa = first ? sif : sjf, sb = first ? sjf : sif;
-          const float h = fmaxf(cut - r, 0.0f);
-          const float fel = (h * sqrtf(h)) / (0.75f * c2f * sqrtf(2.0f / sif + 2.0f / sjf));
-          const float ra = 0.5f * sa, rb = 0.5f * sb;
-          float A, vol;
-          if (D == 3) {
-            const float u = r2f - rb * rb + ra * ra;
-            const float t = sqrtf(4.0f * r2f * (ra * ra) - u * u) / (2.0f * r);
-            A = t > 0.0f ? static_cast<float>(kPi) * (t * t) : 0.0f;
-            vol = A == 0.0f ? 0.0f : (4.0f * static_cast<float>(kPi) * (ra * ra) / 3.0f);
-          } else {
-            const float w = h * (sb - h) / (2.0f * r);
-            const float t = 2.0f * sqrtf(w * (sa - w));
-            A = isnan(t) ? fminf(sa, sb) : t;
-            vol = A;
-          }
-          const float f0 = -fel + adhf * A;
-#pragma unroll
-          for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * df[d]);
-          out[D] = static_cast<R>(vol != 0.0f ? f0 / vol : 0.0f);
-        } else {
-          const double ro = W.rad[o], rj = __ldg(O.rad + tt);
-          double hy, r;
-          if (mid_range(r2)) {
-            const double y = rsqrt_pos(r2);
-            r = sqrt_from(r2, y);
-            hy = 0.5 * y;
-          } else {
-            r = sqrt(r2);
-            hy = 0.5 / r;
-          }
-          const double cut = ro + rj, h = cut - r;
-          // h >= 0 and finite (sign and exponent bits), r not 0
-          if (__double2hiint(h) < 0 || !finite_bits(h) || __double_as_longlong(r) == 0) return;
-          double f0, pr2;
-          contact<D>(C, r, h, hy, cut, first ? ro : rj, first ? rj : ro, &f0, &pr2);
-#pragma unroll
-          for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * rij[d]);
-          out[D] = static_cast<R>(pr2);
-        }
+        contact_terms<D, MIXED>(C, O, W, o, tt, rij, r2, W.idx[o] < __ldg(O.idx + tt), out);
       },
       acc);
   unsigned long long sbits = 0ull;
   if (live && sub == 0) {
-    const int ts = *ts_dev + key_off;
+    const int ts = *ts_dev;
     double F[D];
-    // ---- motility along the velocity (singleCellForce, MD.cu:600-646)
-    {
-      double vi[D], v2 = 0.0;
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        vi[d] = S.v[d * cap + i];
-        v2 = d == 0 ? vi[d] * vi[d] : __fma_rn(vi[d], vi[d], v2);
-      }
-      if (mid_range(v2)) {
-        const double m = C.motility * rsqrt_pos(v2);
-#pragma unroll
-        for (int d = 0; d < D; ++d) F[d] = m * vi[d];
-      } else {
-        double vl = sqrt(v2);
-        if (vl == 0.0) {  // a direction at random, length 1e-11 (BIG_TOL_MP)
-          const u32x4 r = draw(C, i, ts, kCyDir, 0);
-          if (D == 2) {
-            const double ang = 6.283185307179586 * u53(r.v[0], r.v[1]);
-            vi[0] = 1e-11 * cos(ang);
-            vi[1] = 1e-11 * sin(ang);
-          } else {
-            const double z = 2.0 * u53(r.v[0], r.v[1]) - 1.0;
-            const double ang = 6.283185307179586 * u53(r.v[2], r.v[3]);
-            const double s = sqrt(1.0 - z * z);
-            vi[0] = 1e-11 * (s * cos(ang));
-            vi[1] = 1e-11 * (s * sin(ang));
-            vi[D - 1] = 1e-11 * z;
-          }
-          v2 = 0.0;
-#pragma unroll
-          for (int d = 0; d < D; ++d) v2 += vi[d] * vi[d];
-          vl = sqrt(v2);
-        }
-#pragma unroll
-        for (int d = 0; d < D; ++d) F[d] = C.motility * (vi[d] / vl);
-      }
-    }
-    // ---- passive noise (CIL.cu:84-97)
-    if (C.noise_amp > 0.0) {
-      double nz[4];
-      normal2(draw(C, i, ts, kCyNoise, 0), &nz[0], &nz[1]);
-      if (D == 3) normal2(draw(C, i, ts, kCyNoise, 1), &nz[2], &nz[3]);
-#pragma unroll
-      for (int d = 0; d < D; ++d) F[d] += C.zeta * (C.noise_amp * nz[d]);
-    }
+    own_force<D>(C, S, i, ts, F);
     bool finite = true;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -862,18 +877,21 @@ __device__ inline void normal2f(const u32x4 &r, float *n0, float *n1) {
   *n1 = rad * sn;
 }
 
-// Pair dissipative and random forces (cellCellDisRanForce, MD.cu:861-905) over the pairs closer
-// than the lower-index cell's diameter; then, with `kick`, the second half kick into v_out.
+// The conservative forces and the pressure (k_cy_force's) and the pair dissipative and random forces
+// (cellCellDisRanForce, MD.cu:861-905) over the pairs closer than the lower-index cell's diameter, in
+// one walk (a contact's range, the mean diameter, is within the larger one); then, with `kick`, the
+// second half kick into v_out. In two walks 0.15M cells with FP32 pair terms took 25.4 and 22.6 us; in
+// one about 32.
 // MIXED: the pair terms in FP32 on the FP64 separation, FP32 velocities and normals, summed in FP32
 // per cell; the kick stays FP64, and the new velocities' records go to vel_out for k_dpd_dis.
 template <int D, bool MIXED>
-__global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, double *v_out, CyCounters *cnt,
+__global__ void __launch_bounds__(kPairBlock) k_dpd_forces(CyConst C, CySet S, double *v_out, CyCounters *cnt,
                                                          const int *start, const int *ts_dev, int key_off, int kick_on,
                                                          CyOrdered O, float4 *vel_out, int lane_bits) {
   cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
-  __shared__ PairWarp<D, 2 * D, R> s_warp[kPairBlock / 32];
-  PairWarp<D, 2 * D, R> &W = s_warp[threadIdx.x >> 5];
+  __shared__ PairWarp<D, 3 * D + 1, R> s_warp[kPairBlock / 32];
+  PairWarp<D, 3 * D + 1, R> &W = s_warp[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairBlock + threadIdx.x;
   const int n = cnt->n;
   const int L = 1 << lane_bits;
@@ -897,11 +915,10 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
     W.idx[el] = i;
   }
   __syncwarp();
-  const float gdf = static_cast<float>(C.gamma_d), srf = static_cast<float>(C.sigma_r);
-  R acc[2 * D];
+  R acc[3 * D + 1];  // conservative, pressure, dissipative, random
 #pragma unroll
-  for (int k = 0; k < 2 * D; ++k) acc[k] = R(0);
-  walk_pairs<D, 2 * D, R>(
+  for (int k = 0; k < 3 * D + 1; ++k) acc[k] = R(0);
+  walk_pairs<D, 3 * D + 1, R>(
       C, W, O, start, live, q, lane_bits, sigma_max_f(cnt),
       [](const float4 &a, const float4 &b) {
         const float s = fmaxf(a.w, b.w);
@@ -918,6 +935,8 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
         }
         const int io = W.idx[o], j = __ldg(O.idx + tt);
         const uint32_t a = static_cast<uint32_t>(io < j ? io : j), z = static_cast<uint32_t>(io < j ? j : io);
+        contact_terms<D, MIXED>(C, O, W, o, tt, rij, r2, io < j, out);
+        out += D + 1;
 #pragma unroll
         for (int k = 0; k < 2 * D; ++k) out[k] = R(0);
         if (MIXED) {
@@ -940,8 +959,8 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
           for (int d = 0; d < D; ++d) {
             const float nd = df[d] * rinv;
             const float dv = static_cast<float>(W.v[o * D + d]) - f4c(vj4, d);
-            out[d] = static_cast<R>(-(gdf * w * (dv * nd) * nd));
-            out[D + d] = static_cast<R>(srf * sw * nd * xf[d]);
+            out[d] = static_cast<R>(-(C.gdf * w * (dv * nd) * nd));
+            out[D + d] = static_cast<R>(C.srf * sw * nd * xf[d]);
           }
         } else {
           const double rc = 2 * (io < j ? W.rad[o] : __ldg(O.rad + tt));
@@ -972,14 +991,20 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_pair(CyConst C, CySet S, dou
   if (!live || sub != 0) return;
   bool finite = true;
   float vf[3] = {0.0f, 0.0f, 0.0f};
+  double F[D];
+  own_force<D>(C, S, i, static_cast<int>(ts), F);
+  S.p[i] = MIXED ? -static_cast<double>(acc[D]) : -0.5 * static_cast<double>(acc[D]);
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     const size_t k = d * cap + i;
-    const double fd = static_cast<double>(acc[d]), fr = static_cast<double>(acc[D + d]);
+    F[d] += static_cast<double>(acc[d]);
+    finite = finite && finite_bits(F[d]);
+    S.fc[k] = F[d];
+    const double fd = static_cast<double>(acc[D + 1 + d]), fr = static_cast<double>(acc[2 * D + 1 + d]);
     S.fd[k] = fd;
     S.fr[k] = fr;
     if (kick_on) {
-      const double v = kick(C, vi[d], S.fc[k], fd, fr);
+      const double v = kick(C, vi[d], F[d], fd, fr);
       v_out[k] = v;
       vf[d] = static_cast<float>(v);
       finite = finite && finite_bits(v);
@@ -1022,7 +1047,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
   }
   __syncwarp();
   const double rc = C.sigma_core;
-  const float rcf = static_cast<float>(rc), gdf = static_cast<float>(C.gamma_d);
+  const float rcf = static_cast<float>(rc);
   R acc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) acc[d] = R(0);
@@ -1054,7 +1079,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
           for (int d = 0; d < D; ++d) {
             const float nd = -df[d] * rinv;
             const float dv = static_cast<float>(W.v[o * D + d]) - f4c(vj4, d);
-            out[d] = static_cast<R>(-(gdf * w * (dv * nd) * nd));
+            out[d] = static_cast<R>(-(C.gdf * w * (dv * nd) * nd));
           }
         } else {
           const int j = __ldg(O.idx + tt);
@@ -1605,40 +1630,40 @@ int pair_blocks(const cil_cycle *h) {
 }
 
 template <int D>
-void launch_force_d(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
+void launch_force_d(cil_cycle *h, CySet &S, double *frc, int mode) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_cy_force<D, true>, h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_cy_force<D, true>, h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode,
                                                          h->O, h->lane_bits, h->dblk, h->dueq, h->sig_part);
   else
-    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_cy_force<D, false>, h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode, key_off,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_cy_force<D, false>, h->C, S, frc, h->cnt, h->bstart, h->ts_dev, mode,
                                                           h->O, h->lane_bits, h->dblk, h->dueq, h->sig_part);
 }
 
-void launch_force(cil_cycle *h, CySet &S, double *frc, int mode, int key_off) {
+void launch_force(cil_cycle *h, CySet &S, double *frc, int mode) {
   if (h->C.D == 2)
-    launch_force_d<2>(h, S, frc, mode, key_off);
+    launch_force_d<2>(h, S, frc, mode);
   else
-    launch_force_d<3>(h, S, frc, mode, key_off);
+    launch_force_d<3>(h, S, frc, mode);
   h->launches += 1;
 }
 
 template <int D>
-void launch_dpd_pair_d(cil_cycle *h, CySet &S, int key_off, int kick_on) {
+void launch_dpd_forces_d(cil_cycle *h, CySet &S, int key_off, int kick_on) {
   const int g = pair_blocks(h);
   if (h->p.precision == 1)
-    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_pair<D, true>, h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off, kick_on,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_forces<D, true>, h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off, kick_on,
                                                          h->O, h->vel_next, h->lane_bits);
   else
-    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_pair<D, false>, h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off,
+    cil::launch_step(true, g, kPairBlock, 0, h->stream, k_dpd_forces<D, false>, h->C, S, h->vs, h->cnt, h->bstart, h->ts_dev, key_off,
                                                           kick_on, h->O, h->vel_next, h->lane_bits);
 }
 
-void launch_dpd_pair(cil_cycle *h, CySet &S, int key_off, int kick_on) {
+void launch_dpd_forces(cil_cycle *h, CySet &S, int key_off, int kick_on) {
   if (h->C.D == 2)
-    launch_dpd_pair_d<2>(h, S, key_off, kick_on);
+    launch_dpd_forces_d<2>(h, S, key_off, kick_on);
   else
-    launch_dpd_pair_d<3>(h, S, key_off, kick_on);
+    launch_dpd_forces_d<3>(h, S, key_off, kick_on);
   h->launches += 1;
 }
 
@@ -1666,20 +1691,18 @@ void launch_dpd_dis(cil_cycle *h, CySet &S) {
 void dpd_initial_forces(cil_cycle *h) {
   CySet &S = h->set[h->cur];
   bin_cells(h, 0);
-  launch_force(h, S, S.fc, 1, 0);
-  launch_dpd_pair(h, S, 0, 0);
+  launch_dpd_forces(h, S, 0, 0);
 }
 
 cil_status enqueue_step(cil_cycle *h) {
   CySet &S = h->set[h->cur];
   bin_cells(h, h->C.dpd);
   if (h->C.dpd) {  // DPD (CIL.cu:1054-1066); this step's draws are keyed by ts + 1
-    launch_force(h, S, S.fc, 1, 1);
-    launch_dpd_pair(h, S, 1, 1);
+    launch_dpd_forces(h, S, 1, 1);
     std::swap(S.v, h->vs);
     launch_dpd_dis(h, S);
   } else {
-    launch_force(h, S, nullptr, 0, 0);
+    launch_force(h, S, nullptr, 0);
   }
   h->ts += 1;
   if (h->C.divide) {  // also moves the step counter
@@ -1811,6 +1834,8 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   set_bins(h, p->sigma_core, capacity);
   C.hz_c = (1 - p->nu * p->nu) / p->E;
   C.adhesion = p->adhesion;
+  C.c2f = static_cast<float>(C.hz_c + C.hz_c);
+  C.adhf = static_cast<float>(C.adhesion);
   C.motility = p->motility;
   C.zeta = p->zeta;
   C.zeta_p = p->zeta_p;
@@ -1863,6 +1888,8 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   C.gamma_d = p->dis_diff;
   C.gamma_b = p->dis_bg;
   C.sigma_r = std::sqrt(2 * p->dis_diff * p->kbt);  // Sigma (MD.cu:872)
+  C.gdf = static_cast<float>(C.gamma_d);
+  C.srf = static_cast<float>(C.sigma_r);
   C.seed_lo = static_cast<uint32_t>(seed);
   C.seed_hi = static_cast<uint32_t>(seed >> 32);
 
@@ -2066,7 +2093,7 @@ cil_status cil_cycle_download(cil_cycle *h, cil_cycle_view *v) {
     // evaluates at its end (CIL.cu:1019) and writes out; the next step's force pass computes
     // the same values again (same positions, velocities and step key)
     bin_cells(h, 0);
-    launch_force(h, h->set[h->cur], h->frc, 1, 0);
+    launch_force(h, h->set[h->cur], h->frc, 1);
     h->launches = launches;
     CY_TRY(h, cudaGetLastError());
   }
