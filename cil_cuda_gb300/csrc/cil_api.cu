@@ -811,7 +811,8 @@ cudaEvent_t pool_event(cil_handle *h, size_t i) {
 // Lanes per element of the FP64 force pass: as many as keep the walk and the pair evaluation of a
 // small colony spread over every SM, up to 8, while the elements give fewer than two warps per
 // scheduler (nsm x 4 x 2 x 32 lanes). From the cells the host knows of (uploaded, or counted by the
-// last cil_step); the forces do not depend on it. Step of the growth colony with 1, 2, 4, 8 lanes:
+// last cil_step); the forces do not depend on it. Step of the growth colony with 1, 2, 4, 8 lanes
+// (when a step had 15 launches):
 // 500 cells 48, 46, 44, 42 us; 4864 cells 61, 56, 57, 61 us; 19456 cells 72, 73, 87, 107 us.
 void set_lane_bits(cil_handle *h) {
   long long elems = 0;
