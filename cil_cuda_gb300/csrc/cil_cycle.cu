@@ -775,11 +775,14 @@ __device__ __forceinline__ void own_force(const CyConst &C, const CySet &S, int 
 // MIXED: the contact arithmetic in FP32 on the FP64 displacement; the forces and the pressure are
 // summed in FP32 over the contacts and added to the FP64 motility and noise; the position update and
 // the cell state stay FP64.
+// Blocks an SM: 8 (64 registers) with FP32 pair terms, where the walk's loads need the warps (10 steps of
+// 0.6M cells 3.17 -> 3.06 ms against the compiler's 95 registers); 7 (72) in FP64, which is bound by the
+// FP64 pipe (more registers and fewer blocks: 1M cells 7.44 -> 8.34 ms).
 // mode 0 (Euler): the position update with the pressure-dependent friction follows (in place: the
 // other cells read the bin-ordered copies), then the cell cycle; mode 1: the forces go to frc and
 // nothing moves. Draws are keyed by the device step counter.
 template <int D, bool MIXED>
-__global__ void __launch_bounds__(kPairBlock) k_cy_force(CyConst C, CySet S, double *frc, CyCounters *cnt,
+__global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 7) k_cy_force(CyConst C, CySet S, double *frc, CyCounters *cnt,
                                                          const int *start, const int *ts_dev, int mode, CyOrdered O, int lane_bits, int *dblk, int *dueq,
                                                          unsigned long long *sig_part) {
   cil::enter_step_kernel();
@@ -881,11 +884,12 @@ __device__ inline void normal2f(const u32x4 &r, float *n0, float *n1) {
 // (cellCellDisRanForce, MD.cu:861-905) over the pairs closer than the lower-index cell's diameter, in
 // one walk (a contact's range, the mean diameter, is within the larger one); then, with `kick`, the
 // second half kick into v_out. In two walks 0.15M cells with FP32 pair terms took 25.4 and 22.6 us; in
-// one about 32.
+// one about 32. 8 blocks an SM with FP32 pair terms (12 steps of 0.15M cells 1.87 -> 1.82 ms against 95
+// registers); FP64 keeps its registers (10 steps 4.19 -> 4.04 ms).
 // MIXED: the pair terms in FP32 on the FP64 separation, FP32 velocities and normals, summed in FP32
 // per cell; the kick stays FP64, and the new velocities' records go to vel_out for k_dpd_dis.
 template <int D, bool MIXED>
-__global__ void __launch_bounds__(kPairBlock) k_dpd_forces(CyConst C, CySet S, double *v_out, CyCounters *cnt,
+__global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyConst C, CySet S, double *v_out, CyCounters *cnt,
                                                          const int *start, const int *ts_dev, int key_off, int kick_on,
                                                          CyOrdered O, float4 *vel_out, int lane_bits) {
   cil::enter_step_kernel();
