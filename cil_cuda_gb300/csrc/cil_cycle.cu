@@ -66,7 +66,7 @@ struct CyConst {
   double dt;
   int ns[3];
   double bw[3];       // bin width per axis
-  float boxf[3], halff[3];  // FP32 copies for the range tests
+  float bwf[3], boxf[3], halff[3];  // FP32 copies for the range tests and FP32 separations
   double half[3];     // box / 2
   float inv_bwf[3];   // bins per length, rounded up
   float scalef[3];    // and to the nearest
@@ -111,6 +111,8 @@ struct CyOrdered {
   double *rad;  // radius (sigma / 2, exact)
   float4 *rec;  // FP32 position (z 0 in 2D) and diameter, for the range tests
   float4 *vel;  // FP32 velocity (DPD, precision 1)
+  float4 *loc;  // FP32 position relative to the origin of the cell's bin (z 0 in 2D) and diameter (DPD, precision 1)
+  ushort4 *cell;  // the bin's place along each axis (DPD, precision 1)
   int *idx;     // the cell's index
   int *bin;
 };
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(kTile) k_cy_scatter(const CyCounters *cnt, con
 // radius, and the FP32 record (absolute position and diameter) of the range tests. Threads take the
 // cells in arrival order, next to their places: the state is gathered (32 bytes a value where the
 // index order is not the bin order) and the copies are written in full lines (DPD, 0.15M cells: 6.8 us;
-// from the index order, with the copies scattered, 8.2 us).
+// from the index order, with the copies scattered, 8.2 us; without `loc` and `cell`).
 __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounters *cnt, const int *start,
                                                     const int2 *tmp, CyOrdered O, int with_vel) {
   cil::enter_step_kernel();
@@ -350,7 +352,21 @@ __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounte
   O.bin[q] = b;
   O.rec[q] = make_float4(static_cast<float>(x[0]), static_cast<float>(x[1]), static_cast<float>(x[2]),
                          static_cast<float>(sg));
-  if (with_vel) O.vel[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
+  if (with_vel) {
+    O.vel[q] = make_float4(vf[0], vf[1], vf[2], 0.0f);
+    int v[3] = {0, 0, 0}, r = b;
+    float u[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int d = 2; d >= 0; --d) {
+      if (d >= C.D) continue;
+      v[d] = d > 0 ? r % C.ns[d] : r;
+      r /= C.ns[d];
+      u[d] = static_cast<float>(x[d] - v[d] * C.bw[d]);
+    }
+    O.loc[q] = make_float4(u[0], u[1], u[2], static_cast<float>(sg));
+    O.cell[q] = make_ushort4(static_cast<unsigned short>(v[0]), static_cast<unsigned short>(v[1]),
+                             static_cast<unsigned short>(v[2]), 0);
+  }
 }
 
 // ---------------------------------------------------------------- the pair walk
@@ -375,6 +391,8 @@ struct PairWarp {
   R res[kSeg * NRES];
   double x[32 * D];
   R v[32 * D];  // velocities (DPD)
+  float u[32 * D];  // CyOrdered::loc and ::cell (DPD, FP32 pair terms)
+  int cell[32 * D];
   double rad[32];
   float dia[32];
   int idx[32];
@@ -388,6 +406,48 @@ __device__ inline double nearest(double dd, double L, double half) {
   const long long b = __double_as_longlong(dd);
   if ((b & 0x7fffffffffffffffll) > __double_as_longlong(half)) return b < 0 ? dd + L : dd - L;
   return dd;
+}
+
+// DPD's FP32 pair terms take the displacement from coordinates relative to the bins' origins and the
+// bins' offset. Not from the FP64 positions, although those would round better: the random force's
+// sqrt(1 - r / rc) of a pair at the end of its range follows the last bits of r, so with another rounding
+// a velocity differs by up to 2e-3 of their root mean square (0.15M cells, 12 steps) from what this
+// form has always given.
+// Bit d: the search covers axis d whole (each bin once), and an offset may span the axis.
+template <int D>
+__device__ __forceinline__ int whole_axes(const CyConst &C, float radius) {
+  int m = 0;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float kk = ceilf(__fmul_ru(radius, C.inv_bwf[d]));
+    const int k = (kk >= 0.0f && kk < static_cast<float>(C.ns[d])) ? static_cast<int>(kk) : C.ns[d];
+    if (2 * k + 1 >= C.ns[d]) m |= 1 << d;
+  }
+  return m;
+}
+
+// the warp's cell o to the cell at place tt, at the nearest image on periodic axes
+template <int D, int NRES, typename R>
+__device__ __forceinline__ void local_separation(const CyConst &C, const CyOrdered &O, const PairWarp<D, NRES, R> &W,
+                                                 int whole, int o, int tt, float *df) {
+  const float4 uj = __ldg(O.loc + tt);
+  const ushort4 cj = __ldg(O.cell + tt);
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    int off = (d == 0 ? cj.x : (d == 1 ? cj.y : cj.z)) - W.cell[o * D + d];
+    if (C.periodic[d] && !(whole >> d & 1)) {
+      if (2 * off > C.ns[d]) off -= C.ns[d];
+      if (2 * off < -C.ns[d]) off += C.ns[d];
+    }
+    float v = f4c(uj, d) + static_cast<float>(off) * C.bwf[d] - W.u[o * D + d];
+    if (C.periodic[d]) {
+      if (v > C.halff[d])
+        v -= C.boxf[d];
+      else if (v < -C.halff[d])
+        v += C.boxf[d];
+    }
+    df[d] = v;
+  }
 }
 
 // reach2(me, p): the squared range of a pair in FP32 (an upper bound up to rounding);
@@ -658,12 +718,12 @@ __device__ inline void contact(const CyConst &C, double r, double h, double hy, 
   }
 }
 
-// The terms of the pair at displacement rij (r2 its square, FP64 form): the contact force on the cell,
+// The terms of the pair at displacement rij (FP64, or FP32 with FP32 pair terms; r2 its square, FP64 form): the contact force on the cell,
 // and in out[D] the pressure term, -f0 / volume doubled (FP64) or f0 / volume (MIXED); zeros out of
 // contact. The warp's cell o and the cell at place tt; first: the cell has the lower index.
-template <int D, bool MIXED, int NRES, typename R>
+template <int D, bool MIXED, int NRES, typename R, typename X>
 __device__ __forceinline__ void contact_terms(const CyConst &C, const CyOrdered &O, const PairWarp<D, NRES, R> &W, int o,
-                                              int tt, const double *rij, double r2, bool first, R *out) {
+                                              int tt, const X *rij, double r2, bool first, R *out) {
   // the pair's first cell is the one of lower index (the contact length is not symmetric in
   // the two diameters)
 #pragma unroll
@@ -886,7 +946,7 @@ __device__ inline void normal2f(const u32x4 &r, float *n0, float *n1) {
 // second half kick into v_out. In two walks 0.15M cells with FP32 pair terms took 25.4 and 22.6 us; in
 // one about 32. 8 blocks an SM with FP32 pair terms (12 steps of 0.15M cells 1.87 -> 1.82 ms against 95
 // registers); FP64 keeps its registers (10 steps 4.19 -> 4.04 ms).
-// MIXED: the pair terms in FP32 on the FP64 separation, FP32 velocities and normals, summed in FP32
+// MIXED: the pair terms in FP32 on the separations of local_separation, FP32 velocities and normals, summed in FP32
 // per cell; the kick stays FP64, and the new velocities' records go to vel_out for k_dpd_dis.
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyConst C, CySet S, double *v_out, CyCounters *cnt,
@@ -894,6 +954,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
                                                          CyOrdered O, float4 *vel_out, int lane_bits) {
   cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
+  using X = R;  // displacements
   __shared__ PairWarp<D, 3 * D + 1, R> s_warp[kPairBlock / 32];
   PairWarp<D, 3 * D + 1, R> &W = s_warp[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairBlock + threadIdx.x;
@@ -909,9 +970,18 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
 #pragma unroll
   for (int d = 0; d < D; ++d) vi[d] = live ? S.v[d * cap + i] : 0.0;
   if (sub == 0) {
+    if (MIXED) {
+      const float4 u = live ? O.loc[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const ushort4 b = live ? O.cell[q] : make_ushort4(0, 0, 0, 0);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        W.u[el * D + d] = f4c(u, d);
+        W.cell[el * D + d] = d == 0 ? b.x : (d == 1 ? b.y : b.z);
+      }
+    }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
+      if (!MIXED) W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
       W.v[el * D + d] = static_cast<R>(vi[d]);
     }
     W.rad[el] = live ? O.rad[q] : 1.0;
@@ -919,23 +989,30 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
     W.idx[el] = i;
   }
   __syncwarp();
+  const float radius = sigma_max_f(cnt);
+  const int whole = MIXED ? whole_axes<D>(C, radius) : 0;
   R acc[3 * D + 1];  // conservative, pressure, dissipative, random
 #pragma unroll
   for (int k = 0; k < 3 * D + 1; ++k) acc[k] = R(0);
   walk_pairs<D, 3 * D + 1, R>(
-      C, W, O, start, live, q, lane_bits, sigma_max_f(cnt),
+      C, W, O, start, live, q, lane_bits, radius,
       [](const float4 &a, const float4 &b) {
         const float s = fmaxf(a.w, b.w);
         return s * s;
       },
       [&](int o, int tt, R *out) {
-        double rij[D], r2 = 0.0;
+        X rij[D];
+        double r2 = 0.0;
+        if constexpr (MIXED) {
+          local_separation<D>(C, O, W, whole, o, tt, rij);
+        } else {
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-          double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
-          if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
-          rij[d] = v;
-          if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
+          for (int d = 0; d < D; ++d) {
+            double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+            if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
+            rij[d] = v;
+            r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
+          }
         }
         const int io = W.idx[o], j = __ldg(O.idx + tt);
         const uint32_t a = static_cast<uint32_t>(io < j ? io : j), z = static_cast<uint32_t>(io < j ? j : io);
@@ -944,12 +1021,9 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
 #pragma unroll
         for (int k = 0; k < 2 * D; ++k) out[k] = R(0);
         if (MIXED) {
-          float df[D], r2f = 0.0f;
+          float r2f = 0.0f;
 #pragma unroll
-          for (int d = 0; d < D; ++d) {
-            df[d] = static_cast<float>(rij[d]);
-            r2f += df[d] * df[d];
-          }
+          for (int d = 0; d < D; ++d) r2f += rij[d] * rij[d];
           const float rc = io < j ? W.dia[o] : __ldg(O.rec + tt).w;
           if (!(r2f < rc * rc) || r2f == 0.0f) return;
           const float4 vj4 = __ldg(O.vel + tt);
@@ -961,7 +1035,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
           const float sw = sqrtf(w);
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            const float nd = df[d] * rinv;
+            const float nd = rij[d] * rinv;
             const float dv = static_cast<float>(W.v[o * D + d]) - f4c(vj4, d);
             out[d] = static_cast<R>(-(C.gdf * w * (dv * nd) * nd));
             out[D + d] = static_cast<R>(C.srf * sw * nd * xf[d]);
@@ -1029,6 +1103,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
                                                          unsigned long long *sig_part) {
   cil::enter_step_kernel();
   using R = typename std::conditional<MIXED, float, double>::type;
+  using X = R;  // displacements
   __shared__ PairWarp<D, D, R> s_warp[kPairBlock / 32];
   PairWarp<D, D, R> &W = s_warp[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairBlock + threadIdx.x;
@@ -1043,45 +1118,59 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
 #pragma unroll
   for (int d = 0; d < D; ++d) vi[d] = live ? S.v[d * cap + i] : 0.0;
   if (sub == 0) {
+    if (MIXED) {
+      const float4 u = live ? O.loc[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const ushort4 b = live ? O.cell[q] : make_ushort4(0, 0, 0, 0);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        W.u[el * D + d] = f4c(u, d);
+        W.cell[el * D + d] = d == 0 ? b.x : (d == 1 ? b.y : b.z);
+      }
+    }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
+      if (!MIXED) W.x[el * D + d] = live ? O.x[d * cap + q] : 0.0;
       W.v[el * D + d] = static_cast<R>(vi[d]);
     }
   }
   __syncwarp();
   const double rc = C.sigma_core;
   const float rcf = static_cast<float>(rc);
+  const float radius = fmaxf(sigma_max_f(cnt), __double2float_ru(rc));
+  const int whole = MIXED ? whole_axes<D>(C, radius) : 0;
   R acc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) acc[d] = R(0);
   walk_pairs<D, D, R>(
-      C, W, O, start, live, q, lane_bits, fmaxf(sigma_max_f(cnt), __double2float_ru(rc)),
+      C, W, O, start, live, q, lane_bits, radius,
       [&](const float4 &, const float4 &) { return rcf * rcf; },
       [&](int o, int tt, R *out) {
-        double rij[D], r2 = 0.0;
+        X rij[D];
+        double r2 = 0.0;
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-          double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
-          if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
-          rij[d] = v;
-          if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
-          out[d] = R(0);
-        }
-        if (MIXED) {
-          float df[D], r2f = 0.0f;
+        for (int d = 0; d < D; ++d) out[d] = R(0);
+        if constexpr (MIXED) {
+          local_separation<D>(C, O, W, whole, o, tt, rij);
+        } else {
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            df[d] = static_cast<float>(rij[d]);
-            r2f += df[d] * df[d];
+            double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+            if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
+            rij[d] = v;
+            r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
           }
+        }
+        if (MIXED) {
+          float r2f = 0.0f;
+#pragma unroll
+          for (int d = 0; d < D; ++d) r2f += rij[d] * rij[d];
           if (!(r2f < rcf * rcf) || r2f == 0.0f) return;
           const float4 vj4 = __ldg(vel + tt);
           const float rinv = rsqrtf(r2f);
           const float w = 1.0f - r2f / rcf;
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            const float nd = -df[d] * rinv;
+            const float nd = -rij[d] * rinv;
             const float dv = static_cast<float>(W.v[o * D + d]) - f4c(vj4, d);
             out[d] = static_cast<R>(-(C.gdf * w * (dv * nd) * nd));
           }
@@ -1575,6 +1664,7 @@ void set_bins(cil_cycle *h, double smax, int ncells) {
       C.bw[d] = 1.0;
       C.inv_bw[d] = 1.0;
     }
+    C.bwf[d] = static_cast<float>(C.bw[d]);
     C.scalef[d] = static_cast<float>(C.inv_bw[d]);
     C.inv_bwf[d] = std::nextafter(static_cast<float>(C.inv_bw[d]), INFINITY);
     h->nbins *= C.ns[d];
@@ -1928,7 +2018,9 @@ cil_status cil_cycle_create(const cil_cycle_params *p, int32_t capacity, uint64_
   if (ok && p->precision == 1 && C.dpd) {
     h->O.vel = h->alloc<float4>(cap);
     h->vel_next = h->alloc<float4>(cap);
-    ok = h->O.vel && h->vel_next;
+    h->O.loc = h->alloc<float4>(cap);
+    h->O.cell = h->alloc<ushort4>(cap);
+    ok = h->O.vel && h->vel_next && h->O.loc && h->O.cell;
   }
   h->nblocks = (capacity + 31) / 32;  // blocks of the per-cell event kernels at their smallest (32 threads)
   h->nparts = (h->nbins_cap + kScanTile - 1) / kScanTile + 1;
