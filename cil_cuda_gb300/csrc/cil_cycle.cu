@@ -1028,7 +1028,8 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
           if (!(r2f < rc * rc) || r2f == 0.0f) return;
           const float4 vj4 = __ldg(O.vel + tt);
           const float rinv = rsqrtf(r2f);
-          const float w = 1.0f - r2f * rinv / rc;
+          // within the range by a few units of the last place, r2f rinv may pass rc: not below 0
+          const float w = fmaxf(1.0f - r2f * rinv / rc, 0.0f);
           float xf[4];
           normal2f(philox4x32_10(a, ts, kCyDpd0, z, C.seed_lo, C.seed_hi), &xf[0], &xf[1]);
           if (D == 3) normal2f(philox4x32_10(a, ts, kCyDpd1, z, C.seed_lo, C.seed_hi), &xf[2], &xf[3]);

@@ -33,3 +33,30 @@ def test_pairs_at_the_end_of_their_range_keep_their_values(gpu_lib, name, dim, L
         np.testing.assert_allclose(got[k], want, rtol=1e-6, atol=1e-9 * np.abs(want).max(), err_msg=k)
     want = z["%s.out.vel" % name]
     assert np.abs(got["vel"] - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_pairs_within_a_few_units_of_their_range(gpu_lib, dim):
+    """r below rc by 0 to 3 units of 2^-24: the FP32 quotient r / rc rounds past 1 for some per cent of the pairs
+    whose r2 is the number below rc^2 (diameters between 0.9 and 1 have most), and the weight under the root is 0 then, not negative. sqrt(w) is at
+    most sqrt(2^-19) (the units, and the FP32 rounding of coordinates below 2 with their differences), a
+    normal from 24-bit uniforms at most 5.77."""
+    m, L, count = _recipe(), 400.0 if dim == 2 else 88.0, 10000
+    rng = np.random.default_rng(5 + dim)
+    pos, sigma = m.pairs(rng, dim, L, 4.0, count)
+    sigma *= 0.86
+    u = pos[1::2] - pos[0::2]
+    u -= np.round(u / L) * L
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    pos[1::2] = np.mod(pos[0::2] + sigma[0::2, None] * (1 - rng.integers(0, 4, count) * 2.0**-24)[:, None] * u, L)
+    n = len(sigma)
+    st = dict(pos=pos, sigma=sigma, theta=np.zeros(n), rho=np.ones(n), angvel=np.full(n, 1e-4),
+              vel=np.full((n, dim), 0.05))
+    p = m.params(gpu_lib, dim, L)
+    eng = gpu_lib.CycleEngine(p, n, seed=3)
+    eng.upload(**st)
+    ran = eng.download()["force_ran"]
+    eng.step(2)
+    eng.close()
+    assert np.all(np.isfinite(ran)) and np.count_nonzero(ran) > n // 8
+    assert np.abs(ran).max() <= np.sqrt(2 * p["dis_diff"] * p["kbt"]) * np.sqrt(2.0**-19) * 5.77
