@@ -687,12 +687,26 @@ __device__ __forceinline__ float pair_f0_fast(float r2, float si, float sj, floa
   }
 }
 
-// The largest distance at which the law acts between elements of diameters si, sj (the Verlet
-// lists add the skin to it).
-template <int LAW>
-__device__ __forceinline__ float law_cutoff_f(const ColonyConst &C, float si, float sj) {
-  const float sij = 0.5f * (si + sj);
-  return LAW == CIL_FORCE_SC ? C.rcs_f * (sij + C.well_sigma_f) : C.rcs_f * sij;
+// Whether the candidate with record p, `row` of the neighbour rows and l bins away along the last axis
+// (-1, 0, 1), is within the list reach of an element at ui. k_skin_lists counts by it and k_list_flatten
+// repeats it for the candidates past its mask; the count must come out the same, so every operation that
+// the compiler could contract differently in the two is written out.
+template <int D, int LAW>
+__device__ __forceinline__ bool list_reaches(const ColonyConst &C, const float *ui, float si, float skin,
+                                             const float4 &p, int row, int l) {
+  const int oo[3] = {(D == 2 ? row : row / 3) - 1, D == 2 ? l : row % 3 - 1, l};
+  float r2 = 0.0f;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float origin = static_cast<float>(oo[d]) * C.bwf[d];  // exact
+    const float dx = __fadd_rn(pk_c(p, d), __fadd_rn(origin, -ui[d]));
+    r2 = __fmaf_rn(dx, dx, r2);
+  }
+  // the largest separation at which the law acts, plus the skin
+  float sij = 0.5f * __fadd_rn(si, fabsf(p.w));
+  if (LAW == CIL_FORCE_SC) sij = __fadd_rn(sij, C.well_sigma_f);
+  const float cut = __fmaf_rn(C.rcs_f, sij, skin);
+  return r2 < __fmul_rn(cut, cut);
 }
 
 // ---------------------------------------------------------------- kernel argument packs

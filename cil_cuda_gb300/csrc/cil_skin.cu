@@ -335,21 +335,6 @@ __device__ __forceinline__ int candidate_slot(const SkinArgs &a, int at, float z
   return D == 2 ? __float_as_int(z) : static_cast<int>(a.perm[at] & 0xffffffffu);
 }
 
-// whether the candidate with record p, l bins away along the last axis (-1, 0, 1), is within reach
-template <int D, int LAW>
-__device__ __forceinline__ bool list_reaches(const ColonyConst &C, const float *ui, float si, float skin,
-                                             const float4 &p, int row, int l) {
-  const int oo[3] = {(D == 2 ? row : row / 3) - 1, D == 2 ? l : row % 3 - 1, l};
-  float r2 = 0.0f;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const float dx = pk_c(p, d) + (static_cast<float>(oo[d]) * C.bwf[d] - ui[d]);
-    r2 += dx * dx;
-  }
-  const float cut = law_cutoff_f<LAW>(C, si, fabsf(p.w)) + skin;
-  return r2 < cut * cut;
-}
-
 // Bound by its round trips to L2, so the candidates' records are read as ranges, in the bin order's own
 // copy, with kListAhead in flight: one round trip per batch. Through the bin order's slots (slot, then
 // element id and record, two in flight) a build of the 2M-element 2D colony took 400 us and its

@@ -1,0 +1,106 @@
+"""Device functions by themselves: a probe compiled from csrc's headers, with and without FMA contraction
+(the library's translation units use both)."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from cil_cuda_gb300 import build as B
+
+pytestmark = pytest.mark.gpu
+
+PROBE = r"""
+#include "cil_internal.cuh"
+using namespace cil;
+
+template <int LAW>
+__global__ void k_reaches(ColonyConst C, int n, const float4 *p, const float2 *u, float si, float skin, int *in) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float ui[2] = {u[i].x, u[i].y};
+  in[i] = list_reaches<2, LAW>(C, ui, si, skin, p[i], 1, 0) ? 1 : 0;
+}
+
+template <class T>
+static T *up(const void *src, size_t bytes) {
+  void *q = nullptr;
+  if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
+  cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice);
+  return static_cast<T *>(q);
+}
+
+extern "C" int reaches(int well, int n, const float *p, const float *u, float si, float skin, float rcs, float xi,
+                       int *in) {
+  ColonyConst C{};
+  C.rcs_f = rcs;
+  C.well_sigma_f = xi;
+  C.bwf[0] = C.bwf[1] = 2.0f;
+  float4 *dp = up<float4>(p, 16 * size_t(n));
+  float2 *du = up<float2>(u, 8 * size_t(n));
+  int *di = up<int>(in, 4 * size_t(n));
+  if (well)
+    k_reaches<CIL_FORCE_SC><<<(n + 127) / 128, 128>>>(C, n, dp, du, si, skin, di);
+  else
+    k_reaches<CIL_FORCE_SOFTCORE><<<(n + 127) / 128, 128>>>(C, n, dp, du, si, skin, di);
+  const cudaError_t e = cudaMemcpy(in, di, 4 * size_t(n), cudaMemcpyDeviceToHost);
+  cudaFree(dp);
+  cudaFree(du);
+  cudaFree(di);
+  return static_cast<int>(e);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def probes(tmp_path_factory):
+    d = tmp_path_factory.mktemp("probe")
+    src = d / "probe.cu"
+    src.write_text(PROBE)
+    out, running = {}, []
+    for fmad in ("true", "false"):
+        so = str(d / ("probe_%s.so" % fmad))
+        running.append((fmad, so, subprocess.Popen([B.nvcc(), *B.ARCH, "-O3", "-std=c++17", "--fmad=" + fmad, "-shared",
+                                                    "-Xcompiler", "-fPIC", "-I", os.path.join(B.ROOT, "include"),
+                                                    "-I", B.CSRC, str(src), "-o", so])))
+    for fmad, so, p in running:
+        assert p.wait() == 0
+        out[fmad] = C.CDLL(so)
+    return out
+
+
+def _fma32(a, b, c):
+    # products and sums of FP32 numbers within a few binades of each other are exact in 64 bits
+    return (a.astype(np.float64) * b + c).astype(np.float32)
+
+
+@pytest.mark.parametrize("well", [0, 1])
+def test_list_reach_rounds_as_stated(gpu_lib, probes, well):
+    """The list build decides each pair in two kernels, which must agree in the last bit: the sums and
+    products of the decision are the stated ones, whatever the compiler may contract. Pairs within a
+    unit of the last place of the reach, where a sum of rounded squares decides some the other way."""
+    rng = np.random.default_rng(8)
+    f = np.float32
+    si, sj, skin, rcs, xi = f(1.0371), f(0.9713), f(0.31), f(1.0923), f(0.0517)
+    sij = f(0.5) * (si + sj)
+    if well:
+        sij = sij + xi
+    cut = _fma32(np.array([rcs]), np.array([sij]), skin)[0]
+    n = 200000
+    d = np.empty((n, 2), f)
+    d[:, 0] = rng.uniform(0.1, 0.9, n) * cut
+    d[:, 1] = np.sqrt(np.float64(cut) ** 2 - d[:, 0].astype(np.float64) ** 2)
+    u = np.zeros((n, 2), f)  # the element at its bin's origin: the differences are the records' own
+    p = np.zeros((n, 4), f)
+    p[:, :2] = d
+    p[:, 3] = -sj  # a record with its sign set counts by its magnitude
+    want = _fma32(d[:, 1], d[:, 1], d[:, 0] * d[:, 0]) < cut * cut
+    other = d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1] < cut * cut
+    assert 0 < want.sum() < n and (want != other).sum() > n // 100
+    for lib in probes.values():
+        got = np.zeros(n, np.int32)
+        a = [np.ascontiguousarray(v) for v in (p, u)]
+        assert lib.reaches(well, n, a[0].ctypes.data_as(C.c_void_p), a[1].ctypes.data_as(C.c_void_p), C.c_float(si),
+                           C.c_float(skin), C.c_float(rcs), C.c_float(xi), got.ctypes.data_as(C.c_void_p)) == 0
+        np.testing.assert_array_equal(got.astype(bool), want)
