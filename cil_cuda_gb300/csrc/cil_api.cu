@@ -810,15 +810,17 @@ cudaEvent_t pool_event(cil_handle *h, size_t i) {
 
 // Lanes per element of the FP64 force pass: as many as keep the walk and the pair evaluation of a
 // small colony spread over every SM, up to 8, while the elements give fewer than two warps per
-// scheduler (nsm x 4 x 2 x 32 lanes). From the cells the host knows of (uploaded, or counted by the
-// last cil_step); the forces do not depend on it. Step of the growth colony with 1, 2, 4, 8 lanes
+// scheduler (nsm x 4 x 2 x 32 lanes), and while the grid, which covers the capacity, stays within 8192
+// blocks (an empty block costs about 0.9 ns, more than lanes save beyond that: 500 cells at a capacity of 2M
+// took 271 us a step with 262 144 blocks, 51 with 32 768; 29 at a capacity of 664). From the cells the host
+// knows of (uploaded, or counted by the last cil_step); the forces do not depend on it. Step of the growth colony with 1, 2, 4, 8 lanes
 // (when a step had 15 launches):
 // 500 cells 48, 46, 44, 42 us; 4864 cells 61, 56, 57, 61 us; 19456 cells 72, 73, 87, 107 us.
 void set_lane_bits(cil_handle *h) {
   long long elems = 0;
   for (int c = 0; c < h->B; ++c) elems += 2ll * h->hc[c].n_seen;
   int b = 0;
-  while (b < 3 && elems * (2ll << b) <= 2ll * h->nsm * 4 * 32) ++b;
+  while (b < 3 && elems * (2ll << b) <= 2ll * h->nsm * 4 * 32 && h->stiles * (4ll << b) <= 8192) ++b;
   h->lane_bits = b;
   // The list force kernel's default form for more cells than one wave of its first form holds (6
   // blocks of 128 threads an SM): with a third more warps an SM the pass hides more of its loads (legs

@@ -1,0 +1,56 @@
+"""Engines whose capacity is far above their cells: an early colony in an engine sized for its end. The
+force passes' grids follow the cells known of, the results do not depend on them, and a step takes about
+what it takes in a small engine."""
+import time
+
+import numpy as np
+import pytest
+
+import cil_cuda_gb300 as G
+from cil_cuda_gb300 import synthetic as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _early(n=500, dim=2):
+    p = S.growth_params(box=256.0, dt=1e-4, divide=0, apop_rate=0.0, noise_D=0.0)
+    return p, S.disk_colony(n, p, seed=3)
+
+
+def _engine(p, cap, precision, skin):
+    return G.Engine([p], [cap], precision=precision, rng=G.RNG_PHILOX, seed=4, skin=skin)
+
+
+@pytest.mark.parametrize("precision", [G.PREC_FP64, G.PREC_MIXED])
+def test_results_do_not_depend_on_the_capacity(gpu_lib, precision):
+    # FP64: 8 lanes per element, then 2 and 1. Without lists every sum has its order: equal. (With lists their
+    # order is that of the cells' arrival in the bins, which differs from run to run.)
+    p, st = _early()
+    got = []
+    for cap in (600, 200000, 300000):
+        eng = _engine(p, cap, precision, 0.0)
+        eng.upload(0, **st)
+        eng.step(20)
+        got.append(eng.download(0))
+        eng.close()
+    for g in got[1:]:
+        np.testing.assert_array_equal(g["pos"], got[0]["pos"])
+
+
+@pytest.mark.parametrize("precision,skin,cap,most", [(G.PREC_FP64, 0.0, 1000000, 2.0)])
+def test_a_step_costs_about_as_much_in_a_large_engine(gpu_lib, precision, skin, cap, most):
+    # blocks for every tile and lane of the capacity: 5 times the small engine's
+    p, st = _early()
+    best = []
+    for c in (600, cap):
+        eng = _engine(p, c, precision, skin)
+        eng.upload(0, **st)
+        eng.step(40)
+        t = []
+        for _ in range(25):
+            t0 = time.perf_counter()
+            eng.step(40)
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+        eng.close()
+    assert best[1] <= most * best[0]
