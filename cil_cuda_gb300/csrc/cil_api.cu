@@ -48,7 +48,7 @@ struct HostColony {
 }  // namespace
 
 struct GraphSlot {
-  int key;                 // cur | meta << 1 | pu << 2 at the first step, | two steps << 3, | last << 4, lane bits << 5, many << 7
+  int key;                 // cur | meta << 1 | pu << 2 at the first step, | two steps << 3, | last << 4, lane bits << 5, many << 7, list class << 8
   uint64_t gen;
   cudaGraphExec_t exec;
   int64_t launches;        // kernels in the graph
@@ -94,6 +94,8 @@ struct cil_handle {
   float4 *d_rec = nullptr;  // FP64 form: FP32 absolute coordinates and diameter per slot
   int lane_bits = 0;        // FP64 form: log2 of the lanes per element of the force pass
   bool many = false;        // the list force kernel's form for many cells (set_lane_bits)
+  int list_blocks = 0;      // its blocks: 2048 << list_class, at most one per tile of the capacity (set_lane_bits)
+  int list_class = 0;
   double *d_sigma_c = nullptr;  // canonical diameters [2 * CC]
   bool need_exact = true;       // next rebuild takes the FP64 reference path
   bool due_events = false;      // Philox draws, no crawling/dividing cells: events from the due-cell queues
@@ -828,6 +830,18 @@ void set_lane_bits(cil_handle *h) {
   // 33.2), but segments shrink from 544 to 352 entries, which a colony that does not fill the chip pays
   // for (300 cells 2.80 -> 2.90 ms).
   h->many = elems / 2 > 6ll * 128 * h->nsm;
+  // Its blocks: one per tile of the capacity, unless the cells known of leave most of those empty (500
+  // cells at a capacity of 2M: 15 625 blocks took 18.2 us a pass, 2048 that take the tiles in turn 7.6). A
+  // colony that outgrows twice its tiles within a call has several a block until the next call. Blocks of
+  // 256 and 512 cells are a half and a quarter as many and keep one per tile.
+  long long tiles = 0;
+  for (int c = 0; c < h->B; ++c) tiles += (h->hc[c].n_seen + h->cell_block - 1) / h->cell_block;
+  h->list_class = 0;
+  h->list_blocks = h->ptiles;
+  if (h->cell_block == 128) {
+    while ((2048ll << h->list_class) < std::min<long long>(2 * tiles, h->ptiles)) ++h->list_class;
+    h->list_blocks = static_cast<int>(std::min<long long>(2048ll << h->list_class, h->ptiles));
+  }
 }
 
 // Error bits of the colonies' counters as a status (and the handle's message).
@@ -1010,7 +1024,8 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
   fa.heun = heun;
   fa.collect_due = (!oracle && heun != 1) ? 1 : 0;  // the step's events read the due-cell queue
   const int variant = h->list_variant == 0 && h->many ? 4 : h->list_variant;
-  launch_force_list(fa, h->D, h->cfg.force_law, h->ptiles, variant, h->cell_block, h->stream);  // skin mode
+  fa.list_loop = h->list_blocks < h->ptiles;
+  launch_force_list(fa, h->D, h->cfg.force_law, h->list_blocks, variant, h->cell_block, h->stream);  // skin mode
   h->launches += 1;
   h->cur = 1 - h->cur;
   if (h->cfg.precision == CIL_PREC_MIXED) h->pu = 1 - h->pu;
@@ -1077,7 +1092,7 @@ void restore_host_state(cil_handle *h, const HostStepState &s) {
 // switched off for the handle and null is returned.
 cudaGraphExec_t steady_graph(cil_handle *h, int nsteps, bool last, int64_t *launches_per_graph) {
   const int key = h->cur | (h->meta << 1) | (h->pu << 2) | ((nsteps == 2 ? 1 : 0) << 3) | ((last ? 1 : 0) << 4) |
-                  (h->lane_bits << 5) | ((h->many ? 1 : 0) << 7);
+                  (h->lane_bits << 5) | ((h->many ? 1 : 0) << 7) | (h->list_class << 8);
   for (auto &gs : h->graphs)
     if (gs.key == key && gs.gen == h->graph_gen) {
       HostStepState s = host_state(h);

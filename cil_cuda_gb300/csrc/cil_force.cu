@@ -935,9 +935,9 @@ __device__ __forceinline__ void pairs_finish(const ForceArgs &a, const ColonyCon
 // and noise terms are the expressions of the other force kernels, the pair terms are summed in
 // list order, and pairs with fresh elements (created or moved by a division since the last
 // list build, in no list) arrive through facc from k_fresh_pairs.
+// One tile of TILE cells, the whole block.
 template <int D, int LAW, int UNROLL, int MINB, int TILE>
-__global__ void __launch_bounds__(TILE, MINB) k_force_cells(const ForceArgs a) {
-  enter_step_kernel();
+__device__ __forceinline__ void force_tile(const ForceArgs &a, int t) {
   constexpr int SEG = pair_seg<D, MINB, TILE>();
   extern __shared__ __align__(16) unsigned char s_pairs[];
   __shared__ ColonyConst sC;
@@ -947,8 +947,6 @@ __global__ void __launch_bounds__(TILE, MINB) k_force_cells(const ForceArgs a) {
   __shared__ int s_nbuilt;
   __shared__ int s_warps_done;
   __shared__ __align__(16) float s_off[kOffCodes<D> * kOffStride<D>];
-  const int t = blockIdx.x;
-  if (t >= a.tiles[a.B]) return;  // uniform per block (tiles over slot pairs)
   const int tid = threadIdx.x;
   const int c = colony_of_tile(a.tiles, a.B, t);
   {
@@ -1260,7 +1258,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_force_cells(const ForceArgs a) {
       __threadfence_block();
       if (atomicAdd(&s_warps_done, 1) == TILE / 32 - 1) {
         __threadfence_block();
-        StatPart &P = a.spart[c * kStatSlots + (blockIdx.x & (kStatSlots - 1))];
+        StatPart &P = a.spart[c * kStatSlots + (t & (kStatSlots - 1))];
         atomicMax(&P.dmax, atomicOr(&s_dmax, 0u));
         if (a.sched) {
           atomicMax(&P.smax, atomicOr(&s_smax, 0u));
@@ -1271,28 +1269,45 @@ __global__ void __launch_bounds__(TILE, MINB) k_force_cells(const ForceArgs a) {
   }
 }
 
-template <int D, int LAW, int UNROLL, int MINB, int TILE>
+// LOOP: the blocks take the tiles (over slot pairs) in turn, the grid of few cells in a large capacity;
+// otherwise a tile each, which is 0.6 to 1.3 % of a leg faster where most blocks have one.
+template <int D, int LAW, int UNROLL, int MINB, int TILE, bool LOOP>
+__global__ void __launch_bounds__(TILE, MINB) k_force_cells(const ForceArgs a) {
+  enter_step_kernel();
+  if (!LOOP) {
+    if (static_cast<int>(blockIdx.x) < a.tiles[a.B]) force_tile<D, LAW, UNROLL, MINB, TILE>(a, blockIdx.x);
+  } else {
+    for (int t = blockIdx.x; t < a.tiles[a.B]; t += gridDim.x) {
+      force_tile<D, LAW, UNROLL, MINB, TILE>(a, t);
+      __syncthreads();
+    }
+  }
+}
+
+template <int D, int LAW, int UNROLL, int MINB, int TILE, bool LOOP>
 void launch_cells_t(const ForceArgs &a, int grid, cudaStream_t s) {
   constexpr int bytes = (TILE / 32) * pair_smem_warp<D, pair_seg<D, MINB, TILE>()>();
   static bool attr_set = false;  // per instantiation; the attribute is per function
   if (!attr_set) {
-    cudaFuncSetAttribute(k_force_cells<D, LAW, UNROLL, MINB, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_force_cells<D, LAW, UNROLL, MINB, TILE, LOOP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          bytes);
     attr_set = true;
   }
-  launch_step(true, grid, TILE, bytes, s, k_force_cells<D, LAW, UNROLL, MINB, TILE>, a);
+  launch_step(true, grid, TILE, bytes, s, k_force_cells<D, LAW, UNROLL, MINB, TILE, LOOP>, a);
 }
 
 // MINB is the CTAs per SM at 256 threads; 128-thread blocks keep its threads per SM (hence the
 // register budget per thread), 512-thread blocks take at most as many threads per SM
 template <int D, int LAW, int UNROLL, int MINB>
 void launch_cells(const ForceArgs &a, int grid, int block, cudaStream_t s) {
-  if (block == 128)
-    launch_cells_t<D, LAW, UNROLL, 2 * MINB, 128>(a, grid, s);
+  if (block == 128 && a.list_loop)
+    launch_cells_t<D, LAW, UNROLL, 2 * MINB, 128, true>(a, grid, s);
+  else if (block == 128)
+    launch_cells_t<D, LAW, UNROLL, 2 * MINB, 128, false>(a, grid, s);
   else if (block == 512)
-    launch_cells_t<D, LAW, UNROLL, (MINB / 2 > 0 ? MINB / 2 : 1), 512>(a, grid, s);
+    launch_cells_t<D, LAW, UNROLL, (MINB / 2 > 0 ? MINB / 2 : 1), 512, false>(a, grid, s);
   else
-    launch_cells_t<D, LAW, UNROLL, MINB, 256>(a, grid, s);
+    launch_cells_t<D, LAW, UNROLL, MINB, 256, false>(a, grid, s);
 }
 
 template <int D, int LAW>

@@ -780,6 +780,7 @@ struct ForceArgs {
   const int *slot_of;
   // skin mode (null otherwise)
   const int *tiles;        // skin mode: tiles over slot pairs (k_force_cells)
+  bool list_loop;          // and fewer blocks than the capacity has tiles
   ColonySkin *skin;
   const int *ncnt;
   // the lists per warp of 32 cells (64 slots from w0), flattened: entries and their owners

@@ -37,9 +37,32 @@ def test_results_do_not_depend_on_the_capacity(gpu_lib, precision):
         np.testing.assert_array_equal(g["pos"], got[0]["pos"])
 
 
-@pytest.mark.parametrize("precision,skin,cap,most", [(G.PREC_FP64, 0.0, 1000000, 2.0)])
+def test_growth_past_the_grid_within_one_call(gpu_lib):
+    """131 000 cells in lists (1024 tiles of 128, 2048 blocks) that grow past 262 144 (2048 tiles) within
+    one call, so that blocks take several tiles, against calls of 20 steps, whose grids follow. dt 1e-5: a
+    step's displacements agree to 1e-6 of a force below 2e3 (FP32 sums in two orders, as fresh pairs
+    arrive by atomics), and a tile left out would leave stale positions behind."""
+    p = S.growth_params(box=1500.0, dt=1e-5, div_tau_mu=1.2e-3, div_tau_sigma=5e-5, apop_rate=0.0, noise_D=0.0)
+    st = S.disk_colony(131000, p, seed=5, phi=0.15)
+    steps, got = 240, []
+    for call in (steps, 20):
+        eng = _engine(p, 700000, G.PREC_MIXED, 0.3)
+        eng.upload(0, **st)
+        for _ in range(steps // call):
+            eng.step(call)
+        got.append(eng.download(0))
+        eng.close()
+    a, b = got
+    assert a["ncells"] == b["ncells"] > 300000
+    np.testing.assert_array_equal(a["tswitch"], b["tswitch"])
+    d = a["pos"] - b["pos"]
+    d -= np.round(d / 1500.0) * 1500.0
+    assert np.abs(d).max() <= steps * 1e-6 * 2e3 * 1e-5
+
+
+@pytest.mark.parametrize("precision,skin,cap,most", [(G.PREC_FP64, 0.0, 1000000, 2.0), (G.PREC_MIXED, 0.3, 2000000, 1.4)])
 def test_a_step_costs_about_as_much_in_a_large_engine(gpu_lib, precision, skin, cap, most):
-    # blocks for every tile and lane of the capacity: 5 times the small engine's
+    # blocks for every tile and lane of the capacity: 5 times (FP64) and 1.65 times the small engine's
     p, st = _early()
     best = []
     for c in (600, cap):
