@@ -18,7 +18,8 @@ from . import Engine, PREC_MIXED, RNG_PHILOX
 
 BIN_FACTORS = (1.0, 1.15, 1.3)
 BLOCK_SIZES = (128, 256, 512)  # threads (cells) per block of the list force kernel; stage 1 runs the first
-VARIANTS = ((4, 3), (2, 3), (1, 3), (1, 4))  # (chunks of 32 list entries in flight per warp, CTAs per SM)
+# (chunks of 32 list entries in flight per warp, CTAs per SM); (0, 0): the library's choice by the cells
+VARIANTS = ((0, 0), (4, 3), (2, 3), (1, 3), (1, 4))
 
 
 def needed_width(params, states, skin):

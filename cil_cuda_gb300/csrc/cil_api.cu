@@ -75,6 +75,7 @@ struct cil_handle {
   int ptiles = 0;      // tiles over the slot pairs of the capacity (grid of the list force kernel)
   int cell_block = 256;  // threads (cells) per block of the list force kernel
   int list_variant = 0;  // list force kernel: staging depth and CTAs per SM (cil_config.staging/occupancy)
+  bool list_default = false;  // neither was asked for: its form for many cells may take its place (set_lane_bits)
   int nsm = 0;
   bool geometry_ready = false;
   int64_t ts = 0;
@@ -824,12 +825,12 @@ void set_lane_bits(cil_handle *h) {
   int b = 0;
   while (b < 3 && elems * (2ll << b) <= 2ll * h->nsm * 4 * 32 && h->stiles * (4ll << b) <= 8192) ++b;
   h->lane_bits = b;
-  // The list force kernel's default form for more cells than one wave of its first form holds (6
-  // blocks of 128 threads an SM): with a third more warps an SM the pass hides more of its loads (legs
-  // of 1M cells 14.89 -> 14.44 ms, of the 0.4M-cell 3D channel 5.20 -> 5.09, of a sweep of 0.29M 33.8 ->
-  // 33.2), but segments shrink from 544 to 352 entries, which a colony that does not fill the chip pays
-  // for (300 cells 2.80 -> 2.90 ms).
-  h->many = elems / 2 > 6ll * 128 * h->nsm;
+  // The list force kernel's form when none is asked for, at the default 128 cells a block, for more cells
+  // than one wave of its first form holds (6 blocks an SM): with a third more warps an SM the pass hides more
+  // of its loads (legs of 1M cells 14.89 -> 14.44 ms, of the 0.4M-cell 3D channel 5.20 -> 5.09, of a sweep of
+  // 0.29M 33.8 -> 33.2), but segments shrink from 544 to 352 entries, which a colony that does not fill the
+  // chip pays for (300 cells 2.80 -> 2.90 ms).
+  h->many = h->list_default && h->cell_block == 128 && elems / 2 > 6ll * 128 * h->nsm;
   // Its blocks: one per tile of the capacity, unless the cells known of leave most of those empty (500
   // cells at a capacity of 2M: 15 625 blocks took 18.2 us a pass, 2048 that take the tiles in turn 7.6). A
   // colony that outgrows twice its tiles within a call has several a block until the next call. Blocks of
@@ -1023,7 +1024,7 @@ cil_status enqueue_force_pass(cil_handle *h, bool last, int heun, bool first, cu
   ForceArgs fa = force_args(h, noise ? (oracle ? 2 : 1) : 0, 1, last ? h->d_vel : nullptr, nullptr);
   fa.heun = heun;
   fa.collect_due = (!oracle && heun != 1) ? 1 : 0;  // the step's events read the due-cell queue
-  const int variant = h->list_variant == 0 && h->many ? 4 : h->list_variant;
+  const int variant = h->many ? 4 : h->list_variant;
   fa.list_loop = h->list_blocks < h->ptiles;
   launch_force_list(fa, h->D, h->cfg.force_law, h->list_blocks, variant, h->cell_block, h->stream);  // skin mode
   h->launches += 1;
@@ -1212,6 +1213,7 @@ cil_status cil_create(const cil_config *cfg, const cil_colony_params *params, co
   auto *h = new cil_handle();
   h->cfg = *cfg;
   h->list_variant = list_variant;
+  h->list_default = cfg->staging == 0 && cfg->occupancy == 0;
   h->B = cfg->num_colonies;
   h->D = cfg->dim;
   h->hc.resize(h->B);

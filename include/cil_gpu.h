@@ -161,7 +161,8 @@ typedef struct cil_config {
   /* Verlet-list force kernel (skin mode: one thread per cell, each warp's list entries taken as
    * one flattened range): chunks of 32 entries in flight per warp (0 = 4; 1, 2) and CTAs per SM
    * of 256 threads it is compiled for (0 = 3; 4). Supported pairs: (4, 3), (2, 3), (1, 3),
-   * (1, 4). cil_cuda_gb300/autotune.py picks them. */
+   * (1, 4). Both 0 at 128 cells per block: (4, 3), or for more cells than its blocks hold at once a form
+   * with a third more warps an SM. cil_cuda_gb300/autotune.py picks them. */
   int32_t staging;
   int32_t occupancy;
   int32_t integrator;     /* CIL_INTEGRATOR_*: 0 = Euler */
