@@ -322,9 +322,12 @@ __device__ __forceinline__ double wrap_bits(double t, double L) {
 // instructions: one reciprocal square root per root or quotient, products with constants in place
 // of divisions, comparisons and sign tests on bit patterns.
 
-// 1 / sqrt(a) for normal a > 0: the hardware's approximate reciprocal square root y, then the
-// series 1 / sqrt(1 - e) = 1 + e / 2 + 3 e^2 / 8 + ... with e = 1 - a y^2 (its next term is below
-// 2^-53 for a seed good to 2^-18).
+// 1 / sqrt(a) for normal a > 0: an approximate y, then one step of Schroeder's iteration of order three
+// (E. Schroeder, Mathematische Annalen 2, 1870), the series 1 / sqrt(1 - e) = 1 + e / 2 + 3 e^2 / 8 + ... with
+// e = 1 - a y^2. PTX's rsqrt.approx.ftz.f64 takes the upper 32 bits of a and gives those of y, 20 bits of
+// mantissa each, so y is good to 2^-19 (half of the operand's 2^-20, and the result's), e is below 2^-18, and the
+// term left out, 5 e^3 / 16, below 2^-55. With the roundings of e and of the last sum, within 1.75 x 2^-53
+// of the value (1.40e-16 at most over 31M values; CUDA's rsqrt 1.12e-16).
 __device__ __forceinline__ double rsqrt_pos(double a) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
@@ -332,14 +335,17 @@ __device__ __forceinline__ double rsqrt_pos(double a) {
   return __fma_rn(__fma_rn(0.375, e, 0.5), y * e, y);
 }
 
-// sqrt(a) from y = rsqrt_pos(a): a y and one Newton residual
+// sqrt(a) from y = rsqrt_pos(a): a y, within 3 x 2^-53, and one Newton step on its residual a - s^2, whose
+// error is far below the last rounding's (the same as sqrt's over 31M values)
 __device__ __forceinline__ double sqrt_from(double a, double y) {
   const double s = a * y;
   return __fma_rn(__fma_rn(-s, s, a), 0.5 * y, s);
 }
 
-// 1 / a for normal a: the approximate reciprocal y, then 1 / (1 - e) = 1 + e + e^2 + ... with
-// e = 1 - a y
+// 1 / a for normal a: an approximate y and one step of the hyperpower iteration of order three (M. Altman,
+// Pacific Journal of Mathematics 10, 1960), 1 / (1 - e) = 1 + e + e^2 + ... with e = 1 - a y. rcp.approx.ftz.f64
+// is good to 2^-19 (20 bits of mantissa in and out), so e^3, the first term left out, is below 2^-57: within
+// 1.1 x 2^-53 of the value
 __device__ __forceinline__ double rcp_normal(double a) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));

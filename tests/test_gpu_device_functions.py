@@ -31,6 +31,27 @@ static T *up(const void *src, size_t bytes) {
   return static_cast<T *>(q);
 }
 
+// rsqrt_pos, sqrt_from, rcp_normal, CUDA's rsqrt, sqrt and reciprocal, the two approximate seeds, mid_range
+__global__ void k_roots(int n, const double *a, double *out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double x = a[i], y = rsqrt_pos(x);
+  double s, r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(s) : "d"(x));
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double v[9] = {y, sqrt_from(x, y), rcp_normal(x), rsqrt(x), sqrt(x), 1.0 / x, s, r, mid_range(x) ? 1.0 : 0.0};
+  for (int k = 0; k < 9; ++k) out[size_t(k) * n + i] = v[k];
+}
+
+extern "C" int roots(int n, const double *a, double *out) {
+  double *da = up<double>(a, 8 * size_t(n)), *dout = up<double>(out, 72 * size_t(n));
+  k_roots<<<(n + 127) / 128, 128>>>(n, da, dout);
+  const cudaError_t e = cudaMemcpy(out, dout, 72 * size_t(n), cudaMemcpyDeviceToHost);
+  cudaFree(da);
+  cudaFree(dout);
+  return static_cast<int>(e);
+}
+
 extern "C" int reaches(int well, int n, const float *p, const float *u, float si, float skin, float rcs, float xi,
                        int *in) {
   ColonyConst C{};
@@ -104,3 +125,54 @@ def test_list_reach_rounds_as_stated(gpu_lib, probes, well):
         assert lib.reaches(well, n, a[0].ctypes.data_as(C.c_void_p), a[1].ctypes.data_as(C.c_void_p), C.c_float(si),
                            C.c_float(skin), C.c_float(rcs), C.c_float(xi), got.ctypes.data_as(C.c_void_p)) == 0
         np.testing.assert_array_equal(got.astype(bool), want)
+
+
+def _roots(lib, a):
+    a = np.ascontiguousarray(a, np.float64)
+    out = np.empty((9, len(a)))
+    assert lib.roots(len(a), a.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)) == 0
+    return out
+
+
+def _mid_range_values():
+    """Random mantissas at every exponent of mid_range (2^-511 to 2^510), and both ends of each binade."""
+    rng = np.random.default_rng(12)
+    e = np.arange(-511, 510)
+    one = np.ldexp(1.0, e)
+    ends = np.concatenate([one * (1 + k * 2.0**-52) for k in range(4)] + [one * (2 - k * 2.0**-52) for k in range(1, 5)])
+    m = 1 + rng.integers(0, 2**52, 600000) * 2.0**-52
+    # the operand's low 32 bits, which the seeds ignore, all 0 and all 1
+    top = 1 + rng.integers(0, 2**20, 100000) * 2.0**-20
+    m = np.concatenate([m, top, top + 2.0**-20 - 2.0**-52])
+    return np.concatenate([ends, np.ldexp(m, rng.integers(-511, 510, len(m)))])
+
+
+def test_roots_and_reciprocals_within_their_bounds(gpu_lib, probes):
+    """The FP64 kernels' reciprocal square root, root and reciprocal against the values (in longer
+    arithmetic) and CUDA's results over mid_range. Seeds good to 2^-19 leave series terms below 2^-55 and
+    2^-57. rsqrt_pos: the last sum's rounding 2^-53, half of e's 2^-53 and the series 0.16 x 2^-53: 1.75 x
+    2^-53. sqrt_from: the last rounding, and terms below 2^-100: 0.501 units. rcp_normal: 1.1 x 2^-53. CUDA's
+    sqrt and division are correctly rounded and its rsqrt within a unit: at most 1, 1 and 2 units apart."""
+    a = _mid_range_values()
+    x = a.astype(np.longdouble)
+    assert np.finfo(np.longdouble).nmant >= 63
+    for lib in probes.values():
+        rs, sq, rc, c_rs, c_sq, c_rc, seed_rs, seed_rc, mid = _roots(lib, a)
+        assert np.all(mid == 1.0)
+        root = np.sqrt(x)
+        assert np.abs(seed_rs * root - 1).max() <= 2.0**-19
+        assert np.abs(seed_rc * x - 1).max() <= 2.0**-19
+        assert np.abs(rs * root - 1).max() <= 1.75 * 2.0**-53
+        assert (np.abs(sq - root) / np.spacing(sq)).max() <= 0.501
+        assert np.abs(rc * x - 1).max() <= 1.1 * 2.0**-53
+        for got, cuda, units in ((rs, c_rs, 2), (sq, c_sq, 1), (rc, c_rc, 1)):
+            assert (np.abs(got - cuda) / np.spacing(cuda)).max() <= units
+
+
+def test_mid_range_takes_its_range_only(gpu_lib, probes):
+    tiny, big = 2.0**-511, 2.0**510
+    out = [0.0, -0.0, -1.0, np.inf, -np.inf, np.nan, 5e-324, tiny * (1 - 2.0**-53), big, 1e300, 1e-300]
+    ins = [tiny, 1.0, big * (1 - 2.0**-53)]
+    for lib in probes.values():
+        mid = _roots(lib, np.array(out + ins))[8]
+        assert list(mid) == [0.0] * len(out) + [1.0] * len(ins)
