@@ -430,8 +430,8 @@ __device__ __forceinline__ int whole_axes(const CyConst &C, float radius) {
 template <int D, int NRES, typename R>
 __device__ __forceinline__ void local_separation(const CyConst &C, const CyOrdered &O, const PairWarp<D, NRES, R> &W,
                                                  int whole, int o, int tt, float *df) {
-  const float4 uj = __ldg(O.loc + tt);
-  const ushort4 cj = __ldg(O.cell + tt);
+  const float4 uj = O.loc[tt];
+  const ushort4 cj = O.cell[tt];
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     int off = (d == 0 ? cj.x : (d == 1 ? cj.y : cj.z)) - W.cell[o * D + d];
@@ -584,7 +584,7 @@ __device__ __forceinline__ void walk_pairs(const CyConst &C, PairWarp<D, NRES, R
         for (int u = 0; u < kPairAhead; ++u) {
           const int tt = tt0 + u * L + sub;
           there[u] = u < ahead && tt < en && tt != q;
-          p[u] = there[u] ? __ldg(O.rec + tt) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          p[u] = there[u] ? O.rec[tt] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
 #pragma unroll
         for (int u = 0; u < kPairAhead; ++u) {
@@ -735,7 +735,7 @@ __device__ __forceinline__ void contact_terms(const CyConst &C, const CyOrdered 
       df[d] = static_cast<float>(rij[d]);
       r2f += df[d] * df[d];
     }
-    const float sif = W.dia[o], sjf = __ldg(O.rec + tt).w;
+    const float sif = W.dia[o], sjf = O.rec[tt].w;
     const float cut = 0.5f * (sif + sjf);
     if (!(r2f <= cut * cut) || r2f == 0.0f) return;
     const float r = sqrtf(r2f);
@@ -760,7 +760,7 @@ __device__ __forceinline__ void contact_terms(const CyConst &C, const CyOrdered 
     for (int d = 0; d < D; ++d) out[d] = static_cast<R>(f0 * df[d]);
     out[D] = static_cast<R>(vol != 0.0f ? f0 / vol : 0.0f);
   } else {
-    const double ro = W.rad[o], rj = __ldg(O.rad + tt);
+    const double ro = W.rad[o], rj = O.rad[tt];
     double hy, r;
     if (mid_range(r2)) {
       const double y = rsqrt_pos(r2);
@@ -882,12 +882,12 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 7) k_cy_force(CyConst 
         double rij[D], r2 = 0.0;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-          double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+          double v = O.x[d * cap + tt] - W.x[o * D + d];
           if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
           rij[d] = v;
           if (!MIXED) r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
         }
-        contact_terms<D, MIXED>(C, O, W, o, tt, rij, r2, W.idx[o] < __ldg(O.idx + tt), out);
+        contact_terms<D, MIXED>(C, O, W, o, tt, rij, r2, W.idx[o] < O.idx[tt], out);
       },
       acc);
   unsigned long long sbits = 0ull;
@@ -1008,13 +1008,13 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
         } else {
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+            double v = O.x[d * cap + tt] - W.x[o * D + d];
             if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
             rij[d] = v;
             r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
           }
         }
-        const int io = W.idx[o], j = __ldg(O.idx + tt);
+        const int io = W.idx[o], j = O.idx[tt];
         const uint32_t a = static_cast<uint32_t>(io < j ? io : j), z = static_cast<uint32_t>(io < j ? j : io);
         contact_terms<D, MIXED>(C, O, W, o, tt, rij, r2, io < j, out);
         out += D + 1;
@@ -1024,9 +1024,9 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
           float r2f = 0.0f;
 #pragma unroll
           for (int d = 0; d < D; ++d) r2f += rij[d] * rij[d];
-          const float rc = io < j ? W.dia[o] : __ldg(O.rec + tt).w;
+          const float rc = io < j ? W.dia[o] : O.rec[tt].w;
           if (!(r2f < rc * rc) || r2f == 0.0f) return;
-          const float4 vj4 = __ldg(O.vel + tt);
+          const float4 vj4 = O.vel[tt];
           const float rinv = rsqrtf(r2f);
           // within the range by a few units of the last place, r2f rinv may pass rc: not below 0
           const float w = fmaxf(1.0f - r2f * rinv / rc, 0.0f);
@@ -1042,7 +1042,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
             out[D + d] = static_cast<R>(C.srf * sw * nd * xf[d]);
           }
         } else {
-          const double rc = 2 * (io < j ? W.rad[o] : __ldg(O.rad + tt));
+          const double rc = 2 * (io < j ? W.rad[o] : O.rad[tt]);
           double ir, r;
           if (mid_range(r2)) {
             ir = rsqrt_pos(r2);
@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
 #pragma unroll
           for (int d = 0; d < D; ++d) {
             const double nd = rij[d] * ir;
-            const double vj = __ldg(S.v + d * cap + j);
+            const double vj = S.v[d * cap + j];
             out[d] = static_cast<R>(-(gw * ((W.v[o * D + d] - vj) * nd) * nd));
             out[D + d] = static_cast<R>(sw * nd * xn[d]);
           }
@@ -1155,7 +1155,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
         } else {
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            double v = __ldg(O.x + d * cap + tt) - W.x[o * D + d];
+            double v = O.x[d * cap + tt] - W.x[o * D + d];
             if (C.periodic[d]) v = nearest(v, C.box[d], C.half[d]);
             rij[d] = v;
             r2 = d == 0 ? v * v : __fma_rn(v, v, r2);
@@ -1166,7 +1166,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
 #pragma unroll
           for (int d = 0; d < D; ++d) r2f += rij[d] * rij[d];
           if (!(r2f < rcf * rcf) || r2f == 0.0f) return;
-          const float4 vj4 = __ldg(vel + tt);
+          const float4 vj4 = vel[tt];
           const float rinv = rsqrtf(r2f);
           const float w = 1.0f - r2f / rcf;
 #pragma unroll
@@ -1176,7 +1176,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
             out[d] = static_cast<R>(-(C.gdf * w * (dv * nd) * nd));
           }
         } else {
-          const int j = __ldg(O.idx + tt);
+          const int j = O.idx[tt];
           double ir, r;
           if (mid_range(r2)) {
             ir = rsqrt_pos(r2);
@@ -1190,7 +1190,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
 #pragma unroll
           for (int d = 0; d < D; ++d) {
             const double nd = rij[d] * ir;
-            out[d] = static_cast<R>(-(gw * ((W.v[o * D + d] - __ldg(S.v + d * cap + j)) * nd) * nd));
+            out[d] = static_cast<R>(-(gw * ((W.v[o * D + d] - S.v[d * cap + j]) * nd) * nd));
           }
         }
       },

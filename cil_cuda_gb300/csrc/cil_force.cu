@@ -309,13 +309,13 @@ __global__ void __launch_bounds__(kF64Block, 8) k_force_fp64(ForceArgs a_, int l
             double r2 = 0.0;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-              double xj = __ldg(a.x_in + d * SS + tt);
+              double xj = a.x_in[d * SS + tt];
               const int k = (code >> (2 * d)) & 3;  // the neighbour's image: 1 below, 2 above
               if (k) xj = __dadd_rn(xj, k == 1 ? -C.box[d] : C.box[d]);
               dx[d] = xj - W.x[o * D + d];
               r2 += dx[d] * dx[d];
             }
-            const double f0 = pair_force_lean<LAW>(r2, W.hs[o], __ldg(a.sig + tt), eps, rcs, C.well_eps, C.well_sigma,
+            const double f0 = pair_force_lean<LAW>(r2, W.hs[o], a.sig[tt], eps, rcs, C.well_eps, C.well_sigma,
                                                    C.force_shifted);
 #pragma unroll
             for (int d = 0; d < D; ++d) W.res[(f - S) * D + d] = f0 * dx[d];
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(kF64Block, 8) k_force_fp64(ForceArgs a_, int l
           for (int u = 0; u < AHEAD; ++u) {
             const int tt = tt0 + u * L + sub;
             there[u] = tt < en && tt != s && tt != ps;
-            p[u] = there[u] ? __ldg(a.rec + tt) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            p[u] = there[u] ? a.rec[tt] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           }
 #pragma unroll
           for (int u = 0; u < AHEAD; ++u) {
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(kTile, 4) k_force_mixed(ForceArgs a_) {
         for (int t0 = st; t0 < en; t0 += kMixedAhead) {
           float4 pj[kMixedAhead];
 #pragma unroll
-          for (int u = 0; u < kMixedAhead; ++u) pj[u] = __ldg(a.pk + min(t0 + u, en - 1));
+          for (int u = 0; u < kMixedAhead; ++u) pj[u] = a.pk[min(t0 + u, en - 1)];
 #pragma unroll
           for (int u = 0; u < kMixedAhead; ++u) {
             const int tt = t0 + u;
@@ -889,7 +889,7 @@ __device__ __forceinline__ void pairs_finish(const ForceArgs &a, const ColonyCon
       }
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u)
-        pj[u] = own[u] >= 0 ? __ldg(a.pk + (ent[u] & ((1u << kListSlotBits) - 1u)))
+        pj[u] = own[u] >= 0 ? a.pk[ent[u] & ((1u << kListSlotBits) - 1u)]
                             : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
@@ -969,7 +969,7 @@ __device__ __forceinline__ void force_tile(const ForceArgs &a, int t) {
   }
   __syncthreads();
   const ColonyConst &C = sC;
-  const int ts = __ldg(a.ts_dev);
+  const int ts = *a.ts_dev;
   const size_t SS = a.SS;
   const int s0 = C.slot_base + 2 * ((t - a.tiles[c]) * TILE + tid);
   // every load of the cell is issued at once, guarded by the colony's slot capacity only (the
@@ -979,17 +979,17 @@ __device__ __forceinline__ void force_tile(const ForceArgs &a, int t) {
   float4 pr[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
   ushort2 ls = make_ushort2(0, 0);
   if (incap) {
-    ee = __ldg(reinterpret_cast<const int2 *>(a.eid + s0));
-    pr[0] = __ldg(a.pk + s0);
-    pr[1] = __ldg(a.pk + s0 + 1);
-    sb = __ldg(reinterpret_cast<const int2 *>(a.sbin + s0));
-    nn = __ldg(reinterpret_cast<const int2 *>(a.ncnt + s0));
-    ls = __ldg(reinterpret_cast<const ushort2 *>(a.lstart + s0));
-    if (C.divide) cy = __ldg(a.cyc + s0);
+    ee = *reinterpret_cast<const int2 *>(a.eid + s0);
+    pr[0] = a.pk[s0];
+    pr[1] = a.pk[s0 + 1];
+    sb = *reinterpret_cast<const int2 *>(a.sbin + s0);
+    nn = *reinterpret_cast<const int2 *>(a.ncnt + s0);
+    ls = *reinterpret_cast<const ushort2 *>(a.lstart + s0);
+    if (C.divide) cy = a.cyc[s0];
   }
   // the warp's entry count at the last build (warps past the slots of that build have none)
   const int sw0 = s0 - 2 * (tid & 31);
-  const int Tw = sw0 < C.slot_base + s_nbuilt ? __ldg(a.lwarp + (sw0 >> 6)) : 0;
+  const int Tw = sw0 < C.slot_base + s_nbuilt ? a.lwarp[sw0 >> 6] : 0;
   // fresh-pair contributions: one bit per slot; slot bases are 32-aligned and s0 is even, so
   // both bits of the cell sit in one word (16 cells per word)
   const unsigned tword = a.ftouch[s0 >> 5];
@@ -1149,7 +1149,7 @@ __device__ __forceinline__ void force_tile(const ForceArgs &a, int t) {
     } else {
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        const float2 uv = __ldg(reinterpret_cast<const float2 *>(a.uref + d * SS + s0));
+        const float2 uv = *reinterpret_cast<const float2 *>(a.uref + d * SS + s0);
         uref[0][d] = uv.x;
         uref[1][d] = uv.y;
       }

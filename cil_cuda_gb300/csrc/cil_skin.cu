@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kTile, 4) k_skin_lists(SkinArgs a) {
 #pragma unroll
             for (int u = 0; u < kListAhead; ++u) {
               const int at = min(t0 + u, en - 1);
-              pj[u] = __ldg(a.brec + at);
+              pj[u] = a.brec[at];
               tj[u] = candidate_slot<D>(a, at, pj[u].z);
             }
 #pragma unroll
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(kTile) k_list_flatten(SkinArgs a) {
               for (int u = 0; u < kFlatAhead; ++u) {
                 at[u] = bits ? rs + __ffsll(static_cast<long long>(bits)) - 1 : -1;
                 bits &= bits - 1ull;
-                slot[u] = at[u] >= 0 ? candidate_slot<D>(a, at[u], D == 2 ? __ldg(&a.brec[at[u]].z) : 0.0f) : 0;
+                slot[u] = at[u] >= 0 ? candidate_slot<D>(a, at[u], D == 2 ? a.brec[at[u]].z : 0.0f) : 0;
               }
 #pragma unroll
               for (int u = 0; u < kFlatAhead; ++u)
