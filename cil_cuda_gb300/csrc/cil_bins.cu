@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kTile) k_scatter(RebuildArgs a) {
     const ColonyConst &C = a.col[c];
     const int s = C.slot_base + (t - a.tiles_used[c]) * kTile + threadIdx.x;
     // nslot was overwritten by the scan; the used-slot bound is the tile range itself and
-    // every slot past the old nslot carries key -1 (k_clear_tail_keys / the rebin kernel).
+    // every slot past the old nslot carries key -1 (k_bin_keys / the rebin kernel).
     if (s >= C.slot_base + C.slot_cap) continue;
     const int k = a.key[s];
     if (k < 0) continue;

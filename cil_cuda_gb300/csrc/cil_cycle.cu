@@ -378,9 +378,9 @@ __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounte
 //           walk order, so that the sums do not depend on the lane count;
 //   pairs   the warp's survivors as one flattened range, a pair per lane;
 //   sums    a cell's first lane adds its pairs in walk order.
-// The contacts and the cycle of 1M cells (2.6 contacts a cell, FP64) take 498 us, with the FP64 pipe 80 %
-// busy (253 FP64 instructions per cell); one thread per cell with each contact evaluated where it was
-// met took 1079 us, and the cycle's own pass 258 us.
+// The contacts and the cycle of 1M cells (2.6 contacts a cell, FP64) take 509 us (caches flushed), with
+// the FP64 pipe 83 % busy (259 FP64 instructions a warp of 32 cells); one thread per cell with each contact
+// evaluated where it was met took 1079 us, and the cycle's own pass 258 us.
 constexpr int kPairBlock = 128;
 constexpr int kPairNear = 384;  // survivors held per warp (12 per cell at one lane each)
 constexpr int kPairAhead = 4;   // candidates a lane has in flight (one lane per cell)
@@ -391,8 +391,11 @@ struct PairWarp {
   R res[kSeg * NRES];
   double x[32 * D];
   R v[32 * D];  // velocities (DPD)
-  float u[32 * D];  // CyOrdered::loc and ::cell (DPD, FP32 pair terms)
-  int cell[32 * D];
+  // CyOrdered::loc and ::cell, of DPD with FP32 pair terms (the others keep the 2 KB a block: 1 % of a step of
+  // 1024 cells)
+  static constexpr int kLoc = sizeof(R) == sizeof(float) && NRES != D + 1 ? 32 * D : 1;
+  float u[kLoc];
+  int cell[kLoc];
   double rad[32];
   float dia[32];
   int idx[32];
@@ -970,7 +973,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 8 : 1) k_dpd_forces(CyCons
 #pragma unroll
   for (int d = 0; d < D; ++d) vi[d] = live ? S.v[d * cap + i] : 0.0;
   if (sub == 0) {
-    if (MIXED) {
+    if constexpr (MIXED) {
       const float4 u = live ? O.loc[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       const ushort4 b = live ? O.cell[q] : make_ushort4(0, 0, 0, 0);
 #pragma unroll
@@ -1119,7 +1122,7 @@ __global__ void __launch_bounds__(kPairBlock) k_dpd_dis(CyConst C, CySet S, CyCo
 #pragma unroll
   for (int d = 0; d < D; ++d) vi[d] = live ? S.v[d * cap + i] : 0.0;
   if (sub == 0) {
-    if (MIXED) {
+    if constexpr (MIXED) {
       const float4 u = live ? O.loc[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       const ushort4 b = live ? O.cell[q] : make_ushort4(0, 0, 0, 0);
 #pragma unroll
