@@ -698,8 +698,7 @@ __global__ void __launch_bounds__(kTile) k_events_exec(EventArgs a_) {
   apo_colony(a, c, D);
 }
 
-// Ascending bitonic sort of v[0, P) (P a power of two) by the whole block; v in shared or
-// global memory (a block barrier orders both within the block).
+// Ascending bitonic sort of v[0, P) (P a power of two) in shared memory by the whole block.
 __device__ void block_bitonic_sort(int *v, int P) {
   for (int size = 2; size <= P; size <<= 1)
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -718,12 +717,13 @@ __device__ void block_bitonic_sort(int *v, int P) {
     }
 }
 
-constexpr int kDueSort = 2048;  // due cells sorted in shared memory (more: in the queue itself)
+constexpr int kDueSort = 2048;  // due cells sorted in shared memory (more: found again by a scan of the cells)
 constexpr int kDueRank = 512;   // up to this many: sorted by ranks instead of a sorting network
 
 // Philox mode: the step's events from the due-cell queues, one block per colony. The force pass
 // appended the cells whose cycle ends at this step (in no particular order); the block ranks them by
-// cell index (up to kDueRank among themselves, more by a sort), so the first ndiv_allowed in cell order
+// cell index (up to kDueRank among themselves, more by a sort, beyond kDueSort by a scan of the colony's
+// cells: a sort in the queue took 17 ms for 80 000), so the first ndiv_allowed in cell order
 // divide (within the colony's cell and slot room; the ranking of the tile-wise kernels), places the
 // divisions (one thread each: draws, FP64 placement of the four elements, new cycles; daughters take
 // cells n + rank and slots nslot + 2 rank), then the
@@ -758,17 +758,32 @@ __global__ void __launch_bounds__(kTile) k_events_due(EventArgs a_) {
     for (int i = threadIdx.x; i < ((nd + 3) & ~3); i += blockDim.x)
       s_key[i] = i >= nd ? 0x7fffffff : (i == static_cast<int>(threadIdx.x) ? own : q[i]);
     __syncthreads();
-  } else {
+  } else if (nd <= kDueSort) {
     int P = 1;
     while (P < nd) P <<= 1;
-    if (P <= kDueSort) {
-      for (int i = threadIdx.x; i < P; i += blockDim.x) s_key[i] = i < nd ? q[i] : 0x7fffffff;
-    } else {
-      for (int i = nd + static_cast<int>(threadIdx.x); i < P; i += blockDim.x) q[i] = 0x7fffffff;
-      keys = q;
-    }
+    for (int i = threadIdx.x; i < P; i += blockDim.x) s_key[i] = i < nd ? q[i] : 0x7fffffff;
     __syncthreads();
-    block_bitonic_sort(keys, P);
+    block_bitonic_sort(s_key, P);
+  } else {
+    // the colony's cells in order instead: those whose cycle ends at this step, into the queue
+    int found = 0;
+    for (int i0 = 0; i0 < n && found < nd; i0 += kCellTile) {
+      const int i = i0 + static_cast<int>(threadIdx.x) * kCellItems;
+      bool due[kCellItems];
+      int mine = 0;
+#pragma unroll
+      for (int k = 0; k < kCellItems; ++k) due[k] = i + k < n && a.tsw[C.cell_base + i + k] == a.ts;
+#pragma unroll
+      for (int k = 0; k < kCellItems; ++k) mine += due[k] ? 1 : 0;
+      int tot;
+      int at = found + block_excl_scan_ev(mine, &tot);
+#pragma unroll
+      for (int k = 0; k < kCellItems; ++k)
+        if (due[k]) q[at++] = i + k;
+      found += tot;
+    }
+    keys = q;
+    __syncthreads();
   }
   if (threadIdx.x == 0) {  // every thread has read the counters
     if (allowed < nd) K.err |= kErrCap;
