@@ -138,10 +138,7 @@ __device__ __forceinline__ bool no_rebuild(const RebuildArgs &a) {
   return a.any_rebuild != nullptr && a.any_rebuild[*a.ts_dev & 1] == 0;
 }
 
-__global__ void __launch_bounds__(kTile) k_scan_partial(RebuildArgs a) {
-  enter_step_kernel();
-  if (no_rebuild(a)) return;
-  const int sb = blockIdx.x;
+__device__ __forceinline__ void scan_partial_block(const RebuildArgs &a, int sb) {
   if (skip_colony(a, a.scan_col[sb])) return;
   const ColonyConst &C = a.col[a.scan_col[sb]];
   const int b0 = C.bin_base + (sb - C.scan_base) * kScanItems;
@@ -156,6 +153,21 @@ __global__ void __launch_bounds__(kTile) k_scan_partial(RebuildArgs a) {
     int t = 0;
     for (int w = 0; w < kTile / 32; ++w) t += ws[w];
     a.scan_sum[sb] = t;
+  }
+}
+
+// Up to kScanBlocks blocks take the scan blocks in turn. (2000 cells in lists over 73M bins took 137 us a
+// step with 72 000 blocks, which all return when nothing rebuilds; now 35.)
+constexpr int kScanBlocks = 4096;
+
+__global__ void __launch_bounds__(kTile) k_scan_partial(RebuildArgs a) {
+  enter_step_kernel();
+  if (no_rebuild(a)) return;
+  int sb = blockIdx.x;
+  scan_partial_block(a, sb);
+  while ((sb += gridDim.x) < a.nscan) {
+    __syncthreads();
+    scan_partial_block(a, sb);
   }
 }
 
@@ -183,10 +195,8 @@ __global__ void __launch_bounds__(kTile) k_scan_colony(RebuildArgs a) {
 // less (1.6-2 us of a step) against 4 bytes times half the square of the colony's scan blocks read
 // from L2. The last scan block of a colony has its total: nlive (and, re-sorting, nslot); the last
 // colony to have its total writes the tile table over the live slots (a.tiles_live_out).
-__global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
-  enter_step_kernel();
-  if (no_rebuild(a)) return;
-  const int sb = blockIdx.x, c = a.scan_col[sb];
+__device__ __forceinline__ void scan_final_block(const RebuildArgs &a, int sb) {
+  const int c = a.scan_col[sb];
   if (skip_colony(a, c)) return;
   const ColonyConst &C = a.col[c];
   const int b0 = C.bin_base + (sb - C.scan_base) * kScanItems + threadIdx.x * 4;
@@ -237,6 +247,17 @@ __global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
   if (threadIdx.x == 0) {
     a.tiles_live_out[a.B] = carry;
     *a.scan_done = 0;
+  }
+}
+
+__global__ void __launch_bounds__(kTile) k_scan_final(RebuildArgs a) {
+  enter_step_kernel();
+  if (no_rebuild(a)) return;
+  int sb = blockIdx.x;
+  scan_final_block(a, sb);
+  while ((sb += gridDim.x) < a.nscan) {
+    __syncthreads();
+    scan_final_block(a, sb);
   }
 }
 
@@ -483,9 +504,10 @@ void launch_tiles(const ColonyConst *, ColonyCounters *cnt, int B, int which, in
 }
 
 static void launch_scan(const RebuildArgs &a, cudaStream_t s) {
-  launch_step(a.dep, a.nscan, kTile, 0, s, k_scan_partial, a);
+  const int blocks = a.nscan < kScanBlocks ? a.nscan : kScanBlocks;
+  launch_step(a.dep, blocks, kTile, 0, s, k_scan_partial, a);
   if (a.scanned) launch_step(a.dep, a.B, kTile, 0, s, k_scan_colony, a);
-  launch_step(a.dep, a.nscan, kTile, 0, s, k_scan_final, a);
+  launch_step(a.dep, blocks, kTile, 0, s, k_scan_final, a);
 }
 
 void launch_rebuild(const RebuildArgs &a, int grid_slots, cudaStream_t s) {

@@ -77,3 +77,40 @@ def test_a_step_costs_about_as_much_in_a_large_engine(gpu_lib, precision, skin, 
         best.append(min(t))
         eng.close()
     assert best[1] <= most * best[0]
+
+
+def _dilute(box, n=3000):
+    p = S.growth_params(box=box, dt=1e-4, divide=0, apop_rate=0.0, noise_D=0.0)
+    return p, S.disk_colony(n, p, seed=6)
+
+
+def test_lists_over_more_bins_than_scan_blocks(gpu_lib):
+    """13.6M bins, whose 13 300 scan blocks are taken in turn by 4096: two steps in lists against the bins
+    of every step (FP32 pair sums in two orders, 1e-6 of a force below 2e3, times dt / zeta)."""
+    p, st = _dilute(6000.0)
+    pos = []
+    for skin in (0.3, 0.0):
+        eng = _engine(p, 3000, G.PREC_MIXED, skin)
+        eng.upload(0, **st)
+        eng.step(2)
+        pos.append(eng.download(0)["pos"])
+        eng.close()
+    assert np.abs(pos[0] - pos[1]).max() <= 2 * 1e-6 * 2e3 * 1e-4
+
+
+def test_lists_cost_about_as_much_over_many_bins(gpu_lib):
+    # a step that rebuilds nothing passes the scan kernels by: a block per scan block took 1.9 times
+    best = []
+    for box in (1500.0, 6000.0):
+        p, st = _dilute(box)
+        eng = _engine(p, 3000, G.PREC_MIXED, 0.3)
+        eng.upload(0, **st)
+        eng.step(40)
+        t = []
+        for _ in range(25):
+            t0 = time.perf_counter()
+            eng.step(40)
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+        eng.close()
+    assert best[1] <= 1.5 * best[0]
