@@ -1886,6 +1886,20 @@ cil_status graph_step(cil_cycle *h) {
   return CIL_OK;
 }
 
+// Pageable memory that nobody has touched is faulted in here, on the host, before a copy into it: the
+// device faults its pages in one by one (a download of 0.6M cells into new arrays took 51 ms, now 4.2; with a
+// host loop over the vectors 30).
+void touch_pages(void *dst, size_t bytes) {
+  if (bytes < 65536) return;  // a page or two
+  cudaPointerAttributes at{};
+  const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  if (!pageable) return;
+  volatile char *p = static_cast<char *>(dst);
+  for (size_t k = 0; k < bytes; k += 4096) p[k] = 0;
+  p[bytes - 1] = 0;
+}
+
 cil_status read_counters(cil_cycle *h) {
   CY_TRY(h, cudaMemcpyAsync(h->h_cnt, h->cnt, sizeof(CyCounters), cudaMemcpyDeviceToHost, h->stream));
   CY_TRY(h, cudaStreamSynchronize(h->stream));
@@ -2207,11 +2221,14 @@ cil_status cil_cycle_download(cil_cycle *h, cil_cycle_view *v) {
   // rearranged in O.x (free between steps), one vector after the other on the stream
   auto vec = [&](double *dst, const double *src) -> cudaError_t {
     if (!dst || n == 0) return cudaSuccess;
+    touch_pages(dst, sizeof(double) * static_cast<size_t>(n) * D);
     k_cy_to_host<<<blocks_for(n), kTile, 0, h->stream>>>(src, n, D, cap, h->O.x);
     return cudaMemcpyAsync(dst, h->O.x, sizeof(double) * static_cast<size_t>(n) * D, cudaMemcpyDeviceToHost, h->stream);
   };
   auto sca = [&](void *dst, const void *src, size_t es) -> cudaError_t {
-    return dst ? cudaMemcpyAsync(dst, src, es * n, cudaMemcpyDeviceToHost, h->stream) : cudaSuccess;
+    if (!dst || n == 0) return cudaSuccess;
+    touch_pages(dst, es * n);
+    return cudaMemcpyAsync(dst, src, es * n, cudaMemcpyDeviceToHost, h->stream);
   };
   CY_TRY(h, vec(v->pos, S.x));
   CY_TRY(h, vec(v->vel, S.v));
