@@ -816,9 +816,10 @@ cudaEvent_t pool_event(cil_handle *h, size_t i) {
 // scheduler (nsm x 4 x 2 x 32 lanes), and while the grid, which covers the capacity, stays within 8192
 // blocks (an empty block costs about 0.9 ns, more than lanes save beyond that: 500 cells at a capacity of 2M
 // took 271 us a step with 262 144 blocks, 51 with 32 768; 29 at a capacity of 664). From the cells the host
-// knows of (uploaded, or counted by the last cil_step); the forces do not depend on it. Step of the growth colony with 1, 2, 4, 8 lanes
-// (when a step had 15 launches):
-// 500 cells 48, 46, 44, 42 us; 4864 cells 61, 56, 57, 61 us; 19456 cells 72, 73, 87, 107 us.
+// knows of (uploaded, or counted by the last cil_step); the forces do not depend on it. Step with 1, 2, 4
+// and 8 lanes, us: 2D growth of 500 cells 40, 37, 34, 33; 4864: 44, 42, 42, 47; 9728: 50, 52, 57, 59; 19456:
+// 81, 67, 65, 85 (the rule gives 1); 60000: 87, 95, 126, 198; 3D channel of 1000 cells 49, 46, 41, 39; 4000: 51,
+// 49, 50, 56; 20000: 90, 78, 90, 121 (the rule gives 1); 60001: 97, 126, 177, 276.
 void set_lane_bits(cil_handle *h) {
   long long elems = 0;
   for (int c = 0; c < h->B; ++c) elems += 2ll * h->hc[c].n_seen;

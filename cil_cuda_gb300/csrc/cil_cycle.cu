@@ -378,8 +378,8 @@ __global__ void __launch_bounds__(kTile) k_cy_place(CyConst C, CySet S, CyCounte
 //           walk order, so that the sums do not depend on the lane count;
 //   pairs   the warp's survivors as one flattened range, a pair per lane;
 //   sums    a cell's first lane adds its pairs in walk order.
-// The contacts and the cycle of 1M cells (2.6 contacts a cell, FP64) take 509 us (caches flushed), with
-// the FP64 pipe 83 % busy (259 FP64 instructions a warp of 32 cells); one thread per cell with each contact
+// The contacts and the cycle of 1M cells (2.6 contacts a cell, FP64) take 515 us (caches flushed), with
+// the FP64 pipe 83 % busy (260 FP64 instructions a warp of 32 cells); one thread per cell with each contact
 // evaluated where it was met took 1079 us, and the cycle's own pass 258 us.
 constexpr int kPairBlock = 128;
 constexpr int kPairNear = 384;  // survivors held per warp (12 per cell at one lane each)

@@ -110,8 +110,9 @@ __device__ __forceinline__ void collect_due(const ForceArgs &a, const ColonyCons
 // Lanes per element: see set_lane_bits (cil_api.cu). When every candidate's separation was formed
 // in FP64 and each lane evaluated its own pairs, a pass took 879 us for 0.5M elements of the 2D
 // growth colony, 376 us for 0.12M of the 3D channel and 42 us for 8192 WCA elements; now 161, 62
-// and 12.4 us, with the FP64 pipe 70 to 75 % active in the first (137 FP64 instructions a warp's
-// 32 elements); the walk over 9 rows of bins is most of the channel's instructions.
+// and 12.4 us, with the FP64 pipe 77 % active in the first (152 FP64 instructions a warp's 32
+// elements); the walk over 9 rows of bins is most of the channel's instructions. Compiled for 8 blocks
+// an SM; in 3D a block's 28 KB of shared memory let 7 of them fit.
 constexpr int kF64Block = 128;
 constexpr int kF64Near = 512;  // survivors held per warp (16 per element at one lane each)
 constexpr int kF64Seg = 128;   // pairs evaluated before their sums are taken
