@@ -85,19 +85,7 @@ __device__ __forceinline__ void fast_bin(const ColonyConst &C, int home, const f
   int h[D];
   bin_decode<D>(C, home, h);
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const int sh = static_cast<int>(floorf(pk_c(p, d) * C.inv_bwf[d]));
-    int v = h[d] + sh;
-    if (C.periodic[d]) {
-      if (v < 0) v += C.ns[d];
-      if (v >= C.ns[d]) v -= C.ns[d];
-      shift[d] = sh;
-    } else {
-      v = v < 0 ? 0 : (v >= C.ns[d] ? C.ns[d] - 1 : v);
-      shift[d] = v - h[d];
-    }
-    b[d] = v;
-  }
+  for (int d = 0; d < D; ++d) b[d] = moved_bin(C, d, h[d], pk_c(p, d), &shift[d]);
 }
 
 template <int D>

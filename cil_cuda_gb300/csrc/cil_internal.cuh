@@ -449,6 +449,26 @@ __device__ __forceinline__ int floor_scaled(double x, float scale, F exact) {
   return static_cast<int>(exact());
 }
 
+// The bin along axis d of an element at the FP32 coordinate u from its home bin h's origin: *shift whole
+// bin widths further, wrapped along a periodic axis, clamped along an open one. Within the grid whatever u
+// is (an unstable run moves elements by more than a box in a step, and a bin outside the grid would be
+// counted outside the bin arrays); shift is the unwrapped change of the bin coordinate.
+__device__ __forceinline__ int moved_bin(const ColonyConst &C, int d, int h, float u, int *shift) {
+  const float far = 1048576.0f;  // within int, with h added
+  const int sh = static_cast<int>(fminf(fmaxf(floorf(u * C.inv_bwf[d]), -far), far));
+  const int ns = C.ns[d];
+  int v = h + sh;
+  *shift = sh;
+  if (C.periodic[d]) {
+    if (v < 0) v += ns;
+    if (v >= ns) v -= ns;
+  }
+  if (v >= 0 && v < ns) return v;
+  v = v < 0 ? 0 : ns - 1;
+  if (!C.periodic[d]) *shift = v - h;
+  return v;
+}
+
 // Bin coordinates of a position (LinkListOrtho::populate_list, Utils.hpp:990), clamped
 // to the grid along non-periodic axes.
 template <int D>

@@ -251,20 +251,10 @@ __global__ void __launch_bounds__(kTile) k_skin_rebin(SkinArgs a) {
       float4 p = a.pk[s];
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        float u = pk_c(p, d);
-        const int sh = static_cast<int>(floorf(u * C.inv_bwf[d]));
-        int v = h[d] + sh;
-        if (C.periodic[d]) {
-          if (v < 0) v += C.ns[d];
-          if (v >= C.ns[d]) v -= C.ns[d];
-          u -= static_cast<float>(sh) * C.bwf[d];
-        } else {
-          const int vc = v < 0 ? 0 : (v >= C.ns[d] ? C.ns[d] - 1 : v);
-          u -= static_cast<float>(vc - h[d]) * C.bwf[d];
-          v = vc;
-        }
-        b[d] = v;
-        pk_set(p, d, u);
+        const float u = pk_c(p, d);
+        int sh;
+        b[d] = moved_bin(C, d, h[d], u, &sh);
+        pk_set(p, d, u - static_cast<float>(sh) * C.bwf[d]);
       }
       a.pk[s] = p;
       const int id = bin_id<D>(C, b);

@@ -31,6 +31,29 @@ static T *up(const void *src, size_t bytes) {
   return static_cast<T *>(q);
 }
 
+__global__ void k_moved(ColonyConst C, int n, const float *u, const int *h, int *bin, int *shift) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) bin[i] = moved_bin(C, 0, h[i], u[i], shift + i);
+}
+
+extern "C" int moved(int periodic, int ns, float bw, int n, const float *u, const int *h, int *bin, int *shift) {
+  ColonyConst C{};
+  C.ns[0] = ns;
+  C.periodic[0] = periodic;
+  C.bwf[0] = bw;
+  C.inv_bwf[0] = 1.0f / bw;
+  float *du = up<float>(u, 4 * size_t(n));
+  int *dh = up<int>(h, 4 * size_t(n)), *db = up<int>(bin, 4 * size_t(n)), *ds = up<int>(shift, 4 * size_t(n));
+  k_moved<<<(n + 127) / 128, 128>>>(C, n, du, dh, db, ds);
+  cudaMemcpy(bin, db, 4 * size_t(n), cudaMemcpyDeviceToHost);
+  const cudaError_t e = cudaMemcpy(shift, ds, 4 * size_t(n), cudaMemcpyDeviceToHost);
+  cudaFree(du);
+  cudaFree(dh);
+  cudaFree(db);
+  cudaFree(ds);
+  return static_cast<int>(e);
+}
+
 // rsqrt_pos, sqrt_from, rcp_normal, CUDA's rsqrt, sqrt and reciprocal, the two approximate seeds, mid_range
 __global__ void k_roots(int n, const double *a, double *out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -176,3 +199,29 @@ def test_mid_range_takes_its_range_only(gpu_lib, probes):
     for lib in probes.values():
         mid = _roots(lib, np.array(out + ins))[8]
         assert list(mid) == [0.0] * len(out) + [1.0] * len(ins)
+
+
+@pytest.mark.parametrize("periodic", [0, 1])
+@pytest.mark.parametrize("ns", [1, 3, 40])
+def test_a_moved_bin_is_in_the_grid(gpu_lib, probes, periodic, ns):
+    """Whatever an element's FP32 coordinate has become (an unstable run), its bin is one of the grid's;
+    within a grid's length of a periodic axis it is the wrapped one, along an open one the clamped one."""
+    rng = np.random.default_rng(3)
+    bw = np.float32(1.5)  # quotients of multiples of 3/4 are exact enough for their floors
+    near = 0.75 * rng.integers(-2 * ns, 2 * ns + 1, 4000) + 0.3
+    far = np.concatenate([s * 10.0 ** rng.uniform(0, 38, 2000) for s in (-1, 1)])
+    u = np.concatenate([near, far, [np.inf, -np.inf, np.nan, 0.0, -0.0, 3e38, -3e38]]).astype(np.float32)
+    h = rng.integers(0, ns, len(u)).astype(np.int32)
+    for lib in probes.values():
+        b, sh = np.full(len(u), -7, np.int32), np.zeros(len(u), np.int32)
+        p = [x.ctypes.data_as(C.c_void_p) for x in (u, h, b, sh)]
+        assert lib.moved(periodic, ns, C.c_float(bw), len(u), *p) == 0
+        assert b.min() >= 0 and b.max() < ns
+        want = h[:4000] + np.floor(u[:4000] / bw).astype(np.int64)
+        if periodic:
+            inside = (want >= -ns) & (want < 2 * ns)
+            np.testing.assert_array_equal(b[:4000][inside], (want % ns)[inside])
+            np.testing.assert_array_equal(sh[:4000], want - h[:4000])
+        else:
+            np.testing.assert_array_equal(b[:4000], np.clip(want, 0, ns - 1))
+            np.testing.assert_array_equal(sh[:4000], b[:4000] - h[:4000])
