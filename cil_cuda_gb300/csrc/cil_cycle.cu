@@ -722,8 +722,9 @@ __device__ inline void contact(const CyConst &C, double r, double h, double hy, 
 }
 
 // The terms of the pair at displacement rij (FP64, or FP32 with FP32 pair terms; r2 its square, FP64
-// form): the contact force on the cell, and in out[D] the pressure term, -f0 / volume doubled (FP64) or f0 / volume (MIXED); zeros out of
-// contact. The warp's cell o and the cell at place tt; first: the cell has the lower index.
+// form): the contact force on the cell, and in out[D] the pressure term, -f0 / volume doubled (FP64) or
+// f0 / volume (MIXED); zeros out of contact. The warp's cell o and the cell at place tt; first: the cell
+// has the lower index.
 template <int D, bool MIXED, int NRES, typename R, typename X>
 __device__ __forceinline__ void contact_terms(const CyConst &C, const CyOrdered &O, const PairWarp<D, NRES, R> &W, int o,
                                               int tt, const X *rij, double r2, bool first, R *out) {
